@@ -1,73 +1,125 @@
-// FP64-grade complex GEMM on the bf16 tensor cores (tcgen05), for the contractions that
-// must stay FP64-accurate: environment updates, the Rayleigh quotients and residuals of the
-// Krylov refinement.  On this part FP64 runs at about 1.2 TFLOP/s, more than a thousand
-// times below the bf16 tensor rate; this kernel trades that for exact integer arithmetic.
+// FP64-accurate complex GEMM on the bf16 tensor cores (tcgen05): the long-K contractions of
+// the FP64 mode and every product of GTN_PREC_FP64E.  FP64 runs at about 1.2 TFLOP/s on this
+// part, more than a thousand times below the bf16 tensor rate; this kernel trades that for
+// exact integer arithmetic.
 //
 // Method (the fixed-point splitting of Ozaki, Ogita, Oishi and Rump, Numer. Algorithms 59
 // (2012), with exact chunked accumulation):
 //   * every row of the real-expanded A (and every complex row of B') is scaled by a power
-//     of two 2^k so that its entries lie in (-1, 1), then written as S = 7 signed base-128
-//     digits, a = sum_i d_i 2^{-7(i+1)}, |d_0| <= 128, |d_i| <= 64; each digit is an integer
-//     that bf16 holds exactly (the digit planes are built by split_i7 / pack_b_planes_i7);
-//   * the digit products d_i e_j with i + j <= 6 (28 of them) are summed on the tensor
-//     cores, one TMEM accumulator per level s = i + j (7 levels x 64 columns).  Every
-//     product of two digits is an integer below 2^14 and a level gets at most
-//     2 * 2^13 + 5 * 2^12 per k, so over a chunk of 256 k the FP32 sums are exact integers;
-//   * after each chunk the epilogue warps read the levels and add 2^{-7(s+2)} L_s into a
-//     double-float accumulator (pairs of FP32 with error-free TwoSum updates, about 48
-//     significant bits); the result is scaled back by 2^{-(k_row + k_col)} into FP64.
-// The terms left out (i + j >= 7) and the digits beyond the seventh are below 2^-49 of the
-// row maxima, so each output is accurate to about 1e-14 relative to sum_k |a_k| |b_k|.
+//     of two so that its entries lie in (-1/2, 1/2), then written as S = 7 signed base-256
+//     digits, a = sum_i d_i 2^{-8(i+1)}, |d_i| <= 128 (bf16 holds them exactly);
+//   * the digit products d_i e_j of the levels l = i + j < L are summed on the tensor cores,
+//     one TMEM accumulator of 64 columns per level: L = 8 (34 products) in the FP64 mode, L = 7
+//     (28) in FP64E.  A level gets at most min(l + 1, 13 - l) 2^14 per real k, so the FP32 sums are
+//     exact integers (<= 2^24) over 256 real k for the levels 0-3 and over 128 for the others;
+//   * the epilogue warps read the levels from 4 on after every 128 k and the levels 0-3 after
+//     every 256, and add them with their weights into two 64-bit integers per output (units
+//     2^-72 and 2^-40): the sum over all k of the kept digit products is exact.  Its one rounding
+//     is the conversion to FP64 at the end, done on the integers' bits.
+// What is left out (levels from L on, digits beyond the seventh) does not grow with K, unlike the
+// rounding errors of FP64 fused multiply-adds.  Measured against extended precision, relative
+// 2-norm, Gaussian operands: K = 65 5.7e-17 (FP64 pipe 3.7e-16), K = 5120 7.1e-17 (3.4e-15),
+// rows that decay from 1 to 1e-9 along k 1.3e-16 (5.4e-16) and 1.8e-16 (4.9e-15); L = 7 about
+// 3.6e-16 at every K.
+// A row with an infinity, a NaN or a magnitude beyond 2^+-450 has no digits: the split sets a
+// flag, this kernel returns and the FP64 kernel behind it computes the product.
 //
-// Tile: 128 rows x 64 real columns (32 complex) per CTA; stages of 16 k (SWIZZLE_32B rows
-// of 32 bytes) holding all 7 digit planes of A and of B'; warp 0 issues TMA, warp 1 the
-// MMAs (tcgen05.mma.cta_group::1.kind::f16, bf16 x bf16 -> f32), warps 2-9 drain the
-// levels (warp w reads TMEM lanes 32 (w % 4) .. + 31, columns (w - 2) / 4 * 32 .. + 31).
-// Every mbarrier wait is bounded as in the other tcgen05 kernels.
+// Tile: 128 rows x 64 real columns (32 complex); stages of 16 real k hold all 7 planes of A
+// (28 KB) and of B' (14 KB), laid out by the split so that one contiguous bulk copy loads each
+// (rows of 32 bytes, SWIZZLE_32B order).  The planes of B' lie behind each other in a stage, so
+// digit i of A meets the stack e_0, e_1, .. in MMAs up to 256 wide whose columns run through
+// the levels from i on: 10 to 13 instructions a stage instead of 28 or 34 of width 64 (A is read
+// from shared memory once per instruction, and 64-wide instructions are bound by that).  One CTA per SM
+// walks over the tiles: warp 0 copies, warp 1 issues the MMAs, warps 2-9 drain the levels (warp
+// w reads TMEM lanes 32 (w % 4) .. + 31, columns (w - 2) / 4 * 32 .. + 31) and convert and store
+// a tile while the next one's MMAs run.  Every mbarrier wait is bounded as in the other tcgen05
+// kernels.
 #include "gtn_internal.h"
 #include "gtn_tcgen05.h"
 
 #include <algorithm>
+#include <cmath>
 
 namespace {
 using namespace gtn_tc;
 
 constexpr int kS = kF64eSlices;                  // digits per value
-constexpr int kLevels = kS;                      // levels s = i + j <= kS - 1
-constexpr int kBM = 128;
-constexpr int kBN = 64;                          // real columns (32 complex outputs)
-constexpr int kBK = 16;                          // real k per stage (one 32-byte row)
-constexpr int kPlaneA = kBM * kBK * 2;           // 4 KB
-constexpr int kPlaneB = kBN * kBK * 2;           // 2 KB
-constexpr int kStageBytes = kS * (kPlaneA + kPlaneB);
-constexpr int kStages = (228352 - 4096) / kStageBytes > 8 ? 8 : (228352 - 4096) / kStageBytes;
+constexpr int kBM = kF64eRowsA;
+constexpr int kBN = kF64eRowsB;                  // real columns (32 complex outputs)
+constexpr int kPlaneA = kBM * 32;                // 16 real k
+constexpr int kPlaneB = kBN * 32;
+constexpr int kStageA = kS * kPlaneA, kStageB = kS * kPlaneB;
+constexpr int kStageBytes = kStageA + kStageB;
+constexpr int kStages = 5;
 constexpr int kSmem = kStages * kStageBytes + 1024;
-constexpr int kChunkStages = 16;                 // 256 real k per exact chunk
-constexpr uint32_t kTmemCols = 512;              // 7 levels x 64 columns = 448
+constexpr int kChunkStages = 8;                  // 128 real k between drains of the levels 4-6
+constexpr int kHiLevels = 4;                     // levels 0-3: drained every second chunk
+constexpr uint32_t kTmemCols = 512;              // up to 8 levels x 64 columns
 constexpr int kThreads = 320;
-static_assert(kStages >= 3, "operand ring");
-static_assert(kLevels * kBN <= (int)kTmemCols, "TMEM columns");
+constexpr int kGroupM = 8;                       // row tiles walked together (L2 reuse of B')
+static_assert(kSmem <= 227 * 1024 - 1024, "operand ring");
 
-// Power-of-two exponent k with |x| 2^k < 1 for every |x| <= mx (mx a float row maximum).
-__device__ __forceinline__ int row_exp(float mx) {
-  const uint32_t b = __float_as_uint(mx);
-  const int e = (int)((b >> 23) & 0xffu);
-  return mx > 0.f ? 126 - e : 0;
+// hi 2^-40 + lo 2^-72, times 2^(ea + eb - 2 * 1021) (the rows' scales), rounded once to double.
+// |hi| < 2^61, |lo| < 2^63; the exponents keep the result a normal number or zero.
+__device__ __forceinline__ double to_double(long long hi, long long lo, int esum) {
+  long long th = hi + (lo >> 32);          // value = th 2^-40 + tl 2^-72
+  uint32_t tl = (uint32_t)lo;
+  const bool neg = th < 0;
+  if (neg) {
+    tl = 0u - tl;
+    th = ~th + (tl == 0u ? 1 : 0);
+  }
+  int e = esum - 2 * 1021 - 41;            // bit 0 of th is 2^(e + 1), of tl 2^(e - 31)
+  unsigned long long m = (unsigned long long)th;
+  e += 64;                                 // bit 63
+  if (m == 0) {
+    if (tl == 0u) return 0.0;
+    m = tl;
+    tl = 0u;
+    e -= 32;
+  }
+  const int lz = __clzll((long long)m);
+  const unsigned long long w = lz == 0 ? m : (lz < 32 ? (m << lz) | (tl >> (32 - lz)) : (m << lz) | ((unsigned long long)tl << (lz - 32)));
+  const bool sticky = lz < 32 && (tl << lz) != 0u;
+  e -= lz;
+  unsigned long long r = w >> 11;
+  const uint32_t rem = (uint32_t)w & 0x7ffu;
+  if (rem > 0x400u || (rem == 0x400u && (sticky || (r & 1ull)))) ++r;
+  const unsigned long long bits = ((unsigned long long)(e + 1022) << 52) + r;  // r's top bit adds one
+  return __longlong_as_double((long long)(bits | (neg ? 0x8000000000000000ull : 0ull)));
 }
 
-// x = hi + lo (double-float) += v, error-free (Knuth TwoSum) with the error kept in lo.
-__device__ __forceinline__ void df_add(float& hi, float& lo, float v) {
-  const float s = hi + v;
-  const float bb = s - hi;
-  const float err = (hi - (s - bb)) + (v - bb);
-  hi = s;
-  lo += err;
+__device__ __forceinline__ void bulk_load(uint32_t dst, const void* src, uint32_t bytes, uint64_t* bar) {
+  asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(dst),
+               "l"(reinterpret_cast<uint64_t>(src)), "r"(bytes), "r"(smem_u32(bar))
+               : "memory");
 }
 
+// acc[j] += w * (the exact integer in column j), 32 columns.
+__device__ __forceinline__ void drain(uint32_t taddr, int w, long long (&acc)[32]) {
+#pragma unroll
+  for (int h = 0; h < 2; ++h) {
+    uint32_t v[16];
+    tmem_ld16(taddr + (uint32_t)(h * 16), v);
+#pragma unroll
+    for (int j = 0; j < 16; ++j) acc[h * 16 + j] += (long long)__float2int_rn(__uint_as_float(v[j])) * w;
+  }
+}
+
+// Tile t -> (row tile, column tile): groups of kGroupM row tiles, rows fastest.
+__device__ __forceinline__ void tile_of(int64_t t, int64_t tm, int64_t tn, int64_t* mt, int64_t* nt) {
+  const int64_t per = kGroupM * tn, g = t / per, r = t - g * per;
+  const int64_t gm = min((int64_t)kGroupM, tm - g * kGroupM);
+  *nt = r / gm;
+  *mt = g * kGroupM + (r - *nt * gm);
+}
+
+template <int L>
 __global__ void __launch_bounds__(kThreads, 1)
-    f64e_gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB,
-                     double2* __restrict__ C, int64_t M, int64_t N, int nkb, const float* __restrict__ amax,
-                     const float* __restrict__ bmax, int* __restrict__ errflag, int tiles_n) {
+    f64e_gemm_kernel(const unsigned char* __restrict__ A, const unsigned char* __restrict__ B, double2* __restrict__ C,
+                     int64_t M, int64_t N, int nkb, int64_t tiles_m, int64_t tiles_n, const float* __restrict__ a_exp,
+                     const float* __restrict__ b_exp, const int* __restrict__ a_flag, const int* __restrict__ b_flag,
+                     int token, int* __restrict__ errflag) {
   extern __shared__ __align__(1024) uint8_t smem_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) &
                                              ~static_cast<uintptr_t>(1023));
@@ -78,8 +130,9 @@ __global__ void __launch_bounds__(kThreads, 1)
   __shared__ volatile int abort_flag;
   __shared__ int n_issued, n_consumed;
 
+  if (*a_flag == token || *b_flag != 0) return;  // the same for every thread of the launch
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int m0 = (int)(blockIdx.x / tiles_n) * kBM, r0 = (int)(blockIdx.x % tiles_n) * kBN;
+  const int64_t ntiles = tiles_m * tiles_n;
   const int nchunks = (nkb + kChunkStages - 1) / kChunkStages;
   if (threadIdx.x == 0) {
     for (int s = 0; s < kStages; ++s) {
@@ -92,8 +145,6 @@ __global__ void __launch_bounds__(kThreads, 1)
     n_issued = 0;
     n_consumed = 0;
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
-    asm volatile("prefetch.tensormap [%0];" ::"l"(reinterpret_cast<uint64_t>(&tmA)) : "memory");
-    asm volatile("prefetch.tensormap [%0];" ::"l"(reinterpret_cast<uint64_t>(&tmB)) : "memory");
   }
   if (warp == 1) {
     asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(&tmem_slot)),
@@ -108,116 +159,141 @@ __global__ void __launch_bounds__(kThreads, 1)
 
   if (warp == 0 && lane == 0) {
     int it = 0;
-    for (; it < nkb; ++it) {
-      const int s = it % kStages;
-      const uint32_t ph = (uint32_t)(it / kStages) & 1u;
-      if (!mbar_wait(&empty_bar[s], ph ^ 1u, &abort_flag)) {
-        abort_flag = 1;
-        atomicCAS(errflag, 0, DEVERR_TMA_TIMEOUT);
-        break;
-      }
-      const uint32_t sa = smem_u32(smem + s * kStageBytes);
-      const uint32_t sb = sa + kS * kPlaneA;
-      mbar_expect_tx(&full_bar[s], kStageBytes);
-#pragma unroll
-      for (int p = 0; p < kS; ++p) {
-        tma_load_3d(sa + p * kPlaneA, &tmA, &full_bar[s], it * kBK, m0, p);
-        tma_load_3d(sb + p * kPlaneB, &tmB, &full_bar[s], it * kBK, r0, p);
+    bool stop = false;
+    for (int64_t t = blockIdx.x; t < ntiles && !stop; t += gridDim.x) {
+      int64_t mt, nt;
+      tile_of(t, tiles_m, tiles_n, &mt, &nt);
+      const unsigned char* a = A + mt * nkb * kStageA;
+      const unsigned char* b = B + nt * nkb * kStageB;
+      for (int kb = 0; kb < nkb; ++kb, ++it) {
+        const int s = it % kStages;
+        const uint32_t ph = (uint32_t)(it / kStages) & 1u;
+        if (!mbar_wait(&empty_bar[s], ph ^ 1u, &abort_flag)) {
+          abort_flag = 1;
+          atomicCAS(errflag, 0, DEVERR_TMA_TIMEOUT);
+          stop = true;
+          break;
+        }
+        const uint32_t sa = smem_u32(smem + s * kStageBytes);
+        mbar_expect_tx(&full_bar[s], kStageBytes);
+        bulk_load(sa, a + (int64_t)kb * kStageA, kStageA, &full_bar[s]);
+        bulk_load(sa + kStageA, b + (int64_t)kb * kStageB, kStageB, &full_bar[s]);
       }
     }
     n_issued = it;
   } else if (warp == 1 && lane == 0) {
-    constexpr uint32_t idesc = idesc_bf16(kBM, kBN);
-    int it = 0;
+    int it = 0, ev = 0;
     bool stop = false;
-    for (int c = 0; c < nchunks && !stop; ++c) {
-      // the levels are free once the epilogue drained the previous chunk
-      if (!mbar_wait(&chunk_empty, ((uint32_t)c & 1u) ^ 1u, &abort_flag)) {
-        abort_flag = 1;
-        atomicCAS(errflag, 0, DEVERR_MMA_TIMEOUT);
-        break;
-      }
-      fence_after();
-      bool started[kLevels];
-#pragma unroll
-      for (int l = 0; l < kLevels; ++l) started[l] = false;
-      const int kb_end = std::min(nkb, (c + 1) * kChunkStages);
-      for (; it < kb_end; ++it) {
-        const int s = it % kStages;
-        const uint32_t ph = (uint32_t)(it / kStages) & 1u;
-        if (!mbar_wait(&full_bar[s], ph, &abort_flag)) {
+    for (int64_t t = blockIdx.x; t < ntiles && !stop; t += gridDim.x) {
+      int kb = 0;
+      for (int c = 0; c < nchunks && !stop; ++c, ++ev) {
+        // the levels are free once the epilogue drained the previous chunk
+        if (!mbar_wait(&chunk_empty, ((uint32_t)ev & 1u) ^ 1u, &abort_flag)) {
           abort_flag = 1;
           atomicCAS(errflag, 0, DEVERR_MMA_TIMEOUT);
           stop = true;
           break;
         }
         fence_after();
-        const uint32_t sa = smem_u32(smem + s * kStageBytes);
-        const uint32_t sb = sa + kS * kPlaneA;
-#pragma unroll
-        for (int i = 0; i < kS; ++i) {
-#pragma unroll
-          for (int j = 0; j + i < kLevels; ++j) {
-            const int l = i + j;
-            umma_bf16(tmem_base + (uint32_t)(l * kBN), sdesc32(sa + i * kPlaneA), sdesc32(sb + j * kPlaneB), idesc,
-                      started[l] ? 1u : 0u);
-            started[l] = true;
+        const uint32_t acc_hi = (c & 1) ? 1u : 0u;  // the levels 0-3 run over two chunks
+        bool first = true;
+        const int kb_end = std::min(nkb, (c + 1) * kChunkStages);
+        for (; kb < kb_end; ++kb, ++it) {
+          const int s = it % kStages;
+          const uint32_t ph = (uint32_t)(it / kStages) & 1u;
+          if (!mbar_wait(&full_bar[s], ph, &abort_flag)) {
+            abort_flag = 1;
+            atomicCAS(errflag, 0, DEVERR_MMA_TIMEOUT);
+            stop = true;
+            break;
           }
+          fence_after();
+          const uint32_t sa = smem_u32(smem + s * kStageBytes), sb = sa + kStageA;
+          // mma(i, j, n): digit i of A times the digits j .. j+n-1 of B', into the levels i+j ..
+          // i+j+n-1.  The first stage of a chunk overwrites its levels
+          // (digit 0 reaches the levels 0-6, digit 1 the level 7).
+          auto mma = [&](int i, int j, int n, uint32_t acc) {
+            umma_bf16(tmem_base + (uint32_t)((i + j) * kBN), sdesc32(sa + i * kPlaneA), sdesc32(sb + j * kPlaneB),
+                      idesc_bf16(kBM, n * kBN), acc);
+          };
+          mma(0, 0, 4, first ? acc_hi : 1u);
+          mma(0, 4, 3, first ? 0u : 1u);
+          mma(1, 0, 3, 1u);
+          if (L == 7) {
+            mma(1, 3, 3, 1u);
+            mma(2, 0, 3, 1u);
+            mma(2, 3, 2, 1u);
+            mma(3, 0, 4, 1u);
+            mma(4, 0, 3, 1u);
+            mma(5, 0, 2, 1u);
+            mma(6, 0, 1, 1u);
+          } else {
+            if (first) {
+              mma(1, 3, 3, 1u);
+              mma(1, 6, 1, 0u);
+            } else {
+              mma(1, 3, 4, 1u);
+            }
+            mma(2, 0, 3, 1u);
+            mma(2, 3, 3, 1u);
+            mma(3, 0, 3, 1u);
+            mma(3, 3, 2, 1u);
+            mma(4, 0, 4, 1u);
+            mma(5, 0, 3, 1u);
+            mma(6, 0, 2, 1u);
+          }
+          first = false;
+          umma_commit(&empty_bar[s]);
         }
-        umma_commit(&empty_bar[s]);
+        umma_commit(&chunk_full);  // the chunk's levels are complete once its MMAs are
       }
-      umma_commit(&chunk_full);  // the chunk's levels are complete once its MMAs are
     }
     n_consumed = it;
   } else if (warp >= 2) {
     const int q4 = warp & 3;             // TMEM lane quarter
     const int half = (warp - 2) >> 2;    // column half
-    const int row = q4 * 32 + lane;
-    const int64_t m = (int64_t)m0 + row;
-    float hi[32], lo[32];
-#pragma unroll
-    for (int j = 0; j < 32; ++j) hi[j] = lo[j] = 0.f;
+    const uint32_t tm0 = tmem_base + (uint32_t)(half * 32) + ((uint32_t)(q4 * 32) << 16);
+    int ev = 0;
     bool ok = true;
-    for (int c = 0; c < nchunks; ++c) {
-      if (!mbar_wait(&chunk_full, (uint32_t)c & 1u, &abort_flag)) {
-        if (lane == 0) {
-          abort_flag = 1;
-          atomicCAS(errflag, 0, DEVERR_EPI_TIMEOUT);
+    for (int64_t t = blockIdx.x; t < ntiles && ok; t += gridDim.x) {
+      int64_t mt, nt;
+      tile_of(t, tiles_m, tiles_n, &mt, &nt);
+      long long hi[32], lo[32];
+#pragma unroll
+      for (int j = 0; j < 32; ++j) hi[j] = lo[j] = 0;
+      for (int c = 0; c < nchunks; ++c, ++ev) {
+        if (!mbar_wait(&chunk_full, (uint32_t)ev & 1u, &abort_flag)) {
+          if (lane == 0) {
+            abort_flag = 1;
+            atomicCAS(errflag, 0, DEVERR_EPI_TIMEOUT);
+          }
+          ok = false;
+          break;
         }
-        ok = false;
-        break;
-      }
-      __syncwarp();
-      fence_after();
+        __syncwarp();
+        fence_after();
+        // weights 2^{-8(l + 2)}: levels from 4 on in units of 2^-72, levels 0-3 in units of 2^-40
 #pragma unroll 1
-      for (int l = 0; l < kLevels; ++l) {
-        uint32_t v[32];
-        tmem_ld32(tmem_base + (uint32_t)(l * kBN + half * 32) + ((uint32_t)(q4 * 32) << 16), v);
-        const float w = __uint_as_float((uint32_t)(127 - 7 * (l + 2)) << 23);  // 2^{-7(l+2)}, exact
-#pragma unroll
-        for (int j = 0; j < 32; ++j) df_add(hi[j], lo[j], __uint_as_float(v[j]) * w);
+        for (int l = kHiLevels; l < L; ++l) drain(tm0 + (uint32_t)(l * kBN), 1 << (8 * (7 - l)), lo);
+        if ((c & 1) || c == nchunks - 1) {
+#pragma unroll 1
+          for (int l = 0; l < kHiLevels; ++l) drain(tm0 + (uint32_t)(l * kBN), 1 << (8 * (3 - l)), hi);
+        }
+        fence_before();
+        __syncwarp();
+        if (lane == 0) mbar_arrive_local(&chunk_empty);
       }
+      const int64_t m = mt * kBM + q4 * 32 + lane;
+      if (ok && m < M) {
+        const int ea = (int)a_exp[m];
+        const int64_t nb = nt * (kBN / 2) + half * 16;
 #pragma unroll
-      for (int j = 0; j < 32; ++j) {  // renormalise (FastTwoSum, |hi| >= |lo|)
-        const float s = hi[j] + lo[j];
-        lo[j] = lo[j] - (s - hi[j]);
-        hi[j] = s;
-      }
-      fence_before();
-      __syncwarp();
-      if (lane == 0) mbar_arrive_local(&chunk_empty);
-    }
-    if (ok && m < M) {
-      const int ka = row_exp(amax[m]);
-      const int64_t nb = (int64_t)(r0 + half * 32) >> 1;
-#pragma unroll
-      for (int j = 0; j < 16; ++j) {
-        const int64_t n = nb + j;
-        if (n < N) {
-          const int kb = row_exp(bmax[n]);
-          const double sc = ldexp(1.0, -(ka + kb));
-          C[n * M + m] = make_double2(((double)hi[2 * j] + (double)lo[2 * j]) * sc,
-                                      ((double)hi[2 * j + 1] + (double)lo[2 * j + 1]) * sc);
+        for (int j = 0; j < 16; ++j) {
+          const int64_t n = nb + j;
+          if (n < N) {
+            const int es = ea + (int)b_exp[n];
+            C[n * M + m] = make_double2(to_double(hi[2 * j], lo[2 * j], es), to_double(hi[2 * j + 1], lo[2 * j + 1], es));
+          }
         }
       }
     }
@@ -237,54 +313,39 @@ __global__ void __launch_bounds__(kThreads, 1)
   }
 }
 
-// 3-D map over the digit planes: (2Kp elements, rows, planes), box (16, box_rows, 1), 32B swizzle.
-bool make_map32(CUtensorMap* tm, const void* base, int64_t Kp, int64_t rows, int planes, int box_rows,
-                std::string* why) {
-  EncodeTiledFn enc = get_encode();
-  if (!enc) {
-    if (why) *why = "cuTensorMapEncodeTiled unavailable";
-    return false;
-  }
-  cuuint64_t gdim[3] = {(cuuint64_t)(2 * Kp), (cuuint64_t)rows, (cuuint64_t)planes};
-  cuuint64_t gstr[2] = {(cuuint64_t)(2 * Kp * 2), (cuuint64_t)(rows * 2 * Kp * 2)};
-  cuuint32_t box[3] = {(cuuint32_t)kBK, (cuuint32_t)box_rows, 1u};
-  cuuint32_t estr[3] = {1u, 1u, 1u};
-  CUresult r = enc(tm, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 3, const_cast<void*>(base), gdim, gstr, box, estr,
-                   CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_32B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
-                   CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
-  if (r != CUDA_SUCCESS) {
-    if (why) *why = "cuTensorMapEncodeTiled failed (" + std::to_string((int)r) + ")";
-    return false;
-  }
-  return true;
-}
-
 }  // namespace
 
-cudaError_t launch_f64e_gemm(const F64eGemmArgs& a, int* errflag, cudaStream_t s, std::string* why) {
+// Tensor path: the split and its launches, then per wave of 152 tiles about 1000 clocks per
+// stage of 8 complex k and 5000 for the drains and the store; FP64 pipe: 1.15 TFLOP/s.
+bool f64e_worthwhile(int64_t M, int64_t N, int64_t K) {
+  const double waves = (double)(((M + kBM - 1) / kBM) * ((2 * N + kBN - 1) / kBN) + 151) / 152;
+  const double tc = 8e-6 + std::floor(waves) * ((double)((K + 7) / 8) * 1000 + 5000) / 1.9e9 + (double)M * K * 60 / 4e12;
+  return tc < 4e-6 + 8.0 * (double)M * (double)N * (double)K / 1.15e12;
+}
+
+cudaError_t launch_f64e_gemm(const F64eGemmArgs& a, int sm_count, int* errflag, cudaStream_t s, std::string* why) {
   if (a.M <= 0 || a.N <= 0) return cudaSuccess;
-  if (a.Kp % 32 != 0 || !a.A || !a.B || !a.C || !a.a_max || !a.b_max) {
-    if (why) *why = "f64e_gemm: Kp must be a multiple of 32 and every operand given";
+  if (!a.A || !a.B || !a.C || !a.a_exp || !a.b_exp || !a.a_flag || !a.b_flag || a.K <= 0 || a.K > kF64eMaxK) {
+    if (why) *why = "f64e_gemm: every operand given and K at most 2^21";
     return cudaErrorInvalidValue;
   }
   if (reinterpret_cast<uintptr_t>(a.A) % 16 || reinterpret_cast<uintptr_t>(a.B) % 16) {
     if (why) *why = "f64e_gemm: digit planes must be 16-byte aligned";
     return cudaErrorInvalidValue;
   }
-  CUtensorMap tmA, tmB;
-  if (!make_map32(&tmA, a.A, a.Kp, a.M, kS, kBM, why)) return cudaErrorInvalidValue;
-  if (!make_map32(&tmB, a.B, a.Kp, 2 * a.N, kS, kBN, why)) return cudaErrorInvalidValue;
+  auto kern = a.levels == 7 ? f64e_gemm_kernel<7> : f64e_gemm_kernel<8>;
   static bool attr_set = false;
   if (!attr_set) {
-    cudaError_t e = cudaFuncSetAttribute(f64e_gemm_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmem);
+    cudaError_t e = cudaFuncSetAttribute(f64e_gemm_kernel<7>, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmem);
+    if (e == cudaSuccess) e = cudaFuncSetAttribute(f64e_gemm_kernel<8>, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmem);
     if (e != cudaSuccess) return e;
     attr_set = true;
   }
-  const int nkb = (int)(2 * a.Kp / kBK);
-  const int64_t gx = (a.M + kBM - 1) / kBM;
-  const int64_t gy = (2 * a.N + kBN - 1) / kBN;
-  if (gx * gy > 2147483647LL) return cudaErrorInvalidConfiguration;
-  f64e_gemm_kernel<<<(unsigned)(gx * gy), kThreads, kSmem, s>>>(tmA, tmB, a.C, a.M, a.N, nkb, a.a_max, a.b_max,
-                                                               errflag, (int)gy);
+  const int nkb = (int)((a.K + 7) / 8);
+  const int64_t tm = (a.M + kBM - 1) / kBM, tn = (2 * a.N + kBN - 1) / kBN;
+  const int64_t grid = std::min<int64_t>(tm * tn, std::max(1, sm_count));
+  kern<<<(unsigned)grid, kThreads, kSmem, s>>>(
+      static_cast<const unsigned char*>(a.A), static_cast<const unsigned char*>(a.B), a.C, a.M, a.N, nkb, tm, tn,
+      a.a_exp, a.b_exp, a.a_flag, a.b_flag, a.token, errflag);
   return cudaGetLastError();
 }

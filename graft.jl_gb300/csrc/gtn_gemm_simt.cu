@@ -2,6 +2,7 @@
 //   C[n][m] = sum_k A[m][k] * B[n][k]      A: [M][K], B: [N][K], C: [N][M] (row-major)
 // The output is written m-fastest so that each warp's stores are contiguous.
 #include "gtn_internal.h"
+#include "gtn_group.h"
 
 #include <algorithm>
 #include <cstring>
@@ -330,6 +331,103 @@ __global__ void splitk_reduce_kernel(const T* __restrict__ P, int S, int64_t MN,
   }
 }
 
+// FP64 products that read the running tensor in place (no K-major copy): 256 threads compute a
+// TM x TN tile, every thread R x R outputs, in KS slices of each 16-wide k block.  A 64 x 64
+// tile costs 64 * 64 * 4 FMAs per k on one SM, which issues about two FP64 FMAs per clock, so a
+// product with few 64-wide tiles is bound by the SMs it leaves idle and by the padding of its
+// edge tiles, not by loads: the launcher takes the largest tile that still gives every SM two.
+// The slices' partial sums are added in order.
+template <int TM, int TN, int R, int KS>
+__global__ void __launch_bounds__(256) zgemm_view_kernel(const double2* __restrict__ T, GroupSpec mg, GroupSpec kg,
+                                                         const double2* __restrict__ B, double2* __restrict__ C,
+                                                         int64_t M, int64_t N, int64_t K, int64_t tiles_m,
+                                                         int64_t ntiles, const int* __restrict__ a_flag,
+                                                         const int* __restrict__ b_flag, int token) {
+  static_assert((TM / R) * (TN / R) * KS == 256 && BK % KS == 0, "one thread per R x R outputs and slice");
+  if (a_flag && *a_flag != token && *b_flag == 0) return;
+  __shared__ double2 As[BK][TM + 1];
+  __shared__ double2 Bs[BK][TN + 1];
+  __shared__ int64_t offM[TM], offK[BK];
+  const int tid = threadIdx.x;
+  const int ks = tid / ((TM / R) * (TN / R)), q = tid % ((TM / R) * (TN / R));
+  const int tx = q % (TM / R), ty = q / (TM / R);
+  for (int64_t tile = blockIdx.x; tile < ntiles; tile += gridDim.x) {
+    const int64_t m0 = (tile % tiles_m) * TM, n0 = (tile / tiles_m) * TN;
+    double2 acc[R][R];
+#pragma unroll
+    for (int i = 0; i < R; ++i)
+#pragma unroll
+      for (int j = 0; j < R; ++j) acc[i][j] = make_double2(0.0, 0.0);
+    if (tid < TM) offM[tid] = m0 + tid < M ? decompose(m0 + tid, mg) : 0;
+    for (int64_t k0 = 0; k0 < K; k0 += BK) {
+      if (tid < BK) offK[tid] = k0 + tid < K ? decompose(k0 + tid, kg) : 0;
+      __syncthreads();
+      for (int e = tid; e < TM * BK; e += 256) {
+        const int r = e / BK, c = e % BK;
+        As[c][r] = (m0 + r < M && k0 + c < K) ? T[offM[r] + offK[c]] : CT<double2>::zero();
+      }
+      for (int e = tid; e < TN * BK; e += 256) {
+        const int r = e / BK, c = e % BK;
+        Bs[c][r] = (n0 + r < N && k0 + c < K) ? B[(n0 + r) * K + k0 + c] : CT<double2>::zero();
+      }
+      __syncthreads();
+#pragma unroll 4
+      for (int kk = ks; kk < BK; kk += KS) {
+        double2 a[R], b[R];
+#pragma unroll
+        for (int i = 0; i < R; ++i) a[i] = As[kk][tx + (TM / R) * i];
+#pragma unroll
+        for (int j = 0; j < R; ++j) b[j] = Bs[kk][ty + (TN / R) * j];
+#pragma unroll
+        for (int i = 0; i < R; ++i)
+#pragma unroll
+          for (int j = 0; j < R; ++j) {
+            acc[i][j].x = fma(a[i].x, b[j].x, acc[i][j].x);
+            acc[i][j].x = fma(-a[i].y, b[j].y, acc[i][j].x);
+            acc[i][j].y = fma(a[i].x, b[j].y, acc[i][j].y);
+            acc[i][j].y = fma(a[i].y, b[j].x, acc[i][j].y);
+          }
+      }
+      __syncthreads();
+    }
+    if constexpr (KS > 1) {  // one output per thread and slice: R == 1
+      __shared__ double2 part[KS][TM * TN];
+      part[ks][q] = acc[0][0];
+      __syncthreads();
+      if (ks == 0)
+        for (int z = 1; z < KS; ++z) {
+          acc[0][0].x += part[z][q].x;
+          acc[0][0].y += part[z][q].y;
+        }
+      __syncthreads();
+    }
+    if (ks == 0) {
+#pragma unroll
+      for (int j = 0; j < R; ++j) {
+        const int64_t n = n0 + ty + (TN / R) * j;
+#pragma unroll
+        for (int i = 0; i < R; ++i) {
+          const int64_t m = m0 + tx + (TM / R) * i;
+          if (m < M && n < N) C[n * M + m] = acc[i][j];
+        }
+      }
+    }
+    __syncthreads();
+  }
+}
+
+template <int TM, int TN, int R, int KS>
+cudaError_t launch_view(const double2* T, const GroupSpec& mg, const GroupSpec& kg, const double2* B, double2* C,
+                        int64_t M, int64_t N, int64_t K, cudaStream_t s, const int* a_flag, const int* b_flag,
+                        int token) {
+  const int64_t tm = (M + TM - 1) / TM, nt = tm * ((N + TN - 1) / TN);
+  // a launch that usually has nothing to do keeps its grid small
+  const int64_t grid = std::min<int64_t>(nt, a_flag ? 2 * 152 : (int64_t(1) << 30));
+  zgemm_view_kernel<TM, TN, R, KS><<<(unsigned)grid, 256, 0, s>>>(T, mg, kg, B, C, M, N, K, tm, nt, a_flag, b_flag,
+                                                                 token);
+  return cudaGetLastError();
+}
+
 template <typename T>
 cudaError_t launch(const T* A, const T* B, T* C, int64_t M, int64_t N, int64_t K, cudaStream_t s) {
   if (M <= 0 || N <= 0) return cudaSuccess;
@@ -367,6 +465,17 @@ cudaError_t launch_splitk(const T* A, const T* B, T* C, int64_t M, int64_t N, in
 cudaError_t launch_zgemm_simt(const double2* A, const double2* B, double2* C, int64_t M, int64_t N,
                               int64_t K, cudaStream_t s) {
   return launch(A, B, C, M, N, K, s);
+}
+cudaError_t launch_zgemm_view(const double2* T, const GroupSpec& mg, const GroupSpec& kg, const double2* B, double2* C,
+                              int64_t M, int64_t N, int64_t K, cudaStream_t s, const int* a_flag, const int* b_flag,
+                              int token) {
+  if (M <= 0 || N <= 0) return cudaSuccess;
+  auto tiles = [&](int t) { return ((M + t - 1) / t) * ((N + t - 1) / t); };
+  if (tiles(64) >= 2 * 152) return launch_view<64, 64, 4, 1>(T, mg, kg, B, C, M, N, K, s, a_flag, b_flag, token);
+  if (tiles(32) >= 2 * 152) return launch_view<32, 32, 2, 1>(T, mg, kg, B, C, M, N, K, s, a_flag, b_flag, token);
+  if (tiles(16) >= 2 * 152) return launch_view<16, 16, 1, 1>(T, mg, kg, B, C, M, N, K, s, a_flag, b_flag, token);
+  if (tiles(8) >= 2 * 152) return launch_view<8, 8, 1, 4>(T, mg, kg, B, C, M, N, K, s, a_flag, b_flag, token);
+  return launch_view<4, 4, 1, 16>(T, mg, kg, B, C, M, N, K, s, a_flag, b_flag, token);
 }
 int gemm_splitk_slices(int64_t M, int64_t N, int64_t K) {
   const int64_t tiles = ((M + BM - 1) / BM) * (N <= 16 ? 1 : (N + BN - 1) / BN);

@@ -39,6 +39,10 @@ struct gtn_ctx_s {
   std::mutex err_mu;
   int64_t launches = 0;
   int* d_errflag = nullptr;
+  // out-of-range flags of the digit-plane products: product number t writes t to slot
+  // t % kFbSlots, so no slot needs clearing between products (they are ordered on the stream)
+  int* d_fbflag = nullptr;
+  int fb_token = 0;
   int sm_count = 0;
   int cc_major = 0, cc_minor = 0;
   // reduction scratch (device + pinned host)
@@ -62,6 +66,8 @@ struct gtn_ctx_s {
   std::multimap<size_t, void*> blk_free;
   size_t blk_cached = 0;
 };
+
+constexpr int kFbSlots = 1024;
 
 // ---- status helpers -------------------------------------------------------------
 int set_err(gtn_ctx ctx, int code, const std::string& msg);
@@ -135,11 +141,6 @@ cudaError_t launch_split16_rows_tab(const void* T, int is64, const GatherTab& t,
 cudaError_t launch_split16_rows_grp(const void* T, int is64, const GroupSpec& mg, const GroupSpec& kg, int64_t M,
                                     int64_t K, int64_t Kp, int64_t pstride, float* amax, __nv_bfloat16* out,
                                     cudaStream_t s, bool* done);
-cudaError_t launch_split_i7_rows_tab(const double2* T, const GatherTab& t, int64_t M, int64_t K, int64_t Kp,
-                                     int64_t pstride, float* amax, __nv_bfloat16* out, cudaStream_t s, bool* done);
-cudaError_t launch_split_i7_rows_grp(const double2* T, const GroupSpec& mg, const GroupSpec& kg, int64_t M, int64_t K,
-                                     int64_t Kp, int64_t pstride, float* amax, __nv_bfloat16* out, cudaStream_t s,
-                                     bool* done);
 cudaError_t launch_gather_tab_to_c128(const void* T, int is64, const GatherTab& t, int64_t M, int64_t K, int64_t ldo,
                                       double2* out, cudaStream_t s);
 // fp16 slice planes (2 planes, hi + lo) of a K-major gather, rows scaled by
@@ -342,27 +343,51 @@ __host__ __device__ inline float fp16_row_scale_inv(float mx) {
 }
 cudaError_t launch_tc_gemm(const TcGemmArgs& a, int* errflag, cudaStream_t s, std::string* why);
 
-// ---- FP64-grade GEMM on the tensor cores (gtn_gemm_f64e.cu) ------------------------------
-// C (complex FP64, [N][M]) = A B^T from integer digit planes: A [S][M][2Kp] (rows scaled by
-// 2^k(a_max[m])), B' [S][2N][2Kp] (complex rows scaled by 2^k(b_max[n])), S = kF64eSlices.
+// ---- FP64-accurate GEMM on the tensor cores (gtn_gemm_f64e.cu) ---------------------------
+// C (complex FP64, [N][M]) = A B^T from integer digit planes (7 base-256 digits): A in blocks
+// [row tile of 128][16 real k][plane][128][32 bytes], the real-expanded B' in blocks of 64
+// rows; row m of A scaled by 2^(1021 - a_exp[m]), complex row n of B by 2^(1021 - b_exp[n])
+// (biased exponents of the rows' largest entries).  A row whose exponent lies outside
+// [kF64eMinExp, kF64eMaxExp] (infinities, NaN, magnitudes beyond 2^+-450) sets a flag, the GEMM
+// then leaves C alone and the FP64 kernel launched behind it computes the product.
 constexpr int kF64eSlices = 7;
+constexpr int kF64eRowsA = 128, kF64eRowsB = 64;
+constexpr int64_t kF64eMaxK = int64_t(1) << 21;  // the 64-bit sums hold 2^22 real k
+constexpr int kF64eMinExp = 1023 - 450, kF64eMaxExp = 1023 + 450;
+inline size_t f64e_a_bytes(int64_t M, int64_t K) {
+  return (size_t)((M + kF64eRowsA - 1) / kF64eRowsA) * ((K + 7) / 8) * kF64eSlices * kF64eRowsA * 32;
+}
+inline size_t f64e_b_bytes(int64_t N, int64_t K) {
+  return (size_t)((2 * N + kF64eRowsB - 1) / kF64eRowsB) * ((K + 7) / 8) * kF64eSlices * kF64eRowsB * 32;
+}
+// When the digit-plane GEMM takes an FP64 step (M, N, K) from the FP64 pipe.
+bool f64e_worthwhile(int64_t M, int64_t N, int64_t K);
 struct F64eGemmArgs {
-  const __nv_bfloat16* A = nullptr;
-  const __nv_bfloat16* B = nullptr;
+  const void* A = nullptr;
+  const void* B = nullptr;
   double2* C = nullptr;
-  int64_t M = 0, N = 0, Kp = 0;
-  const float* a_max = nullptr;
-  const float* b_max = nullptr;
+  int64_t M = 0, N = 0, K = 0;
+  const float* a_exp = nullptr;
+  const float* b_exp = nullptr;
+  const int* a_flag = nullptr;  // == token: a row of A out of range
+  const int* b_flag = nullptr;  // != 0: a row of B out of range
+  int token = 0;
+  int levels = 8;               // digit products d_i e_j with i + j < levels (7 or 8)
 };
-cudaError_t launch_f64e_gemm(const F64eGemmArgs& a, int* errflag, cudaStream_t s, std::string* why);
-// digit planes of the running tensor's K-major view (c128), rows scaled by amax (from
-// launch_rowmax_*), and of a static B [N][K] (bmax written here)
-cudaError_t launch_split_i7_tab(const double2* T, const GatherTab& t, int64_t M, int64_t K, int64_t Kp,
-                               int64_t pstride, const float* amax, __nv_bfloat16* out, cudaStream_t s);
-cudaError_t launch_split_i7_c128(const double2* T, const GroupSpec& mg, const GroupSpec& kg, int64_t M, int64_t K,
-                                 int64_t Kp, int64_t pstride, const float* amax, __nv_bfloat16* out, cudaStream_t s);
-cudaError_t launch_pack_b_planes_i7(const double2* B, int64_t N, int64_t K, int64_t Kp, int64_t pstride,
-                                    __nv_bfloat16* out, float* bmax, cudaStream_t s);
+cudaError_t launch_f64e_gemm(const F64eGemmArgs& a, int sm_count, int* errflag, cudaStream_t s, std::string* why);
+// Digit planes and row exponents of the running tensor's K-major view (c128; *flag = token when
+// a row is out of range), and of a static B [N][K] (*flag = 1 when a row is out of range).
+cudaError_t launch_split_digits_tab(const double2* T, const GatherTab& t, int64_t M, int64_t K, float* rexp, void* out,
+                                    int* flag, int token, cudaStream_t s, int* launches);
+cudaError_t launch_split_digits_grp(const double2* T, const GroupSpec& mg, const GroupSpec& kg, int64_t M, int64_t K,
+                                    float* rexp, void* out, int* flag, int token, cudaStream_t s, int* launches);
+cudaError_t launch_pack_b_digits(const double2* B, int64_t N, int64_t K, void* out, float* bexp, int* flag,
+                                 cudaStream_t s);
+// C[n][m] = sum_k T[offM(m) + offK(k)] B[n][k] on the FP64 pipe, T read in place; with a_flag
+// set the launch does its work only if *a_flag == token or *b_flag != 0.
+cudaError_t launch_zgemm_view(const double2* T, const GroupSpec& mg, const GroupSpec& kg, const double2* B, double2* C,
+                              int64_t M, int64_t N, int64_t K, cudaStream_t s, const int* a_flag = nullptr,
+                              const int* b_flag = nullptr, int token = 0);
 bool tc_gemm_supported(int cc_major, int cc_minor);
 // Independent problems in one launch per 56 problems (same product list for all).
 cudaError_t launch_tc_gemm_grouped(const TcGemmArgs* probs, int nprob, int* errflag, cudaStream_t s,
@@ -425,6 +450,12 @@ struct PlanStep {
   float* bmax = nullptr;           // [N] row maxima of the static (fp16 planes)
   GatherTab tab;                   // offset tables of the running tensor's [M, K] view (tc steps)
   int splitk = 1;                  // K slices of the SIMT GEMM (few output tiles, long K)
+  // FP64-accurate digit-plane GEMM (FP64 and FP64E plans): planes, row exponents and
+  // out-of-range flag of the static; bdig stays null where the FP64 pipe keeps the step
+  bool dg = false;
+  void* bdig = nullptr;
+  float* bexp = nullptr;
+  int* bflag = nullptr;
   double macs = 0;
 };
 
@@ -458,7 +489,8 @@ struct gtn_map_s {
   int64_t max_t = 0;       // largest running tensor (elements)
   int64_t max_a = 0;       // largest A operand (elements, for permuted / split staging)
   int64_t max_apl = 0;     // largest split-plane staging (bf16 elements per plane * planes)
-  int64_t max_mtc = 0;     // largest M of a tensor-core step (fp16 row maxima)
+  int64_t max_mtc = 0;     // largest M of a tensor-core step (fp16 row maxima, digit row exponents)
+  size_t max_adg = 0;      // largest digit-plane operand (bytes)
   int64_t max_splitk = 0;  // largest split-K partial-sum workspace (complex elements)
   bool oneshot = false;    // a one-shot contraction (gtn_contract): arena allocations, no tables
   char* arena = nullptr;   // allocations come from here first (one-shot contractions)

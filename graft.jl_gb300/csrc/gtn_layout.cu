@@ -3,6 +3,7 @@
 // HBM-bound; tiles are 32x32 through shared memory so that both the read and the write
 // side are coalesced.
 #include "gtn_internal.h"
+#include "gtn_group.h"
 
 #include <algorithm>
 #include <cstdlib>
@@ -10,18 +11,6 @@
 #include <type_traits>
 
 namespace {
-
-__device__ __forceinline__ int64_t decompose(int64_t i, const GroupSpec& g) {
-  int64_t off = 0;
-#pragma unroll 1
-  for (int j = g.n - 1; j >= 0; --j) {
-    const int64_t d = g.dim[j];
-    const int64_t q = i / d;
-    off += (i - q * d) * g.str[j];
-    i = q;
-  }
-  return off;
-}
 
 template <typename T> struct Zero;
 template <> struct Zero<double2> { __device__ static double2 v() { return make_double2(0.0, 0.0); } };
@@ -319,6 +308,11 @@ __device__ __forceinline__ float absmax2(double2 v) {
   return __uint_as_float((static_cast<uint32_t>(fe) << 23) | static_cast<uint32_t>((m >> 29) & 0x7fffffu));
 }
 
+// The row "maximum" of a split: magnitudes here, binary exponents for the digit planes.
+struct AbsMag {
+  template <typename T> __device__ static float of(T v) { return absmax2(v); }
+};
+
 // Element (m, k) as two fp16 planes, the row scaled by fp16_row_scale of its maximum.
 template <typename Tin>
 __device__ __forceinline__ void put16(__half* out, int64_t ld2, int64_t pstride, int64_t m, int64_t k, Tin v,
@@ -344,6 +338,9 @@ struct Split16Writer {
 // The same, handed the row maximum (the fused split computes it in shared memory), for two
 // adjacent columns k, k + 1 (k even): one 8-byte store per plane.
 struct Split16RowWriter {
+  using Mag = AbsMag;
+  static constexpr int kCols = 2;
+  __device__ void row(float) const {}
   __half* out;
   int64_t ld2;
   int64_t pstride;
@@ -366,109 +363,161 @@ struct Split16RowWriter {
 };
 
 // ---- integer digit planes of the FP64-grade tensor-core GEMM (gtn_gemm_f64e.cu) ---------
-// x 2^k (|x| 2^k < 1, k from the row maximum) as kF64eSlices signed base-128 digits,
-// x 2^k = sum_i d_i 2^{-7(i+1)}: the fixed-point value N = round(x 2^{k + 7 S}) is formed
-// from the double's bits with integer operations (no FP64 arithmetic), then peeled from the
-// top digit down with round-half-up shifts; |d_0| <= 128, |d_i| <= 64, all exact in bf16.
-__device__ __forceinline__ int f64e_row_exp(float mx) {
-  const uint32_t b = __float_as_uint(mx);
-  const int e = (int)((b >> 23) & 0xffu);
-  return mx > 0.f ? 126 - e : 0;
-}
-__device__ __forceinline__ void i7_digits(double x, int k, __nv_bfloat16* d) {
-  constexpr int NB = 7 * kF64eSlices;
+// x 2^k (|x| 2^k < 1/2, k from the row's largest binary exponent) as kF64eSlices signed
+// base-256 digits, x 2^k = sum_i d_i 2^{-8(i+1)}: the fixed-point value N = round(x 2^{k+56})
+// is formed from the double's bits with integer operations (no FP64 arithmetic).  Adding 128
+// to every digit position turns the balanced digits into the bytes of one 56-bit number
+// (only the top one may reach 128 after the rounding), so a digit costs one byte extraction
+// and one FP32 add of 2^23 + byte instead of 64-bit shifts; |d_i| <= 128, exact in bf16.
+// Row "maxima" of these planes are the biased binary exponents of the largest entry (0 for a
+// zero or subnormal row, 2047 for a row with an infinity or NaN), held as floats.
+struct ExpMag {  // exponent of max(|re|, |im|)
+  __device__ static float of(double2 v) {
+    const int a = (__double2hiint(v.x) >> 20) & 0x7ff, c = (__double2hiint(v.y) >> 20) & 0x7ff;
+    return (float)max(a, c);
+  }
+};
+
+// N + 0x80808080808080 (56 bits, a carry into bit 56 possible) of x under row exponent E.
+__device__ __forceinline__ unsigned long long digit_word(double x, int E) {
   const long long bits = __double_as_longlong(x);
-  const int E = (int)((bits >> 52) & 0x7ff);
-  long long N = 0;
-  if (E != 0 && E != 0x7ff) {
-    const long long mant = (bits & 0xFFFFFFFFFFFFFLL) | (1LL << 52);
-    const int r = 1075 - E - k - NB;  // >= 4 whenever |x| 2^k < 1
-    if (r <= 0) N = mant << (r < -10 ? 10 : -r);
-    else if (r < 63) N = (mant + (1LL << (r - 1))) >> r;
-    if (bits < 0) N = -N;
-  }
-#pragma unroll
-  for (int i = 0; i < kF64eSlices; ++i) {
-    const int w = 7 * (kF64eSlices - 1 - i);
-    long long di;
-    if (w > 0) {
-      di = (N + (1LL << (w - 1))) >> w;
-      N -= di << w;
-    } else {
-      di = N;
-    }
-    d[i] = __float2bfloat16_rn((float)di);
-  }
+  const int e = (int)((bits >> 52) & 0x7ff);
+  unsigned long long mant = ((unsigned long long)bits & 0xFFFFFFFFFFFFFull) | (1ull << 52);
+  // x 2^k = mant 2^{e - 1075} 2^{1021 - E}; N = mant 2^{e - E + 2} rounded half up
+  const int r = E - e - 2;
+  unsigned long long N = 0;
+  if (e != 0 && r < 60) N = r <= 0 ? mant << -r : (mant + (1ull << (r - 1))) >> r;
+  return 0x80808080808080ull + (bits < 0 ? 0ull - N : N);
 }
-__device__ __forceinline__ void i7_digits(float x, int k, __nv_bfloat16* d) { i7_digits((double)x, k, d); }
-
-// Element (m, k) as kF64eSlices digit planes, the row scaled by 2^k of its maximum.
-template <typename Tin>
-__device__ __forceinline__ void put_i7(__nv_bfloat16* out, int64_t ld2, int64_t pstride, int64_t m, int64_t k,
-                                       Tin v, float rowmax) {
-  const int e = f64e_row_exp(rowmax);
-  __nv_bfloat16 dr[kF64eSlices], di[kF64eSlices];
-  i7_digits(v.x, e, dr);
-  i7_digits(v.y, e, di);
-  __nv_bfloat16* row = out + m * ld2 + 2 * k;
-#pragma unroll
-  for (int p = 0; p < kF64eSlices; ++p) {
-    __nv_bfloat162 pr;
-    pr.x = dr[p];
-    pr.y = di[p];
-    *reinterpret_cast<__nv_bfloat162*>(row + p * pstride) = pr;
+// Digits i of two numbers as a bf16 pair (first in the low half).
+__device__ __forceinline__ uint32_t digit_pair(unsigned long long a, unsigned long long b, int i) {
+  float fa, fb;
+  if (i == 0) {
+    fa = (float)((int)(a >> 48) - 128);
+    fb = (float)((int)(b >> 48) - 128);
+  } else {
+    const uint32_t wa = i < 3 ? (uint32_t)(a >> 32) : (uint32_t)a, wb = i < 3 ? (uint32_t)(b >> 32) : (uint32_t)b;
+    const uint32_t sel = 0x7440u + (uint32_t)(i < 3 ? 2 - i : 6 - i);  // byte of w, zeros, 0x4B
+    fa = __uint_as_float(__byte_perm(wa, 0x4B000000u, sel)) - 8388736.f;  // 2^23 + byte - (2^23 + 128)
+    fb = __uint_as_float(__byte_perm(wb, 0x4B000000u, sel)) - 8388736.f;
   }
+  return __byte_perm(__float_as_uint(fa), __float_as_uint(fb), 0x7632);  // the bf16 halves: exact
+}
+// Byte offset, within the digit planes of an operand with `rows` rows per tile, of plane 0 of
+// the 16-byte chunk `chunk` (8 real k) of row r: blocks [row tile][16 k][plane][rows][32 bytes],
+// each (row tile, 16 k) block contiguous so that one bulk copy loads a pipeline stage; the
+// two chunks of a row are swapped in rows 4-7 of every 8 (the 32-byte swizzle of the MMA).
+__device__ __forceinline__ int64_t digit_chunk(int64_t r, int64_t chunk, int rows, int64_t nkb) {
+  const int64_t rt = r / rows;
+  const int rr = (int)(r - rt * rows);
+  return ((rt * nkb + (chunk >> 1)) * kF64eSlices * rows + rr) * 32 + (((int)chunk ^ (rr >> 2)) & 1) * 16;
+}
+__device__ __forceinline__ void digit_check(float E, int token, int* flag) {
+  if (E != 0.f && !(E >= (float)kF64eMinExp && E <= (float)kF64eMaxExp)) *flag = token;
 }
 
-struct Int7Writer {
-  __nv_bfloat16* out;
-  int64_t ld2;      // row pitch (= 2 Kp)
-  int64_t pstride;  // plane pitch
-  const float* amax;
-  template <typename Tin> __device__ void operator()(int64_t m, int64_t k, Tin v) const {
-    put_i7(out, ld2, pstride, m, k, v, amax[m]);
+// Element (m, k) of the A operand: its digits in the planes (4 bytes each).
+struct DigitWriter {
+  unsigned char* out;
+  int64_t nkb;
+  const float* rexp;
+  int* flag;
+  int token;
+  __device__ void operator()(int64_t m, int64_t k, double2 v) const {
+    const float E = rexp[m];
+    digit_check(E, token, flag);
+    const unsigned long long a = digit_word(v.x, (int)E), b = digit_word(v.y, (int)E);
+    unsigned char* p = out + digit_chunk(m, k >> 2, kF64eRowsA, nkb) + (k & 3) * 4;
+#pragma unroll
+    for (int i = 0; i < kF64eSlices; ++i) *reinterpret_cast<uint32_t*>(p + i * kF64eRowsA * 32) = digit_pair(a, b, i);
   }
 };
-struct Int7RowWriter {
-  __nv_bfloat16* out;
-  int64_t ld2;
-  int64_t pstride;
-  template <typename Tin> __device__ void operator()(int64_t m, int64_t k, Tin v0, Tin v1, float rowmax) const {
-    put_i7(out, ld2, pstride, m, k, v0, rowmax);
-    put_i7(out, ld2, pstride, m, k + 1, v1, rowmax);
+// The same for four adjacent columns (k a multiple of 4), the row exponent in hand: one
+// 16-byte store per plane.
+struct DigitRowWriter {
+  unsigned char* out;
+  int64_t nkb;
+  int* flag;
+  int token;
+  using Mag = ExpMag;
+  static constexpr int kCols = 4;
+  __device__ void row(float E) const { digit_check(E, token, flag); }
+  __device__ void operator()(int64_t m, int64_t k, const double2* v, float E) const {
+    unsigned long long w[8];
+#pragma unroll
+    for (int j = 0; j < 4; ++j) {
+      w[2 * j] = digit_word(v[j].x, (int)E);
+      w[2 * j + 1] = digit_word(v[j].y, (int)E);
+    }
+    unsigned char* p = out + digit_chunk(m, k >> 2, kF64eRowsA, nkb);
+#pragma unroll
+    for (int i = 0; i < kF64eSlices; ++i)
+      *reinterpret_cast<uint4*>(p + i * kF64eRowsA * 32) =
+          make_uint4(digit_pair(w[0], w[1], i), digit_pair(w[2], w[3], i), digit_pair(w[4], w[5], i),
+                     digit_pair(w[6], w[7], i));
   }
 };
 
-__global__ void pack_b_planes_i7_kernel(const double2* __restrict__ B, int64_t N, int64_t K, int64_t Kp,
-                                        int64_t pstride, const float* __restrict__ bmax,
-                                        __nv_bfloat16* __restrict__ out) {
-  const int64_t total = 2 * N * Kp;
-  for (int64_t idx = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; idx < total;
-       idx += (int64_t)gridDim.x * blockDim.x) {
-    const int64_t row = idx / Kp;
-    const int64_t k = idx - row * Kp;
-    const int64_t n = row >> 1;
-    const int e = f64e_row_exp(bmax[n]);
-    double v0 = 0.0, v1 = 0.0;
-    if (k < K) {
-      const double2 b = B[n * K + k];
-      if ((row & 1) == 0) { v0 = b.x; v1 = -b.y; } else { v0 = b.y; v1 = b.x; }
+// B' = [[Br, -Bi], [Bi, Br]] of a static B [N][K]: CTA b takes the complex rows 8b .. 8b + 7,
+// one warp per row for the exponents, then every thread the digits of 4 columns of a row for
+// both real rows (the digits of -Bi are the negated digits of Bi).
+__global__ void __launch_bounds__(256) pack_b_digits_kernel(const double2* __restrict__ B, int64_t N, int64_t K,
+                                                            int64_t nkb, float* __restrict__ bexp,
+                                                            unsigned char* __restrict__ out, int* flag) {
+  __shared__ float se[8];
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int64_t n0 = (int64_t)blockIdx.x * 8;
+  {
+    const int64_t n = n0 + warp;
+    float x = 0.f;
+    if (n < N)
+      for (int64_t k = lane; k < K; k += 32) x = fmaxf(x, ExpMag::of(B[n * K + k]));
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) x = fmaxf(x, __shfl_xor_sync(0xffffffffu, x, o));
+    if (lane == 0) {
+      se[warp] = x;
+      if (n < N) {
+        bexp[n] = x;
+        digit_check(x, 1, flag);
+      }
     }
-    __nv_bfloat16 d0[kF64eSlices], d1[kF64eSlices];
-    i7_digits(v0, e, d0);
-    i7_digits(v1, e, d1);
-    for (int p = 0; p < kF64eSlices; ++p) {
-      __nv_bfloat162 pr;
-      pr.x = d0[p];
-      pr.y = d1[p];
-      *reinterpret_cast<__nv_bfloat162*>(out + p * pstride + row * (2 * Kp) + 2 * k) = pr;
+  }
+  __syncthreads();
+  const int nr = (int)min((int64_t)8, N - n0);
+  const int64_t total = 2 * nkb * 8;  // (16-k block, row, chunk), chunk fastest
+  for (int64_t e = threadIdx.x; e < total; e += 256) {
+    const int r = (int)((e >> 1) & 7);
+    if (r >= nr) continue;
+    const int64_t chunk = (e >> 4) * 2 + (e & 1), k = chunk * 4, n = n0 + r;
+    const int E = (int)se[r];
+    unsigned long long w[8];
+#pragma unroll
+    for (int j = 0; j < 4; ++j) {
+      const double2 v = k + j < K ? B[n * K + k + j] : make_double2(0.0, 0.0);
+      w[2 * j] = digit_word(v.x, E);
+      w[2 * j + 1] = digit_word(v.y, E);
+    }
+    // (the two real rows share a swizzle group: 2n and 2n + 1 differ in bit 0 only)
+    unsigned char* p = out + digit_chunk(2 * n, chunk, kF64eRowsB, nkb);
+#pragma unroll
+    for (int i = 0; i < kF64eSlices; ++i) {
+      uint32_t q[4], t[4];
+#pragma unroll
+      for (int j = 0; j < 4; ++j) {
+        const uint32_t d = digit_pair(w[2 * j], w[2 * j + 1], i);
+        q[j] = d ^ 0x80000000u;                 // (re, -im)
+        t[j] = __byte_perm(d, d, 0x1032);       // (im, re)
+      }
+      unsigned char* o = p + i * kF64eRowsB * 32;
+      *reinterpret_cast<uint4*>(o) = make_uint4(q[0], q[1], q[2], q[3]);
+      *reinterpret_cast<uint4*>(o + 32) = make_uint4(t[0], t[1], t[2], t[3]);
     }
   }
 }
 
 // amax[m] = max over k of max(|re|, |im|) of the K-major gather (atomic max of the
 // non-negative float bits; amax zeroed before the launch).
-template <typename Tin, class Off, int TM, int TK>
+template <typename Tin, class Off, int TM, int TK, class Mag = AbsMag>
 __device__ __forceinline__ void rowmax_tile(const Tin* __restrict__ T, const Off& off, int64_t M, int64_t K, int m_fast,
                                             float* __restrict__ amax, int64_t m0, int64_t k0) {
   // TM x TK = 2048 elements per tile (8 loads in flight per thread); 256 x 8 when the rows
@@ -491,7 +540,7 @@ __device__ __forceinline__ void rowmax_tile(const Tin* __restrict__ T, const Off
     const int e = it * 256 + tid;
     const int im = m_fast ? (e % TM) : (e / TK);
     const int ik = m_fast ? (e / TM) : (e % TK);
-    v[it] = (m0 + im < M && k0 + ik < K) ? absmax2(T[offM[im] + offK[ik]]) : 0.f;
+    v[it] = (m0 + im < M && k0 + ik < K) ? Mag::of(T[offM[im] + offK[ik]]) : 0.f;
   }
 #pragma unroll
   for (int it = 0; it < 8; ++it) {
@@ -513,10 +562,10 @@ __device__ __forceinline__ void rowmax_tile(const Tin* __restrict__ T, const Off
   }
 }
 
-template <typename Tin, class Off, int TM, int TK>
+template <typename Tin, class Off, int TM, int TK, class Mag>
 __global__ void __launch_bounds__(256) rowmax_kernel(const Tin* __restrict__ T, Off off, int64_t M, int64_t K,
                                                      int m_fast, float* __restrict__ amax) {
-  rowmax_tile<Tin, Off, TM, TK>(T, off, M, K, m_fast, amax, (int64_t)blockIdx.x * TM, (int64_t)blockIdx.y * TK);
+  rowmax_tile<Tin, Off, TM, TK, Mag>(T, off, M, K, m_fast, amax, (int64_t)blockIdx.x * TM, (int64_t)blockIdx.y * TK);
 }
 
 // bmax[n] = max over k of max(|re|, |im|) of B[n][:], one CTA per row
@@ -571,6 +620,7 @@ __device__ __forceinline__ void cfma(float2& acc, float2 a, float2 b) {
 }
 
 constexpr int kSmallSmemBytes = 48 * 1024;
+__host__ __device__ constexpr size_t small_offk_bytes(int K) { return ((size_t)K * sizeof(int64_t) + 15) / 16 * 16; }
 
 // C[n][m] = sum_k T[offM(m) + offK(k)] * B[n][k]; B and the K offsets live in shared memory.
 template <typename T, int NB>
@@ -580,7 +630,7 @@ __device__ __forceinline__ void small_contract_body(const T* __restrict__ A, con
                                                     int64_t nblk) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
   int64_t* offK = reinterpret_cast<int64_t*>(smem_raw);
-  T* Bs = reinterpret_cast<T*>(smem_raw + ((K * sizeof(int64_t) + 15) / 16) * 16);
+  T* Bs = reinterpret_cast<T*>(smem_raw + small_offk_bytes(K));
   for (int i = threadIdx.x; i < K; i += blockDim.x) offK[i] = decompose(i, kg);
   for (int i = threadIdx.x; i < N * K; i += blockDim.x) Bs[i] = B[i];
   __syncthreads();
@@ -615,7 +665,7 @@ template <typename T>
 cudaError_t launch_small(const T* A, const GroupSpec& mg, const GroupSpec& kg, int64_t M, int K,
                          int N, const T* B, T* C, cudaStream_t s) {
   if (M <= 0) return cudaSuccess;
-  const size_t smem = ((K * sizeof(int64_t) + 15) / 16) * 16 + (size_t)N * K * sizeof(T);
+  const size_t smem = small_offk_bytes(K) + (size_t)N * K * sizeof(T);
   if (smem > (size_t)kSmallSmemBytes) return cudaErrorInvalidValue;
   int64_t blocks = (M + 255) / 256;
   if (blocks > 152 * 16) blocks = 152 * 16;
@@ -1150,7 +1200,7 @@ __global__ void __launch_bounds__(256) split_rows_kernel(const Tin* __restrict__
   const int warp = tid >> 5, lane = tid & 31;
   for (int r = warp; r < TR; r += 8) {
     float x = 0.f;
-    for (int c = lane; c < kv; c += 32) x = fmaxf(x, absmax2(tile[r * pitch + c]));
+    for (int c = lane; c < kv; c += 32) x = fmaxf(x, W::Mag::of(tile[r * pitch + c]));
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) x = fmaxf(x, __shfl_xor_sync(0xffffffffu, x, o));
     if (lane == 0) pmax[r] = x;
@@ -1169,16 +1219,33 @@ __global__ void __launch_bounds__(256) split_rows_kernel(const Tin* __restrict__
     if (tid < TR) rmax[tid] = pmax[tid];
     __syncthreads();
   }
-  if (rank == 0 && tid < TR && m0 + tid < M) amax[m0 + tid] = rmax[tid];
-  // columns in pairs (kc, Kp and k0 are even): 8-byte stores per plane; (row, pair) indices
-  // run jointly over the threads, so short rows still keep every thread busy
-  const int hw = kw / 2;
-  const FastDiv dhw = make_fastdiv((uint32_t)(hw > 0 ? hw : 1));
+  if (rank == 0 && tid < TR && m0 + tid < M) {
+    amax[m0 + tid] = rmax[tid];
+    w.row(rmax[tid]);
+  }
   const int nrows = (int)min((int64_t)TR, M - m0);
-  for (int e = tid; e < nrows * hw; e += 256) {
-    const int r = (int)fast_div((uint32_t)e, dhw), c = 2 * (e - r * hw);
-    w(m0 + r, k0 + c, c < kv ? tile[r * pitch + c] : Zero<Tin>::v(),
-      c + 1 < kv ? tile[r * pitch + c + 1] : Zero<Tin>::v(), rmax[r]);
+  if constexpr (W::kCols == 4) {
+    // digit planes: 16-byte chunks of 4 columns (kc, Kp and k0 are multiples of 8), the two
+    // chunks of a row's 32 bytes and then the rows on consecutive threads
+    const FastDiv drow = make_fastdiv((uint32_t)nrows);
+    for (int e = tid; e < nrows * (kw / 4); e += 256) {
+      const int rk = e >> 1;
+      const int kb = (int)fast_div((uint32_t)rk, drow), r = rk - kb * nrows, c = kb * 8 + (e & 1) * 4;
+      Tin v[4];
+#pragma unroll
+      for (int j = 0; j < 4; ++j) v[j] = c + j < kv ? tile[r * pitch + c + j] : Zero<Tin>::v();
+      w(m0 + r, k0 + c, v, rmax[r]);
+    }
+  } else {
+    // columns in pairs (kc, Kp and k0 are even): 8-byte stores per plane; (row, pair) indices
+    // run jointly over the threads, so short rows still keep every thread busy
+    const int hw = kw / 2;
+    const FastDiv dhw = make_fastdiv((uint32_t)(hw > 0 ? hw : 1));
+    for (int e = tid; e < nrows * hw; e += 256) {
+      const int r = (int)fast_div((uint32_t)e, dhw), c = 2 * (e - r * hw);
+      w(m0 + r, k0 + c, c < kv ? tile[r * pitch + c] : Zero<Tin>::v(),
+        c + 1 < kv ? tile[r * pitch + c + 1] : Zero<Tin>::v(), rmax[r]);
+    }
   }
   if (cs > 1) cluster_wait();  // peers may read this CTA's maxima until they have arrived
 }
@@ -1565,7 +1632,7 @@ cudaError_t launch_split_c64(const float2* T, const GroupSpec& mg, const GroupSp
                              __nv_bfloat16* out, cudaStream_t s) {
   return launch_gather(T, mg, kg, M, K, Kp, SplitWriter{out, 2 * Kp, pstride, nplanes}, s);
 }
-template <typename Tin, class Off>
+template <class Mag = AbsMag, typename Tin, class Off>
 static cudaError_t launch_rowmax(const Tin* T, const Off& off, int m_fast, int64_t M, int64_t K, float* amax,
                                  cudaStream_t s) {
   static_assert(!std::is_same<Off, GrpOff>::value, "kernel parameters hold index groups by value (GrpOffV)");
@@ -1575,13 +1642,13 @@ static cudaError_t launch_rowmax(const Tin* T, const Off& off, int m_fast, int64
   if (m_fast) {
     const int64_t gx = (M + 255) / 256, gy = (K + 7) / 8;
     if (gy > 65535 || gx > 2147483647LL) return cudaErrorInvalidConfiguration;
-    rowmax_kernel<Tin, Off, 256, 8><<<dim3((unsigned)gx, (unsigned)gy), dim3(32, 8), 0, s>>>(T, off, M, K, m_fast,
-                                                                                           amax);
+    rowmax_kernel<Tin, Off, 256, 8, Mag><<<dim3((unsigned)gx, (unsigned)gy), dim3(32, 8), 0, s>>>(T, off, M, K,
+                                                                                                m_fast, amax);
   } else {
     const int64_t gx = (M + 63) / 64, gy = (K + 31) / 32;
     if (gy > 65535 || gx > 2147483647LL) return cudaErrorInvalidConfiguration;
-    rowmax_kernel<Tin, Off, 64, 32><<<dim3((unsigned)gx, (unsigned)gy), dim3(32, 8), 0, s>>>(T, off, M, K, m_fast,
-                                                                                           amax);
+    rowmax_kernel<Tin, Off, 64, 32, Mag><<<dim3((unsigned)gx, (unsigned)gy), dim3(32, 8), 0, s>>>(T, off, M, K,
+                                                                                                m_fast, amax);
   }
   return cudaGetLastError();
 }
@@ -1632,37 +1699,43 @@ cudaError_t launch_split16_rows_grp(const void* T, int is64, const GroupSpec& mg
   return is64 ? launch_split_rows(static_cast<const double2*>(T), off, M, K, Kp, mf, w, amax, s, done)
               : launch_split_rows(static_cast<const float2*>(T), off, M, K, Kp, mf, w, amax, s, done);
 }
-cudaError_t launch_split_i7_rows_tab(const double2* T, const GatherTab& t, int64_t M, int64_t K, int64_t Kp,
-                                     int64_t pstride, float* amax, __nv_bfloat16* out, cudaStream_t s, bool* done) {
-  return launch_split_rows(T, TabOff{t.om, t.ok}, M, K, Kp, t.m_fast, Int7RowWriter{out, 2 * Kp, pstride}, amax, s,
-                           done);
-}
-cudaError_t launch_split_i7_rows_grp(const double2* T, const GroupSpec& mg, const GroupSpec& kg, int64_t M, int64_t K,
-                                     int64_t Kp, int64_t pstride, float* amax, __nv_bfloat16* out, cudaStream_t s,
-                                     bool* done) {
-  return launch_split_rows(T, GrpOffV{mg, kg}, M, K, Kp, choose_m_fast(mg, kg) ? 1 : 0,
-                           Int7RowWriter{out, 2 * Kp, pstride}, amax, s, done);
-}
-cudaError_t launch_split_i7_tab(const double2* T, const GatherTab& t, int64_t M, int64_t K, int64_t Kp,
-                               int64_t pstride, const float* amax, __nv_bfloat16* out, cudaStream_t s) {
-  const Int7Writer w{out, 2 * Kp, pstride, amax};
-  return launch_gather_tab(T, t.om, t.ok, M, K, Kp, t.m_fast, w, s);
-}
-cudaError_t launch_split_i7_c128(const double2* T, const GroupSpec& mg, const GroupSpec& kg, int64_t M, int64_t K,
-                                 int64_t Kp, int64_t pstride, const float* amax, __nv_bfloat16* out, cudaStream_t s) {
-  const Int7Writer w{out, 2 * Kp, pstride, amax};
-  return launch_gather(T, mg, kg, M, K, Kp, w, s);
-}
-cudaError_t launch_pack_b_planes_i7(const double2* B, int64_t N, int64_t K, int64_t Kp, int64_t pstride,
-                                    __nv_bfloat16* out, float* bmax, cudaStream_t s) {
-  if (N <= 0) return cudaSuccess;
-  if (N > 2147483647LL) return cudaErrorInvalidConfiguration;
-  bmax_kernel<<<(unsigned)N, 256, 0, s>>>(B, K, bmax);
-  cudaError_t e = cudaGetLastError();
+// Digit planes of the running tensor's K-major view and its row exponents: the one-pass
+// split, or row exponents first and then the planes when a row is too long for it.
+template <class Off>
+static cudaError_t split_digits(const double2* T, const Off& off, int m_fast, const GroupSpec* mg, const GroupSpec* kg,
+                                int64_t M, int64_t K, float* rexp, unsigned char* out, int* flag, int token,
+                                cudaStream_t s, int* launches) {
+  const int64_t Kp = (K + 7) / 8 * 8, nkb = Kp / 8;
+  bool done = false;
+  cudaError_t e = launch_split_rows(T, off, M, K, Kp, m_fast, DigitRowWriter{out, nkb, flag, token}, rexp, s, &done);
+  *launches = 1;
+  if (e != cudaSuccess || done) return e;
+  *launches = 2;
+  e = launch_rowmax<ExpMag>(T, off, m_fast, M, K, rexp, s);
   if (e != cudaSuccess) return e;
-  const int64_t total = 2 * N * Kp;
-  int64_t blocks = std::min<int64_t>(std::max<int64_t>((total + 255) / 256, 1), 152 * 32);
-  pack_b_planes_i7_kernel<<<(unsigned)blocks, 256, 0, s>>>(B, N, K, Kp, pstride, bmax, out);
+  const DigitWriter w{out, nkb, rexp, flag, token};
+  if constexpr (std::is_same<Off, TabOff>::value)
+    return launch_gather_tab(T, off.om, off.ok, M, K, Kp, m_fast, w, s);
+  else
+    return launch_gather(T, *mg, *kg, M, K, Kp, w, s);
+}
+cudaError_t launch_split_digits_tab(const double2* T, const GatherTab& t, int64_t M, int64_t K, float* rexp, void* out,
+                                    int* flag, int token, cudaStream_t s, int* launches) {
+  return split_digits(T, TabOff{t.om, t.ok}, t.m_fast, nullptr, nullptr, M, K, rexp, static_cast<unsigned char*>(out),
+                      flag, token, s, launches);
+}
+cudaError_t launch_split_digits_grp(const double2* T, const GroupSpec& mg, const GroupSpec& kg, int64_t M, int64_t K,
+                                    float* rexp, void* out, int* flag, int token, cudaStream_t s, int* launches) {
+  return split_digits(T, GrpOffV{mg, kg}, choose_m_fast(mg, kg) ? 1 : 0, &mg, &kg, M, K, rexp,
+                      static_cast<unsigned char*>(out), flag, token, s, launches);
+}
+cudaError_t launch_pack_b_digits(const double2* B, int64_t N, int64_t K, void* out, float* bexp, int* flag,
+                                 cudaStream_t s) {
+  if (N <= 0) return cudaSuccess;
+  const int64_t blocks = (N + 7) / 8;
+  if (blocks > 2147483647LL) return cudaErrorInvalidConfiguration;
+  pack_b_digits_kernel<<<(unsigned)blocks, 256, 0, s>>>(B, N, K, (K + 7) / 8, bexp, static_cast<unsigned char*>(out),
+                                                       flag);
   return cudaGetLastError();
 }
 cudaError_t launch_gather_tab_to_c128(const void* T, int is64, const GatherTab& t, int64_t M, int64_t K, int64_t ldo,

@@ -115,6 +115,33 @@ int fill_offset_tables(gtn_map map) {
   return e == cudaSuccess ? GTN_OK : set_err(map->ctx, GTN_ERR_CUDA, std::string("offset tables: ") + cudaGetErrorString(e));
 }
 
+// Digit planes of the statics of the plan's digit-plane steps.  They are optional in an FP64
+// plan (a step without them stays on the FP64 pipe) and needed in an FP64E one.
+int pack_digits(gtn_map map, bool required) {
+  gtn_ctx ctx = map->ctx;
+  int* flags = nullptr;
+  cudaError_t e = dalloc(map, &flags, map->steps.size() * sizeof(int));
+  if (e == cudaSuccess) e = cudaMemsetAsync(flags, 0, map->steps.size() * sizeof(int), ctx->stream);
+  for (size_t i = 0; i < map->steps.size() && e == cudaSuccess; ++i) {
+    PlanStep& st = map->steps[i];
+    if (!st.dg) continue;
+    void* planes = nullptr;
+    cudaError_t a = dalloc(map, &planes, f64e_b_bytes(st.N, st.K));
+    if (a == cudaSuccess) a = dalloc(map, &st.bexp, (size_t)st.N * sizeof(float));
+    if (a != cudaSuccess) {
+      if (required) return set_err(ctx, GTN_ERR_MEMORY, "static packing allocation failed");
+      cudaGetLastError();
+      continue;
+    }
+    st.bflag = flags + i;
+    e = launch_pack_b_digits(st.b64, st.N, st.K, planes, st.bexp, st.bflag, ctx->stream);
+    ctx->launches++;
+    st.bdig = planes;
+  }
+  if (e != cudaSuccess) return set_err(ctx, GTN_ERR_CUDA, std::string("digit planes: ") + cudaGetErrorString(e));
+  return GTN_OK;
+}
+
 // Offset tables of an [M, K] gather, or none (index-group decomposition) when they would
 // exceed 256 MiB.
 cudaError_t make_tab(gtn_map map, const GroupSpec& mg, const GroupSpec& kg, int64_t M, int64_t K, GatherTab* t) {
@@ -316,7 +343,9 @@ int plan_build(gtn_ctx ctx, int n, const int* ranks, const int64_t* dims, const 
   map->max_apl = 0;
   const bool tc = is_tc(precision);
   const bool f64e = is_f64e(precision);
-  const int P = tc ? nplanes_of(precision) : (f64e ? kF64eSlices : 0);
+  const int P = tc ? nplanes_of(precision) : 0;
+  // FP64 plans that own a workspace run their long products on the tensor cores too
+  const bool dg64 = precision == GTN_PREC_FP64 && alloc_ws && statics && tc_gemm_supported(ctx->cc_major, ctx->cc_minor);
 
   // ---- the reference's env-first chain and the grouped chain we execute ------------------
   ChainOp X{L[0], D[0]};
@@ -453,7 +482,8 @@ int plan_build(gtn_ctx ctx, int n, const int* ranks, const int64_t* dims, const 
     if (!make_group(DT, freeT, &st.mg) || !make_group(DT, sh, &st.kg))
       return set_err(ctx, GTN_ERR_UNSUPPORTED, "too many non-contiguous leg groups");
     st.small = st.K <= kSmallK && small_contract_fits((int)st.K, (int)std::min<int64_t>(st.N, 1 << 20), sizeof(double2));
-    st.tc = (tc || f64e) && !st.small;
+    st.tc = tc && !st.small;
+    st.dg = !st.small && st.K <= kF64eMaxK && ((f64e && statics) || (dg64 && f64e_worthwhile(st.M, st.N, st.K)));
     st.Kp = ((st.K + 31) / 32) * 32;
     // C legs: S free (S order), then T free (T order)
     for (int b : freeS) { st.out_labels.push_back(LS[b]); st.out_dims.push_back(DS[b]); }
@@ -463,7 +493,8 @@ int plan_build(gtn_ctx ctx, int n, const int* ranks, const int64_t* dims, const 
     if (!st.small) {
       map->max_a = std::max(map->max_a, st.M * st.K);
       if (st.tc) map->max_apl = std::max(map->max_apl, (int64_t)P * st.M * 2 * st.Kp);
-      if (st.tc) map->max_mtc = std::max(map->max_mtc, st.M);
+      if (st.tc || st.dg) map->max_mtc = std::max(map->max_mtc, st.M);
+      if (st.dg) map->max_adg = std::max(map->max_adg, f64e_a_bytes(st.M, st.K));
       st.splitk = gemm_splitk_slices(st.M, st.N, st.K);
       if (st.splitk > 1) map->max_splitk = std::max(map->max_splitk, (int64_t)st.splitk * st.M * st.N);
     }
@@ -497,13 +528,7 @@ int plan_build(gtn_ctx ctx, int n, const int* ranks, const int64_t* dims, const 
         st.bplanes = P;
         const int64_t pstride = 2 * st.N * 2 * st.Kp;
         e = dalloc(map, &st.bpl, (size_t)P * pstride * sizeof(__nv_bfloat16));
-        if (e == cudaSuccess && f64e) {
-          st.bfp16 = 2;  // integer digit planes
-          e = dalloc(map, &st.bmax, (size_t)st.N * sizeof(float));
-          if (e == cudaSuccess) e = launch_pack_b_planes_i7(st.b64, st.N, st.K, st.Kp, pstride, st.bpl, st.bmax,
-                                                            ctx->stream);
-          ctx->launches += 2;
-        } else if (e == cudaSuccess && is_fp16(precision)) {
+        if (e == cudaSuccess && is_fp16(precision)) {
           st.bfp16 = 1;
           e = dalloc(map, &st.bmax, (size_t)st.N * sizeof(float));
           if (e == cudaSuccess) e = launch_pack_b_planes_f16(st.b64, st.N, st.K, st.Kp, pstride, st.bpl, st.bmax,
@@ -516,7 +541,7 @@ int plan_build(gtn_ctx ctx, int n, const int* ranks, const int64_t* dims, const 
       }
       if (e != cudaSuccess) return set_err(ctx, GTN_ERR_CUDA, std::string("static packing: ") + cudaGetErrorString(e));
     }
-    if (statics && st.tc && !map->oneshot) {
+    if (statics && (st.tc || st.dg) && !map->oneshot) {
       cudaError_t e = make_tab(map, st.mg, st.kg, st.M, st.K, &st.tab);
       if (e != cudaSuccess) return set_err(ctx, GTN_ERR_CUDA, std::string("offset tables: ") + cudaGetErrorString(e));
     }
@@ -577,14 +602,19 @@ int plan_build(gtn_ctx ctx, int n, const int* ranks, const int64_t* dims, const 
     max_sk = std::max(max_sk, map->fp64_alt->max_splitk);
   }
   const size_t tbytes = (size_t)max_t * sizeof(double2);
-  const size_t abytes = std::max<size_t>((size_t)max_a * sizeof(double2),
-                                         (size_t)map->max_apl * sizeof(__nv_bfloat16));
+  size_t abytes = std::max<size_t>((size_t)max_a * sizeof(double2), (size_t)map->max_apl * sizeof(__nv_bfloat16));
   size_t freeb = 0, totalb = 0;
   if (map->oneshot) freeb = SIZE_MAX;  // one-shot contraction: the arena or a failing cudaMalloc decides
   else {
     cudaMemGetInfo(&freeb, &totalb);
     freeb += ctx->blk_cached;  // cached blocks are reused or given back on demand
   }
+  if (dg64 && map->max_adg > abytes && 2 * tbytes + map->max_adg + (size_t)(1u << 30) > freeb) {
+    // the digit planes do not fit: the FP64 pipe, which reads the running tensor in place, runs
+    for (auto& st : map->steps) st.dg = false;
+    map->max_adg = 0;
+  }
+  abytes = std::max(abytes, map->max_adg);
   const size_t need = 2 * tbytes + abytes + (size_t)(1u << 30);
   if (need > freeb)
     return set_err(ctx, GTN_ERR_MEMORY, "memory admission refused: map workspace " +
@@ -593,12 +623,16 @@ int plan_build(gtn_ctx ctx, int n, const int* ranks, const int64_t* dims, const 
   if (dalloc(map, &map->buf0, tbytes) != cudaSuccess || dalloc(map, &map->buf1, tbytes) != cudaSuccess ||
       dalloc(map, &map->abuf, std::max<size_t>(abytes, 256)) != cudaSuccess)
     return set_err(ctx, GTN_ERR_MEMORY, "map workspace allocation failed");
-  if ((is_fp16(precision) || f64e) && map->max_mtc > 0 &&
+  if ((is_fp16(precision) || map->max_adg > 0) && map->max_mtc > 0 &&
       dalloc(map, &map->amax, (size_t)map->max_mtc * sizeof(float)) != cudaSuccess)
     return set_err(ctx, GTN_ERR_MEMORY, "map workspace allocation failed");
   if (max_sk > 0 && dalloc(map, reinterpret_cast<double2**>(&map->skbuf), (size_t)max_sk * sizeof(double2)) !=
                         cudaSuccess)
     return set_err(ctx, GTN_ERR_MEMORY, "map workspace allocation failed");
+  if (statics && map->max_adg > 0) {
+    const int st = pack_digits(map, f64e);
+    if (st != GTN_OK) return st;
+  }
   if (map->fp64_alt) {
     map->fp64_alt->buf0 = map->buf0;
     map->fp64_alt->buf1 = map->buf1;
@@ -672,7 +706,7 @@ int map_run(gtn_map map, int precision, const double2* x, double2* y) {
   const bool f64e = is_f64e(precision);
   if (f64e) {
     for (auto& st : map->steps)
-      if (!st.small && (!st.bpl || st.bplanes != kF64eSlices || st.bfp16 != 2 || !map->amax))
+      if (!st.small && st.K <= kF64eMaxK && (!st.bdig || !map->amax))
         return set_err(ctx, GTN_ERR_INVALID, "map was not created for the FP64-grade tensor-core precision");
   }
   const bool fp64 = precision == GTN_PREC_FP64 || f64e;  // complex FP64 running tensors
@@ -692,64 +726,59 @@ int map_run(gtn_map map, int precision, const double2* x, double2* y) {
                                        (int)st.N, st.b64, static_cast<double2*>(out), s);
         prof_end(s, GTN_KERNEL_SMALL, 8.0 * st.macs);
         ctx->launches++;
-      } else if (f64e) {
-        // integer digit planes of the running tensor (row maxima first), then the exact
-        // chunked digit-product GEMM straight into complex FP64
-        __nv_bfloat16* Apl = static_cast<__nv_bfloat16*>(map->abuf);
-        const int64_t pstride = st.M * 2 * st.Kp;
+      } else if (st.bdig && map->amax) {
+        // digit planes of the running tensor, the exact digit-product GEMM straight into
+        // complex FP64, and the FP64 kernel that takes over when a row was out of range
+        const double2* T = static_cast<const double2*>(cur);
+        ctx->fb_token = ctx->fb_token == INT32_MAX ? 1 : ctx->fb_token + 1;
+        F64eGemmArgs a;
+        a.A = map->abuf;
+        a.B = st.bdig;
+        a.C = static_cast<double2*>(out);
+        a.M = st.M;
+        a.N = st.N;
+        a.K = st.K;
+        a.a_exp = map->amax;
+        a.b_exp = st.bexp;
+        a.token = ctx->fb_token;
+        a.levels = f64e ? 7 : 8;
+        a.a_flag = ctx->d_fbflag + ctx->fb_token % kFbSlots;
+        a.b_flag = st.bflag;
+        int* flag = ctx->d_fbflag + ctx->fb_token % kFbSlots;
+        int nl = 0;
         prof_begin(s);
-        bool fused = false;
-        if (st.tab.om)
-          e = launch_split_i7_rows_tab(static_cast<const double2*>(cur), st.tab, st.M, st.K, st.Kp, pstride,
-                                       map->amax, Apl, s, &fused);
-        else
-          e = launch_split_i7_rows_grp(static_cast<const double2*>(cur), st.mg, st.kg, st.M, st.K, st.Kp, pstride,
-                                       map->amax, Apl, s, &fused);
-        if (e == cudaSuccess && !fused) {  // rows too long for the clusters: maxima first, then the split
-          if (st.tab.om) {
-            e = launch_rowmax_tab(cur, 1, st.tab, st.M, st.K, map->amax, s);
-            if (e == cudaSuccess)
-              e = launch_split_i7_tab(static_cast<const double2*>(cur), st.tab, st.M, st.K, st.Kp, pstride,
-                                      map->amax, Apl, s);
-          } else {
-            e = launch_rowmax_c128(static_cast<const double2*>(cur), st.mg, st.kg, st.M, st.K, map->amax, s);
-            if (e == cudaSuccess)
-              e = launch_split_i7_c128(static_cast<const double2*>(cur), st.mg, st.kg, st.M, st.K, st.Kp, pstride,
-                                       map->amax, Apl, s);
-          }
-        }
+        if (st.tab.om) e = launch_split_digits_tab(T, st.tab, st.M, st.K, map->amax, map->abuf, flag, a.token, s, &nl);
+        else e = launch_split_digits_grp(T, st.mg, st.kg, st.M, st.K, map->amax, map->abuf, flag, a.token, s, &nl);
         prof_end(s, GTN_KERNEL_SPLIT, 0.0);
-        ctx->launches += fused ? 1 : 2;
+        ctx->launches += nl;
         if (e == cudaSuccess) {
-          F64eGemmArgs a;
-          a.A = Apl;
-          a.B = st.bpl;
-          a.C = static_cast<double2*>(out);
-          a.M = st.M;
-          a.N = st.N;
-          a.Kp = st.Kp;
-          a.a_max = map->amax;
-          a.b_max = st.bmax;
           std::string why;
           prof_begin(s);
-          e = launch_f64e_gemm(a, ctx->d_errflag, s, &why);
+          e = launch_f64e_gemm(a, ctx->sm_count, ctx->d_errflag, s, &why);
           prof_end(s, GTN_KERNEL_TC_GEMM, 8.0 * st.macs);
-          ctx->launches++;
           if (e != cudaSuccess) return set_err(ctx, GTN_ERR_CUDA, "f64e_gemm: " + why + " " + cudaGetErrorString(e));
+          prof_begin(s);
+          e = launch_zgemm_view(T, st.mg, st.kg, st.b64, a.C, st.M, st.N, st.K, s, a.a_flag, a.b_flag, a.token);
+          prof_end(s, GTN_KERNEL_ZGEMM, 0.0);
+          ctx->launches += 2;
         }
-      } else {
+      } else if (st.splitk > 1 && map->skbuf) {
         double2* A = static_cast<double2*>(map->abuf);
         prof_begin(s);
         e = launch_gather_c128_to_c128(static_cast<const double2*>(cur), st.mg, st.kg, st.M, st.K, st.K, A, s);
         prof_end(s, GTN_KERNEL_GATHER, 0.0);
         prof_begin(s);
-        if (e == cudaSuccess && st.splitk > 1 && map->skbuf)
+        if (e == cudaSuccess)
           e = launch_zgemm_simt_splitk(A, st.b64, static_cast<double2*>(out), st.M, st.N, st.K, st.splitk,
                                        static_cast<double2*>(map->skbuf), s);
-        else if (e == cudaSuccess)
-          e = launch_zgemm_simt(A, st.b64, static_cast<double2*>(out), st.M, st.N, st.K, s);
         prof_end(s, GTN_KERNEL_ZGEMM, 8.0 * st.macs);
-        ctx->launches += 2;
+        ctx->launches += 3;
+      } else {
+        prof_begin(s);
+        e = launch_zgemm_view(static_cast<const double2*>(cur), st.mg, st.kg, st.b64, static_cast<double2*>(out), st.M,
+                              st.N, st.K, s);
+        prof_end(s, GTN_KERNEL_ZGEMM, 8.0 * st.macs);
+        ctx->launches++;
       }
     } else {
       if (cur64 && (st.small || !tc)) {
