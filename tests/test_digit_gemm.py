@@ -160,3 +160,25 @@ def test_products_read_in_place_match_numpy(ctx):
         got = ctx.download(ctx.contract([ctx.upload(T), ctx.upload(B)], [[-1, 1, -3], [-2, 1]], None, None, 0))
         ref = np.einsum("abc,nb->anc", T, B)
         assert np.all(np.abs(got - ref) <= b * 2.0 ** -51 * np.einsum("abc,nb->anc", np.abs(T), np.abs(B)))
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("kn", [(1, 1), (3, 8), (25, 9), (50, 10), (64, 17), (64, 48), (10, 300)])
+def test_short_contractions_skip_zeros_exactly(ctx, kn):
+    """Short FP64 contractions with a mostly zero static: the sums of numpy, and infinities and
+    NaN meet the zeros as 0 * inf and 0 * nan do."""
+    K, N = kn
+    rng = np.random.default_rng(K * N)
+    for M in (1, 31, 700):
+        T, B = crandn(rng, (M, K)), crandn(rng, (N, K))
+        B[rng.random((N, K)) < 0.8] = 0
+        B.real[rng.random((N, K)) < 0.3] = 0
+        B.imag[rng.random((N, K)) < 0.3] = 0
+        got = contract(ctx, T, np.ascontiguousarray(B.T), "fp64")
+        assert np.all(np.abs(got - T @ B.T) <= (K + 1) * 2.0 ** -51 * (np.abs(T) @ np.abs(B.T)))
+        T[M // 2, K // 2] = np.inf
+        T[0, 0] = np.nan
+        got = contract(ctx, T, np.ascontiguousarray(B.T), "fp64")
+        assert not np.isfinite(got[M // 2]).any() and np.isnan(got[0]).all()
+        ok = [i for i in range(M) if i not in (0, M // 2)]
+        assert np.isfinite(got[ok]).all()
