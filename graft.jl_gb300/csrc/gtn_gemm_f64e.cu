@@ -315,13 +315,13 @@ __global__ void __launch_bounds__(kThreads, 1)
 
 }  // namespace
 
-// Tensor path: the split and its launches, then per wave of 152 tiles about 1000 clocks per
-// stage of 8 complex k and 5000 for the drains and the store; FP64 pipe: 1.15 TFLOP/s.
-bool f64e_worthwhile(int64_t M, int64_t N, int64_t K) {
-  const double waves = (double)(((M + kBM - 1) / kBM) * ((2 * N + kBN - 1) / kBN) + 151) / 152;
-  const double tc = 8e-6 + std::floor(waves) * ((double)((K + 7) / 8) * 1000 + 5000) / 1.9e9 + (double)M * K * 60 / 4e12;
-  return tc < 4e-6 + 8.0 * (double)M * (double)N * (double)K / 1.15e12;
+// Digit planes: the split and the launches, then per wave of 152 tiles about 1000 clocks per
+// stage of 8 complex k and 5000 for the drains and the store.  FP64 pipe: 1.15 TFLOP/s.
+double f64e_time(double M, double N, double K) {
+  const double tiles = std::ceil(M / kBM) * std::ceil(2 * N / kBN);
+  return 8e-6 + std::ceil(tiles / 152) * (std::ceil(K / 8) * 1000 + 5000) / 1.9e9 + M * K * 60 / 4e12;
 }
+double f64_pipe_time(double M, double N, double K) { return 4e-6 + 8.0 * M * N * K / 1.15e12; }
 
 cudaError_t launch_f64e_gemm(const F64eGemmArgs& a, int sm_count, int* errflag, cudaStream_t s, std::string* why) {
   if (a.M <= 0 || a.N <= 0) return cudaSuccess;

@@ -360,8 +360,10 @@ inline size_t f64e_a_bytes(int64_t M, int64_t K) {
 inline size_t f64e_b_bytes(int64_t N, int64_t K) {
   return (size_t)((2 * N + kF64eRowsB - 1) / kF64eRowsB) * ((K + 7) / 8) * kF64eSlices * kF64eRowsB * 32;
 }
-// When the digit-plane GEMM takes an FP64 step (M, N, K) from the FP64 pipe.
-bool f64e_worthwhile(int64_t M, int64_t N, int64_t K);
+// Modelled seconds of an FP64 step (M, N, K) on digit planes (split and GEMM) and on the FP64
+// pipe; the step takes the faster one.
+double f64e_time(double M, double N, double K);
+double f64_pipe_time(double M, double N, double K);
 struct F64eGemmArgs {
   const void* A = nullptr;
   const void* B = nullptr;
@@ -518,6 +520,7 @@ struct gtn_map_s {
   double2* kcoef = nullptr; double2* kscratch = nullptr; int kscratch_cap = 0;
 };
 
+double plan_step_time(int precision, double M, double K, double N, bool oneshot);
 int plan_build(gtn_ctx ctx, int n_operands, const int* ranks, const int64_t* dims,
                const int* labels, const int* conj, const int* order, const void* const* statics,
                int precision, gtn_map map, bool allow_group = true, bool alloc_ws = true);

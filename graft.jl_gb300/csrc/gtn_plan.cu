@@ -187,6 +187,18 @@ double est_step_time(int prec, double M, double K, double N) {
   return t + flops / rate + (M * K * e + M * 2 * Kp * P * 2 + M * N * 8) / hbm;
 }
 
+}  // namespace
+
+// Time of one pair step as it will run: est_step_time, with the choice between the FP64 pipe
+// and the digit planes in FP64; a one-shot contraction packs the absorbed operand too.
+double plan_step_time(int precision, double M, double K, double N, bool oneshot) {
+  const double pack = oneshot ? 10e-6 + N * K * 90.0 / 4e12 : 0.0;
+  const bool small = K <= kSmallK && small_contract_fits((int)K, (int)std::min(N, 1048576.0), sizeof(double2));
+  if (precision != GTN_PREC_FP64 || small) return est_step_time(precision, M, K, N) + pack;
+  return std::min(f64e_time(M, N, K), f64_pipe_time(M, N, K)) + M * N * 16.0 / 5e12 + pack;
+}
+
+namespace {
 struct ChainOp {
   std::vector<int> L;
   std::vector<int64_t> D;
@@ -483,7 +495,7 @@ int plan_build(gtn_ctx ctx, int n, const int* ranks, const int64_t* dims, const 
       return set_err(ctx, GTN_ERR_UNSUPPORTED, "too many non-contiguous leg groups");
     st.small = st.K <= kSmallK && small_contract_fits((int)st.K, (int)std::min<int64_t>(st.N, 1 << 20), sizeof(double2));
     st.tc = tc && !st.small;
-    st.dg = !st.small && st.K <= kF64eMaxK && ((f64e && statics) || (dg64 && f64e_worthwhile(st.M, st.N, st.K)));
+    st.dg = !st.small && st.K <= kF64eMaxK && ((f64e && statics) || (dg64 && f64e_time(st.M, st.N, st.K) < f64_pipe_time(st.M, st.N, st.K)));
     st.Kp = ((st.K + 31) / 32) * 32;
     // C legs: S free (S order), then T free (T order)
     for (int b : freeS) { st.out_labels.push_back(LS[b]); st.out_dims.push_back(DS[b]); }

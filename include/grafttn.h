@@ -285,7 +285,7 @@ int gtn_contract(gtn_ctx ctx, int n_operands, const int* ranks, const int64_t* d
  * for every perturbation of op_slot as it enters the contraction (after its conj flag):
  * G = contract(ybar, conj(op_i), i != slot).  It runs through the same contraction engine
  * (tcgen05 steps in the mixed precisions).  order (may be NULL) orders the rewritten
- * operand list [ybar, op_i for i != slot]; NULL picks a greedy chain from ybar. */
+ * operand list [ybar, op_i for i != slot]; NULL picks the cheapest chain from ybar. */
 int gtn_contract_vjp(gtn_ctx ctx, int n_operands, const int* ranks, const int64_t* dims, const int* labels,
                      const int* conj, const int* order, const void* const* operands, int slot, const void* ybar,
                      void* out, int precision);

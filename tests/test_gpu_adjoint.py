@@ -139,3 +139,23 @@ def test_ttno_gradients_under_env_budget(ctx, xxz_bin31):
     g_small = GR.ttno_gradients(psi, H, max_env_bytes=3 * 32 * 5 * 32 * 16)
     for a, b in zip(g_full, g_small):
         assert ctx.norm(ctx.axpby(1.0, a, -1.0, b.clone())) <= 1e-13 * max(1.0, ctx.norm(a))
+
+
+@pytest.mark.parametrize("n", [5, 12, 15])
+def test_vjp_of_a_matrix_chain_for_every_slot(ctx, n):
+    """The adjoint's own chain: compared with all others up to 13 operands, greedy beyond."""
+    rng = np.random.default_rng(n)
+    dims = [int(rng.integers(2, 7)) for _ in range(n + 1)]
+    mats = [O.randn_c(rng, (dims[i], dims[i + 1])) / 2 for i in range(n)]
+    labels = [[-1 if i == 0 else i, -2 if i == n - 1 else i + 1] for i in range(n)]
+    ybar = O.randn_c(rng, (dims[0], dims[n]))
+    dev = [ctx.upload(m) for m in mats]
+    for slot in (0, n // 2, n - 1):
+        left, right = np.eye(dims[0]), np.eye(dims[n])
+        for m in mats[:slot]:
+            left = left @ m
+        for m in reversed(mats[slot + 1:]):
+            right = m @ right
+        ref = left.conj().T @ ybar @ right.conj().T
+        got = ctx.download(ctx.contract_vjp(dev, labels, ctx.upload(ybar), slot))
+        assert np.linalg.norm(got - ref) <= 1e-13 * np.linalg.norm(ref)
