@@ -331,6 +331,38 @@ __global__ void splitk_reduce_kernel(const T* __restrict__ P, int S, int64_t MN,
   }
 }
 
+template <typename T>
+cudaError_t launch(const T* A, const T* B, T* C, int64_t M, int64_t N, int64_t K, cudaStream_t s) {
+  if (M <= 0 || N <= 0) return cudaSuccess;
+  const int64_t gx = (M + BM - 1) / BM, gy = (N + BN - 1) / BN;
+  if (gy > 65535) return cudaErrorInvalidConfiguration;
+  gemm_simt_kernel<T><<<dim3((unsigned)gx, (unsigned)gy), 256, 0, s>>>(A, B, C, M, N, K);
+  return cudaGetLastError();
+}
+
+template <typename T>
+cudaError_t launch_splitk(const T* A, const T* B, T* C, int64_t M, int64_t N, int64_t K, int S, T* P,
+                          cudaStream_t s) {
+  if (M <= 0 || N <= 0) return cudaSuccess;
+  const int64_t gx = (M + BM - 1) / BM, gy = (N + BN - 1) / BN;
+  if (gy > 65535 || S < 1 || S > 65535) return cudaErrorInvalidConfiguration;
+  int64_t kchunk = (K + S - 1) / S;
+  kchunk = (kchunk + BK - 1) / BK * BK;
+  const int Se = (int)((K + kchunk - 1) / kchunk);
+  if (N <= 16)
+    gemm_simt_splitk_kernel<T, true><<<dim3((unsigned)gx, 1u, (unsigned)Se), 256, 0, s>>>(A, B, P, M, N, K, kchunk);
+  else
+    gemm_simt_splitk_kernel<T, false><<<dim3((unsigned)gx, (unsigned)gy, (unsigned)Se), 256, 0, s>>>(A, B, P, M, N, K,
+                                                                                                   kchunk);
+  cudaError_t e = cudaGetLastError();
+  if (e != cudaSuccess) return e;
+  const int64_t MN = M * N;
+  int64_t blocks = (MN + 255) / 256;
+  if (blocks > 152 * 8) blocks = 152 * 8;
+  splitk_reduce_kernel<T><<<(unsigned)(blocks < 1 ? 1 : blocks), 256, 0, s>>>(P, Se, MN, C);
+  return cudaGetLastError();
+}
+
 // FP64 products that read the running tensor in place (no K-major copy): 256 threads compute a
 // TM x TN tile, every thread R x R outputs, in KS slices of each 16-wide k block.  A 64 x 64
 // tile costs 64 * 64 * 4 FMAs per k on one SM, which issues about two FP64 FMAs per clock, so a
@@ -341,8 +373,12 @@ template <int TM, int TN, int R, int KS>
 __global__ void __launch_bounds__(256) zgemm_view_kernel(const double2* __restrict__ T, GroupSpec mg, GroupSpec kg,
                                                          const double2* __restrict__ B, double2* __restrict__ C,
                                                          int64_t M, int64_t N, int64_t K, int64_t tiles_m,
-                                                         int64_t ntiles, const int* __restrict__ a_flag,
+                                                         int64_t ntiles, int64_t kchunk,
+                                                         const int* __restrict__ a_flag,
                                                          const int* __restrict__ b_flag, int token) {
+  // slice blockIdx.y of the k range writes its partial product to C + blockIdx.y * M * N
+  const int64_t kb = (int64_t)blockIdx.y * kchunk, ke = kb + kchunk < K ? kb + kchunk : K;
+  C += (int64_t)blockIdx.y * M * N;
   static_assert((TM / R) * (TN / R) * KS == 256 && BK % KS == 0, "one thread per R x R outputs and slice");
   if (a_flag && *a_flag != token && *b_flag == 0) return;
   __shared__ double2 As[BK][TM + 1];
@@ -359,16 +395,16 @@ __global__ void __launch_bounds__(256) zgemm_view_kernel(const double2* __restri
 #pragma unroll
       for (int j = 0; j < R; ++j) acc[i][j] = make_double2(0.0, 0.0);
     if (tid < TM) offM[tid] = m0 + tid < M ? decompose(m0 + tid, mg) : 0;
-    for (int64_t k0 = 0; k0 < K; k0 += BK) {
-      if (tid < BK) offK[tid] = k0 + tid < K ? decompose(k0 + tid, kg) : 0;
+    for (int64_t k0 = kb; k0 < ke; k0 += BK) {
+      if (tid < BK) offK[tid] = k0 + tid < ke ? decompose(k0 + tid, kg) : 0;
       __syncthreads();
       for (int e = tid; e < TM * BK; e += 256) {
         const int r = e / BK, c = e % BK;
-        As[c][r] = (m0 + r < M && k0 + c < K) ? T[offM[r] + offK[c]] : CT<double2>::zero();
+        As[c][r] = (m0 + r < M && k0 + c < ke) ? T[offM[r] + offK[c]] : CT<double2>::zero();
       }
       for (int e = tid; e < TN * BK; e += 256) {
         const int r = e / BK, c = e % BK;
-        Bs[c][r] = (n0 + r < N && k0 + c < K) ? B[(n0 + r) * K + k0 + c] : CT<double2>::zero();
+        Bs[c][r] = (n0 + r < N && k0 + c < ke) ? B[(n0 + r) * K + k0 + c] : CT<double2>::zero();
       }
       __syncthreads();
 #pragma unroll 4
@@ -418,64 +454,43 @@ __global__ void __launch_bounds__(256) zgemm_view_kernel(const double2* __restri
 
 template <int TM, int TN, int R, int KS>
 cudaError_t launch_view(const double2* T, const GroupSpec& mg, const GroupSpec& kg, const double2* B, double2* C,
-                        int64_t M, int64_t N, int64_t K, cudaStream_t s, const int* a_flag, const int* b_flag,
-                        int token) {
+                        int64_t M, int64_t N, int64_t K, int64_t kchunk, cudaStream_t s, const int* a_flag,
+                        const int* b_flag, int token) {
   const int64_t tm = (M + TM - 1) / TM, nt = tm * ((N + TN - 1) / TN);
   // a launch that usually has nothing to do keeps its grid small
   const int64_t grid = std::min<int64_t>(nt, a_flag ? 2 * 152 : (int64_t(1) << 30));
-  zgemm_view_kernel<TM, TN, R, KS><<<(unsigned)grid, 256, 0, s>>>(T, mg, kg, B, C, M, N, K, tm, nt, a_flag, b_flag,
-                                                                 token);
-  return cudaGetLastError();
-}
-
-template <typename T>
-cudaError_t launch(const T* A, const T* B, T* C, int64_t M, int64_t N, int64_t K, cudaStream_t s) {
-  if (M <= 0 || N <= 0) return cudaSuccess;
-  const int64_t gx = (M + BM - 1) / BM, gy = (N + BN - 1) / BN;
-  if (gy > 65535) return cudaErrorInvalidConfiguration;
-  gemm_simt_kernel<T><<<dim3((unsigned)gx, (unsigned)gy), 256, 0, s>>>(A, B, C, M, N, K);
-  return cudaGetLastError();
-}
-
-template <typename T>
-cudaError_t launch_splitk(const T* A, const T* B, T* C, int64_t M, int64_t N, int64_t K, int S, T* P,
-                          cudaStream_t s) {
-  if (M <= 0 || N <= 0) return cudaSuccess;
-  const int64_t gx = (M + BM - 1) / BM, gy = (N + BN - 1) / BN;
-  if (gy > 65535 || S < 1 || S > 65535) return cudaErrorInvalidConfiguration;
-  int64_t kchunk = (K + S - 1) / S;
-  kchunk = (kchunk + BK - 1) / BK * BK;
-  const int Se = (int)((K + kchunk - 1) / kchunk);
-  if (N <= 16)
-    gemm_simt_splitk_kernel<T, true><<<dim3((unsigned)gx, 1u, (unsigned)Se), 256, 0, s>>>(A, B, P, M, N, K, kchunk);
-  else
-    gemm_simt_splitk_kernel<T, false><<<dim3((unsigned)gx, (unsigned)gy, (unsigned)Se), 256, 0, s>>>(A, B, P, M, N, K,
-                                                                                                   kchunk);
-  cudaError_t e = cudaGetLastError();
-  if (e != cudaSuccess) return e;
-  const int64_t MN = M * N;
-  int64_t blocks = (MN + 255) / 256;
-  if (blocks > 152 * 8) blocks = 152 * 8;
-  splitk_reduce_kernel<T><<<(unsigned)(blocks < 1 ? 1 : blocks), 256, 0, s>>>(P, Se, MN, C);
+  const int64_t slices = (K + kchunk - 1) / kchunk;
+  zgemm_view_kernel<TM, TN, R, KS><<<dim3((unsigned)grid, (unsigned)slices), 256, 0, s>>>(T, mg, kg, B, C, M, N, K, tm, nt, kchunk, a_flag, b_flag, token);
   return cudaGetLastError();
 }
 
 }  // namespace
 
-cudaError_t launch_zgemm_simt(const double2* A, const double2* B, double2* C, int64_t M, int64_t N,
-                              int64_t K, cudaStream_t s) {
-  return launch(A, B, C, M, N, K, s);
-}
 cudaError_t launch_zgemm_view(const double2* T, const GroupSpec& mg, const GroupSpec& kg, const double2* B, double2* C,
                               int64_t M, int64_t N, int64_t K, cudaStream_t s, const int* a_flag, const int* b_flag,
-                              int token) {
+                              int token, int slices, double2* P) {
   if (M <= 0 || N <= 0) return cudaSuccess;
   auto tiles = [&](int t) { return ((M + t - 1) / t) * ((N + t - 1) / t); };
-  if (tiles(64) >= 2 * 152) return launch_view<64, 64, 4, 1>(T, mg, kg, B, C, M, N, K, s, a_flag, b_flag, token);
-  if (tiles(32) >= 2 * 152) return launch_view<32, 32, 2, 1>(T, mg, kg, B, C, M, N, K, s, a_flag, b_flag, token);
-  if (tiles(16) >= 2 * 152) return launch_view<16, 16, 1, 1>(T, mg, kg, B, C, M, N, K, s, a_flag, b_flag, token);
-  if (tiles(8) >= 2 * 152) return launch_view<8, 8, 1, 4>(T, mg, kg, B, C, M, N, K, s, a_flag, b_flag, token);
-  return launch_view<4, 4, 1, 16>(T, mg, kg, B, C, M, N, K, s, a_flag, b_flag, token);
+  if (tiles(64) >= 2 * 152) return launch_view<64, 64, 4, 1>(T, mg, kg, B, C, M, N, K, K, s, a_flag, b_flag, token);
+  if (tiles(32) >= 2 * 152) return launch_view<32, 32, 2, 1>(T, mg, kg, B, C, M, N, K, K, s, a_flag, b_flag, token);
+  if (tiles(16) >= 2 * 152) return launch_view<16, 16, 1, 1>(T, mg, kg, B, C, M, N, K, K, s, a_flag, b_flag, token);
+  if (slices > 1 && P) {
+    const int64_t kchunk = ((K + slices - 1) / slices + BK - 1) / BK * BK;
+    cudaError_t e = launch_view<16, 16, 1, 1>(T, mg, kg, B, P, M, N, K, kchunk, s, a_flag, b_flag, token);
+    if (e != cudaSuccess) return e;
+    const int64_t blocks = std::min<int64_t>((M * N + 255) / 256, 152 * 8);
+    splitk_reduce_kernel<double2><<<(unsigned)blocks, 256, 0, s>>>(P, (int)((K + kchunk - 1) / kchunk), M * N, C);
+    return cudaGetLastError();
+  }
+  if (tiles(8) >= 2 * 152) return launch_view<8, 8, 1, 4>(T, mg, kg, B, C, M, N, K, K, s, a_flag, b_flag, token);
+  return launch_view<4, 4, 1, 16>(T, mg, kg, B, C, M, N, K, K, s, a_flag, b_flag, token);
+}
+int zgemm_view_slices(int64_t M, int64_t N, int64_t K) {
+  const int64_t t16 = ((M + 15) / 16) * ((N + 15) / 16), t4 = ((M + 3) / 4) * ((N + 3) / 4);
+  if (t16 >= 2 * 152 || K < 512) return 1;
+  // the 4 x 4 tiles without slices already fill the chip when there are enough of them
+  const int64_t S = std::min<int64_t>(std::min<int64_t>((4 * 152) / t16, K / 128), 256);
+  return S < 2 || (t4 >= 2 * 152 && t16 * S < 152) ? 1 : (int)S;
 }
 int gemm_splitk_slices(int64_t M, int64_t N, int64_t K) {
   const int64_t tiles = ((M + BM - 1) / BM) * (N <= 16 ? 1 : (N + BN - 1) / BN);
@@ -485,10 +500,6 @@ int gemm_splitk_slices(int64_t M, int64_t N, int64_t K) {
   if (S > kmax) S = kmax;
   if (S > 256) S = 256;
   return S < 2 ? 1 : (int)S;
-}
-cudaError_t launch_zgemm_simt_splitk(const double2* A, const double2* B, double2* C, int64_t M, int64_t N, int64_t K,
-                                     int S, double2* P, cudaStream_t s) {
-  return launch_splitk(A, B, C, M, N, K, S, P, s);
 }
 cudaError_t launch_cgemm_simt_splitk(const float2* A, const float2* B, float2* C, int64_t M, int64_t N, int64_t K,
                                      int S, float2* P, cudaStream_t s) {

@@ -269,8 +269,6 @@ cudaError_t launch_small_contract_c64(const float2* T, const GroupSpec& mg, cons
 bool small_contract_fits(int K, int N, size_t elem_bytes);
 
 // ---- SIMT GEMMs (gtn_gemm_simt.cu): C[n][m] = sum_k A[m][k] B[n][k] -----------------
-cudaError_t launch_zgemm_simt(const double2* A, const double2* B, double2* C, int64_t M, int64_t N,
-                              int64_t K, cudaStream_t s);
 cudaError_t launch_cgemm_simt(const float2* A, const float2* B, float2* C, int64_t M, int64_t N,
                               int64_t K, cudaStream_t s);
 
@@ -285,8 +283,6 @@ cudaError_t launch_gemm_simt_grouped(const GemmJob* jobs, int njobs, int is64, c
 // Split-K for GEMMs with few output tiles and a long K: the number of K slices (1 = no
 // split), and the launchers with a partial-sum workspace P of slices * M * N elements.
 int gemm_splitk_slices(int64_t M, int64_t N, int64_t K);
-cudaError_t launch_zgemm_simt_splitk(const double2* A, const double2* B, double2* C, int64_t M, int64_t N, int64_t K,
-                                     int S, double2* P, cudaStream_t s);
 cudaError_t launch_cgemm_simt_splitk(const float2* A, const float2* B, float2* C, int64_t M, int64_t N, int64_t K,
                                      int S, float2* P, cudaStream_t s);
 // Skinny grouped GEMM (same contraction) for N <= 32; every job must pass gemm_skinny_fits.
@@ -386,10 +382,13 @@ cudaError_t launch_split_digits_grp(const double2* T, const GroupSpec& mg, const
 cudaError_t launch_pack_b_digits(const double2* B, int64_t N, int64_t K, void* out, float* bexp, int* flag,
                                  cudaStream_t s);
 // C[n][m] = sum_k T[offM(m) + offK(k)] B[n][k] on the FP64 pipe, T read in place; with a_flag
-// set the launch does its work only if *a_flag == token or *b_flag != 0.
+// set the launch does its work only if *a_flag == token or *b_flag != 0.  With slices > 1 (of
+// zgemm_view_slices: few outputs, long K) the k range is cut into that many partial products
+// P[slice][n][m], summed in order.
+int zgemm_view_slices(int64_t M, int64_t N, int64_t K);
 cudaError_t launch_zgemm_view(const double2* T, const GroupSpec& mg, const GroupSpec& kg, const double2* B, double2* C,
                               int64_t M, int64_t N, int64_t K, cudaStream_t s, const int* a_flag = nullptr,
-                              const int* b_flag = nullptr, int token = 0);
+                              const int* b_flag = nullptr, int token = 0, int slices = 1, double2* P = nullptr);
 bool tc_gemm_supported(int cc_major, int cc_minor);
 // Independent problems in one launch per 56 problems (same product list for all).
 cudaError_t launch_tc_gemm_grouped(const TcGemmArgs* probs, int nprob, int* errflag, cudaStream_t s,
@@ -451,7 +450,8 @@ struct PlanStep {
   int bfp16 = 0;                   // planes hold fp16 slices scaled per complex row by bmax
   float* bmax = nullptr;           // [N] row maxima of the static (fp16 planes)
   GatherTab tab;                   // offset tables of the running tensor's [M, K] view (tc steps)
-  int splitk = 1;                  // K slices of the SIMT GEMM (few output tiles, long K)
+  int splitk = 1;                  // K slices of the FP32 SIMT GEMM (few output tiles, long K)
+  int vslices = 1;                 // K slices of the FP64 product
   // FP64-accurate digit-plane GEMM (FP64 and FP64E plans): planes, row exponents and
   // out-of-range flag of the static; bdig stays null where the FP64 pipe keeps the step
   bool dg = false;

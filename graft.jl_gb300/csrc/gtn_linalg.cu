@@ -128,29 +128,33 @@ int64_t trunc_rank(const std::vector<double>& hs, int64_t maxdim, double atol, d
 }
 
 // C[n][m] = sum_k X[m][k] Y'[n][k] for row-major X (M x K) and Y (N x K), Y' = conj(Y) when
-// conj_y: FP64 SIMT, or the FP64-grade tensor-core GEMM (a one-shot contraction) when the
-// context's linear-algebra precision is GTN_PREC_FP64E.  tmp (M x K when conj_y, SIMT only)
-// holds conj(Y).
+// conj_y: a one-shot contraction in the context's linear-algebra precision (GTN_PREC_FP64 or
+// GTN_PREC_FP64E; long products run on digit planes in both), or without the memory for its
+// copies the FP64 pipe in place (tmp, N x K, then holds conj(Y)).
 int linalg_gemm(gtn_ctx ctx, const double2* X, const double2* Y, double2* C, int64_t M, int64_t N, int64_t K,
-                bool conj_y, double2* tmp) {
-  cudaStream_t s = ctx->stream;
-  if (ctx->linalg_prec == GTN_PREC_FP64E) {
-    const int ranks[2] = {2, 2};
-    const int64_t dims[4] = {M, K, N, K};
-    const int labels[4] = {-2, 1, -1, 1};
-    const int conj[2] = {0, conj_y ? 1 : 0};
-    const int order[2] = {0, 1};
-    const void* ops[2] = {X, Y};
-    return gtn_contract(ctx, 2, ranks, dims, labels, conj, order, ops, C, GTN_PREC_FP64E);
-  }
-  const double2* Yc = Y;
+                bool conj_y = false, double2* tmp = nullptr) {
+  const int ranks[2] = {2, 2};
+  const int64_t dims[4] = {M, K, N, K};
+  const int labels[4] = {-2, 1, -1, 1};
+  const int conj[2] = {0, conj_y ? 1 : 0};
+  const int order[2] = {0, 1};
+  const void* ops[2] = {X, Y};
+  const int prec = ctx->linalg_prec == GTN_PREC_FP64E ? GTN_PREC_FP64E : GTN_PREC_FP64;
+  const int st = gtn_contract(ctx, 2, ranks, dims, labels, conj, order, ops, C, prec);
+  if (st != GTN_ERR_MEMORY) return st;
+  cudaGetLastError();
   if (conj_y) {
-    GTN_CUDA_TRY(ctx, cudaMemcpyAsync(tmp, Y, N * K * sizeof(double2), cudaMemcpyDeviceToDevice, s));
-    GTN_CUDA_TRY(ctx, launch_conj_inplace(tmp, N * K, s));
+    GTN_CUDA_TRY(ctx, cudaMemcpyAsync(tmp, Y, N * K * sizeof(double2), cudaMemcpyDeviceToDevice, ctx->stream));
+    GTN_CUDA_TRY(ctx, launch_conj_inplace(tmp, N * K, ctx->stream));
     ctx->launches++;
-    Yc = tmp;
+    Y = tmp;
   }
-  GTN_CUDA_TRY(ctx, launch_zgemm_simt(X, Yc, C, M, N, K, s));
+  GroupSpec mg, kg;
+  std::memset(&mg, 0, sizeof(mg));
+  std::memset(&kg, 0, sizeof(kg));
+  mg.n = 1; mg.dim[0] = M; mg.str[0] = K;
+  kg.n = 1; kg.dim[0] = K; kg.str[0] = 1;
+  GTN_CUDA_TRY(ctx, launch_zgemm_view(X, mg, kg, Y, C, M, N, K, ctx->stream));
   ctx->launches++;
   return GTN_OK;
 }
@@ -219,7 +223,7 @@ int svd_gram(gtn_ctx ctx, cusolverDnHandle_t h, int64_t m, int64_t n, const doub
   // Vh[i][l] = sum_a Ut[i][a] A[a][l]: C[nn=i][mm=l] = sum_k X[l][k] Y[i][k], X = A^T, Y = Ut
   GTN_CUDA_TRY(ctx, launch_transpose_c128(A, m, n, At, s));
   {
-    const int st = linalg_gemm(ctx, At, Ut, Vh, n, r, m, false, nullptr);
+    const int st = linalg_gemm(ctx, At, Ut, Vh, n, r, m);
     if (st != GTN_OK) return st;
   }
   // s_i = ||A^H u_i|| (absolute accuracy ~ eps * s_max instead of the eigenvalues'
@@ -275,7 +279,7 @@ int64_t subspace_dim(int64_t m, int64_t maxdim) {
 // 2011, algorithm 4.4) on a kk-dimensional subspace, iterated until the leading maxdim
 // Rayleigh-Ritz singular values stop moving (1e-13 of the largest).  Their vectors have
 // then converged to ~1e-7 in angle; the split is the exact orthogonal projection of A on
-// the kept left vectors whatever the angle.  Every product is an FP64 SIMT GEMM of
+// the kept left vectors whatever the angle.  Every product is an FP64 GEMM of
 // m x n x kk (two per iteration) instead of the m x m x n Gram product and an m x m
 // eigenproblem.  *done is false when the values have not settled within the iteration
 // cap, or when the truncation would keep the whole subspace; the caller then takes the
@@ -296,8 +300,6 @@ int svd_subspace(gtn_ctx ctx, cusolverDnHandle_t h, int64_t m, int64_t n, const 
   GTN_CUDA_TRY(ctx, cudaMemcpyAsync(&tot2, ctx->d_red, sizeof(double2), cudaMemcpyDeviceToHost, s));
   GTN_CUDA_TRY(ctx, cudaStreamSynchronize(s));
   const double tot = tot2.x;
-  const int sk1 = gemm_splitk_slices(m, kk, n), sk2 = gemm_splitk_slices(n, kk, m);
-  const size_t pcap = (size_t)std::max(sk1 > 1 ? sk1 : 0, sk2 > 1 ? sk2 : 0) * std::max(m, n) * kk;
   CallBuffers buf(s);
   double2* Ah = buf.get<double2>(m * n);     // conj(A)^T, n x m
   double2* Qt = buf.get<double2>(kk * m);    // basis of the range, rows of length m
@@ -309,9 +311,8 @@ int svd_subspace(gtn_ctx ctx, cusolverDnHandle_t h, int64_t m, int64_t n, const 
   double* w = buf.get<double>(kk);
   double* dnorm = buf.get<double>(kk);
   double2* tau = buf.get<double2>(kk);
-  double2* P = pcap ? buf.get<double2>(pcap) : nullptr;
   int* dinfo = buf.get<int>(1);
-  if (!Ah || !Qt || !Zt || !Zc || !Gc || !Wr || !Qr || !w || !dnorm || !tau || !dinfo || (pcap && !P))
+  if (!Ah || !Qt || !Zt || !Zc || !Gc || !Wr || !Qr || !w || !dnorm || !tau || !dinfo)
     return set_err(ctx, GTN_ERR_MEMORY, "svd subspace: staging allocation failed");
   int lq = 0, lq2 = 0, lu = 0, lu2 = 0, le = 0;
   if (sv.geqrf_bs(h, (int)m, ik, reinterpret_cast<cuDoubleComplex*>(Qt), (int)m, &lq) != CUSOLVER_STATUS_SUCCESS ||
@@ -326,12 +327,6 @@ int svd_subspace(gtn_ctx ctx, cusolverDnHandle_t h, int64_t m, int64_t n, const 
   const int lwork = std::max({lq, lq2, lu, lu2, le, 1});
   double2* work = buf.get<double2>(lwork);
   if (!work) return set_err(ctx, GTN_ERR_MEMORY, "svd subspace: workspace allocation failed");
-  auto gemm = [&](const double2* X, const double2* Y, double2* C, int64_t M, int64_t N, int64_t K) {
-    const int sl = gemm_splitk_slices(M, N, K);
-    ctx->launches += sl > 1 ? 2 : 1;
-    if (sl > 1 && P && (size_t)sl * M * N <= pcap) return launch_zgemm_simt_splitk(X, Y, C, M, N, K, sl, P, s);
-    return launch_zgemm_simt(X, Y, C, M, N, K, s);
-  };
   // Householder QR of a column-major rows x kk block (a row-major kk x rows one), in place: Q
   auto orth = [&](double2* Y, int64_t rows) -> int {
     if (sv.geqrf(h, (int)rows, ik, reinterpret_cast<cuDoubleComplex*>(Y), (int)rows,
@@ -347,17 +342,17 @@ int svd_subspace(gtn_ctx ctx, cusolverDnHandle_t h, int64_t m, int64_t n, const 
   GTN_CUDA_TRY(ctx, launch_conj_inplace(Ah, m * n, s));
   GTN_CUDA_TRY(ctx, launch_fill_uniform_c128(Zt, kk * n, 0x5eed5eedull + (uint64_t)m * 131 + (uint64_t)n, s));
   ctx->launches += 3;
-  GTN_CUDA_TRY(ctx, gemm(A, Zt, Qt, m, kk, n));  // Y = A Omega
+  if (const int st = linalg_gemm(ctx, A, Zt, Qt, m, kk, n)) return st;  // Y = A Omega
   int st = orth(Qt, m);
   if (st != GTN_OK) return st;
   std::vector<double> hw(kk), sig(kk), prev;
   const int64_t rchk = std::min(maxdim, kk);
   bool settled = false;
   for (int it = 0; it <= max_it; ++it) {
-    GTN_CUDA_TRY(ctx, gemm(Ah, Qt, Zt, n, kk, m));  // Z = A^H Q
+    if (const int st = linalg_gemm(ctx, Ah, Qt, Zt, n, kk, m)) return st;  // Z = A^H Q
     GTN_CUDA_TRY(ctx, cudaMemcpyAsync(Zc, Zt, kk * n * sizeof(double2), cudaMemcpyDeviceToDevice, s));
     GTN_CUDA_TRY(ctx, launch_conj_inplace(Zc, kk * n, s));
-    GTN_CUDA_TRY(ctx, gemm(Zc, Zt, Gc, kk, kk, n));  // Z^H Z, column-major
+    if (const int st = linalg_gemm(ctx, Zc, Zt, Gc, kk, kk, n)) return st;  // Z^H Z, column-major
     ctx->launches++;
     if (sv.heevd(h, CUSOLVER_EIG_MODE_VECTOR, CUBLAS_FILL_MODE_LOWER, ik, reinterpret_cast<cuDoubleComplex*>(Gc), ik, w,
                  reinterpret_cast<cuDoubleComplex*>(work), lwork, dinfo) != CUSOLVER_STATUS_SUCCESS)
@@ -380,7 +375,7 @@ int svd_subspace(gtn_ctx ctx, cusolverDnHandle_t h, int64_t m, int64_t n, const 
     prev = sig;
     st = orth(Zt, n);  // P = orth(Z)
     if (st != GTN_OK) return st;
-    GTN_CUDA_TRY(ctx, gemm(A, Zt, Qt, m, kk, n));  // Y = A P
+    if (const int st = linalg_gemm(ctx, A, Zt, Qt, m, kk, n)) return st;  // Y = A P
     st = orth(Qt, m);
     if (st != GTN_OK) return st;
   }
@@ -400,10 +395,10 @@ int svd_subspace(gtn_ctx ctx, cusolverDnHandle_t h, int64_t m, int64_t n, const 
   GTN_CUDA_TRY(ctx, launch_gather_c128_to_c128(Gc + (kk - 1) * kk, mg, kg, r, kk, kk, Wr, s));
   // U = Q W (m x r)
   GTN_CUDA_TRY(ctx, launch_transpose_c128(Qt, kk, m, Qr, s));
-  GTN_CUDA_TRY(ctx, gemm(Wr, Qr, U, r, m, kk));
+  if (const int st = linalg_gemm(ctx, Wr, Qr, U, r, m, kk)) return st;
   // Vh = S^-1 W^H Q^H A = S^-1 conj(W^T Z^T): C[c][l] = sum_j Z^T[l][j] Wr[c][j], conjugated
   GTN_CUDA_TRY(ctx, launch_transpose_c128(Zt, kk, n, Zc, s));
-  GTN_CUDA_TRY(ctx, gemm(Zc, Wr, Vh, n, r, kk));
+  if (const int st = linalg_gemm(ctx, Zc, Wr, Vh, n, r, kk)) return st;
   GTN_CUDA_TRY(ctx, launch_conj_inplace(Vh, r * n, s));
   GTN_CUDA_TRY(ctx, launch_row_norms(Vh, r, n, dnorm, s));
   ctx->launches += 5;

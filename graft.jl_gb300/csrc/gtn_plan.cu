@@ -508,7 +508,9 @@ int plan_build(gtn_ctx ctx, int n, const int* ranks, const int64_t* dims, const 
       if (st.tc || st.dg) map->max_mtc = std::max(map->max_mtc, st.M);
       if (st.dg) map->max_adg = std::max(map->max_adg, f64e_a_bytes(st.M, st.K));
       st.splitk = gemm_splitk_slices(st.M, st.N, st.K);
-      if (st.splitk > 1) map->max_splitk = std::max(map->max_splitk, (int64_t)st.splitk * st.M * st.N);
+      st.vslices = zgemm_view_slices(st.M, st.N, st.K);
+      const int sk = std::max(st.splitk, st.vslices);
+      if (sk > 1) map->max_splitk = std::max(map->max_splitk, (int64_t)sk * st.M * st.N);
     }
 
     // ---- pack the static: B[n][k] = S[freeS(n), shared(k)] (conj applied) -------------
@@ -774,23 +776,13 @@ int map_run(gtn_map map, int precision, const double2* x, double2* y) {
           prof_end(s, GTN_KERNEL_ZGEMM, 0.0);
           ctx->launches += 2;
         }
-      } else if (st.splitk > 1 && map->skbuf) {
-        double2* A = static_cast<double2*>(map->abuf);
-        prof_begin(s);
-        e = launch_gather_c128_to_c128(static_cast<const double2*>(cur), st.mg, st.kg, st.M, st.K, st.K, A, s);
-        prof_end(s, GTN_KERNEL_GATHER, 0.0);
-        prof_begin(s);
-        if (e == cudaSuccess)
-          e = launch_zgemm_simt_splitk(A, st.b64, static_cast<double2*>(out), st.M, st.N, st.K, st.splitk,
-                                       static_cast<double2*>(map->skbuf), s);
-        prof_end(s, GTN_KERNEL_ZGEMM, 8.0 * st.macs);
-        ctx->launches += 3;
       } else {
+        const int slices = map->skbuf ? st.vslices : 1;
         prof_begin(s);
         e = launch_zgemm_view(static_cast<const double2*>(cur), st.mg, st.kg, st.b64, static_cast<double2*>(out), st.M,
-                              st.N, st.K, s);
+                              st.N, st.K, s, nullptr, nullptr, 0, slices, static_cast<double2*>(map->skbuf));
         prof_end(s, GTN_KERNEL_ZGEMM, 8.0 * st.macs);
-        ctx->launches++;
+        ctx->launches += slices > 1 ? 2 : 1;
       }
     } else {
       if (cur64 && (st.small || !tc)) {

@@ -182,3 +182,14 @@ def test_short_contractions_skip_zeros_exactly(ctx, kn):
         assert not np.isfinite(got[M // 2]).any() and np.isnan(got[0]).all()
         ok = [i for i in range(M) if i not in (0, M // 2)]
         assert np.isfinite(got[ok]).all()
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("mkn", [(7, 511, 3), (7, 512, 3), (100, 5625, 5), (33, 1025, 47), (250, 640, 60), (1, 9000, 1)])
+def test_few_outputs_with_a_long_sum(ctx, mkn):
+    """The FP64 product in k slices, with remainders in m, n, k and the slices."""
+    M, K, N = mkn
+    rng = np.random.default_rng(K)
+    A, B = crandn(rng, (M, K)), crandn(rng, (K, N))
+    got = contract(ctx, A, B, "fp64")
+    assert np.all(np.abs(got - A @ B) <= K * 2.0 ** -52 * (np.abs(A) @ np.abs(B)))
