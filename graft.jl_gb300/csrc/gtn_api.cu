@@ -262,6 +262,7 @@ int gtn_ctx_destroy(gtn_ctx ctx) {
   if (ctx->d_red) cudaFree(ctx->d_red);
   if (ctx->h_red) cudaFreeHost(ctx->h_red);
   if (ctx->d_errflag) cudaFree(ctx->d_errflag);
+  if (ctx->f64e_part) cudaFree(ctx->f64e_part);
   if (ctx->own_stream) cudaStreamDestroy(ctx->stream);
   delete ctx;
   return GTN_OK;

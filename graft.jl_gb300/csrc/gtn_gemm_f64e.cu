@@ -30,8 +30,8 @@
 // digit i of A meets the stack e_0, e_1, .. in MMAs up to 256 wide whose columns run through
 // the levels from i on: 10 to 13 instructions a stage instead of 28 or 34 of width 64 (A is read
 // from shared memory once per instruction, and 64-wide instructions are bound by that).  One CTA per SM
-// walks over the tiles: warp 0 copies, warp 1 issues the MMAs, warps 2-9 drain the levels (warp
-// w reads TMEM lanes 32 (w % 4) .. + 31, columns (w - 2) / 4 * 32 .. + 31) and convert and store
+// walks over the tiles: warp 0 copies, warp 1 issues the MMAs, warps 2-17 drain the levels (warp
+// w reads TMEM lanes 32 (w % 4) .. + 31, columns (w - 2) / 4 * 16 .. + 15) and convert and store
 // a tile while the next one's MMAs run.  Every mbarrier wait is bounded as in the other tcgen05
 // kernels.
 #include "gtn_internal.h"
@@ -55,7 +55,9 @@ constexpr int kSmem = kStages * kStageBytes + 1024;
 constexpr int kChunkStages = 8;                  // 128 real k between drains of the levels 4-6
 constexpr int kHiLevels = 4;                     // levels 0-3: drained every second chunk
 constexpr uint32_t kTmemCols = 512;              // up to 8 levels x 64 columns
-constexpr int kThreads = 320;
+constexpr int kEpiWarps = 16;                    // four per TMEM lane quarter
+constexpr int kCols = kBN / (kEpiWarps / 4);     // real columns per epilogue thread
+constexpr int kThreads = 64 + 32 * kEpiWarps;
 // Stages of a chunk whose levels 0-3 are multiplied before the other levels are free again: the MMAs
 // hide most of their drain (8192 x 1024 x 1024: 1673 -> 1533 us with 34 products, 1468 -> 1353 with 28).
 constexpr int kAhead = 4;
@@ -98,15 +100,13 @@ __device__ __forceinline__ void bulk_load(uint32_t dst, const void* src, uint32_
                : "memory");
 }
 
-// acc[j] += w * (the exact integer in column j), 32 columns.
-__device__ __forceinline__ void drain(uint32_t taddr, int w, long long (&acc)[32]) {
+// acc[j] += w * (the exact integer in column j).
+__device__ __forceinline__ void drain(uint32_t taddr, int w, long long (&acc)[kCols]) {
+  static_assert(kCols == 16, "one 16-column load");
+  uint32_t v[16];
+  tmem_ld16(taddr, v);
 #pragma unroll
-  for (int h = 0; h < 2; ++h) {
-    uint32_t v[16];
-    tmem_ld16(taddr + (uint32_t)(h * 16), v);
-#pragma unroll
-    for (int j = 0; j < 16; ++j) acc[h * 16 + j] += (long long)__float2int_rn(__uint_as_float(v[j])) * w;
-  }
+  for (int j = 0; j < 16; ++j) acc[j] += (long long)__float2int_rn(__uint_as_float(v[j])) * w;
 }
 
 // Tile t -> (row tile, column tile): groups of kGroupM row tiles, rows fastest.
@@ -117,12 +117,49 @@ __device__ __forceinline__ void tile_of(int64_t t, int64_t tm, int64_t tn, int64
   *mt = g * kGroupM + (r - *nt * gm);
 }
 
-template <int L>
+// A CTA's share of the product: whole tiles in turn (neighbouring CTAs on neighbouring tiles).  With
+// Split the tiles of the last, incomplete wave (from `whole` on) are cut: their chunks, in tile
+// order, are dealt evenly, CTA b of G getting [U b / G, U (b+1) / G) of the U chunks.
+__device__ __forceinline__ int64_t unit_begin(int64_t U, int64_t b, int64_t G) { return U * b / G; }
+template <bool Split>
+struct Segments {
+  int nchunks;
+  int64_t t, whole, u, u0, end;
+  int64_t tile = 0;
+  int c0 = 0, c1 = 0, slot = 0;  // chunks [c0, c1) of the tile; where its partial sums go
+  __device__ Segments(int64_t ntiles, int nch) : nchunks(nch), t(blockIdx.x), whole(ntiles) {
+    if (Split) {
+      whole = ntiles / gridDim.x * gridDim.x;
+      const int64_t U = (ntiles - whole) * nch;
+      u0 = u = unit_begin(U, blockIdx.x, gridDim.x);
+      end = unit_begin(U, (int64_t)blockIdx.x + 1, gridDim.x);
+    }
+  }
+  __device__ bool next() {
+    if (t < whole) {
+      tile = t;
+      c0 = 0;
+      c1 = nchunks;
+      t += gridDim.x;
+      return true;
+    }
+    if (!Split || u >= end) return false;
+    const int64_t q = u / nchunks;
+    tile = whole + q;
+    c0 = (int)(u - q * nchunks);
+    c1 = (int)(end - u < nchunks - c0 ? c0 + (end - u) : nchunks);
+    slot = 2 * (int)blockIdx.x + (u == u0 ? 0 : 1);
+    u += c1 - c0;
+    return true;
+  }
+};
+
+template <int L, bool Split>
 __global__ void __launch_bounds__(kThreads, 1)
     f64e_gemm_kernel(const unsigned char* __restrict__ A, const unsigned char* __restrict__ B, double2* __restrict__ C,
                      int64_t M, int64_t N, int nkb, int64_t tiles_m, int64_t tiles_n, const float* __restrict__ a_exp,
                      const float* __restrict__ b_exp, const int* __restrict__ a_flag, const int* __restrict__ b_flag,
-                     int token, int* __restrict__ errflag) {
+                     int token, longlong2* __restrict__ part, int* __restrict__ errflag) {
   extern __shared__ __align__(1024) uint8_t smem_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) &
                                              ~static_cast<uintptr_t>(1023));
@@ -143,8 +180,8 @@ __global__ void __launch_bounds__(kThreads, 1)
       mbar_init(&empty_bar[s], 1);
     }
     mbar_init(&chunk_full, 1);
-    mbar_init(&hi_empty, 8);
-    mbar_init(&lo_empty, 8);
+    mbar_init(&hi_empty, kEpiWarps);
+    mbar_init(&lo_empty, kEpiWarps);
     abort_flag = 0;
     n_issued = 0;
     n_consumed = 0;
@@ -164,12 +201,14 @@ __global__ void __launch_bounds__(kThreads, 1)
   if (warp == 0 && lane == 0) {
     int it = 0;
     bool stop = false;
-    for (int64_t t = blockIdx.x; t < ntiles && !stop; t += gridDim.x) {
+    Segments<Split> seg(ntiles, nchunks);
+    while (!stop && seg.next()) {
       int64_t mt, nt;
-      tile_of(t, tiles_m, tiles_n, &mt, &nt);
+      tile_of(seg.tile, tiles_m, tiles_n, &mt, &nt);
       const unsigned char* a = A + mt * nkb * kStageA;
       const unsigned char* b = B + nt * nkb * kStageB;
-      for (int kb = 0; kb < nkb; ++kb, ++it) {
+      const int kb_end = seg.c1 * kChunkStages < nkb ? seg.c1 * kChunkStages : nkb;
+      for (int kb = seg.c0 * kChunkStages; kb < kb_end; ++kb, ++it) {
         const int s = it % kStages;
         const uint32_t ph = (uint32_t)(it / kStages) & 1u;
         if (!mbar_wait(&empty_bar[s], ph ^ 1u, &abort_flag)) {
@@ -198,9 +237,10 @@ __global__ void __launch_bounds__(kThreads, 1)
       fence_after();
       return !stop;
     };
-    for (int64_t t = blockIdx.x; t < ntiles && !stop; t += gridDim.x) {
-      int kb = 0;
-      for (int c = 0; c < nchunks && !stop; ++c, ++ev) {
+    Segments<Split> seg(ntiles, nchunks);
+    while (!stop && seg.next()) {
+      int kb = seg.c0 * kChunkStages;
+      for (int c = 0; c < seg.c1 - seg.c0 && !stop; ++c, ++ev) {
         const int n = nkb - kb < kChunkStages ? nkb - kb : kChunkStages;
         // the levels 0-3 run over two chunks: a pair's first one overwrites them
         if (!(c & 1) && !wait(&hi_empty, (hi_ev++ & 1u) ^ 1u)) break;
@@ -255,17 +295,17 @@ __global__ void __launch_bounds__(kThreads, 1)
     n_consumed = it;
   } else if (warp >= 2) {
     const int q4 = warp & 3;             // TMEM lane quarter
-    const int half = (warp - 2) >> 2;    // column half
-    const uint32_t tm0 = tmem_base + (uint32_t)(half * 32) + ((uint32_t)(q4 * 32) << 16);
+    const int cg = (warp - 2) >> 2;      // column group
+    const uint32_t tm0 = tmem_base + (uint32_t)(cg * kCols) + ((uint32_t)(q4 * 32) << 16);
     int ev = 0;
     bool ok = true;
-    for (int64_t t = blockIdx.x; t < ntiles && ok; t += gridDim.x) {
-      int64_t mt, nt;
-      tile_of(t, tiles_m, tiles_n, &mt, &nt);
-      long long hi[32], lo[32];
+    Segments<Split> seg(ntiles, nchunks);
+    while (ok && seg.next()) {
+      const int nc = seg.c1 - seg.c0;
+      long long hi[kCols], lo[kCols];
 #pragma unroll
-      for (int j = 0; j < 32; ++j) hi[j] = lo[j] = 0;
-      for (int c = 0; c < nchunks; ++c, ++ev) {
+      for (int j = 0; j < kCols; ++j) hi[j] = lo[j] = 0;
+      for (int c = 0; c < nc; ++c, ++ev) {
         if (!mbar_wait(&chunk_full, (uint32_t)ev & 1u, &abort_flag)) {
           if (lane == 0) {
             abort_flag = 1;
@@ -277,7 +317,7 @@ __global__ void __launch_bounds__(kThreads, 1)
         __syncwarp();
         fence_after();
         // weights 2^{-8(l + 2)}: levels 0-3 in units of 2^-40, the others in units of 2^-72
-        if ((c & 1) || c == nchunks - 1) {
+        if ((c & 1) || c == nc - 1) {
 #pragma unroll 1
           for (int l = 0; l < kHiLevels; ++l) drain(tm0 + (uint32_t)(l * kBN), 1 << (8 * (3 - l)), hi);
           fence_before();
@@ -290,12 +330,21 @@ __global__ void __launch_bounds__(kThreads, 1)
         __syncwarp();
         if (lane == 0) mbar_arrive_local(&lo_empty);
       }
-      const int64_t m = mt * kBM + q4 * 32 + lane;
-      if (ok && m < M) {
-        const int ea = (int)a_exp[m];
-        const int64_t nb = nt * (kBN / 2) + half * 16;
+      if (!ok) break;
+      if (Split && nc < nchunks) {  // part of a tile: f64e_finish_kernel adds the parts and converts
+        longlong2* p = part + (int64_t)seg.slot * kBM * kBN + (warp - 2) * 32 + lane;
 #pragma unroll
-        for (int j = 0; j < 16; ++j) {
+        for (int j = 0; j < kCols; ++j) p[j * 32 * kEpiWarps] = make_longlong2(hi[j], lo[j]);
+        continue;
+      }
+      int64_t mt, nt;
+      tile_of(seg.tile, tiles_m, tiles_n, &mt, &nt);
+      const int64_t m = mt * kBM + q4 * 32 + lane;
+      if (m < M) {
+        const int ea = (int)a_exp[m];
+        const int64_t nb = nt * (kBN / 2) + cg * (kCols / 2);
+#pragma unroll
+        for (int j = 0; j < kCols / 2; ++j) {
           const int64_t n = nb + j;
           if (n < N) {
             const int es = ea + (int)b_exp[n];
@@ -320,17 +369,69 @@ __global__ void __launch_bounds__(kThreads, 1)
   }
 }
 
+// The tiles that several CTAs shared: CTA (tile, jp) adds the parts of the column pair jp of each
+// epilogue thread (exact integer sums, any order gives the same), rounds and stores.
+__global__ void __launch_bounds__(32 * kEpiWarps)
+    f64e_finish_kernel(const longlong2* __restrict__ part, double2* __restrict__ C, int64_t M, int64_t N, int nchunks,
+                       int64_t tiles_m, int64_t tiles_n, int G, const float* __restrict__ a_exp,
+                       const float* __restrict__ b_exp, const int* __restrict__ a_flag, const int* __restrict__ b_flag,
+                       int token) {
+  if (*a_flag == token || *b_flag != 0) return;
+  constexpr int kPairs = kCols / 2, kT = 32 * kEpiWarps;
+  const int64_t whole = tiles_m * tiles_n / G * G, t = blockIdx.x / kPairs;  // tile whole + t
+  const int64_t U = (tiles_m * tiles_n - whole) * nchunks;
+  const int jp = blockIdx.x % kPairs;
+  auto owner = [&](int64_t u) { return ((u + 1) * G + U - 1) / U - 1; };  // the CTA of unit u
+  const int64_t b0 = owner(t * nchunks), b1 = owner(t * nchunks + nchunks - 1);
+  if (b0 == b1) return;
+  longlong2 re = make_longlong2(0, 0), im = make_longlong2(0, 0);
+  for (int64_t b = b0; b <= b1; ++b) {
+    const int64_t ub = unit_begin(U, b, G);
+    if (ub == unit_begin(U, b + 1, G)) continue;  // fewer chunks than CTAs: this one had none
+    const int64_t slot = 2 * b + (ub / nchunks == t ? 0 : 1);
+    const longlong2* p = part + slot * kBM * kBN + 2 * jp * kT + threadIdx.x;
+    const longlong2 x = p[0], y = p[kT];
+    re.x += x.x;
+    re.y += x.y;
+    im.x += y.x;
+    im.y += y.y;
+  }
+  int64_t mt, nt;
+  tile_of(whole + t, tiles_m, tiles_n, &mt, &nt);
+  const int warp = (threadIdx.x >> 5) + 2, lane = threadIdx.x & 31;
+  const int64_t m = mt * kBM + (warp & 3) * 32 + lane, n = nt * (kBN / 2) + ((warp - 2) >> 2) * kPairs + jp;
+  if (m < M && n < N) {
+    const int es = (int)a_exp[m] + (int)b_exp[n];
+    C[n * M + m] = make_double2(to_double(re.x, re.y, es), to_double(im.x, im.y, es));
+  }
+}
+
 }  // namespace
 
-// Digit planes: the split and the launches, then per wave of 152 tiles about 1000 clocks per
-// stage of 8 complex k and 5000 for the drains and the store.  FP64 pipe: 1.15 TFLOP/s.
-double f64e_time(double M, double N, double K) {
-  const double tiles = std::ceil(M / kBM) * std::ceil(2 * N / kBN);
-  return 8e-6 + std::ceil(tiles / 152) * (std::ceil(K / 8) * 1000 + 5000) / 1.9e9 + M * K * 60 / 4e12;
+// Seconds of a chunk (128 real k) and of a tile's end, and whether the last wave's tiles are shared:
+// when whole ones would leave more idle than the shared tiles' sums cost (about 10 us: 128 KB a part
+// written and read back, one more launch).  Measured, 34 products: M, N, K = 384, 96, 480 (9 tiles)
+// 63 -> 25 us, 250, 250, 1250 (16 tiles) 143 -> 39 us.
+constexpr double kChunk = 6e-6, kTileEnd = 2.5e-6, kShareCost = 10e-6;
+static double f64e_waves(double M, double N, double K, int sms, bool* share) {
+  const double tiles = std::ceil(M / kBM) * std::ceil(2 * N / kBN), chunks = std::ceil(K / 64);
+  const double tile = std::min(chunks, K / 64 + 0.125) * kChunk + kTileEnd;
+  const double rest = tiles - std::floor(tiles / sms) * sms;
+  const double cut = std::ceil(rest * chunks / sms) * kChunk + kTileEnd + kShareCost;
+  *share = rest > 0 && chunks > 1 && cut < tile;
+  return std::floor(tiles / sms) * tile + (rest > 0 ? std::min(tile, cut) : 0.0);
 }
+// Digit planes: the split and the launches, then the waves of tiles.  FP64 pipe: 1.15 TFLOP/s.
+double f64e_time(double M, double N, double K) {
+  bool share;
+  return 8e-6 + f64e_waves(M, N, K, 152, &share) + M * K * 60 / 4e12;
+}
+size_t f64e_part_bytes(int sm_count) { return (size_t)2 * std::max(1, sm_count) * kBM * kBN * sizeof(longlong2); }
 double f64_pipe_time(double M, double N, double K) { return 4e-6 + 8.0 * M * N * K / 1.15e12; }
 
-cudaError_t launch_f64e_gemm(const F64eGemmArgs& a, int sm_count, int* errflag, cudaStream_t s, std::string* why) {
+cudaError_t launch_f64e_gemm(const F64eGemmArgs& a, int sm_count, int* errflag, cudaStream_t s, std::string* why,
+                             int* launches) {
+  *launches = 0;
   if (a.M <= 0 || a.N <= 0) return cudaSuccess;
   if (!a.A || !a.B || !a.C || !a.a_exp || !a.b_exp || !a.a_flag || !a.b_flag || a.K <= 0 || a.K > kF64eMaxK) {
     if (why) *why = "f64e_gemm: every operand given and K at most 2^21";
@@ -340,19 +441,37 @@ cudaError_t launch_f64e_gemm(const F64eGemmArgs& a, int sm_count, int* errflag, 
     if (why) *why = "f64e_gemm: digit planes must be 16-byte aligned";
     return cudaErrorInvalidValue;
   }
-  auto kern = a.levels == 7 ? f64e_gemm_kernel<7> : f64e_gemm_kernel<8>;
-  static bool attr_set = false;
-  if (!attr_set) {
-    cudaError_t e = cudaFuncSetAttribute(f64e_gemm_kernel<7>, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmem);
-    if (e == cudaSuccess) e = cudaFuncSetAttribute(f64e_gemm_kernel<8>, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmem);
-    if (e != cudaSuccess) return e;
-    attr_set = true;
-  }
   const int nkb = (int)((a.K + 7) / 8);
   const int64_t tm = (a.M + kBM - 1) / kBM, tn = (2 * a.N + kBN - 1) / kBN;
-  const int64_t grid = std::min<int64_t>(tm * tn, std::max(1, sm_count));
-  kern<<<(unsigned)grid, kThreads, kSmem, s>>>(
+  const int nchunks = (nkb + kChunkStages - 1) / kChunkStages, sms = std::max(1, sm_count);
+  bool share = false;
+  f64e_waves((double)a.M, (double)a.N, (double)a.K, sms, &share);
+  share = share && a.part;
+  const int64_t grid = std::min<int64_t>(share && tm * tn < sms ? tm * tn * nchunks : tm * tn, sms);
+  using Kern = void (*)(const unsigned char*, const unsigned char*, double2*, int64_t, int64_t, int, int64_t, int64_t,
+                        const float*, const float*, const int*, const int*, int, longlong2*, int*);
+  static const Kern kerns[4] = {f64e_gemm_kernel<8, false>, f64e_gemm_kernel<8, true>, f64e_gemm_kernel<7, false>,
+                                f64e_gemm_kernel<7, true>};
+  static bool attr_set = false;
+  if (!attr_set) {
+    for (Kern k : kerns) {
+      const cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmem);
+      if (e != cudaSuccess) return e;
+    }
+    attr_set = true;
+  }
+  kerns[(a.levels == 7 ? 2 : 0) + (share ? 1 : 0)]<<<(unsigned)grid, kThreads, kSmem, s>>>(
       static_cast<const unsigned char*>(a.A), static_cast<const unsigned char*>(a.B), a.C, a.M, a.N, nkb, tm, tn,
-      a.a_exp, a.b_exp, a.a_flag, a.b_flag, a.token, errflag);
-  return cudaGetLastError();
+      a.a_exp, a.b_exp, a.a_flag, a.b_flag, a.token, share ? static_cast<longlong2*>(a.part) : nullptr, errflag);
+  cudaError_t e = cudaGetLastError();
+  *launches = 1;
+  if (e == cudaSuccess && share) {
+    *launches = 2;
+    const int64_t rest = tm * tn - tm * tn / grid * grid;
+    f64e_finish_kernel<<<(unsigned)(rest * (kCols / 2)), 32 * kEpiWarps, 0, s>>>(static_cast<const longlong2*>(a.part), a.C, a.M, a.N,
+                                                             nchunks, tm, tn, (int)grid, a.a_exp, a.b_exp, a.a_flag,
+                                                             a.b_flag, a.token);
+    e = cudaGetLastError();
+  }
+  return e;
 }

@@ -42,6 +42,7 @@ struct gtn_ctx_s {
   // out-of-range flags of the digit-plane products: product number t writes t to slot
   // t % kFbSlots, so no slot needs clearing between products (they are ordered on the stream)
   int* d_fbflag = nullptr;
+  void* f64e_part = nullptr;  // partial sums of the digit-plane products (first plan that has one)
   int fb_token = 0;
   int sm_count = 0;
   int cc_major = 0, cc_minor = 0;
@@ -371,8 +372,11 @@ struct F64eGemmArgs {
   const int* b_flag = nullptr;  // != 0: a row of B out of range
   int token = 0;
   int levels = 8;               // digit products d_i e_j with i + j < levels (7 or 8)
+  void* part = nullptr;         // f64e_part_bytes, or null: no tile is shared
 };
-cudaError_t launch_f64e_gemm(const F64eGemmArgs& a, int sm_count, int* errflag, cudaStream_t s, std::string* why);
+cudaError_t launch_f64e_gemm(const F64eGemmArgs& a, int sm_count, int* errflag, cudaStream_t s, std::string* why,
+                             int* launches);
+size_t f64e_part_bytes(int sm_count);  // partial sums of tiles that CTAs share
 // Digit planes and row exponents of the running tensor's K-major view (c128; *flag = token when
 // a row is out of range), and of a static B [N][K] (*flag = 1 when a row is out of range).
 cudaError_t launch_split_digits_tab(const double2* T, const GatherTab& t, int64_t M, int64_t K, float* rexp, void* out,

@@ -119,6 +119,10 @@ int fill_offset_tables(gtn_map map) {
 // plan (a step without them stays on the FP64 pipe) and needed in an FP64E one.
 int pack_digits(gtn_map map, bool required) {
   gtn_ctx ctx = map->ctx;
+  if (!ctx->f64e_part && cudaMalloc(&ctx->f64e_part, f64e_part_bytes(ctx->sm_count)) != cudaSuccess) {
+    cudaGetLastError();  // without it no tile is shared
+    ctx->f64e_part = nullptr;
+  }
   int* flags = nullptr;
   cudaError_t e = dalloc(map, &flags, map->steps.size() * sizeof(int));
   if (e == cudaSuccess) e = cudaMemsetAsync(flags, 0, map->steps.size() * sizeof(int), ctx->stream);
@@ -756,6 +760,7 @@ int map_run(gtn_map map, int precision, const double2* x, double2* y) {
         a.b_exp = st.bexp;
         a.token = ctx->fb_token;
         a.levels = f64e ? 7 : 8;
+        a.part = ctx->f64e_part;
         a.a_flag = ctx->d_fbflag + ctx->fb_token % kFbSlots;
         a.b_flag = st.bflag;
         int* flag = ctx->d_fbflag + ctx->fb_token % kFbSlots;
@@ -768,13 +773,13 @@ int map_run(gtn_map map, int precision, const double2* x, double2* y) {
         if (e == cudaSuccess) {
           std::string why;
           prof_begin(s);
-          e = launch_f64e_gemm(a, ctx->sm_count, ctx->d_errflag, s, &why);
+          e = launch_f64e_gemm(a, ctx->sm_count, ctx->d_errflag, s, &why, &nl);
           prof_end(s, GTN_KERNEL_TC_GEMM, 8.0 * st.macs);
           if (e != cudaSuccess) return set_err(ctx, GTN_ERR_CUDA, "f64e_gemm: " + why + " " + cudaGetErrorString(e));
           prof_begin(s);
           e = launch_zgemm_view(T, st.mg, st.kg, st.b64, a.C, st.M, st.N, st.K, s, a.a_flag, a.b_flag, a.token);
           prof_end(s, GTN_KERNEL_ZGEMM, 0.0);
-          ctx->launches += 2;
+          ctx->launches += nl + 1;
         }
       } else {
         const int slices = map->skbuf ? st.vslices : 1;
