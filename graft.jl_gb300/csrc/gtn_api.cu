@@ -95,9 +95,9 @@ cudaError_t ctx_red(gtn_ctx ctx, size_t n2) {
     ctx->red_cap = n2;
   }
   if (!ctx->h_red) {
-    cudaError_t e = cudaMallocHost(&ctx->h_red, 256 * sizeof(double2));
+    cudaError_t e = cudaMallocHost(&ctx->h_red, 408 * sizeof(double2));
     if (e != cudaSuccess) return e;
-    ctx->hred_cap = 256;
+    ctx->hred_cap = 408;
   }
   return cudaSuccess;
 }
@@ -261,6 +261,8 @@ int gtn_ctx_destroy(gtn_ctx ctx) {
   if (ctx->carena) cudaFree(ctx->carena);
   if (ctx->d_red) cudaFree(ctx->d_red);
   if (ctx->h_red) cudaFreeHost(ctx->h_red);
+  for (auto& ev : ctx->step_ev)
+    if (ev) cudaEventDestroy(ev);
   if (ctx->d_errflag) cudaFree(ctx->d_errflag);
   if (ctx->f64e_part) cudaFree(ctx->f64e_part);
   if (ctx->own_stream) cudaStreamDestroy(ctx->stream);

@@ -11,10 +11,6 @@ namespace {
 constexpr int kMaxJ = 64;
 constexpr int kDotThreads = 256;
 
-__device__ __forceinline__ double2 cmul_conj(double2 a, double2 b) {  // conj(a) * b
-  return make_double2(a.x * b.x + a.y * b.y, a.x * b.y - a.y * b.x);
-}
-
 // double -> float by bit manipulation on the integer pipe: mantissa truncated to 23 bits,
 // magnitudes below float's normal range flushed to signed zero, finite values above it
 // clamped to the largest float.  Inf stays Inf and NaN stays NaN (a quiet NaN), so a
@@ -37,147 +33,196 @@ __device__ __forceinline__ float dtof_trunc(double d) {
   return __uint_as_float(bits);
 }
 
-// Per-block partial sums of conj(V_j) . w for j < J, written to part[block * J + j].
-template <int JB>
-__global__ void __launch_bounds__(kDotThreads) multidot_partial_kernel(const double2* __restrict__ V,
-                                                                       int64_t ldv, int J, int j0,
-                                                                       const double2* __restrict__ w,
-                                                                       int64_t n,
-                                                                       double2* __restrict__ part) {
-  double2 acc[JB];
+// acc += conj(v) w: four FMAs, in FP64 or, with F32, on inputs rounded to float.
+template <bool F32> struct DotAcc;
+template <> struct DotAcc<false> {
+  using T = double2;
+  __device__ static T load(double2 v) { return v; }
+  __device__ static void add(T& acc, T v, T w) {
+    acc.x = fma(v.x, w.x, fma(v.y, w.y, acc.x));
+    acc.y = fma(v.x, w.y, fma(-v.y, w.x, acc.y));
+  }
+};
+template <> struct DotAcc<true> {
+  using T = float2;
+  __device__ static T load(double2 v) { return make_float2(dtof_trunc(v.x), dtof_trunc(v.y)); }
+  __device__ static void add(T& acc, T v, T w) {
+    acc.x = fmaf(v.x, w.x, fmaf(v.y, w.y, acc.x));
+    acc.y = fmaf(v.x, w.y, fmaf(-v.y, w.x, acc.y));
+  }
+};
+
+// Sums of R rows of 256 doubles (row r, thread t at sm[r * 256 + t]) by 16 threads per row; the
+// first of each row's 16 threads returns the sum (r = tid / 16).  An FP64 addition costs a warp
+// about 15 clocks of the SM's FP64 pipe, and the usual five shuffle rounds per value kept it busy
+// for longer than the vectors took to stream; 16 threads add 16 values each and then take four
+// rounds, a quarter of the additions.
+__device__ __forceinline__ double row_sum16(const double* sm, int R) {
+  const int r = threadIdx.x >> 4, l = threadIdx.x & 15;
+  double x = 0.0;
+  if (r < R) {
+    const double* p = sm + r * kDotThreads;
 #pragma unroll
-  for (int j = 0; j < JB; ++j) acc[j] = make_double2(0.0, 0.0);
-  for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n;
-       i += (int64_t)gridDim.x * blockDim.x) {
-    const double2 wi = w[i];
+    for (int i = 0; i < 16; ++i) x += p[i * 16 + l];
 #pragma unroll
-    for (int j = 0; j < JB; ++j) {
-      if (j0 + j < J) {
-        const double2 v = V[(int64_t)(j0 + j) * ldv + i];
-        const double2 p = cmul_conj(v, wi);
-        acc[j].x += p.x;
-        acc[j].y += p.y;
-      }
+    for (int o = 8; o > 0; o >>= 1) x += __shfl_down_sync(0xffffu << (threadIdx.x & 16), x, o, 16);
+  }
+  return x;
+}
+
+// Per-block partial sums of conj(V_j) . w for the JB vectors from j0 on, written to
+// part[block * J + j].  U elements in flight per vector, so that narrow groups keep as many
+// loads outstanding as wide ones.
+template <int JB, bool F32>
+__device__ __forceinline__ void dot_group(const double2* __restrict__ V, int64_t ldv, int J, int j0,
+                                          const double2* __restrict__ w, int64_t n, double2* __restrict__ part,
+                                          double* sm) {
+  using D = DotAcc<F32>;
+  constexpr int U = JB >= 5 ? 1 : JB >= 3 ? 2 : 4;
+  typename D::T acc[JB];
+#pragma unroll
+  for (int j = 0; j < JB; ++j) acc[j].x = acc[j].y = 0;
+  const int64_t step = (int64_t)gridDim.x * kDotThreads;
+  const double2* Vj = V + (int64_t)j0 * ldv;
+  int64_t i = (int64_t)blockIdx.x * kDotThreads + threadIdx.x;
+  for (; i + (U - 1) * step < n; i += U * step) {
+    double2 wi[U], v[U][JB];
+#pragma unroll
+    for (int u = 0; u < U; ++u) {
+      wi[u] = w[i + u * step];
+#pragma unroll
+      for (int j = 0; j < JB; ++j) v[u][j] = Vj[(int64_t)j * ldv + i + u * step];
+    }
+#pragma unroll
+    for (int u = 0; u < U; ++u) {
+      const typename D::T x = D::load(wi[u]);
+#pragma unroll
+      for (int j = 0; j < JB; ++j) D::add(acc[j], D::load(v[u][j]), x);
     }
   }
-  __shared__ double2 red[kDotThreads / 32][JB];
-  const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
+  for (; i < n; i += step) {
+    const typename D::T x = D::load(w[i]);
+#pragma unroll
+    for (int j = 0; j < JB; ++j) D::add(acc[j], D::load(Vj[(int64_t)j * ldv + i]), x);
+  }
 #pragma unroll
   for (int j = 0; j < JB; ++j) {
-    double x = acc[j].x, y = acc[j].y;
-    for (int o = 16; o > 0; o >>= 1) {
-      x += __shfl_down_sync(0xffffffffu, x, o);
-      y += __shfl_down_sync(0xffffffffu, y, o);
-    }
-    if (lane == 0) red[wid][j] = make_double2(x, y);
+    sm[(2 * j) * kDotThreads + threadIdx.x] = acc[j].x;
+    sm[(2 * j + 1) * kDotThreads + threadIdx.x] = acc[j].y;
   }
   __syncthreads();
-  if (threadIdx.x < JB && j0 + (int)threadIdx.x < J) {
-    double x = 0, y = 0;
-    for (int q = 0; q < kDotThreads / 32; ++q) {
-      x += red[q][threadIdx.x].x;
-      y += red[q][threadIdx.x].y;
-    }
-    part[(int64_t)blockIdx.x * J + j0 + threadIdx.x] = make_double2(x, y);
+  const double x = row_sum16(sm, 2 * JB);
+  const int r = threadIdx.x >> 4;
+  if (r < 2 * JB && (threadIdx.x & 15) == 0)
+    reinterpret_cast<double*>(part + (int64_t)blockIdx.x * J + j0 + (r >> 1))[r & 1] = x;
+}
+
+// All J projections in one launch, eight vectors per grid row; a row with fewer runs code for
+// exactly that many (a guarded slot of wider code would still cost its FP64 work).  F32: products
+// of inputs rounded to float, per-thread sums in float, block sums in double, for the
+// reorthogonalisation passes of mixed-precision Krylov bases, whose coefficients only need to be
+// accurate well below the map's own error.
+template <bool F32>
+__global__ void __launch_bounds__(kDotThreads, 3) multidot_partial_kernel(const double2* __restrict__ V, int64_t ldv,
+                                                                          int J, const double2* __restrict__ w,
+                                                                          int64_t n, double2* __restrict__ part) {
+  __shared__ double sm[16 * kDotThreads];
+  const int j0 = blockIdx.y * 8;
+  switch (min(8, J - j0)) {
+    case 1: dot_group<1, F32>(V, ldv, J, j0, w, n, part, sm); break;
+    case 2: dot_group<2, F32>(V, ldv, J, j0, w, n, part, sm); break;
+    case 3: dot_group<3, F32>(V, ldv, J, j0, w, n, part, sm); break;
+    case 4: dot_group<4, F32>(V, ldv, J, j0, w, n, part, sm); break;
+    case 5: dot_group<5, F32>(V, ldv, J, j0, w, n, part, sm); break;
+    case 6: dot_group<6, F32>(V, ldv, J, j0, w, n, part, sm); break;
+    case 7: dot_group<7, F32>(V, ldv, J, j0, w, n, part, sm); break;
+    default: dot_group<8, F32>(V, ldv, J, j0, w, n, part, sm); break;
   }
 }
 
-// The same projections with FP32 products (inputs rounded to float, per-thread sums in
-// float, block sums in double): for reorthogonalisation passes of mixed-precision Krylov
-// bases, whose coefficients only need to be accurate well below the map's own error.  The
-// vector kernels are FP64-ALU bound on this part, not HBM bound.
-template <int JB>
-__global__ void __launch_bounds__(kDotThreads) multidot_f32_partial_kernel(const double2* __restrict__ V,
-                                                                           int64_t ldv, int J, int j0,
-                                                                           const double2* __restrict__ w,
-                                                                           int64_t n,
-                                                                           double2* __restrict__ part) {
-  float2 acc[JB];
-#pragma unroll
-  for (int j = 0; j < JB; ++j) acc[j] = make_float2(0.f, 0.f);
-  for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n;
-       i += (int64_t)gridDim.x * blockDim.x) {
-    const double2 wd = w[i];
-    const float wx = dtof_trunc(wd.x), wy = dtof_trunc(wd.y);
-#pragma unroll
-    for (int j = 0; j < JB; ++j) {
-      if (j0 + j < J) {
-        const double2 vd = V[(int64_t)(j0 + j) * ldv + i];
-        const float vx = dtof_trunc(vd.x), vy = dtof_trunc(vd.y);
-        acc[j].x = fmaf(vx, wx, fmaf(vy, wy, acc[j].x));
-        acc[j].y = fmaf(vx, wy, fmaf(-vy, wx, acc[j].y));
-      }
-    }
-  }
-  __shared__ double2 red[kDotThreads / 32][JB];
-  const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
-#pragma unroll
-  for (int j = 0; j < JB; ++j) {
-    double x = acc[j].x, y = acc[j].y;
-    for (int o = 16; o > 0; o >>= 1) {
-      x += __shfl_down_sync(0xffffffffu, x, o);
-      y += __shfl_down_sync(0xffffffffu, y, o);
-    }
-    if (lane == 0) red[wid][j] = make_double2(x, y);
-  }
-  __syncthreads();
-  if (threadIdx.x < JB && j0 + (int)threadIdx.x < J) {
-    double x = 0, y = 0;
-    for (int q = 0; q < kDotThreads / 32; ++q) {
-      x += red[q][threadIdx.x].x;
-      y += red[q][threadIdx.x].y;
-    }
-    part[(int64_t)blockIdx.x * J + j0 + threadIdx.x] = make_double2(x, y);
-  }
-}
-
-// w -= sum_j coef[j] V_j with FP32 products and one FP64 subtraction per element: the
-// update of a reorthogonalisation pass, whose coefficients are small next to |w|.
-__global__ void reorth_update_f32_kernel(double2* __restrict__ w, const double2* __restrict__ V, int64_t ldv,
-                                         int J, const double2* __restrict__ coef, int64_t n) {
-  __shared__ float2 c[kMaxJ];
+// w -= sum_j coef[j] V_j, and the block sums of |w|^2 of the result when part is given.  F32: FP32
+// products and one FP64 subtraction per element (a reorthogonalisation pass, whose coefficients
+// are small next to |w|).
+template <bool F32>
+__global__ void __launch_bounds__(kDotThreads) update_kernel(double2* __restrict__ w, const double2* __restrict__ V,
+                                                             int64_t ldv, int J, const double2* __restrict__ coef,
+                                                             int64_t n, double2* __restrict__ part) {
+  __shared__ double2 c[kMaxJ];
+  __shared__ float2 cf[kMaxJ];
+  __shared__ double sm[kDotThreads];
   if ((int)threadIdx.x < J) {
-    const double2 a = coef[threadIdx.x];
-    c[threadIdx.x] = make_float2((float)a.x, (float)a.y);
+    c[threadIdx.x] = coef[threadIdx.x];
+    cf[threadIdx.x] = make_float2((float)coef[threadIdx.x].x, (float)coef[threadIdx.x].y);
   }
   __syncthreads();
-  for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n;
-       i += (int64_t)gridDim.x * blockDim.x) {
-    float ax = 0.f, ay = 0.f;
-    for (int j = 0; j < J; ++j) {
-      const double2 vd = V[(int64_t)j * ldv + i];
-      const float vx = dtof_trunc(vd.x), vy = dtof_trunc(vd.y);
-      ax = fmaf(c[j].x, vx, fmaf(-c[j].y, vy, ax));
-      ay = fmaf(c[j].x, vy, fmaf(c[j].y, vx, ay));
-    }
+  double nn = 0.0;
+  for (int64_t i = (int64_t)blockIdx.x * kDotThreads + threadIdx.x; i < n; i += (int64_t)gridDim.x * kDotThreads) {
     double2 wi = w[i];
-    wi.x -= (double)ax;
-    wi.y -= (double)ay;
+    if constexpr (F32) {
+      float ax = 0.f, ay = 0.f;
+#pragma unroll 4
+      for (int j = 0; j < J; ++j) {
+        const float2 v = DotAcc<true>::load(V[(int64_t)j * ldv + i]);
+        ax = fmaf(cf[j].x, v.x, fmaf(-cf[j].y, v.y, ax));
+        ay = fmaf(cf[j].x, v.y, fmaf(cf[j].y, v.x, ay));
+      }
+      wi.x -= (double)ax;
+      wi.y -= (double)ay;
+    } else {
+#pragma unroll 4
+      for (int j = 0; j < J; ++j) {
+        const double2 v = V[(int64_t)j * ldv + i];
+        wi.x = fma(-c[j].x, v.x, fma(c[j].y, v.y, wi.x));
+        wi.y = fma(-c[j].x, v.y, fma(-c[j].y, v.x, wi.y));
+      }
+    }
     w[i] = wi;
+    nn = fma(wi.x, wi.x, fma(wi.y, wi.y, nn));
+  }
+  if (!part) return;
+  sm[threadIdx.x] = nn;
+  __syncthreads();
+  const double x = row_sum16(sm, 1);
+  if (threadIdx.x == 0) part[blockIdx.x] = make_double2(x, 0.0);
+}
+
+// w /= sqrt(nrm2) with the squared norm on the device (left alone where that is not positive).
+__global__ void __launch_bounds__(kDotThreads) unit_scale_kernel(double2* __restrict__ w,
+                                                                 const double2* __restrict__ nrm2, int64_t n) {
+  __shared__ double f;
+  if (threadIdx.x == 0) f = nrm2->x > 0.0 ? 1.0 / sqrt(nrm2->x) : 1.0;
+  __syncthreads();
+  const double s = f;
+  for (int64_t i = (int64_t)blockIdx.x * kDotThreads + threadIdx.x; i < n; i += (int64_t)gridDim.x * kDotThreads) {
+    const double2 v = w[i];
+    w[i] = make_double2(s * v.x, s * v.y);
   }
 }
 
-// out[j] = sum over blocks of part[b * J + j] (fixed order: deterministic).
-__global__ void multidot_final_kernel(const double2* __restrict__ part, int nblk, int J,
-                                      double2* __restrict__ out) {
+// out[j] = sum over blocks of part[b * J + j] (fixed order: deterministic); with errflag also the
+// device error flag in out[J], so that one copy brings a step's results to the host.  (Adding the
+// partials in the projection's last CTA instead, found by a counter, measured 9 us slower a launch.)
+__global__ void __launch_bounds__(128) multidot_final_kernel(const double2* __restrict__ part, int nblk, int J,
+                                                             double2* __restrict__ out,
+                                                             const int* __restrict__ errflag) {
   const int j = blockIdx.x;
   double x = 0, y = 0;
-  for (int b = threadIdx.x; b < nblk; b += blockDim.x) {
-    x += part[(int64_t)b * J + j].x;
-    y += part[(int64_t)b * J + j].y;
+  for (int b = threadIdx.x; b < nblk; b += 128) {
+    const double2 p = part[(int64_t)b * J + j];
+    x += p.x;
+    y += p.y;
   }
-  __shared__ double sx[256], sy[256];
-  sx[threadIdx.x] = x;
-  sy[threadIdx.x] = y;
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) {
+    x += __shfl_down_sync(0xffffffffu, x, o);
+    y += __shfl_down_sync(0xffffffffu, y, o);
+  }
+  __shared__ double2 sw[4];
+  if ((threadIdx.x & 31) == 0) sw[threadIdx.x >> 5] = make_double2(x, y);
   __syncthreads();
-  for (int o = blockDim.x / 2; o > 0; o >>= 1) {
-    if ((int)threadIdx.x < o) {
-      sx[threadIdx.x] += sx[threadIdx.x + o];
-      sy[threadIdx.x] += sy[threadIdx.x + o];
-    }
-    __syncthreads();
-  }
-  if (threadIdx.x == 0) out[j] = make_double2(sx[0], sy[0]);
+  if (threadIdx.x == 0 && errflag) *reinterpret_cast<int*>(out + J) = *errflag;
+  if (threadIdx.x == 0)
+    out[j] = make_double2((sw[0].x + sw[1].x) + (sw[2].x + sw[3].x), (sw[0].y + sw[1].y) + (sw[2].y + sw[3].y));
 }
 
 // w = beta*w + cscale * sum_j coef[j] V_j
@@ -201,10 +246,11 @@ __global__ void lincomb_kernel(double2* __restrict__ w, double2 beta, const doub
       const double2 wi = w[i];
       acc = make_double2(beta.x * wi.x - beta.y * wi.y, beta.x * wi.y + beta.y * wi.x);
     }
+#pragma unroll 4
     for (int j = 0; j < J; ++j) {
       const double2 v = V[(int64_t)j * ldv + i];
-      acc.x += c[j].x * v.x - c[j].y * v.y;
-      acc.y += c[j].x * v.y + c[j].y * v.x;
+      acc.x = fma(c[j].x, v.x, fma(-c[j].y, v.y, acc.x));
+      acc.y = fma(c[j].x, v.y, fma(c[j].y, v.x, acc.y));
     }
     w[i] = acc;
   }
@@ -380,66 +426,55 @@ inline unsigned grid_for(int64_t n) {
 
 int multidot_blocks(gtn_ctx ctx) { return (ctx->sm_count > 0 ? ctx->sm_count : 152) * 2; }
 
-int multidot_launch_count(int J) {
-  int c = J > 0 ? 1 : 0;  // the final reduction
-  for (int j0 = 0; j0 < J;) {
-    const int rem = J - j0;
-    j0 += rem >= 8 ? 8 : rem >= 4 ? 4 : rem >= 2 ? 2 : 1;
-    ++c;
-  }
-  return c;
+int multidot_launch_count(int J) { return J > 0 ? 2 : 0; }
+
+// Blocks of a projection or update over n elements: about eight elements per thread (fewer
+// FP64 block sums than elements), at most nblk, or up to four times that where the partials
+// (blocks * J entries) fit the caller's scratch: few vectors need more CTAs to fill the memory
+// pipe (scratch_cap 0: nblk).
+static int dot_blocks(int64_t n, int nblk, int J, int64_t scratch_cap) {
+  int64_t cap = nblk;
+  if (scratch_cap > 0 && J <= 8)
+    for (int f : {4, 2})
+      if ((int64_t)nblk * f * J <= scratch_cap) {
+        cap = (int64_t)nblk * f;
+        break;
+      }
+  const int64_t want = (n + 4 * kDotThreads - 1) / (4 * kDotThreads);
+  return (int)(want < 1 ? 1 : want < cap ? want : cap);
 }
 
-// Grid widening for latency-bound projections: the FP32 kernels and the 1-2 vector FP64 ones
-// keep too few loads in flight with 2 CTAs per SM.  The partials need nb * J entries, so the
-// grid only widens as far as the caller's scratch capacity allows (0: exactly nblk * J).
-int widened_blocks(int nblk, int J, int64_t scratch_cap, bool f32) {
-  if (scratch_cap <= 0 || (!f32 && J > 2)) return nblk;
-  for (int f : {4, 2})
-    if ((int64_t)nblk * f * J <= scratch_cap) return nblk * f;
-  return nblk;
-}
-
-cudaError_t launch_multidot(const double2* V, int64_t ldv, int J, const double2* w, int64_t n,
-                            double2* out, double2* scratch, int nblk, cudaStream_t s, int64_t scratch_cap) {
+template <bool F32>
+static cudaError_t multidot(const double2* V, int64_t ldv, int J, const double2* w, int64_t n, double2* out,
+                            double2* scratch, int nblk, cudaStream_t s, int64_t scratch_cap) {
   if (J <= 0) return cudaSuccess;
   if (J > kMaxJ) return cudaErrorInvalidValue;
-  nblk = widened_blocks(nblk, J, scratch_cap, false);
-  // vectors in groups of 8, 4, 2, 1: a guarded slot of a wider kernel still costs its FP64 work
-  for (int j0 = 0; j0 < J;) {
-    const int rem = J - j0;
-    if (rem >= 8) multidot_partial_kernel<8><<<nblk, kDotThreads, 0, s>>>(V, ldv, J, j0, w, n, scratch);
-    else if (rem >= 4) multidot_partial_kernel<4><<<nblk, kDotThreads, 0, s>>>(V, ldv, J, j0, w, n, scratch);
-    else if (rem >= 2) multidot_partial_kernel<2><<<nblk, kDotThreads, 0, s>>>(V, ldv, J, j0, w, n, scratch);
-    else multidot_partial_kernel<1><<<nblk, kDotThreads, 0, s>>>(V, ldv, J, j0, w, n, scratch);
-    j0 += rem >= 8 ? 8 : rem >= 4 ? 4 : rem >= 2 ? 2 : 1;
-  }
-  multidot_final_kernel<<<J, 256, 0, s>>>(scratch, nblk, J, out);
+  const int nb = dot_blocks(n, nblk, J, scratch_cap);
+  multidot_partial_kernel<F32><<<dim3((unsigned)nb, (unsigned)((J + 7) / 8)), kDotThreads, 0, s>>>(
+      V, ldv, J, w, n, scratch);
+  multidot_final_kernel<<<J, 128, 0, s>>>(scratch, nb, J, out, nullptr);
   return cudaGetLastError();
 }
-
-cudaError_t launch_multidot_f32(const double2* V, int64_t ldv, int J, const double2* w, int64_t n,
-                                double2* out, double2* scratch, int nblk, cudaStream_t s, int64_t scratch_cap) {
-  if (J <= 0) return cudaSuccess;
-  if (J > kMaxJ) return cudaErrorInvalidValue;
-  nblk = widened_blocks(nblk, J, scratch_cap, true);
-  for (int j0 = 0; j0 < J;) {
-    const int rem = J - j0;
-    if (rem >= 8) multidot_f32_partial_kernel<8><<<nblk, kDotThreads, 0, s>>>(V, ldv, J, j0, w, n, scratch);
-    else if (rem >= 4) multidot_f32_partial_kernel<4><<<nblk, kDotThreads, 0, s>>>(V, ldv, J, j0, w, n, scratch);
-    else if (rem >= 2) multidot_f32_partial_kernel<2><<<nblk, kDotThreads, 0, s>>>(V, ldv, J, j0, w, n, scratch);
-    else multidot_f32_partial_kernel<1><<<nblk, kDotThreads, 0, s>>>(V, ldv, J, j0, w, n, scratch);
-    j0 += rem >= 8 ? 8 : rem >= 4 ? 4 : rem >= 2 ? 2 : 1;
-  }
-  multidot_final_kernel<<<J, 256, 0, s>>>(scratch, nblk, J, out);
+cudaError_t launch_multidot(const double2* V, int64_t ldv, int J, const double2* w, int64_t n, double2* out,
+                            double2* scratch, int nblk, cudaStream_t s, int64_t scratch_cap) {
+  return multidot<false>(V, ldv, J, w, n, out, scratch, nblk, s, scratch_cap);
+}
+cudaError_t launch_multidot_f32(const double2* V, int64_t ldv, int J, const double2* w, int64_t n, double2* out,
+                                double2* scratch, int nblk, cudaStream_t s, int64_t scratch_cap) {
+  return multidot<true>(V, ldv, J, w, n, out, scratch, nblk, s, scratch_cap);
+}
+cudaError_t launch_update(double2* w, const double2* V, int64_t ldv, int J, const double2* coef, int64_t n, bool f32,
+                          double2* nrm2, double2* scratch, int nblk, int64_t scratch_cap,
+                          const int* errflag, cudaStream_t s) {
+  if (J <= 0 || J > kMaxJ) return cudaErrorInvalidValue;
+  const int nb = dot_blocks(n, nblk, 1, scratch_cap);
+  double2* part = nrm2 ? scratch : nullptr;
+  (f32 ? update_kernel<true> : update_kernel<false>)<<<nb, kDotThreads, 0, s>>>(w, V, ldv, J, coef, n, part);
+  if (nrm2) multidot_final_kernel<<<1, 128, 0, s>>>(part, nb, 1, nrm2, errflag);
   return cudaGetLastError();
 }
-
-cudaError_t launch_reorth_update_f32(double2* w, const double2* V, int64_t ldv, int J, const double2* coef,
-                                     int64_t n, cudaStream_t s) {
-  if (J > kMaxJ) return cudaErrorInvalidValue;
-  if (J <= 0) return cudaSuccess;
-  reorth_update_f32_kernel<<<grid_for(n), 256, 0, s>>>(w, V, ldv, J, coef, n);
+cudaError_t launch_unit_scale(double2* w, const double2* nrm2, int64_t n, cudaStream_t s) {
+  unit_scale_kernel<<<grid_for(n), kDotThreads, 0, s>>>(w, nrm2, n);
   return cudaGetLastError();
 }
 

@@ -378,17 +378,23 @@ __global__ void __launch_bounds__(32 * kEpiWarps)
                        int token) {
   if (*a_flag == token || *b_flag != 0) return;
   constexpr int kPairs = kCols / 2, kT = 32 * kEpiWarps;
-  const int64_t whole = tiles_m * tiles_n / G * G, t = blockIdx.x / kPairs;  // tile whole + t
-  const int64_t U = (tiles_m * tiles_n - whole) * nchunks;
+  const int64_t whole = tiles_m * tiles_n / G * G;
+  // fewer than G tiles of at most 2^15 chunks are shared: 32 bits hold U b
+  const int t = blockIdx.x / kPairs, U = (int)(tiles_m * tiles_n - whole) * nchunks;  // tile whole + t
   const int jp = blockIdx.x % kPairs;
-  auto owner = [&](int64_t u) { return ((u + 1) * G + U - 1) / U - 1; };  // the CTA of unit u
-  const int64_t b0 = owner(t * nchunks), b1 = owner(t * nchunks + nchunks - 1);
+  auto begin = [&](int b) { return (int)((uint32_t)U * (uint32_t)b / (uint32_t)G); };
+  auto owner = [&](int u) { return (int)(((uint32_t)(u + 1) * (uint32_t)G + U - 1) / (uint32_t)U) - 1; };  // CTA of u
+  const int b0 = owner(t * nchunks), b1 = owner(t * nchunks + nchunks - 1);
   if (b0 == b1) return;
   longlong2 re = make_longlong2(0, 0), im = make_longlong2(0, 0);
-  for (int64_t b = b0; b <= b1; ++b) {
-    const int64_t ub = unit_begin(U, b, G);
-    if (ub == unit_begin(U, b + 1, G)) continue;  // fewer chunks than CTAs: this one had none
-    const int64_t slot = 2 * b + (ub / nchunks == t ? 0 : 1);
+  int next = begin(b0);
+#pragma unroll 4
+  for (int b = b0; b <= b1; ++b) {
+    const int ub = next;
+    next = begin(b + 1);
+    if (ub == next) continue;  // fewer chunks than CTAs: this one had none
+    // its first segment where it begins in this tile, else (b == b0) its second
+    const int64_t slot = 2 * b + (ub >= t * nchunks ? 0 : 1);
     const longlong2* p = part + slot * kBM * kBN + 2 * jp * kT + threadIdx.x;
     const longlong2 x = p[0], y = p[kT];
     re.x += x.x;

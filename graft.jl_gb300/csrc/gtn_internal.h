@@ -51,6 +51,7 @@ struct gtn_ctx_s {
   size_t red_cap = 0;
   double2* h_red = nullptr;
   size_t hred_cap = 0;
+  cudaEvent_t step_ev[2] = {nullptr, nullptr};  // the Krylov steps in flight
   // transient workspace for one-shot contractions / factorisations
   void* ws = nullptr;
   size_t ws_bytes = 0;
@@ -414,8 +415,13 @@ int multidot_launch_count(int J);  // kernels one launch_multidot[_f32] of J vec
 cudaError_t launch_multidot_f32(const double2* V, int64_t ldv, int J, const double2* w, int64_t n,
                                 double2* out /*[J]*/, double2* scratch, int nblk, cudaStream_t s,
                                 int64_t scratch_cap = 0);
-cudaError_t launch_reorth_update_f32(double2* w, const double2* V, int64_t ldv, int J,
-                                     const double2* coef /*device [J]*/, int64_t n, cudaStream_t s);
+// w -= sum_j coef[j] V_j (f32: FP32 products); with nrm2 also nrm2[0] = |w|^2 of the result, by way
+// of scratch (blocks as for launch_multidot of one vector), and nrm2[1] = *errflag.
+cudaError_t launch_update(double2* w, const double2* V, int64_t ldv, int J, const double2* coef /*device [J]*/,
+                          int64_t n, bool f32, double2* nrm2, double2* scratch, int nblk, int64_t scratch_cap,
+                          const int* errflag, cudaStream_t s);
+// w /= sqrt(nrm2), the squared norm read on the device.
+cudaError_t launch_unit_scale(double2* w, const double2* nrm2, int64_t n, cudaStream_t s);
 // In place: V_j <- sum_{i<m} Q[i * k + j] V_i for j < k (k <= m <= 64, Q real, device).
 cudaError_t launch_basis_rotate(double2* V, int64_t ldv, int m, int k, const double* Q, int64_t n,
                                 cudaStream_t s);

@@ -17,10 +17,17 @@
 #include <algorithm>
 #include <cmath>
 #include <complex>
+#include <cstring>
 
 namespace {
 
 constexpr int kMaxKrylov = 63;
+// Pinned slots of 136 entries behind the 136 that fetch and push share: one per step in flight.
+constexpr int kStepSlot = 136;
+// A solve that may stop at any step queues the next one ahead only for vectors of up to 2^20
+// elements: the step that is then queued in vain once per expansion costs less than the gaps that
+// the others close (40-70 us a step against a map application).
+constexpr int64_t kAheadElems = int64_t(1) << 20;
 
 // Cyclic Jacobi eigen-decomposition of a symmetric n x n matrix (row-major A, destroyed).
 // On return w holds eigenvalues ascending and V's columns the matching eigenvectors.
@@ -121,6 +128,8 @@ int krylov_setup(gtn_map map, int kd, Krylov* K) {
   K->part = map->kscratch;
   K->part_cap = map->kscratch_cap;
   GTN_CUDA_TRY(ctx, ctx_red(ctx, 64));
+  for (auto& ev : ctx->step_ev)
+    if (!ev) GTN_CUDA_TRY(ctx, cudaEventCreateWithFlags(&ev, cudaEventDisableTiming));
   return GTN_OK;
 }
 
@@ -163,12 +172,58 @@ int normalize(Krylov& K, double2* x, double* nrm) {
   return GTN_OK;
 }
 
+// The step of a Lanczos expansion that applies the map to V[j]: orthogonalises w = V[j+1], brings
+// the projections, |w|^2 and the device error flag to the pinned slot j % 2, records its event and
+// normalises w on the device.
+int lanczos_step(Krylov& K, int j, bool first, int precision) {
+  gtn_ctx ctx = K.ctx;
+  cudaStream_t s = ctx->stream;
+  double2* w = K.V + (int64_t)(j + 1) * K.n;
+  const int st = map_run(K.map, precision, K.V + (int64_t)j * K.n, w);
+  if (st != GTN_OK) return st;
+  auto dots = [&](const double2* V, int J, double2* out, bool f32) {
+    ctx->launches += multidot_launch_count(J);
+    return (f32 ? launch_multidot_f32 : launch_multidot)(V, K.n, J, w, K.n, out, K.part, K.nblk, s, K.part_cap);
+  };
+  auto update = [&](const double2* V, int J, const double2* c, bool f32, double2* nrm2) {
+    ctx->launches += nrm2 ? 2 : 1;
+    return launch_update(w, V, K.n, J, c, K.n, f32, nrm2, K.part, K.nblk, K.part_cap, ctx->d_errflag, s);
+  };
+  if (first) {
+    // first vector of an expansion (couples to every kept Ritz vector): two classical
+    // Gram-Schmidt passes against V[0..j] in FP64
+    GTN_CUDA_TRY(ctx, dots(K.V, j + 1, K.coef, false));
+    GTN_CUDA_TRY(ctx, update(K.V, j + 1, K.coef, false, nullptr));
+    GTN_CUDA_TRY(ctx, dots(K.V, j + 1, K.coef + 64, false));
+    GTN_CUDA_TRY(ctx, update(K.V, j + 1, K.coef + 64, false, K.coef + 128));
+  } else {
+    // local three-term step against V[j-1], V[j] in FP64, then one full reorthogonalisation
+    // pass (FP32 products for mixed-precision maps, whose error sits far above the
+    // coefficients this pass removes)
+    const double2* vprev = K.V + (int64_t)(j - 1) * K.n;
+    const bool f32 = precision != GTN_PREC_FP64;
+    GTN_CUDA_TRY(ctx, dots(vprev, 2, K.coef, false));
+    GTN_CUDA_TRY(ctx, update(vprev, 2, K.coef, false, nullptr));
+    GTN_CUDA_TRY(ctx, dots(K.V, j + 1, K.coef + 64, f32));
+    GTN_CUDA_TRY(ctx, update(K.V, j + 1, K.coef + 64, f32, K.coef + 128));
+  }
+  double2* slot = ctx->h_red + kStepSlot * (1 + (j & 1));
+  GTN_CUDA_TRY(ctx, cudaMemcpyAsync(slot, K.coef, 130 * sizeof(double2), cudaMemcpyDeviceToHost, s));
+  GTN_CUDA_TRY(ctx, cudaEventRecord(ctx->step_ev[j & 1], s));
+  GTN_CUDA_TRY(ctx, launch_unit_scale(w, K.coef + 128, K.n, s));
+  ctx->launches++;
+  return GTN_OK;
+}
+
 // Lanczos expansion of the basis from column j0 (V[j0] unit norm and orthogonal to V[0..j0))
 // up to kd columns.  Fills a[j0..m), b[j0..m) and returns m (the number of basis vectors);
 // V[m] then holds the normalised residual direction and b[m-1] its norm.  Stops early at an
-// invariant subspace, or when `stop` says so.
+// invariant subspace, or when `stop` says so.  With `ahead` the next step is queued before the
+// host has looked at this one, so that the GPU does not wait for the host's projected problem; a
+// step queued past the end of the expansion, or before a repeated pass, is dropped (its vector is
+// outside the basis or computed again).
 template <class Stop>
-int lanczos_expand(Krylov& K, int j0, int kd, int precision, std::vector<double>& a, std::vector<double>& b,
+int lanczos_expand(Krylov& K, int j0, int kd, int precision, bool ahead, std::vector<double>& a, std::vector<double>& b,
                    int* m_out, int* matvecs, bool* breakdown, Stop stop) {
   gtn_ctx ctx = K.ctx;
   cudaStream_t s = ctx->stream;
@@ -176,43 +231,25 @@ int lanczos_expand(Krylov& K, int j0, int kd, int precision, std::vector<double>
   b.resize(kd, 0.0);
   for (int j = j0; j < kd; ++j) a[j] = b[j] = 0.0;
   *breakdown = false;
-  const bool fast_reorth = precision != GTN_PREC_FP64;
   int m = kd;
+  int queued = j0;  // steps queued so far: j0 .. queued - 1
   for (int j = j0; j < kd; ++j) {
-    double2* vj = K.V + (int64_t)j * K.n;
-    double2* w = K.V + (int64_t)(j + 1) * K.n;
-    int st = map_run(K.map, precision, vj, w);
-    if (st != GTN_OK) return st;
-    (*matvecs)++;
-    double2 hbuf[130];
-    double hh = 0.0;  // squared norm of the full-pass coefficients (local steps only)
-    if (j == j0) {
-      // first vector of an expansion (couples to every kept Ritz vector): two classical
-      // Gram-Schmidt passes against V[0..j] in FP64
-      GTN_CUDA_TRY(ctx, launch_multidot(K.V, K.n, j + 1, w, K.n, K.coef, K.part, K.nblk, s, K.part_cap));
-      GTN_CUDA_TRY(ctx, launch_lincomb(w, make_double2(1.0, 0.0), K.V, K.n, j + 1, K.coef, make_double2(-1.0, 0.0), K.n, s));
-      GTN_CUDA_TRY(ctx, launch_multidot(K.V, K.n, j + 1, w, K.n, K.coef + 64, K.part, K.nblk, s, K.part_cap));
-      GTN_CUDA_TRY(ctx, launch_lincomb(w, make_double2(1.0, 0.0), K.V, K.n, j + 1, K.coef + 64, make_double2(-1.0, 0.0), K.n, s));
-      ctx->launches += 2 * (multidot_launch_count(j + 1) + 1);
-    } else {
-      // local three-term step against V[j-1], V[j] in FP64, then one full reorthogonalisation
-      // pass (FP32 products for mixed-precision maps, whose error sits far above the
-      // coefficients this pass removes)
-      const double2* vprev = K.V + (int64_t)(j - 1) * K.n;
-      GTN_CUDA_TRY(ctx, launch_multidot(vprev, K.n, 2, w, K.n, K.coef, K.part, K.nblk, s, K.part_cap));
-      GTN_CUDA_TRY(ctx, launch_lincomb(w, make_double2(1.0, 0.0), vprev, K.n, 2, K.coef, make_double2(-1.0, 0.0), K.n, s));
-      if (fast_reorth) {
-        GTN_CUDA_TRY(ctx, launch_multidot_f32(K.V, K.n, j + 1, w, K.n, K.coef + 64, K.part, K.nblk, s, K.part_cap));
-        GTN_CUDA_TRY(ctx, launch_reorth_update_f32(w, K.V, K.n, j + 1, K.coef + 64, K.n, s));
-      } else {
-        GTN_CUDA_TRY(ctx, launch_multidot(K.V, K.n, j + 1, w, K.n, K.coef + 64, K.part, K.nblk, s, K.part_cap));
-        GTN_CUDA_TRY(ctx, launch_lincomb(w, make_double2(1.0, 0.0), K.V, K.n, j + 1, K.coef + 64, make_double2(-1.0, 0.0), K.n, s));
-      }
-      ctx->launches += multidot_launch_count(2) + multidot_launch_count(j + 1) + 2;
+    while (queued <= j || (ahead && queued <= j + 1 && queued < kd)) {
+      const int st = lanczos_step(K, queued, queued == j0, precision);
+      if (st != GTN_OK) return st;
+      ++queued;
     }
-    GTN_CUDA_TRY(ctx, norm2_dev(K, w, K.coef + 128));
-    int st2 = fetch(K, K.coef, 130, hbuf);  // h (0..63), h2 (64..127), |w|^2 (128)
-    if (st2 != GTN_OK) return st2;
+    GTN_CUDA_TRY(ctx, cudaEventSynchronize(ctx->step_ev[j & 1]));
+    double2 hbuf[130];
+    std::copy(ctx->h_red + kStepSlot * (1 + (j & 1)), ctx->h_red + kStepSlot * (1 + (j & 1)) + 130, hbuf);
+    int flag = 0;
+    memcpy(&flag, &hbuf[129], sizeof(int));
+    if (flag != 0) {
+      const int st = gtn_ctx_sync(ctx);
+      if (st != GTN_OK) return st;
+    }
+    (*matvecs)++;
+    double hh = 0.0;  // squared norm of the full-pass coefficients (local steps only)
     double nn = hbuf[128].x;
     if (j == j0) {
       a[j] = hbuf[j].x + hbuf[64 + j].x;
@@ -221,15 +258,20 @@ int lanczos_expand(Krylov& K, int j0, int kd, int precision, std::vector<double>
       for (int i = 0; i <= j; ++i) hh += hbuf[64 + i].x * hbuf[64 + i].x + hbuf[64 + i].y * hbuf[64 + i].y;
       if (nn < hh) {
         // DGKS criterion: the pass removed more than half of |w|^2, so V[0..j] and w were far
-        // from orthogonal; repeat it in FP64
+        // from orthogonal; repeat it in FP64 on the normalised w
+        double2* w = K.V + (int64_t)(j + 1) * K.n;
         GTN_CUDA_TRY(ctx, launch_multidot(K.V, K.n, j + 1, w, K.n, K.coef + 64, K.part, K.nblk, s, K.part_cap));
-        GTN_CUDA_TRY(ctx, launch_lincomb(w, make_double2(1.0, 0.0), K.V, K.n, j + 1, K.coef + 64, make_double2(-1.0, 0.0), K.n, s));
-        GTN_CUDA_TRY(ctx, norm2_dev(K, w, K.coef + 128));
-        ctx->launches += multidot_launch_count(j + 1) + 1;
-        st2 = fetch(K, K.coef + 64, 65, hbuf + 64);
-        if (st2 != GTN_OK) return st2;
-        a[j] += hbuf[64 + j].x;
-        nn = hbuf[128].x;
+        GTN_CUDA_TRY(ctx, launch_update(w, K.V, K.n, j + 1, K.coef + 64, K.n, false, K.coef + 128, K.part, K.nblk,
+                                        K.part_cap, ctx->d_errflag, s));
+        ctx->launches += multidot_launch_count(j + 1) + 2;
+        const int st = fetch(K, K.coef + 64, 65, hbuf + 64);
+        if (st != GTN_OK) return st;
+        GTN_CUDA_TRY(ctx, launch_unit_scale(w, K.coef + 128, K.n, s));
+        ctx->launches++;
+        const double scale = nn > 0.0 ? std::sqrt(nn) : 1.0;
+        a[j] += scale * hbuf[64 + j].x;
+        nn = scale * scale * hbuf[128].x;
+        queued = j + 1;
       }
     }
     const double beta = std::sqrt(std::max(nn, 0.0));
@@ -239,8 +281,6 @@ int lanczos_expand(Krylov& K, int j0, int kd, int precision, std::vector<double>
       *breakdown = true;
       break;
     }
-    GTN_CUDA_TRY(ctx, launch_axpby(K.n, make_double2(1.0 / beta, 0.0), w, make_double2(0.0, 0.0), w, s));
-    ctx->launches++;
     if (stop(j + 1, a, b)) {
       m = j + 1;
       break;
@@ -328,7 +368,7 @@ extern "C" int gtn_lanczos_min(gtn_map map, void* xv, int krylovdim, double tol,
       const double r = std::fabs(bb[mm - 1] * QQ[(size_t)(mm - 1) * mm + 0]);
       return small_enough(r, ww[0]);
     };
-    st = lanczos_expand(K, k, kd, map->precision, a, b, &m, &matvecs, &brk, stop);
+    st = lanczos_expand(K, k, kd, map->precision, K.n <= kAheadElems, a, b, &m, &matvecs, &brk, stop);
     if (st != GTN_OK) return st;
     projected_eig(m, k, a, b, s, w, Q);
     theta = w[0];
@@ -374,7 +414,7 @@ extern "C" int gtn_lanczos_min(gtn_map map, void* xv, int krylovdim, double tol,
     st = map_run(map, GTN_PREC_FP64, x, y);
     if (st != GTN_OK) return st;
     matvecs++;
-    GTN_CUDA_TRY(ctx, launch_multidot(x, 0, 1, y, K.n, K.coef + 130, K.part, K.nblk, ctx->stream));
+    GTN_CUDA_TRY(ctx, launch_multidot(x, 0, 1, y, K.n, K.coef + 130, K.part, K.nblk, ctx->stream, K.part_cap));
     ctx->launches += 2;
     double2 h;
     st = fetch(K, K.coef + 130, 1, &h);
@@ -476,7 +516,7 @@ extern "C" int gtn_lanczos_refine(gtn_map map, void* xv, int inner_dim, double t
       return rin <= std::max(tol, 1e-2 * rnorm);
     };
     int mv = 0;
-    st = lanczos_expand(K, 1, m_max, map->precision, a, b, &m, &mv, &brk, stop);
+    st = lanczos_expand(K, 1, m_max, map->precision, K.n <= kAheadElems, a, b, &m, &mv, &brk, stop);
     if (st != GTN_OK) return st;
     mixed_mv += mv;
     a[0] = theta;
@@ -529,7 +569,7 @@ extern "C" int gtn_expm_apply(gtn_map map, double dz_re, double dz_im, void* xv,
     if (beta0 == 0) break;
     int m = 0;
     bool brk = false;
-    st = lanczos_expand(K, 0, kd, map->precision, a, b, &m, &matvecs, &brk,
+    st = lanczos_expand(K, 0, kd, map->precision, true, a, b, &m, &matvecs, &brk,
                         [](int, const std::vector<double>&, const std::vector<double>&) { return false; });
     if (st != GTN_OK) return st;
     tridiag_eig(m, a, b, w, Q);
@@ -636,11 +676,11 @@ int arnoldi_expand(Krylov& K, int kd, int precision, std::vector<cplx>& Hm, int*
     if (st != GTN_OK) return st;
     (*matvecs)++;
     GTN_CUDA_TRY(ctx, launch_multidot(K.V, K.n, j + 1, w, K.n, K.coef, K.part, K.nblk, s, K.part_cap));
-    GTN_CUDA_TRY(ctx, launch_lincomb(w, make_double2(1.0, 0.0), K.V, K.n, j + 1, K.coef, make_double2(-1.0, 0.0), K.n, s));
+    GTN_CUDA_TRY(ctx, launch_update(w, K.V, K.n, j + 1, K.coef, K.n, false, nullptr, nullptr, K.nblk, K.part_cap,
+                                    nullptr, s));
     GTN_CUDA_TRY(ctx, launch_multidot(K.V, K.n, j + 1, w, K.n, K.coef + 64, K.part, K.nblk, s, K.part_cap));
-    GTN_CUDA_TRY(ctx, launch_lincomb(w, make_double2(1.0, 0.0), K.V, K.n, j + 1, K.coef + 64, make_double2(-1.0, 0.0), K.n, s));
-    GTN_CUDA_TRY(ctx, norm2_dev(K, w, K.coef + 128));
-    ctx->launches += 2 * (multidot_launch_count(j + 1) + 1);
+    GTN_CUDA_TRY(ctx, launch_update(w, K.V, K.n, j + 1, K.coef + 64, K.n, false, K.coef + 128, K.part, K.nblk, K.part_cap, ctx->d_errflag, s));
+    ctx->launches += 2 * (multidot_launch_count(j + 1) + 1) + 1;
     double2 hbuf[130];
     st = fetch(K, K.coef, 130, hbuf);
     if (st != GTN_OK) return st;
