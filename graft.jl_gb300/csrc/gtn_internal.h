@@ -97,6 +97,13 @@ bool small_qr_applies(int64_t m, int64_t n);
 // S (k, descending), U (m x k row-major), Vh (k x n row-major), k = min(m, n), on the device.
 bool small_svd_applies(int64_t m, int64_t n);
 int svd_small_launch(gtn_ctx ctx, int64_t m, int64_t n, const double2* A, double* S, double2* U, double2* Vh);
+// One-sided Jacobi SVD over the whole chip (gtn_jacobi.cu), min(m, n) <= 384 and max(m, n) <= 768:
+// run computes all singular values (host, descending), store the leading r vectors from the same
+// workspace of jacobi_svd_bytes.
+bool jacobi_svd_applies(int64_t m, int64_t n);
+size_t jacobi_svd_bytes(int64_t m, int64_t n);
+int jacobi_svd_run(gtn_ctx ctx, int64_t m, int64_t n, const double2* A, void* ws, std::vector<double>* S);
+int jacobi_svd_store(gtn_ctx ctx, int64_t m, int64_t n, void* ws, int64_t r, double2* U, double2* Vh);
 int qr_small(gtn_ctx ctx, int64_t m, int64_t n, const double2* A, double2* Q, double2* R);
 int qr_tall_cholesky(gtn_ctx ctx, int64_t m, int64_t n, const double2* A, double2* Q, double2* R);
 cudaError_t ctx_red(gtn_ctx ctx, size_t n2);   // ensure d_red/h_red hold n2 double2

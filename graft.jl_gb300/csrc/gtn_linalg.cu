@@ -484,6 +484,78 @@ static int orthonormalize_rows(gtn_ctx ctx, int64_t r, int64_t n, double2* Vh) {
   return st;
 }
 
+// Truncated SVD by one-sided Jacobi rotations (gtn_jacobi.cu); a longer side than it holds goes
+// through a thin QR first: the rotations then work on the triangular factor, and U = Q U_R (A^H =
+// Q R for a wide A).  GTN_ERR_UNSUPPORTED where it does not apply.
+static int svd_jacobi(gtn_ctx ctx, int64_t m, int64_t n, const double2* A, int64_t maxdim, double atol, double rtol,
+               double dw, double2* U, double* S, double2* Vh, int64_t* rank, double* discarded) {
+  cudaStream_t s = ctx->stream;
+  const int64_t k = std::min(m, n), lng = std::max(m, n);
+  const bool qr = !jacobi_svd_applies(m, n);
+  const int64_t jm = qr ? k : m, jn = qr ? k : n;
+  if (!jacobi_svd_applies(jm, jn)) return GTN_ERR_UNSUPPORTED;
+  CallBuffers buf(s);
+  void* ws = nullptr;
+  if (qr) ws = buf.get<char>(jacobi_svd_bytes(jm, jn));  // gtn_qr has the context's workspace
+  else GTN_CUDA_TRY(ctx, ctx_workspace(ctx, jacobi_svd_bytes(jm, jn), &ws));
+  double2 *T = nullptr, *Q = nullptr, *R = nullptr, *UR = nullptr, *VR = nullptr;
+  if (qr) {
+    T = buf.get<double2>(m >= n ? 1 : lng * k);  // A^H of a wide A
+    Q = buf.get<double2>(lng * k);
+    R = buf.get<double2>(k * k);
+    UR = buf.get<double2>(k * k);
+    VR = buf.get<double2>(k * k);
+  }
+  if (!ws || (qr && (!T || !Q || !R || !UR || !VR))) return set_err(ctx, GTN_ERR_MEMORY, "svd: staging allocation failed");
+  int st = GTN_OK;
+  const double2* J = A;
+  if (qr) {
+    const double2* X = A;
+    if (m < n) {
+      GTN_CUDA_TRY(ctx, launch_transpose_c128(A, m, n, T, s));
+      GTN_CUDA_TRY(ctx, launch_conj_inplace(T, m * n, s));
+      ctx->launches += 2;
+      X = T;
+    }
+    if ((st = gtn_qr(ctx, lng, k, X, Q, R)) != GTN_OK) return st;
+    J = R;
+  }
+  std::vector<double> hs;
+  if ((st = jacobi_svd_run(ctx, jm, jn, J, ws, &hs)) != GTN_OK) return st;
+  const int64_t r = trunc_rank(hs, maxdim, atol, rtol, dw);
+  // a kept value of zero (or so small that products of its column underflow) needs an orthonormal completion,
+  // and NaN has no order: cuSOLVER's
+  if (!(hs[r - 1] > 1e-60 * hs[0])) return GTN_ERR_UNSUPPORTED;
+  double disc = 0;
+  for (int64_t i = r; i < k; ++i) disc += hs[i] * hs[i];
+  for (int64_t i = 0; i < r; ++i) S[i] = hs[i];
+  *rank = r;
+  if (discarded) *discarded = std::sqrt(disc);
+  if (!qr) {
+    if ((st = jacobi_svd_store(ctx, m, n, ws, r, U, Vh)) != GTN_OK) return st;
+    return gtn_ctx_sync(ctx);
+  }
+  // X = Q R = (Q U_R) S V_R^H with X = A, or A^H: then A = V_R S (Q U_R)^H
+  if ((st = jacobi_svd_store(ctx, k, k, ws, r, UR, VR)) != GTN_OK) return st;
+  const int ranks[2] = {2, 2};
+  const int64_t dims[4] = {lng, k, k, r};
+  const int labels[4] = {-1, 1, 1, -2}, order[2] = {0, 1};
+  const void* ops[2] = {Q, UR};
+  if (m >= n) {
+    if ((st = gtn_contract(ctx, 2, ranks, dims, labels, nullptr, order, ops, U, GTN_PREC_FP64)) != GTN_OK) return st;
+    GTN_CUDA_TRY(ctx, cudaMemcpyAsync(Vh, VR, r * k * sizeof(double2), cudaMemcpyDeviceToDevice, s));
+  } else {
+    double2* L = T;  // Q U_R, n x r
+    if ((st = gtn_contract(ctx, 2, ranks, dims, labels, nullptr, order, ops, L, GTN_PREC_FP64)) != GTN_OK) return st;
+    GTN_CUDA_TRY(ctx, launch_transpose_c128(L, n, r, Vh, s));
+    GTN_CUDA_TRY(ctx, launch_conj_inplace(Vh, r * n, s));
+    GTN_CUDA_TRY(ctx, launch_transpose_c128(VR, r, k, U, s));  // V_R = (V_R^H)^H
+    GTN_CUDA_TRY(ctx, launch_conj_inplace(U, k * r, s));
+    ctx->launches += 4;
+  }
+  return gtn_ctx_sync(ctx);
+}
+
 extern "C" int gtn_svd_trunc(gtn_ctx ctx, int64_t m, int64_t n, const void* A, int64_t maxdim, double atol,
                              double rtol, double discarded_weight, void* U, double* S, void* Vh,
                              int64_t* rank, double* discarded) {
@@ -554,6 +626,11 @@ extern "C" int gtn_svd_trunc(gtn_ctx ctx, int64_t m, int64_t n, const void* A, i
                                         cudaMemcpyDeviceToDevice, s));
     GTN_CUDA_TRY(ctx, cudaMemcpyAsync(Vh, dV, r * n * sizeof(double2), cudaMemcpyDeviceToDevice, s));
     return gtn_ctx_sync(ctx);
+  }
+  if (!(ssv && ssv[0] == '0')) {
+    st = svd_jacobi(ctx, m, n, static_cast<const double2*>(A), maxdim, atol, rtol, discarded_weight,
+                    static_cast<double2*>(U), S, static_cast<double2*>(Vh), rank, discarded);
+    if (st != GTN_ERR_UNSUPPORTED) return st;
   }
   // Column-major problem B (rows >= cols): for n >= m, B = A^T (the same buffer); else B =
   // column-major copy of A (a transpose).
