@@ -58,6 +58,7 @@ struct gtn_blockmap_s {
   void* T[2] = {nullptr, nullptr};
   void* A = nullptr;
   int64_t x_elems = 0, y_elems = 0;
+  int wide = 0;  // a buffer of 2^31 elements or more: 64-bit band offsets
   double flops = 0;
   int n_problems = 0, n_tc = 0;
   // statics B_q [N][K]
@@ -175,7 +176,7 @@ cudaError_t upload_bands(gtn_blockmap bm, const BandSet& bs, int fp64, BMStep* s
   st->band_maxn = bs.maxn;
   st->band_smem = 0;  // the launch's padding and rows per pass follow its largest N
   for (const DevBand& D : bs.bands)
-    st->band_smem = std::max(st->band_smem, block_band_smem(bs.maxn, D.Kq, D.nrect, D.ng, fp64));
+    st->band_smem = std::max(st->band_smem, block_band_smem(bs.maxn, D.Kq, D.nrect, fp64, bm->wide));
   if (bs.bands.empty()) return cudaSuccess;
   auto put = [&](void** dst, const void* src, size_t bytes) {
     cudaError_t e = cudaMalloc(dst, std::max<size_t>(bytes, 16));
@@ -366,7 +367,7 @@ int run(gtn_blockmap bm, const double2* x, double2* y) {
     auto bands = [&](cudaStream_t bs) {
       ctx->launches++;
       return launch_block_band(st.bands, st.bwork, st.nbwork, st.cols, st.rstr, bases, st.src_is64, fp64 ? 1 : 0,
-                               st.band_maxn, st.band_smem, bs);
+                               st.band_maxn, bm->wide, st.band_smem, bs);
     };
     if (fork) {
       e = cudaEventRecord(bm->ev_fork[si], s);
@@ -504,6 +505,7 @@ int gtn_blockmap_create(gtn_ctx ctx, int nsteps, const int* step_ngather, const 
   bm->flops = flops;
   bm->x_elems = buffer_elems[0];
   bm->y_elems = buffer_elems[1];
+  for (int i = 0; i < 4; ++i) bm->wide |= buffer_elems[i] >= ((int64_t)1 << 31);
   const bool fp64 = precision == GTN_PREC_FP64;
   const bool tc = is_tc_p(precision);
   const bool f16 = precision == GTN_PREC_FP16X3;

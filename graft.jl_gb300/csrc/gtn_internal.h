@@ -253,7 +253,7 @@ struct DevBandWork {
 };
 bool block_band_fits(int64_t N, int64_t Kq, int fp64);
 int block_band_rows_per_pass(int maxn);  // rows a CTA covers per pass (one thread per row)
-size_t block_band_smem(int maxn, int Kq, int nrect, int ng, int fp64);
+size_t block_band_smem(int maxn, int Kq, int nrect, int fp64, int wide);
 // Split bands: the slice planes of a tensor-core problem's A_q built band by band (rows of
 // up to 1024 columns staged whole, row maxima reduced in the CTA for fp16), replacing the
 // row-maxima pass, the block moves and the K padding of that problem.
@@ -263,8 +263,9 @@ size_t block_split_band_smem(int Kp, int nrect, int ng, int ncol, int src_is64);
 cudaError_t launch_block_split_band(const DevBand* bands, const DevBandWork* work, int nwork, const DevBandCol* cols,
                                     const int64_t* rstr, const BlockBases& bases, int src_is64, int fp16,
                                     size_t smem, cudaStream_t s);
+// wide: 64-bit element offsets (a source buffer of 2^31 elements or more).
 cudaError_t launch_block_band(const DevBand* bands, const DevBandWork* work, int nwork, const DevBandCol* cols,
-                              const int64_t* rstr, const BlockBases& bases, int src_is64, int fp64, int maxn,
+                              const int64_t* rstr, const BlockBases& bases, int src_is64, int fp64, int maxn, int wide,
                               size_t smem, cudaStream_t s);
 cudaError_t launch_small_grouped(const SmallJob* jobs, int njobs, int is64, cudaStream_t s);
 

@@ -970,7 +970,42 @@ constexpr int kBandMaxN64 = 32, kBandMaxN32 = 64, kBandMaxSmem = 96 * 1024, kBan
 __host__ __device__ constexpr int band_npt(int maxn) { return maxn <= 1 ? 1 : maxn <= 2 ? 2 : maxn <= 4 ? 4 : 8; }
 __host__ __device__ constexpr int band_npad(int n, int npt) { return (n + npt - 1) / npt * npt; }
 
-template <typename Tin, typename T, int NPT>
+// The digits of row m in a band's common groups, and its base offset in rectangle q: O is 32 bits
+// wide where the source buffer has fewer than 2^31 elements: the kernel is bound by its issue
+// slots (73 % taken, DRAM 46 %, at 898 MB read and 238 MB written for N = 4), and 64-bit
+// multiply-adds per group and rectangle and 64-bit offsets per element were most of them (that
+// launch: 308 us with 64-bit offsets, 250 us with 32-bit ones).  Strides are padded with zeros
+// to kBandMaxGroups + 2 per rectangle: eight, read as vectors.
+constexpr int kBandStr = kBandMaxGroups + 2;
+__device__ __forceinline__ void band_digits(uint32_t m, int ng, const uint32_t* sdim, const uint32_t* smag,
+                                            const uint32_t* ssh, int (&dig)[kBandMaxGroups]) {
+#pragma unroll
+  for (int t = kBandMaxGroups - 1; t >= 0; --t) {
+    dig[t] = 0;
+    if (t < ng) {
+      const uint32_t q = sdim[t] == 1u ? m : (__umulhi(m, smag[t]) >> ssh[t]);
+      dig[t] = (int)(m - q * sdim[t]);
+      m = q;
+    }
+  }
+}
+template <typename O>
+__device__ __forceinline__ O band_base(const int (&dig)[kBandMaxGroups], const O* st) {
+  O v[kBandStr];
+#pragma unroll
+  for (int t = 0; t < kBandStr; t += 16 / (int)sizeof(O))
+    *reinterpret_cast<int4*>(v + t) = *reinterpret_cast<const int4*>(st + t);
+  O o = 0;
+#pragma unroll
+  for (int t = 0; t < kBandMaxGroups; ++t) o += (O)dig[t] * v[t];
+  return o;
+}
+template <typename O> struct __align__(16) BandCol {
+  O src;           // element offset of the column
+  int rect, bcol;  // its rectangle's first base offset and its row of B_q, as element indices
+};
+
+template <typename Tin, typename T, int NPT, typename O>
 __global__ void __launch_bounds__(256, 4) block_band_kernel(const DevBand* __restrict__ bands,
                                                             const DevBandWork* __restrict__ work,
                                                             const DevBandCol* __restrict__ cols,
@@ -981,9 +1016,9 @@ __global__ void __launch_bounds__(256, 4) block_band_kernel(const DevBand* __res
   const DevBand& D = bands[W.band];
   const int N = D.N, Kq = D.Kq, ng = D.ng, nrect = D.nrect, ncol = D.ncol, NPAD = band_npad(N, NPT);
   T* Bt = reinterpret_cast<T*>(band_smem);                                // [Kq][NPAD]
-  int64_t* rs = reinterpret_cast<int64_t*>(Bt + (size_t)Kq * NPAD);      // [nrect][ng]
-  int64_t* base = rs + nrect * ng;                                        // [nrect][kBandRows]
-  DevBandCol* cc = reinterpret_cast<DevBandCol*>(base + nrect * kBandRows);  // [ncol]
+  O* rs = reinterpret_cast<O*>(Bt + (Kq * NPAD * (int)sizeof(T) + 15) / 16 * 16 / (int)sizeof(T));  // [nrect][kBandStr]
+  O* base = rs + nrect * kBandStr;                                        // [nrect][kBandRows]
+  BandCol<O>* cc = reinterpret_cast<BandCol<O>*>(base + nrect * kBandRows);  // [ncol]
   __shared__ uint32_t sdim[kBandMaxGroups], smag[kBandMaxGroups], ssh[kBandMaxGroups];
   const int r = threadIdx.x;
   const T* __restrict__ B = static_cast<const T*>(D.B);
@@ -991,8 +1026,14 @@ __global__ void __launch_bounds__(256, 4) block_band_kernel(const DevBand* __res
     const int k = i / NPAD, n = i - k * NPAD;
     Bt[i] = n < N ? B[(size_t)n * Kq + k] : Zero<T>::v();
   }
-  for (int i = r; i < nrect * ng; i += 256) rs[i] = rstr[D.rs0 + i];
-  for (int i = r; i < ncol; i += 256) cc[i] = cols[D.col0 + i];
+  for (int i = r; i < nrect * kBandStr; i += 256) {
+    const int q = i / kBandStr, t = i - q * kBandStr;
+    rs[i] = t < ng ? (O)rstr[D.rs0 + q * ng + t] : (O)0;
+  }
+  for (int i = r; i < ncol; i += 256) {
+    const DevBandCol c = cols[D.col0 + i];
+    cc[i] = BandCol<O>{(O)c.src, c.rect * kBandRows, c.bcol * NPAD};
+  }
   if (r < ng) {
     sdim[r] = D.dim[r];
     smag[r] = D.mag[r];
@@ -1005,24 +1046,9 @@ __global__ void __launch_bounds__(256, 4) block_band_kernel(const DevBand* __res
     const int64_t m = W.m0 + mr;
     {
       int dig[kBandMaxGroups];
-      uint32_t i = (uint32_t)m;
-#pragma unroll
-      for (int t = kBandMaxGroups - 1; t >= 0; --t) {
-        dig[t] = 0;
-        if (t < ng) {
-          const uint32_t q = sdim[t] == 1u ? i : (__umulhi(i, smag[t]) >> ssh[t]);
-          dig[t] = (int)(i - q * sdim[t]);
-          i = q;
-        }
-      }
-      for (int q = 0; q < nrect; ++q) {
-        const int64_t* st = rs + q * ng;
-        int64_t o = 0;
-#pragma unroll
-        for (int t = 0; t < kBandMaxGroups; ++t)
-          if (t < ng) o += (int64_t)dig[t] * st[t];
-        base[q * kBandRows + r] = o;
-      }
+      band_digits((uint32_t)m, ng, sdim, smag, ssh, dig);
+#pragma unroll 1
+      for (int q = 0; q < nrect; ++q) base[q * kBandRows + r] = band_base(dig, rs + q * kBandStr);
     }
     for (int n0 = 0; n0 < N; n0 += NPT) {
       T acc[NPT];
@@ -1036,15 +1062,16 @@ __global__ void __launch_bounds__(256, 4) block_band_kernel(const DevBand* __res
           v[u] = Zero<Tin>::v();
           bc[u] = 0;
           if (j0 + u < ncol) {
-            const DevBandCol c = cc[j0 + u];
+            const BandCol<O> c = cc[j0 + u];
             bc[u] = c.bcol;
-            v[u] = src[c.src + base[c.rect * kBandRows + r]];
+            v[u] = src[c.src + base[c.rect + r]];
           }
         }
 #pragma unroll
         for (int u = 0; u < LB; ++u) {
+          if (j0 + u >= ncol) break;
           const T a = cvt(v[u], (T*)nullptr);
-          const T* bp = Bt + (size_t)bc[u] * NPAD + n0;
+          const T* bp = Bt + bc[u] + n0;
 #pragma unroll
           for (int j = 0; j < NPT; ++j) cfma(acc[j], a, bp[j]);
         }
@@ -1083,11 +1110,29 @@ struct SplitRowWriter {
   }
 };
 
+// q = floor(i / d) for i < 2^31 by a multiply and a shift (Granlund and Montgomery's
+// round-up method, as in decompose_fast); the magic number is made once per CTA.
+struct FastDiv {
+  uint32_t d, mag, sh;
+};
+__device__ __forceinline__ FastDiv make_fastdiv(uint32_t d) {
+  if (d <= 1) return FastDiv{1u, 0u, 0u};
+  uint32_t l = 0;
+  while ((1u << l) < d) ++l;
+  return FastDiv{d, (uint32_t)((1ull << (31 + l)) / d + 1ull), l - 1};
+}
+__device__ __forceinline__ uint32_t fast_div(uint32_t i, const FastDiv& f) {
+  return f.d == 1u ? i : (__umulhi(i, f.mag) >> f.sh);
+}
+
 // Split bands of the tensor-core problems (Kp <= 1024): a CTA stages TR whole rows of A_q
 // (every present column read straight from the running tensor, absent blocks and the K
 // padding zero), reduces the fp16 row maxima over the staged rows, and writes the rows'
 // slice planes with one 8-byte store per plane and column pair.  The values and the split
 // functions are those of the block moves, so the planes equal the staged path's.
+// Latency and issue bound rather than by memory: integer divisions by TR, the column count and
+// Kp / 2 became shifts and multiplications, and a row's maximum is taken by 256 / TR lanes at
+// once instead of a warp per row (Kp = 64 to 128 launches: 87, 198 and 132 us -> 76, 156 and 123).
 // Rows staged per pass: as many as fit 33 KB of the tile, at most 32.
 __host__ __device__ inline int split_band_tr(int Kp, int elem) {
   int tr = 32;
@@ -1104,14 +1149,15 @@ __global__ void __launch_bounds__(256) block_split_band_kernel(const DevBand* __
   const DevBandWork W = work[blockIdx.x];
   const DevBand& D = bands[W.band];
   const int Kp = D.Kp, P = Kp + 1, ng = D.ng, nrect = D.nrect, ncol = D.ncol;
-  const int TR = split_band_tr(Kp, (int)sizeof(Tin));
+  const int TR = split_band_tr(Kp, (int)sizeof(Tin)), lt = 31 - __clz(TR);  // a power of two
+  const FastDiv dcol = make_fastdiv((uint32_t)(ncol > 0 ? ncol : 1)), dhw = make_fastdiv((uint32_t)(Kp / 2));
   Tin* tile = reinterpret_cast<Tin*>(band_smem);                           // [TR][Kp + 1]
   int64_t* rs = reinterpret_cast<int64_t*>(tile + TR * P);                // [nrect][ng]
   int64_t* base = rs + nrect * ng;                                        // [nrect][TR]
   DevBandCol* cc = reinterpret_cast<DevBandCol*>(base + nrect * TR);     // [ncol]
   __shared__ float rmax[32];
   __shared__ uint32_t sdim[kBandMaxGroups], smag[kBandMaxGroups], ssh[kBandMaxGroups];
-  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  const int tid = threadIdx.x;
   for (int i = tid; i < nrect * ng; i += 256) rs[i] = rstr[D.rs0 + i];
   for (int i = tid; i < ncol; i += 256) cc[i] = cols[D.col0 + i];
   if (tid < ng) {
@@ -1128,7 +1174,7 @@ __global__ void __launch_bounds__(256) block_split_band_kernel(const DevBand* __
     __syncthreads();  // (first pass: strides, columns, groups; then the previous pass's tile)
     for (int e = tid; e < TR * P; e += 256) tile[e] = Zero<Tin>::v();
     for (int e = tid; e < TR * nrect; e += 256) {  // row i's base offset in rectangle q
-      const int i = e % TR, q = e / TR;
+      const int i = e & (TR - 1), q = e >> lt;
       uint32_t x = (uint32_t)(m0 + (i < rows ? i : 0));
       int64_t o = 0;
       for (int t = ng - 1; t >= 0; --t) {
@@ -1148,11 +1194,11 @@ __global__ void __launch_bounds__(256) block_split_band_kernel(const DevBand* __
         const int e = e0 + u * 256 + tid;
         int i, j;
         if (D.m_fast) {
-          i = e % TR;
-          j = e / TR;
+          i = e & (TR - 1);
+          j = e >> lt;
         } else {
-          j = e % ncol;
-          i = e / ncol;
+          i = (int)fast_div((uint32_t)e, dcol);
+          j = e - i * ncol;
         }
         slot[u] = -1;
         off[u] = 0;
@@ -1170,21 +1216,21 @@ __global__ void __launch_bounds__(256) block_split_band_kernel(const DevBand* __
         if (slot[u] >= 0) tile[slot[u]] = v[u];
     }
     __syncthreads();
-    if (F16) {  // row maxima, one warp per row
-      for (int i = warp; i < rows; i += 8) {
-        float mx = 0.f;
-        for (int k = lane; k < Kp; k += 32) mx = fmaxf(mx, absmax2(tile[i * P + k]));
-        for (int o = 16; o > 0; o >>= 1) mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, o));
-        if (lane == 0) {
-          rmax[i] = mx;
-          static_cast<float*>(bases.buf[5])[D.amax_off + m0 + i] = mx;
-        }
+    if (F16) {  // row maxima, 256 / TR lanes (at most a warp) per row
+      const int G = TR >= 8 ? 256 >> lt : 32, i = tid / G, l = tid & (G - 1);
+      float mx = 0.f;
+      if (i < rows)
+        for (int k = l; k < Kp; k += G) mx = fmaxf(mx, absmax2(tile[i * P + k]));
+      for (int o = G >> 1; o > 0; o >>= 1) mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, o));
+      if (l == 0 && i < rows) {
+        rmax[i] = mx;
+        static_cast<float*>(bases.buf[5])[D.amax_off + m0 + i] = mx;
       }
       __syncthreads();
     }
     const int hw = Kp / 2;
     for (int e = tid; e < rows * hw; e += 256) {
-      const int i = e / hw, c = 2 * (e - i * hw);
+      const int i = (int)fast_div((uint32_t)e, dhw), c = 2 * (e - i * hw);
       const int64_t m = D.row_off + m0 + i;
       if (F16) {
         Split16RowWriter w{out, ld2, D.pstride};
@@ -1252,21 +1298,6 @@ __device__ __forceinline__ void cp_async_el(double2* dst, const double2* src) {
                : "memory");
 }
 __device__ __forceinline__ void cp_async_wait_all() { asm volatile("cp.async.wait_all;" ::: "memory"); }
-
-// q = floor(i / d) for i < 2^31 by a multiply and a shift (Granlund and Montgomery's
-// round-up method, as in decompose_fast); the magic number is made once per CTA.
-struct FastDiv {
-  uint32_t d, mag, sh;
-};
-__device__ __forceinline__ FastDiv make_fastdiv(uint32_t d) {
-  if (d <= 1) return FastDiv{1u, 0u, 0u};
-  uint32_t l = 0;
-  while ((1u << l) < d) ++l;
-  return FastDiv{d, (uint32_t)((1ull << (31 + l)) / d + 1ull), l - 1};
-}
-__device__ __forceinline__ uint32_t fast_div(uint32_t i, const FastDiv& f) {
-  return f.d == 1u ? i : (__umulhi(i, f.mag) >> f.sh);
-}
 
 template <typename Tin> __host__ __device__ constexpr int split_rows_pitch(int kc) { return kc | 1; }
 template <typename Tin> __host__ __device__ constexpr size_t split_rows_smem(int TR, int kc) {
@@ -1498,10 +1529,11 @@ cudaError_t launch_block_gather(const DevGatherJob* jobs, const int2* tile_map, 
   return cudaGetLastError();
 }
 
-size_t block_band_smem(int maxn, int Kq, int nrect, int ng, int fp64) {
+size_t block_band_smem(int maxn, int Kq, int nrect, int fp64, int wide) {
   const size_t e = fp64 ? sizeof(double2) : sizeof(float2);
-  return (size_t)Kq * band_npad(maxn, band_npt(maxn)) * e + (size_t)nrect * ng * sizeof(int64_t) +
-         (size_t)nrect * kBandRows * sizeof(int64_t) + (size_t)Kq * sizeof(DevBandCol);
+  return ((size_t)Kq * band_npad(maxn, band_npt(maxn)) * e + 15) / 16 * 16 +
+         (size_t)nrect * (kBandStr + kBandRows) * (wide ? sizeof(int64_t) : sizeof(int32_t)) +
+         (size_t)Kq * sizeof(BandCol<int64_t>);
 }
 
 int block_band_rows_per_pass(int) { return kBandRows; }
@@ -1511,44 +1543,50 @@ int block_band_rows_per_pass(int) { return kBandRows; }
 bool block_band_fits(int64_t N, int64_t Kq, int fp64) {
   const int nmax = fp64 ? kBandMaxN64 : kBandMaxN32;
   if (N < 1 || Kq < 1 || N > nmax || Kq > 4096) return false;
-  return block_band_smem(nmax, (int)Kq, kBandMaxRects, kBandMaxGroups, fp64) <= (size_t)kBandMaxSmem;
+  return block_band_smem(nmax, (int)Kq, kBandMaxRects, fp64, 1) <= (size_t)kBandMaxSmem;
 }
 
 namespace {
-template <typename Tin, typename T, int NPT>
+template <typename Tin, typename T, int NPT, typename O>
 cudaError_t launch_band_t(const DevBand* bands, const DevBandWork* work, int nwork, const DevBandCol* cols,
                           const int64_t* rstr, const BlockBases& bases, size_t smem, cudaStream_t s) {
   static bool attr_set = false;
   if (!attr_set) {
-    cudaError_t e = cudaFuncSetAttribute(block_band_kernel<Tin, T, NPT>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+    cudaError_t e = cudaFuncSetAttribute(block_band_kernel<Tin, T, NPT, O>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                          kBandMaxSmem);
     if (e != cudaSuccess) return e;
     attr_set = true;
   }
-  block_band_kernel<Tin, T, NPT><<<nwork, 256, smem, s>>>(bands, work, cols, rstr, bases);
+  block_band_kernel<Tin, T, NPT, O><<<nwork, 256, smem, s>>>(bands, work, cols, rstr, bases);
   return cudaGetLastError();
 }
-
-template <typename Tin, typename T>
-cudaError_t launch_band_n(const DevBand* bands, const DevBandWork* work, int nwork, const DevBandCol* cols,
+template <typename Tin, typename T, typename O>
+cudaError_t launch_band_o(const DevBand* bands, const DevBandWork* work, int nwork, const DevBandCol* cols,
                           const int64_t* rstr, const BlockBases& bases, int maxn, size_t smem, cudaStream_t s) {
   switch (band_npt(maxn)) {
-    case 1: return launch_band_t<Tin, T, 1>(bands, work, nwork, cols, rstr, bases, smem, s);
-    case 2: return launch_band_t<Tin, T, 2>(bands, work, nwork, cols, rstr, bases, smem, s);
-    case 4: return launch_band_t<Tin, T, 4>(bands, work, nwork, cols, rstr, bases, smem, s);
-    default: return launch_band_t<Tin, T, 8>(bands, work, nwork, cols, rstr, bases, smem, s);
+    case 1: return launch_band_t<Tin, T, 1, O>(bands, work, nwork, cols, rstr, bases, smem, s);
+    case 2: return launch_band_t<Tin, T, 2, O>(bands, work, nwork, cols, rstr, bases, smem, s);
+    case 4: return launch_band_t<Tin, T, 4, O>(bands, work, nwork, cols, rstr, bases, smem, s);
+    default: return launch_band_t<Tin, T, 8, O>(bands, work, nwork, cols, rstr, bases, smem, s);
   }
+}
+template <typename Tin, typename T>
+cudaError_t launch_band_n(const DevBand* bands, const DevBandWork* work, int nwork, const DevBandCol* cols,
+                          const int64_t* rstr, const BlockBases& bases, int maxn, int wide, size_t smem,
+                          cudaStream_t s) {
+  return wide ? launch_band_o<Tin, T, int64_t>(bands, work, nwork, cols, rstr, bases, maxn, smem, s)
+              : launch_band_o<Tin, T, int32_t>(bands, work, nwork, cols, rstr, bases, maxn, smem, s);
 }
 }  // namespace
 
 cudaError_t launch_block_band(const DevBand* bands, const DevBandWork* work, int nwork, const DevBandCol* cols,
-                              const int64_t* rstr, const BlockBases& bases, int src_is64, int fp64, int maxn,
+                              const int64_t* rstr, const BlockBases& bases, int src_is64, int fp64, int maxn, int wide,
                               size_t smem, cudaStream_t s) {
   if (nwork <= 0) return cudaSuccess;
   if (smem > (size_t)kBandMaxSmem || maxn > (fp64 ? kBandMaxN64 : kBandMaxN32)) return cudaErrorInvalidValue;
-  if (fp64) return launch_band_n<double2, double2>(bands, work, nwork, cols, rstr, bases, maxn, smem, s);
-  if (src_is64) return launch_band_n<double2, float2>(bands, work, nwork, cols, rstr, bases, maxn, smem, s);
-  return launch_band_n<float2, float2>(bands, work, nwork, cols, rstr, bases, maxn, smem, s);
+  if (fp64) return launch_band_n<double2, double2>(bands, work, nwork, cols, rstr, bases, maxn, wide, smem, s);
+  if (src_is64) return launch_band_n<double2, float2>(bands, work, nwork, cols, rstr, bases, maxn, wide, smem, s);
+  return launch_band_n<float2, float2>(bands, work, nwork, cols, rstr, bases, maxn, wide, smem, s);
 }
 
 int block_split_band_rows(int Kp, int src_is64) { return split_band_tr(Kp, src_is64 ? 16 : 8); }
