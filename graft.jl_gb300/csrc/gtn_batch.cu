@@ -182,9 +182,8 @@ int map_run_batched(gtn_map* maps_in, int n, int precision, const double2* const
       ctx->launches += (int64_t)((gemm.size() + kGemmJobMax - 1) / kGemmJobMax);
     }
     if (e == cudaSuccess && !tcp.empty()) {
-      std::stable_sort(tcp.begin(), tcp.end(), [](const TcGemmArgs& a, const TcGemmArgs& b) { return a.Kp > b.Kp; });
       e = launch_tc_gemm_grouped(tcp.data(), (int)tcp.size(), ctx->d_errflag, s, &why);
-      ctx->launches += (int64_t)((tcp.size() + 55) / 56);
+      ctx->launches += (int64_t)((tcp.size() + kTcGroupMax - 1) / kTcGroupMax);
     }
     if (e != cudaSuccess)
       return set_err(ctx, GTN_ERR_CUDA, "batched step " + std::to_string(si) + ": " + why + " " + cudaGetErrorString(e));

@@ -393,7 +393,7 @@ int run(gtn_blockmap bm, const double2* x, double2* y) {
     }
     if (e == cudaSuccess && !st.tcp.empty()) {
       e = launch_tc_gemm_grouped(st.tcp.data(), (int)st.tcp.size(), ctx->d_errflag, s, &why);
-      ctx->launches += (int64_t)((st.tcp.size() + 55) / 56);
+      ctx->launches += (int64_t)((st.tcp.size() + kTcGroupMax - 1) / kTcGroupMax);
     }
     if (e == cudaSuccess && !st.simt.empty()) {
       e = launch_gemm_simt_grouped(st.simt.data(), (int)st.simt.size(), fp64 ? 1 : 0, s);
@@ -754,7 +754,6 @@ int gtn_blockmap_create(gtn_ctx ctx, int nsteps, const int* step_ngather, const 
       }
       bm->n_problems++;
     }
-    std::stable_sort(st.tcp.begin(), st.tcp.end(), [](const TcGemmArgs& a, const TcGemmArgs& b) { return a.Kp > b.Kp; });
     st.src_is64 = (s == 0 || fp64) ? 1 : 0;
     if (upload_jobs(bm, jobs, &st) != cudaSuccess) return fail(GTN_ERR_CUDA, "job table upload");
     if (upload_bands(bm, step_bands[s], fp64 ? 1 : 0, &st) != cudaSuccess ||

@@ -25,6 +25,7 @@
 #include <map>
 #include <mutex>
 #include <tuple>
+#include <vector>
 
 namespace {
 using namespace gtn_tc;
@@ -32,8 +33,6 @@ using namespace gtn_tc;
 constexpr int BM = 128;
 constexpr int BKE = 64;  // bf16 elements per k-block = 128 bytes = one SW128 row
 constexpr int A_BYTES = BM * BKE * 2;
-
-constexpr int kTcGroupMax = 56;
 
 struct ProdList {
   int n;
@@ -226,6 +225,42 @@ struct PlaneScales {
   int fp16;
 };
 
+// Columns c0 .. c1 - 1 (multiples of 16) of a tile's lead and correction accumulators (TMEM
+// addresses tlead, tcorr of this warp's lane quarter) summed, scaled and stored to row m of C:
+// W columns of both at a time, loaded together and waited for once.  The epilogue is a chain
+// of TMEM round trips: at 16 columns with a wait after each load it took four times as many,
+// which held back the steps of short K (see the persistent kernel).  Reads up to W - 16 columns past c1 (not stored).
+template <int W>
+__device__ __forceinline__ void drain_columns(uint32_t tlead, uint32_t tcorr, bool has_corr, int c0, int c1, int r0,
+                                              float2* __restrict__ C, int64_t M, int64_t N, int64_t m, float ainv,
+                                              const float* binv) {
+  const int64_t nend = (int64_t)(r0 + c1) >> 1 < N ? (int64_t)(r0 + c1) >> 1 : N;
+#pragma unroll 1
+  for (int c = c0; c < c1; c += W) {
+    uint32_t v[W], w[W];
+    tmem_ld_async<W>(tlead + (uint32_t)c, v);
+    if (has_corr) {
+      tmem_ld_async<W>(tcorr + (uint32_t)c, w);
+    } else {
+#pragma unroll
+      for (int j = 0; j < W; ++j) w[j] = 0u;
+    }
+    tmem_ld_wait<W>(v, w);
+    if (m < M) {
+      const int64_t nb = (int64_t)(r0 + c) >> 1;
+      const int nv = (int)(nend - nb < W / 2 ? nend - nb : W / 2);
+      float2* out = C + nb * M + m;
+#pragma unroll
+      for (int j = 0; j < W / 2; ++j)
+        if (j < nv) {
+          const float f = binv ? ainv * binv[((c - c0) >> 1) + j] : ainv;
+          out[(int64_t)j * M] = make_float2((__uint_as_float(v[2 * j]) + __uint_as_float(w[2 * j])) * f,
+                                            (__uint_as_float(v[2 * j + 1]) + __uint_as_float(w[2 * j + 1])) * f);
+        }
+    }
+  }
+}
+
 template <int BN, int P, int CPS>
 __device__ __forceinline__ void tc_tile_ps(const CUtensorMap* tmA, const CUtensorMap* tmB, float2* __restrict__ C,
                                            int64_t M, int64_t N, int nkb, const ProdList& prods, int m0, int r0,
@@ -345,29 +380,8 @@ __device__ __forceinline__ void tc_tile_ps(const CUtensorMap* tmA, const CUtenso
     bool has_corr = false;
     for (int q = 0; q < prods.n; ++q) has_corr |= !(prods.a[q] == 0 && prods.b[q] == 0);
     const float ainv = (sc.amax && m < M) ? fp16_row_scale_inv(sc.amax[m]) : 1.0f;
-#pragma unroll 1
-    for (int c = c0; c < c0 + BN / 2; c += 16) {
-      uint32_t v[16], w[16];
-      tmem_ld16(taddr + (uint32_t)c, v);
-      if (has_corr) {
-        tmem_ld16(taddr + CF::ACC_COLS + (uint32_t)c, w);
-      } else {
-#pragma unroll
-        for (int j = 0; j < 16; ++j) w[j] = 0u;
-      }
-      if (m < M) {
-        const int64_t nb = (int64_t)(r0 + c) >> 1;
-#pragma unroll
-        for (int j = 0; j < 8; ++j) {
-          const int64_t n = nb + j;
-          if (n < N) {
-            const float f = sc.bmax ? ainv * s_binv[(c >> 1) + j] : ainv;
-            C[n * M + m] = make_float2((__uint_as_float(v[2 * j]) + __uint_as_float(w[2 * j])) * f,
-                                       (__uint_as_float(v[2 * j + 1]) + __uint_as_float(w[2 * j + 1])) * f);
-          }
-        }
-      }
-    }
+    drain_columns<(BN < 64 ? 16 : 32)>(taddr, taddr + CF::ACC_COLS, has_corr, c0, c0 + BN / 2, r0, C, M, N, m, ainv,
+                                       sc.bmax ? s_binv + (c0 >> 1) : nullptr);
   }
   fence_before();
   __syncthreads();
@@ -626,29 +640,8 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(128, 1)
     bool has_corr = false;
     for (int q = 0; q < prods.n; ++q) has_corr |= !(prods.a[q] == 0 && prods.b[q] == 0);
     const float ainv = (sc.amax && m < M) ? fp16_row_scale_inv(sc.amax[m]) : 1.0f;
-#pragma unroll 1
-    for (int c = 0; c < CF::TILE_N; c += 16) {
-      uint32_t v[16], w[16];
-      tmem_ld16(taddr + (uint32_t)c, v);
-      if (has_corr) {
-        tmem_ld16(taddr + CF::ACC_COLS + (uint32_t)c, w);
-      } else {
-#pragma unroll
-        for (int j = 0; j < 16; ++j) w[j] = 0u;
-      }
-      if (m < M) {
-        const int64_t nb = (int64_t)(n0 + c) >> 1;
-#pragma unroll
-        for (int j = 0; j < 8; ++j) {
-          const int64_t n = nb + j;
-          if (n < N) {
-            const float f = sc.bmax ? ainv * s_binv[(c >> 1) + j] : ainv;
-            C[n * M + m] = make_float2((__uint_as_float(v[2 * j]) + __uint_as_float(w[2 * j])) * f,
-                                       (__uint_as_float(v[2 * j + 1]) + __uint_as_float(w[2 * j + 1])) * f);
-          }
-        }
-      }
-    }
+    drain_columns<32>(taddr, taddr + CF::ACC_COLS, has_corr, 0, CF::TILE_N, n0, C, M, N, m, ainv,
+                      sc.bmax ? s_binv : nullptr);
   }
   fence_before();
   __syncthreads();
@@ -680,73 +673,95 @@ __global__ void __launch_bounds__(128, 1)
               errflag);
 }
 
-// Many independent problems in one launch: CTA b works on tile b - tile_start[p] of the
-// problem p whose tile range holds b (problems listed largest K first).
-struct GroupedTc {
-  CUtensorMap tmA[kTcGroupMax];
-  CUtensorMap tmB[kTcGroupMax];
-  float2* C[kTcGroupMax];
-  int64_t M[kTcGroupMax];
-  int64_t N[kTcGroupMax];
-  int nkb[kTcGroupMax];
-  int tiles_n[kTcGroupMax];
-  int tile_start[kTcGroupMax + 1];
-  const float* amax[kTcGroupMax];
-  const float* bmax[kTcGroupMax];
+// Up to G independent problems of one launch, the costliest tiles first; tile t belongs to
+// the problem p whose range tile_start[p] .. tile_start[p + 1] holds it.  A launch of one
+// problem passes 0.4 KB of parameters (G = 1), a group 20 KB.
+template <int G> struct GroupedTc {
+  CUtensorMap tmA[G];
+  CUtensorMap tmB[G];
+  float2* C[G];
+  int64_t M[G];
+  int64_t N[G];
+  int nkb[G];
+  int tiles_n[G];
+  int bw[G];  // real columns per tile
+  int tile_start[G + 1];
+  const float* amax[G];
+  const float* bmax[G];
   int nprob;
   int fp16;
   ProdList prods;
 };
 
-template <int BN, int P>
-__global__ void __launch_bounds__(kPsThreads, 1) tc_gemm_grouped_ps_kernel(const __grid_constant__ GroupedTc g,
-                                                                    int* __restrict__ errflag) {
-  constexpr int CPS = 1;
-  const int b = blockIdx.x;
-  int p = 0;
-  while (p + 1 < g.nprob && g.tile_start[p + 1] <= b) ++p;
-  const int t = b - g.tile_start[p];
-  const int tn = t % g.tiles_n[p], tm = t / g.tiles_n[p];  // N tile fastest
-  const PlaneScales sc{g.amax[p], g.bmax[p], g.fp16};
-  tc_tile_ps<BN, P, CPS>(&g.tmA[p], &g.tmB[p], g.C[p], g.M[p], g.N[p], g.nkb[p], g.prods, tm * BM, tn * BN, errflag,
-                         sc);
-}
-
 // ---- persistent grouped kernel -----------------------------------------------------------
 // One launch of at most one CTA per SM runs every tile of every problem of the group (the
-// coupled-charge GEMMs of a block-sparse step, or one dense problem): CTA c takes tiles c,
-// c + grid, ...  Six warps with fixed roles:
+// coupled-charge GEMMs of a block-sparse step, or one dense problem); persist_tile deals
+// them.  Ten warps with fixed roles:
 //   warp 0 (one lane) : TMA producer over the CTA's (tile, k-block) sequence, one ring of
 //                       stages shared by all its tiles (no pipeline drain between tiles)
 //   warp 1 (one lane) : MMA issuer; warp 1 also allocates and frees TMEM
 //   warps 2-9         : epilogue; warp w reads TMEM lanes 32 (w % 4) .. + 31 and one half of
 //                       the tile's columns (two warps per lane quarter keep twice the
 //                       TMEM loads and stores in flight)
-// With 128-wide (or narrower) tiles TMEM holds two accumulator sets (lead + corrections
-// each), so the epilogue of tile i runs while the MMAs of tile i + 1 proceed; 256-wide tiles
-// fill TMEM with one set.  Accumulator hand-off: full barriers (one MMA commit) and empty
+// TMEM holds two accumulator sets (lead + corrections each) of 128 columns at most, so the
+// epilogue of tile i runs while the MMAs of tile i + 1 proceed; a tile wider than that takes
+// both sets (AccSets).  Step 1 of the two-site map at bond 1024 (M = 262144, 2N = 1280,
+// K = 128) went from 674 to 602 us with the wider drain and to 554 with both sets in use.  A problem's 2N columns are cut into tiles of equal width (the
+// narrowest multiple of 16 that takes no more tiles than BN does), so that a ragged N costs
+// no padding: 2N = 280 runs as two tiles of 144 columns instead of two of 256.  Every MMA of
+// a tile has that N and every stage loads that many rows of B'.  Accumulator hand-off: full barriers (one MMA commit) and empty
 // barriers (one arrival per epilogue warp).  Every wait is bounded as in tc_tile_ps.
 template <int BN, int P> struct CfgPersist {
   using Base = Cfg2<BN, P, 1>;
   static constexpr int STAGE_BYTES = Base::STAGE_BYTES;
   static constexpr int STAGES = Base::STAGES;
   static constexpr int SMEM = Base::SMEM;
-  static constexpr uint32_t ACC_COLS = Base::ACC_COLS;
-  static constexpr int NACC = (4 * ACC_COLS <= 512) ? 2 : 1;  // accumulator sets
-  static constexpr uint32_t TMEM_COLS = (uint32_t)NACC * 2 * ACC_COLS;
+  static constexpr uint32_t ACC_COLS = Base::ACC_COLS < 128 ? Base::ACC_COLS : 128;  // of a narrow tile
+  static constexpr uint32_t TMEM_COLS = 4 * ACC_COLS;
 };
 
-__device__ __forceinline__ int find_problem(const GroupedTc& g, int t) {
-  int p = 0;
-  while (p + 1 < g.nprob && g.tile_start[p + 1] <= t) ++p;
+// The accumulator sets in the order of a CTA's tiles, as the MMA issuer and every epilogue warp
+// count them: narrow tiles alternate between the two, a wide one takes both.  Its lead
+// accumulator is columns `lead` .., its corrections columns lead + corr ..
+struct AccSets {
+  uint32_t use[2] = {0u, 0u};  // tiles that have used each set
+  int next = 0;
+  bool s[2];  // sets of the present tile
+  uint32_t lead, corr;
+  template <class CF> __device__ __forceinline__ void take(int bw) {
+    const bool wide = (uint32_t)bw > CF::ACC_COLS;
+    s[0] = wide || next == 0;
+    s[1] = wide || next == 1;
+    lead = !wide && next == 1 ? 2 * CF::ACC_COLS : 0u;
+    corr = wide ? 2 * CF::ACC_COLS : CF::ACC_COLS;
+    next = wide ? 0 : next ^ 1;
+  }
+  __device__ __forceinline__ void done() {
+    use[0] += s[0];
+    use[1] += s[1];
+  }
+};
+
+// The problem of tile t, searched from p on: a CTA's tiles come in ascending order, so each
+// role walks the list once instead of once per tile.
+template <int G> __device__ __forceinline__ int find_problem(const GroupedTc<G>& g, int t, int p) {
+  while (G > 1 && p + 1 < g.nprob && g.tile_start[p + 1] <= t) ++p;
   return p;
+}
+
+// The i-th tile of this CTA: waves of gridDim.x tiles, every second one dealt in reverse.
+// The tiles are sorted by cost, so the CTA with the costliest tile of a wave has the cheapest
+// of the next (64 uneven one-site maps: the long step 304 -> 278 us, the others 134 -> 125 and
+// 44 -> 38).
+__device__ __forceinline__ int persist_tile(int i) {
+  return i * (int)gridDim.x + ((i & 1) ? (int)gridDim.x - 1 - (int)blockIdx.x : (int)blockIdx.x);
 }
 
 constexpr int kPersistEpiWarps = 8;
 constexpr int kPersistThreads = 32 * (2 + kPersistEpiWarps);
 
-template <int BN, int P>
-__global__ void __launch_bounds__(kPersistThreads, 1) tc_gemm_persist_kernel(const __grid_constant__ GroupedTc g,
+template <int BN, int P, int G>
+__global__ void __launch_bounds__(kPersistThreads, 1) tc_gemm_persist_kernel(const __grid_constant__ GroupedTc<G> g,
                                                                              int* __restrict__ errflag) {
   using CF = CfgPersist<BN, P>;
   using B2 = Cfg2<BN, P, 1>;
@@ -757,7 +772,7 @@ __global__ void __launch_bounds__(kPersistThreads, 1) tc_gemm_persist_kernel(con
   __shared__ __align__(8) uint64_t empty_bar[CF::STAGES];
   __shared__ __align__(8) uint64_t accf_bar[2];
   __shared__ __align__(8) uint64_t acce_bar[2];
-  __shared__ float s_binv[kPersistEpiWarps][BN / 4 > 0 ? BN / 4 : 1];
+  __shared__ float s_binv[kPersistEpiWarps][BN / 4];
   __shared__ uint32_t tmem_slot;
   __shared__ volatile int abort_flag;
   __shared__ int n_issued, n_consumed;
@@ -792,10 +807,10 @@ __global__ void __launch_bounds__(kPersistThreads, 1) tc_gemm_persist_kernel(con
   if (warp == 0 && lane == 0) {
     int gk = 0;
     bool stop = false;
-    for (int t = blockIdx.x; t < total && !stop; t += gridDim.x) {
-      const int p = find_problem(g, t);
+    for (int i = 0, p = 0, t; (t = persist_tile(i)) < total && !stop; ++i) {
+      p = find_problem(g, t, p);
       const int tl = t - g.tile_start[p];
-      const int m0 = (tl / g.tiles_n[p]) * BM, r0 = (tl % g.tiles_n[p]) * BN;
+      const int bw = g.bw[p], m0 = (tl / g.tiles_n[p]) * BM, r0 = (tl % g.tiles_n[p]) * bw;
       asm volatile("prefetch.tensormap [%0];" ::"l"(reinterpret_cast<uint64_t>(&g.tmA[p])) : "memory");
       asm volatile("prefetch.tensormap [%0];" ::"l"(reinterpret_cast<uint64_t>(&g.tmB[p])) : "memory");
       for (int kb = 0; kb < g.nkb[p]; ++kb, ++gk) {
@@ -809,7 +824,7 @@ __global__ void __launch_bounds__(kPersistThreads, 1) tc_gemm_persist_kernel(con
         }
         const uint32_t sa = smem_u32(smem + s * CF::STAGE_BYTES);
         const uint32_t sb = sa + P * B2::A_PLANE;
-        mbar_expect_tx(&full_bar[s], CF::STAGE_BYTES);
+        mbar_expect_tx(&full_bar[s], (uint32_t)(P * (B2::A_PLANE + bw * BKE2 * 2)));
 #pragma unroll
         for (int pl = 0; pl < P; ++pl) {
           tma_load_3d(sa + pl * B2::A_PLANE, &g.tmA[p], &full_bar[s], kb * BKE2, m0, pl);
@@ -819,20 +834,23 @@ __global__ void __launch_bounds__(kPersistThreads, 1) tc_gemm_persist_kernel(con
     }
     n_issued = gk;
   } else if (warp == 1 && lane == 0) {
-    const uint32_t idesc = g.fp16 ? idesc_f16(BM, BN) : idesc_bf16(BM, BN);
-    int gk = 0, i = 0;
+    int gk = 0;
     bool stop = false;
-    for (int t = blockIdx.x; t < total && !stop; t += gridDim.x, ++i) {
-      const int p = find_problem(g, t);
-      const int b = i % CF::NACC;
-      const uint32_t use = (uint32_t)(i / CF::NACC);
-      if (!mbar_wait(&acce_bar[b], (use & 1u) ^ 1u, &abort_flag)) {  // the epilogue freed set b
+    AccSets acc;
+    for (int i = 0, p = 0, t; (t = persist_tile(i)) < total && !stop; ++i) {
+      p = find_problem(g, t, p);
+      const uint32_t idesc = g.fp16 ? idesc_f16(BM, g.bw[p]) : idesc_bf16(BM, g.bw[p]);
+      acc.take<CF>(g.bw[p]);
+      bool free = true;  // the epilogue has freed the tile's sets
+      for (int b = 0; b < 2; ++b)
+        free = free && (!acc.s[b] || mbar_wait(&acce_bar[b], (acc.use[b] & 1u) ^ 1u, &abort_flag));
+      if (!free) {
         abort_flag = 1;
         atomicCAS(errflag, 0, DEVERR_MMA_TIMEOUT);
         break;
       }
       fence_after();
-      const uint32_t dlead = tmem_base + (uint32_t)b * 2u * CF::ACC_COLS, dcorr = dlead + CF::ACC_COLS;
+      const uint32_t dlead = tmem_base + acc.lead, dcorr = dlead + acc.corr;
       bool lead_started = false, corr_started = false;
       for (int kb = 0; kb < g.nkb[p]; ++kb, ++gk) {
         const int s = gk % CF::STAGES;
@@ -859,23 +877,39 @@ __global__ void __launch_bounds__(kPersistThreads, 1) tc_gemm_persist_kernel(con
         }
         umma_commit(&empty_bar[s]);
       }
-      umma_commit(&accf_bar[b]);  // set b complete once every MMA issued so far has
+      for (int b = 0; b < 2; ++b)
+        if (acc.s[b]) umma_commit(&accf_bar[b]);  // complete once every MMA issued so far is
+      acc.done();
     }
     n_consumed = gk;
   } else if (warp >= 2) {
     const int q4 = warp & 3;                // TMEM lane quarter of this warp
-    const int c0 = ((warp - 2) >> 2) * (BN / 2);  // its half of the tile's columns
-    int i = 0;
+    const int half = (warp - 2) >> 2;       // its half of the tile's columns
     bool has_corr = false;
     for (int q = 0; q < g.prods.n; ++q) has_corr |= !(g.prods.a[q] == 0 && g.prods.b[q] == 0);
-    for (int t = blockIdx.x; t < total; t += gridDim.x, ++i) {
-      const int p = find_problem(g, t);
+    AccSets acc;
+    for (int i = 0, p = 0, t; (t = persist_tile(i)) < total; ++i) {
+      p = find_problem(g, t, p);
       const int tl = t - g.tile_start[p];
-      const int m0 = (tl / g.tiles_n[p]) * BM, r0 = (tl % g.tiles_n[p]) * BN;
-      const int b = i % CF::NACC;
-      const uint32_t use = (uint32_t)(i / CF::NACC);
-      const bool ok = mbar_wait(&accf_bar[b], use & 1u, &abort_flag);
-      if (!ok) {
+      const int bw = g.bw[p], m0 = (tl / g.tiles_n[p]) * BM, r0 = (tl % g.tiles_n[p]) * bw;
+      const int64_t M = g.M[p], N = g.N[p];
+      const int h1 = (bw / 16 + 1) / 2 * 16, c0 = half ? h1 : 0, c1 = half ? bw : h1;
+      const int64_t m = (int64_t)m0 + q4 * 32 + lane;
+      // scales: this row's, and this warp's copy of its columns' (read once per tile, before the wait)
+      const float ainv = (g.amax[p] && m < M) ? fp16_row_scale_inv(g.amax[p][m]) : 1.0f;
+      const float* bmx = g.bmax[p];
+      float* binv = s_binv[warp - 2];
+      if (bmx) {
+        for (int t = lane; t < (c1 - c0) / 2; t += 32) {
+          const int64_t n = (int64_t)((r0 + c0) >> 1) + t;
+          binv[t] = n < N ? fp16_row_scale_inv(bmx[n]) : 1.0f;
+        }
+      }
+      acc.take<CF>(bw);
+      bool full = true;
+      for (int b = 0; b < 2; ++b)
+        full = full && (!acc.s[b] || mbar_wait(&accf_bar[b], acc.use[b] & 1u, &abort_flag));
+      if (!full) {
         if (lane == 0) {
           abort_flag = 1;
           atomicCAS(errflag, 0, DEVERR_EPI_TIMEOUT);
@@ -884,48 +918,14 @@ __global__ void __launch_bounds__(kPersistThreads, 1) tc_gemm_persist_kernel(con
       }
       __syncwarp();
       fence_after();
-      const int64_t M = g.M[p], N = g.N[p];
-      float2* __restrict__ C = g.C[p];
-      const int row = q4 * 32 + lane;
-      const int64_t m = (int64_t)m0 + row;
-      const uint32_t taddr = tmem_base + (uint32_t)b * 2u * CF::ACC_COLS + ((uint32_t)(q4 * 32) << 16);
-      const float ainv = (g.amax[p] && m < M) ? fp16_row_scale_inv(g.amax[p][m]) : 1.0f;
-      const float* bmx = g.bmax[p];
-      // this warp's copy of its columns' inverse scales (read once per tile)
-      float* binv = s_binv[warp - 2];
-      if (bmx) {
-        for (int t = lane; t < BN / 4; t += 32) {
-          const int64_t n = (int64_t)((r0 + c0) >> 1) + t;
-          binv[t] = n < N ? fp16_row_scale_inv(bmx[n]) : 1.0f;
-        }
-        __syncwarp();
-      }
-#pragma unroll 1
-      for (int c = c0; c < c0 + BN / 2; c += 16) {
-        uint32_t v[16], w[16];
-        tmem_ld16(taddr + (uint32_t)c, v);
-        if (has_corr) {
-          tmem_ld16(taddr + CF::ACC_COLS + (uint32_t)c, w);
-        } else {
-#pragma unroll
-          for (int j = 0; j < 16; ++j) w[j] = 0u;
-        }
-        if (m < M) {
-          const int64_t nb = (int64_t)(r0 + c) >> 1;
-#pragma unroll
-          for (int j = 0; j < 8; ++j) {
-            const int64_t n = nb + j;
-            if (n < N) {
-              const float f = bmx ? ainv * binv[((c - c0) >> 1) + j] : ainv;
-              C[n * M + m] = make_float2((__uint_as_float(v[2 * j]) + __uint_as_float(w[2 * j])) * f,
-                                         (__uint_as_float(v[2 * j + 1]) + __uint_as_float(w[2 * j + 1])) * f);
-            }
-          }
-        }
-      }
+      const uint32_t taddr = tmem_base + acc.lead + ((uint32_t)(q4 * 32) << 16);
+      drain_columns<(BN < 64 ? 16 : 32)>(taddr, taddr + acc.corr, has_corr, c0, c1, r0, g.C[p], M, N, m, ainv,
+                                         bmx ? binv : nullptr);
       fence_before();
       __syncwarp();
-      if (lane == 0) mbar_arrive_local(&acce_bar[b]);
+      for (int b = 0; b < 2; ++b)
+        if (acc.s[b] && lane == 0) mbar_arrive_local(&acce_bar[b]);
+      acc.done();
     }
   }
   fence_before();
@@ -945,7 +945,7 @@ __global__ void __launch_bounds__(kPersistThreads, 1) tc_gemm_persist_kernel(con
 }
 
 template <int BN>
-__global__ void __launch_bounds__(128, 1) tc_gemm_grouped_kernel(const __grid_constant__ GroupedTc g,
+__global__ void __launch_bounds__(128, 1) tc_gemm_grouped_kernel(const __grid_constant__ GroupedTc<kTcGroupMax> g,
                                                                  int* __restrict__ errflag) {
   const int b = blockIdx.x;
   int p = 0;
@@ -1030,57 +1030,66 @@ int device_sm_count() {
   return sms[dev];
 }
 
-// Grouped problems, at most kTcGroupMax per launch.  Persist: one persistent launch of
-// min(tiles, SM count) CTAs of 320 threads (tc_gemm_persist_kernel); otherwise one CTA per
-// tile (tc_gemm_grouped_ps_kernel).
-template <int BN, int P, bool Persist>
-cudaError_t launch_grouped_ps(const TcGemmArgs* probs, int nprob, int* errflag, cudaStream_t s, std::string* why) {
+// Problems, at most G per launch: one persistent launch of min(tiles, SM count) CTAs of 320
+// threads, the problems with the costliest tiles first.
+template <int BN, int P, int G>
+cudaError_t launch_persist_g(const TcGemmArgs* probs, int nprob, int* errflag, cudaStream_t s, std::string* why) {
   using CF = Cfg2<BN, P>;
   static bool attr_set = false;
   if (!attr_set) {
-    cudaError_t e = Persist ? cudaFuncSetAttribute(tc_gemm_persist_kernel<BN, P>,
-                                                   cudaFuncAttributeMaxDynamicSharedMemorySize, CF::SMEM)
-                            : cudaFuncSetAttribute(tc_gemm_grouped_ps_kernel<BN, P>,
-                                                   cudaFuncAttributeMaxDynamicSharedMemorySize, CF::SMEM);
+    cudaError_t e = cudaFuncSetAttribute(tc_gemm_persist_kernel<BN, P, G>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                         CF::SMEM);
     if (e != cudaSuccess) return e;
     attr_set = true;
   }
-  for (int base = 0; base < nprob; base += kTcGroupMax) {
-    const int cnt = std::min(kTcGroupMax, nprob - base);
-    GroupedTc g;
+  const int grid = device_sm_count();
+  auto tiles_n = [](const TcGemmArgs& a) { return (int)((2 * a.N + BN - 1) / BN); };
+  auto width = [&](const TcGemmArgs& a) {
+    return (int)(((2 * a.N + tiles_n(a) - 1) / tiles_n(a) + 15) / 16 * 16);
+  };
+  auto cost = [&](const TcGemmArgs& a) { return (a.Kp + 96) * width(a); };  // 96: about the epilogue's time
+  std::vector<int> order(nprob);
+  for (int q = 0; q < nprob; ++q) order[q] = q;
+  std::stable_sort(order.begin(), order.end(), [&](int x, int y) { return cost(probs[x]) > cost(probs[y]); });
+  for (int base = 0; base < nprob; base += G) {
+    const int cnt = std::min(G, nprob - base);
+    GroupedTc<G> g;
     std::memset(&g, 0, sizeof(g));
     int tiles = 0;
     for (int q = 0; q < cnt; ++q) {
-      const TcGemmArgs& a = probs[base + q];
+      const TcGemmArgs& a = probs[order[base + q]];
+      g.tiles_n[q] = tiles_n(a);
+      g.bw[q] = width(a);
       if (!make_map(&g.tmA[q], a.A, a.Kp, a.M, a.a_planes, BM, why, BKE2)) return cudaErrorInvalidValue;
-      if (!make_map(&g.tmB[q], a.B, a.Kp, 2 * a.N, a.b_planes, BN, why, BKE2)) return cudaErrorInvalidValue;
+      if (!make_map(&g.tmB[q], a.B, a.Kp, 2 * a.N, a.b_planes, g.bw[q], why, BKE2)) return cudaErrorInvalidValue;
       g.C[q] = a.C;
       g.M[q] = a.M;
       g.N[q] = a.N;
       g.amax[q] = a.a_max;
       g.bmax[q] = a.b_max;
       g.nkb[q] = (int)((2 * a.Kp + BKE2 - 1) / BKE2);
-      g.tiles_n[q] = (int)((2 * a.N + BN - 1) / BN);
       g.tile_start[q] = tiles;
       tiles += (int)((a.M + BM - 1) / BM) * g.tiles_n[q];
     }
     g.tile_start[cnt] = tiles;
     g.nprob = cnt;
-    g.fp16 = probs[base].fp16;
-    g.prods.n = probs[base].nprod;
+    g.fp16 = probs[0].fp16;
+    g.prods.n = probs[0].nprod;
     for (int i = 0; i < 9; ++i) {
-      g.prods.a[i] = i < probs[base].nprod ? probs[base].prod_a[i] : 0;
-      g.prods.b[i] = i < probs[base].nprod ? probs[base].prod_b[i] : 0;
+      g.prods.a[i] = i < probs[0].nprod ? probs[0].prod_a[i] : 0;
+      g.prods.b[i] = i < probs[0].nprod ? probs[0].prod_b[i] : 0;
     }
     if (tiles == 0) continue;
-    if (Persist)
-      tc_gemm_persist_kernel<BN, P><<<std::min(tiles, device_sm_count()), kPersistThreads, CF::SMEM, s>>>(g, errflag);
-    else
-      tc_gemm_grouped_ps_kernel<BN, P><<<tiles, kPsThreads, CF::SMEM, s>>>(g, errflag);
+    tc_gemm_persist_kernel<BN, P, G><<<std::min(tiles, grid), kPersistThreads, CF::SMEM, s>>>(g, errflag);
     cudaError_t e = cudaGetLastError();
     if (e != cudaSuccess) return e;
   }
   return cudaSuccess;
+}
+template <int BN, int P>
+cudaError_t launch_persist(const TcGemmArgs* probs, int nprob, int* errflag, cudaStream_t s, std::string* why) {
+  if (nprob == 1) return launch_persist_g<BN, P, 1>(probs, nprob, errflag, s, why);
+  return launch_persist_g<BN, P, kTcGroupMax>(probs, nprob, errflag, s, why);
 }
 
 template <int P>
@@ -1158,8 +1167,8 @@ cudaError_t launch_variant(int v, const TcGemmArgs& a, int* errflag, cudaStream_
     case TCV_PS128: return launch_ps<128, P>(a, errflag, s, why);
     case TCV_PS128X2: return launch_ps<128, P, 2>(a, errflag, s, why);
     case TCV_PS256: return launch_ps<256, P>(a, errflag, s, why);
-    case TCV_PERSIST128: return launch_grouped_ps<128, P, true>(&a, 1, errflag, s, why);
-    case TCV_PERSIST256: return launch_grouped_ps<256, P, true>(&a, 1, errflag, s, why);
+    case TCV_PERSIST128: return launch_persist<128, P>(&a, 1, errflag, s, why);
+    case TCV_PERSIST256: return launch_persist<256, P>(&a, 1, errflag, s, why);
     default: return launch_pair<P>(a, errflag, s, why);
   }
 }
@@ -1283,10 +1292,10 @@ template <int P>
 cudaError_t launch_grouped_persist_bn(int bn, const TcGemmArgs* probs, int nprob, int* errflag, cudaStream_t s,
                               std::string* why) {
   switch (bn) {
-    case 32: return launch_grouped_ps<32, P, true>(probs, nprob, errflag, s, why);
-    case 64: return launch_grouped_ps<64, P, true>(probs, nprob, errflag, s, why);
-    case 128: return launch_grouped_ps<128, P, true>(probs, nprob, errflag, s, why);
-    default: return launch_grouped_ps<256, P, true>(probs, nprob, errflag, s, why);
+    case 32: return launch_persist<32, P>(probs, nprob, errflag, s, why);
+    case 64: return launch_persist<64, P>(probs, nprob, errflag, s, why);
+    case 128: return launch_persist<128, P>(probs, nprob, errflag, s, why);
+    default: return launch_persist<256, P>(probs, nprob, errflag, s, why);
   }
 }
 
@@ -1399,7 +1408,7 @@ cudaError_t launch_grouped_bn(const TcGemmArgs* probs, int nprob, int* errflag, 
   }
   for (int base = 0; base < nprob; base += kTcGroupMax) {
     const int cnt = std::min(kTcGroupMax, nprob - base);
-    GroupedTc g;
+    GroupedTc<kTcGroupMax> g;
     std::memset(&g, 0, sizeof(g));
     int tiles = 0;
     for (int q = 0; q < cnt; ++q) {

@@ -403,7 +403,8 @@ cudaError_t launch_zgemm_view(const double2* T, const GroupSpec& mg, const Group
                               int64_t M, int64_t N, int64_t K, cudaStream_t s, const int* a_flag = nullptr,
                               const int* b_flag = nullptr, int token = 0, int slices = 1, double2* P = nullptr);
 bool tc_gemm_supported(int cc_major, int cc_minor);
-// Independent problems in one launch per 56 problems (same product list for all).
+// Independent problems in one launch per kTcGroupMax problems (same product list for all).
+constexpr int kTcGroupMax = 64;
 cudaError_t launch_tc_gemm_grouped(const TcGemmArgs* probs, int nprob, int* errflag, cudaStream_t s,
                                    std::string* why);
 
