@@ -118,6 +118,7 @@ int map_run_batched(gtn_map* maps_in, int n, int precision, const double2* const
       G.M = st.M;
       G.K = st.K;
       G.out = m->abuf;
+      G.tab = st.tab;
       if (tc) {
         G.Kw = st.Kp;
         G.ld = st.Kp;
@@ -175,7 +176,7 @@ int map_run_batched(gtn_map* maps_in, int n, int precision, const double2* const
     for (int t = 0; t < 2 && e == cudaSuccess; ++t)
       if (!gath[t].empty()) {
         e = launch_gather_grouped(gath[t].data(), (int)gath[t].size(), t, fp64 ? 1 : 0, s);
-        ctx->launches += (int64_t)((gath[t].size() + kGatherJobMax - 1) / kGatherJobMax);
+        ctx->launches += gather_grouped_launches(gath[t].data(), (int)gath[t].size());
       }
     if (e == cudaSuccess && !gemm.empty()) {
       e = launch_gemm_simt_grouped(gemm.data(), (int)gemm.size(), fp64 ? 1 : 0, s);
@@ -207,12 +208,13 @@ int map_run_batched(gtn_map* maps_in, int n, int precision, const double2* const
     G.Kw = m->fin_K;
     G.out = ys[i];
     G.ld = m->fin_K;
+    G.tab = m->fin_tab;
     fin[cur64[i] ? 1 : 0].push_back(G);
   }
   for (int t = 0; t < 2 && e == cudaSuccess; ++t)
     if (!fin[t].empty()) {
       e = launch_gather_grouped(fin[t].data(), (int)fin[t].size(), t, 1, s);
-      ctx->launches += (int64_t)((fin[t].size() + kGatherJobMax - 1) / kGatherJobMax);
+      ctx->launches += gather_grouped_launches(fin[t].data(), (int)fin[t].size());
     }
   if (e != cudaSuccess) return set_err(ctx, GTN_ERR_CUDA, std::string("batched output: ") + cudaGetErrorString(e));
   return GTN_OK;

@@ -169,7 +169,7 @@ cudaError_t launch_pack_b_planes(const double2* B, int64_t N, int64_t K, int64_t
                                  int64_t pstride, __nv_bfloat16* out, cudaStream_t s);
 
 // Grouped variants: independent jobs in one launch (per 48 jobs).
-constexpr int kGatherJobMax = 48;
+constexpr int kGatherJobMax = 48, kGatherTabJobMax = 128;  // jobs per launch: a 4 to 30 KB parameter
 struct GatherJob {
   const void* T;
   GroupSpec mg, kg;
@@ -179,6 +179,7 @@ struct GatherJob {
   int64_t pstride;   // split output: plane pitch (bf16 elements)
   int nplanes;       // 0: complex output, 2 or 3: bf16 slice planes (row pitch 2*Kw)
   const float* amax = nullptr;  // with nplanes == 2: fp16 planes scaled by these row maxima
+  GatherTab tab;                // offset tables, or none
 };
 struct SmallJob {
   const void* A;
@@ -189,6 +190,7 @@ struct SmallJob {
   void* C;
 };
 cudaError_t launch_gather_grouped(const GatherJob* jobs, int njobs, int in_is64, int out_is64, cudaStream_t s);
+int gather_grouped_launches(const GatherJob* jobs, int njobs);  // that it makes
 // out[i] = offset of index i of the group (i < n), computed on the device.
 cudaError_t launch_offsets_table(const GroupSpec& g, int64_t n, int64_t* out, cudaStream_t s);
 // Row maxima of the jobs that carry amax (zeroed first), for their fp16 splits.

@@ -47,6 +47,7 @@ __device__ __forceinline__ double2 cvt(float2 a, double2*) { return make_double2
 
 // Writer for complex outputs: out[m*ldo + k].
 template <typename Tout> struct ComplexWriter {
+  static constexpr bool kPair = false;
   Tout* out;
   int64_t ldo;
   template <typename Tin> __device__ void operator()(int64_t m, int64_t k, Tin v) const {
@@ -55,35 +56,44 @@ template <typename Tout> struct ComplexWriter {
 };
 
 // Splits x into 3 bf16 slices x = s0 + s1 + s2 (round-to-nearest each step; exact for a float,
-// whose 24 significant bits the three 8-bit slices hold).
-__device__ __forceinline__ void split3(float x, __nv_bfloat16* s) {
-  __nv_bfloat16 a = __float2bfloat16_rn(x);
-  float r = x - __bfloat162float(a);
-  __nv_bfloat16 b = __float2bfloat16_rn(r);
-  r -= __bfloat162float(b);
-  s[0] = a; s[1] = b; s[2] = __float2bfloat16_rn(r);
+// whose 24 significant bits the three 8-bit slices hold).  A double is first rounded to float
+// (nearest, from its bits): the slices then hold x to a relative 2^-25, below the dropped
+// products of the six-product bf16 GEMM.
+// Both parts of a complex value: slice p holds (re, im) as one word, by packed conversions.
+__device__ __forceinline__ void split3c(float2 v, uint32_t (&s)[3]) {
+#pragma unroll
+  for (int p = 0; p < 3; ++p) {
+    const __nv_bfloat162 a = __floats2bfloat162_rn(v.x, v.y);
+    s[p] = *reinterpret_cast<const uint32_t*>(&a);
+    v.x -= __uint_as_float(s[p] << 16);
+    v.y -= __uint_as_float(s[p] & 0xffff0000u);
+  }
 }
-// A double is first rounded to float (nearest, from its bits): the slices then hold x to a
-// relative 2^-25, below the dropped products of the six-product bf16 GEMM.
-__device__ __forceinline__ void split3(double x, __nv_bfloat16* s) { split3(d2f_scaled_rn(x, 0), s); }
+__device__ __forceinline__ void split3c(double2 v, uint32_t (&s)[3]) { split3c(cvt(v, (float2*)nullptr), s); }
 
-// Writer for bf16 slice planes.
+// Writer for bf16 slice planes; pair() takes columns k and k + 1 (k even, rows of whole words).
 struct SplitWriter {
+  static constexpr bool kPair = true;
   __nv_bfloat16* out;
   int64_t ld2;      // row pitch in bf16 elements (= 2*Kp)
   int64_t pstride;  // plane pitch in bf16 elements
   int nplanes;
   template <typename Tin> __device__ void operator()(int64_t m, int64_t k, Tin v) const {
-    __nv_bfloat16 sr[3], si[3];
-    split3(v.x, sr);
-    split3(v.y, si);
-    __nv_bfloat162* row = reinterpret_cast<__nv_bfloat162*>(out + m * ld2 + 2 * k);
-    for (int p = 0; p < nplanes; ++p) {
-      __nv_bfloat162 pr;
-      pr.x = sr[p];
-      pr.y = si[p];
-      *reinterpret_cast<__nv_bfloat162*>(reinterpret_cast<__nv_bfloat16*>(row) + p * pstride) = pr;
-    }
+    uint32_t s[3];
+    split3c(v, s);
+    __nv_bfloat16* row = out + m * ld2 + 2 * k;
+#pragma unroll
+    for (int p = 0; p < 3; ++p)
+      if (p < nplanes) *reinterpret_cast<uint32_t*>(row + p * pstride) = s[p];
+  }
+  template <typename Tin> __device__ void pair(int64_t m, int64_t k, Tin v0, Tin v1) const {
+    uint32_t s0[3], s1[3];
+    split3c(v0, s0);
+    split3c(v1, s1);
+    __nv_bfloat16* row = out + m * ld2 + 2 * k;
+#pragma unroll
+    for (int p = 0; p < 3; ++p)
+      if (p < nplanes) *reinterpret_cast<uint2*>(row + p * pstride) = make_uint2(s0[p], s1[p]);
   }
 };
 
@@ -166,20 +176,22 @@ constexpr int kTabRows = 64;
 // TM x TK tile of 2048 elements (8 loads in flight per thread).  64 x 32 in general; 256 x 8
 // when the rows are the unit-stride index, so that every k reads a 4 KB contiguous run
 // (a 32-wide tile over far-apart k legs touches 32 pages per tile).
+template <typename Tin, int TM, int TK> struct SmemTab {
+  int64_t offM[TM];
+  int64_t offK[TK];
+  Tin tile[TM][TK + 1];
+};
 template <typename Tin, class Writer, int TM, int TK>
-__global__ void __launch_bounds__(256) gather_tab_kernel(const Tin* __restrict__ T, TabOff off, int64_t M,
-                                                         int64_t K, int64_t Kw, int m_fast, Writer w) {
+__device__ __forceinline__ void gather_tab_tile(const Tin* __restrict__ T, const TabOff& off, int64_t M, int64_t K,
+                                                int64_t Kw, int m_fast, const Writer& w, int64_t m0, int64_t k0,
+                                                SmemTab<Tin, TM, TK>& sm) {
   static_assert(TM * TK == 2048, "2048 elements per tile");
-  __shared__ int64_t offM[TM];
-  __shared__ int64_t offK[TK];
-  __shared__ Tin tile[TM][TK + 1];
   const int tid = threadIdx.x + 32 * threadIdx.y;
-  const int64_t m0 = (int64_t)blockIdx.x * TM, k0 = (int64_t)blockIdx.y * TK;
   for (int i = tid; i < TM + TK; i += 256) {
     if (i < TM)
-      offM[i] = m0 + i < M ? off.m(m0 + i) : 0;
+      sm.offM[i] = m0 + i < M ? off.m(m0 + i) : 0;
     else
-      offK[i - TM] = k0 + (i - TM) < K ? off.k(k0 + (i - TM)) : 0;
+      sm.offK[i - TM] = k0 + (i - TM) < K ? off.k(k0 + (i - TM)) : 0;
   }
   __syncthreads();
   Tin v[8];
@@ -188,22 +200,38 @@ __global__ void __launch_bounds__(256) gather_tab_kernel(const Tin* __restrict__
     const int e = it * 256 + tid;
     const int im = m_fast ? (e % TM) : (e / TK);
     const int ik = m_fast ? (e / TM) : (e % TK);
-    v[it] = (m0 + im < M && k0 + ik < K) ? T[offM[im] + offK[ik]] : Zero<Tin>::v();
+    v[it] = (m0 + im < M && k0 + ik < K) ? T[sm.offM[im] + sm.offK[ik]] : Zero<Tin>::v();
   }
 #pragma unroll
   for (int it = 0; it < 8; ++it) {
     const int e = it * 256 + tid;
     const int im = m_fast ? (e % TM) : (e / TK);
     const int ik = m_fast ? (e / TM) : (e % TK);
-    tile[im][ik] = v[it];
+    sm.tile[im][ik] = v[it];
   }
   __syncthreads();
+  if constexpr (Writer::kPair) {  // Kw is even
 #pragma unroll
-  for (int it = 0; it < 8; ++it) {
-    const int e = it * 256 + tid;
-    const int r = e / TK, c = e % TK;
-    if (m0 + r < M && k0 + c < Kw) w(m0 + r, k0 + c, tile[r][c]);
+    for (int it = 0; it < 4; ++it) {
+      const int e = it * 256 + tid;
+      const int r = e / (TK / 2), c = 2 * (e % (TK / 2));
+      if (m0 + r < M && k0 + c < Kw) w.pair(m0 + r, k0 + c, sm.tile[r][c], sm.tile[r][c + 1]);
+    }
+  } else {
+#pragma unroll
+    for (int it = 0; it < 8; ++it) {
+      const int e = it * 256 + tid;
+      const int r = e / TK, c = e % TK;
+      if (m0 + r < M && k0 + c < Kw) w(m0 + r, k0 + c, sm.tile[r][c]);
+    }
   }
+}
+template <typename Tin, class Writer, int TM, int TK>
+__global__ void __launch_bounds__(256) gather_tab_kernel(const Tin* __restrict__ T, TabOff off, int64_t M,
+                                                         int64_t K, int64_t Kw, int m_fast, Writer w) {
+  __shared__ SmemTab<Tin, TM, TK> sm;
+  gather_tab_tile<Tin, Writer, TM, TK>(T, off, M, K, Kw, m_fast, w, (int64_t)blockIdx.x * TM,
+                                       (int64_t)blockIdx.y * TK, sm);
 }
 
 template <typename Tin, class Writer>
@@ -266,30 +294,30 @@ __global__ void pack_b_planes_kernel(const double2* __restrict__ B, int64_t N, i
       const double2 b = B[n * K + k];
       if (c_out == 0) { v0 = b.x; v1 = -b.y; } else { v0 = b.y; v1 = b.x; }
     }
-    __nv_bfloat16 s0[3], s1[3];
-    split3(v0, s0);
-    split3(v1, s1);
-    for (int p = 0; p < nplanes; ++p) {
-      __nv_bfloat162 pr;
-      pr.x = s0[p];
-      pr.y = s1[p];
-      *reinterpret_cast<__nv_bfloat162*>(out + p * pstride + row * (2 * Kp) + 2 * k) = pr;
-    }
+    uint32_t w[3];
+    split3c(make_double2(v0, v1), w);
+    for (int p = 0; p < nplanes; ++p)
+      *reinterpret_cast<uint32_t*>(out + p * pstride + row * (2 * Kp) + 2 * k) = w[p];
   }
 }
 
 // ---- fp16 slice planes: x * s = hi + lo, s a power-of-two row scale ---------------------
-__device__ __forceinline__ void split16(float x, __half* h, __half* l) {
-  *h = __float2half_rn(x);
-  *l = __float2half_rn(x - __half2float(*h));
+// Both parts of a complex value scaled by a power of two: (re, im) of each plane as one word, by
+// packed conversions.
+__device__ __forceinline__ void split16_words(float2 x, uint32_t* hi, uint32_t* lo) {
+  const __half2 h = __floats2half2_rn(x.x, x.y);
+  const float2 f = __half22float2(h);
+  const __half2 l = __floats2half2_rn(x.x - f.x, x.y - f.y);
+  *hi = *reinterpret_cast<const uint32_t*>(&h);
+  *lo = *reinterpret_cast<const uint32_t*>(&l);
 }
-// The same scaled split as the float overload, for a double and a power-of-two scale s.
-__device__ __forceinline__ void split16_scaled(double x, float s, __half* h, __half* l) {
-  const float xf = d2f_scaled_rn(x, (int)((__float_as_uint(s) >> 23) & 0xffu) - 127);
-  *h = __float2half_rn(xf);
-  *l = __float2half_rn(xf - __half2float(*h));
+__device__ __forceinline__ void split16c(float2 v, float s, uint32_t* hi, uint32_t* lo) {
+  split16_words(make_float2(v.x * s, v.y * s), hi, lo);
 }
-__device__ __forceinline__ void split16_scaled(float x, float s, __half* h, __half* l) { split16(x * s, h, l); }
+__device__ __forceinline__ void split16c(double2 v, float s, uint32_t* hi, uint32_t* lo) {
+  const int e = (int)((__float_as_uint(s) >> 23) & 0xffu) - 127;
+  split16_words(make_float2(d2f_scaled_rn(v.x, e), d2f_scaled_rn(v.y, e)), hi, lo);
+}
 __device__ __forceinline__ float absmax2(float2 v) { return fmaxf(fabsf(v.x), fabsf(v.y)); }
 // max(|re|, |im|) of a complex double as a float upper bound with the same binary exponent
 // (truncated mantissa), from the bits: NaN entries are ignored like fmax does, a magnitude
@@ -317,22 +345,36 @@ struct AbsMag {
 template <typename Tin>
 __device__ __forceinline__ void put16(__half* out, int64_t ld2, int64_t pstride, int64_t m, int64_t k, Tin v,
                                       float rowmax) {
+  uint32_t hi, lo;
+  split16c(v, fp16_row_scale(rowmax), &hi, &lo);
+  __half* row = out + m * ld2 + 2 * k;
+  *reinterpret_cast<uint32_t*>(row) = hi;
+  *reinterpret_cast<uint32_t*>(row + pstride) = lo;
+}
+// Elements (m, k) and (m, k + 1), k even: one 8-byte store per plane.
+template <typename Tin>
+__device__ __forceinline__ void put16_pair(__half* out, int64_t ld2, int64_t pstride, int64_t m, int64_t k, Tin v0,
+                                           Tin v1, float rowmax) {
   const float s = fp16_row_scale(rowmax);
-  __half2 hi, lo;
-  split16_scaled(v.x, s, &hi.x, &lo.x);
-  split16_scaled(v.y, s, &hi.y, &lo.y);
-  __half2* row = reinterpret_cast<__half2*>(out + m * ld2 + 2 * k);
-  row[0] = hi;
-  *reinterpret_cast<__half2*>(reinterpret_cast<__half*>(row) + pstride) = lo;
+  uint2 hi, lo;
+  split16c(v0, s, &hi.x, &lo.x);
+  split16c(v1, s, &hi.y, &lo.y);
+  __half* row = out + m * ld2 + 2 * k;
+  *reinterpret_cast<uint2*>(row) = hi;
+  *reinterpret_cast<uint2*>(row + pstride) = lo;
 }
 
 struct Split16Writer {
+  static constexpr bool kPair = true;
   __half* out;
   int64_t ld2;      // row pitch in halves (= 2*Kp)
   int64_t pstride;  // plane pitch in halves
   const float* amax;
   template <typename Tin> __device__ void operator()(int64_t m, int64_t k, Tin v) const {
     put16(out, ld2, pstride, m, k, v, amax[m]);
+  }
+  template <typename Tin> __device__ void pair(int64_t m, int64_t k, Tin v0, Tin v1) const {
+    put16_pair(out, ld2, pstride, m, k, v0, v1, amax[m]);
   }
 };
 // The same, handed the row maximum (the fused split computes it in shared memory), for two
@@ -345,20 +387,7 @@ struct Split16RowWriter {
   int64_t ld2;
   int64_t pstride;
   template <typename Tin> __device__ void operator()(int64_t m, int64_t k, Tin v0, Tin v1, float rowmax) const {
-    const float s = fp16_row_scale(rowmax);
-    __half2 h0, l0, h1, l1;
-    split16_scaled(v0.x, s, &h0.x, &l0.x);
-    split16_scaled(v0.y, s, &h0.y, &l0.y);
-    split16_scaled(v1.x, s, &h1.x, &l1.x);
-    split16_scaled(v1.y, s, &h1.y, &l1.y);
-    __half* row = out + m * ld2 + 2 * k;
-    uint2 hv, lv;
-    hv.x = *reinterpret_cast<uint32_t*>(&h0);
-    hv.y = *reinterpret_cast<uint32_t*>(&h1);
-    lv.x = *reinterpret_cast<uint32_t*>(&l0);
-    lv.y = *reinterpret_cast<uint32_t*>(&l1);
-    *reinterpret_cast<uint2*>(row) = hv;
-    *reinterpret_cast<uint2*>(row + pstride) = lv;
+    put16_pair(out, ld2, pstride, m, k, v0, v1, rowmax);
   }
 };
 
@@ -418,6 +447,7 @@ __device__ __forceinline__ void digit_check(float E, int token, int* flag) {
 
 // Element (m, k) of the A operand: its digits in the planes (4 bytes each).
 struct DigitWriter {
+  static constexpr bool kPair = false;
   unsigned char* out;
   int64_t nkb;
   const float* rexp;
@@ -598,11 +628,10 @@ __global__ void pack_b_planes_f16_kernel(const double2* __restrict__ B, int64_t 
       const double2 b = B[n * K + k];
       if ((row & 1) == 0) { v0 = b.x; v1 = -b.y; } else { v0 = b.y; v1 = b.x; }
     }
-    __half2 hi, lo;
-    split16_scaled(v0, s, &hi.x, &lo.x);
-    split16_scaled(v1, s, &hi.y, &lo.y);
-    *reinterpret_cast<__half2*>(out + row * (2 * Kp) + 2 * k) = hi;
-    *reinterpret_cast<__half2*>(out + pstride + row * (2 * Kp) + 2 * k) = lo;
+    uint32_t hi, lo;
+    split16c(make_double2(v0, v1), s, &hi, &lo);
+    *reinterpret_cast<uint32_t*>(out + row * (2 * Kp) + 2 * k) = hi;
+    *reinterpret_cast<uint32_t*>(out + pstride + row * (2 * Kp) + 2 * k) = lo;
   }
 }
 
@@ -819,6 +848,57 @@ __global__ void __launch_bounds__(256) gather_grouped_kernel(const __grid_consta
     gather_tile<Tin, ComplexWriter<Tout>>(static_cast<const Tin*>(J.T), J.mg, J.kg, J.M, J.K, J.Kw, g.m_fast[p], w,
                                           m0, k0, sm);
   }
+}
+
+// The same jobs with offset tables (maps that keep them): no index decomposition, and tiles of
+// 2048 elements with eight loads in flight per thread (64 x 32, or 256 x 8 where the rows are
+// the unit-stride index).  The 32 x 32 tiles above spend their time on 64-bit divisions and one
+// load's latency after the other: 64 uneven one-site maps, the longest split (320 MB moved)
+// 115 us there, 99 us here, and 66 us with the packed conversions and pairs of SplitWriter.
+struct GatherTabJob {
+  const void* T;
+  const int64_t *om, *ok;
+  void* out;
+  const float* amax;
+  int64_t M, K, Kw, ld, pstride;
+  int nplanes, m_fast;
+};
+struct GatherTabJobsP {
+  GatherTabJob j[kGatherTabJobMax];
+  int tile_start[kGatherTabJobMax + 1];
+  int tiles_m[kGatherTabJobMax];
+  int n;
+};
+template <typename Tin> union SmemTabs {
+  SmemTab<Tin, 64, 32> a;
+  SmemTab<Tin, 256, 8> b;
+  __device__ SmemTabs() {}
+};
+template <typename Tin, class Writer>
+__device__ __forceinline__ void gather_tab_job(const GatherTabJob& J, const Writer& w, int tm, int tk,
+                                               SmemTabs<Tin>& sm) {
+  const Tin* T = static_cast<const Tin*>(J.T);
+  const TabOff off{J.om, J.ok};
+  if (J.m_fast)
+    gather_tab_tile<Tin, Writer, 256, 8>(T, off, J.M, J.K, J.Kw, 1, w, (int64_t)tm * 256, (int64_t)tk * 8, sm.b);
+  else
+    gather_tab_tile<Tin, Writer, 64, 32>(T, off, J.M, J.K, J.Kw, 0, w, (int64_t)tm * 64, (int64_t)tk * 32, sm.a);
+}
+template <typename Tin, typename Tout>
+__global__ void __launch_bounds__(256) gather_tab_grouped_kernel(const __grid_constant__ GatherTabJobsP g) {
+  __shared__ SmemTabs<Tin> sm;
+  const int b = blockIdx.x;
+  int p = 0;  // the last job with tile_start <= b
+  for (int h = kGatherTabJobMax / 2; h > 0; h >>= 1)
+    if (p + h < g.n && g.tile_start[p + h] <= b) p += h;
+  const GatherTabJob& J = g.j[p];
+  const int t = b - g.tile_start[p], tm = t % g.tiles_m[p], tk = t / g.tiles_m[p];
+  if (J.nplanes > 0 && J.amax)
+    gather_tab_job<Tin>(J, Split16Writer{static_cast<__half*>(J.out), 2 * J.ld, J.pstride, J.amax}, tm, tk, sm);
+  else if (J.nplanes > 0)
+    gather_tab_job<Tin>(J, SplitWriter{static_cast<__nv_bfloat16*>(J.out), 2 * J.ld, J.pstride, J.nplanes}, tm, tk, sm);
+  else
+    gather_tab_job<Tin>(J, ComplexWriter<Tout>{static_cast<Tout*>(J.out), J.ld}, tm, tk, sm);
 }
 
 struct SmallJobsP {
@@ -1090,23 +1170,7 @@ struct SplitRowWriter {
   int64_t pstride;
   int nplanes;
   template <typename Tin> __device__ void operator()(int64_t m, int64_t k, Tin v0, Tin v1, float) const {
-    __nv_bfloat16 r0[3], i0[3], r1[3], i1[3];
-    split3(v0.x, r0);
-    split3(v0.y, i0);
-    split3(v1.x, r1);
-    split3(v1.y, i1);
-    __nv_bfloat16* row = out + m * ld2 + 2 * k;
-    for (int p = 0; p < nplanes; ++p) {
-      __nv_bfloat162 a, b;
-      a.x = r0[p];
-      a.y = i0[p];
-      b.x = r1[p];
-      b.y = i1[p];
-      uint2 w;
-      w.x = *reinterpret_cast<uint32_t*>(&a);
-      w.y = *reinterpret_cast<uint32_t*>(&b);
-      *reinterpret_cast<uint2*>(row + p * pstride) = w;
-    }
+    SplitWriter{out, ld2, pstride, nplanes}.pair(m, k, v0, v1);
   }
 };
 
@@ -1667,7 +1731,50 @@ static cudaError_t launch_gather_grouped_t(const GatherJob* jobs, int njobs, cud
   return cudaSuccess;
 }
 
+template <typename Tin, typename Tout>
+static cudaError_t launch_gather_tab_grouped_t(const GatherJob* jobs, int njobs, cudaStream_t s) {
+  for (int base = 0; base < njobs; base += kGatherTabJobMax) {
+    const int cnt = std::min(kGatherTabJobMax, njobs - base);
+    GatherTabJobsP g;
+    std::memset(&g, 0, sizeof(g));
+    int64_t tiles = 0;
+    for (int q = 0; q < cnt; ++q) {
+      const GatherJob& J = jobs[base + q];
+      const int TM = J.tab.m_fast ? 256 : 64, TK = 2048 / TM;
+      g.j[q] = GatherTabJob{J.T, J.tab.om, J.tab.ok, J.out, J.amax, J.M, J.K, J.Kw, J.ld > 0 ? J.ld : J.Kw,
+                            J.pstride, J.nplanes, J.tab.m_fast};
+      g.tiles_m[q] = (int)((J.M + TM - 1) / TM);
+      g.tile_start[q] = (int)tiles;
+      tiles += (int64_t)g.tiles_m[q] * ((J.Kw + TK - 1) / TK);
+      if (tiles > 2147483647LL) return cudaErrorInvalidConfiguration;
+    }
+    g.tile_start[cnt] = (int)tiles;
+    g.n = cnt;
+    if (tiles == 0) continue;
+    gather_tab_grouped_kernel<Tin, Tout><<<(unsigned)tiles, dim3(32, 8), 0, s>>>(g);
+    cudaError_t e = cudaGetLastError();
+    if (e != cudaSuccess) return e;
+  }
+  return cudaSuccess;
+}
+// Every job has offset tables.
+static bool all_tabs(const GatherJob* jobs, int njobs) {
+  for (int q = 0; q < njobs; ++q)
+    if (!jobs[q].tab.om) return false;
+  return true;
+}
+int gather_grouped_launches(const GatherJob* jobs, int njobs) {
+  const int per = all_tabs(jobs, njobs) ? kGatherTabJobMax : kGatherJobMax;
+  return (njobs + per - 1) / per;
+}
+
 cudaError_t launch_gather_grouped(const GatherJob* jobs, int njobs, int in_is64, int out_is64, cudaStream_t s) {
+  if (all_tabs(jobs, njobs)) {
+    if (in_is64 && out_is64) return launch_gather_tab_grouped_t<double2, double2>(jobs, njobs, s);
+    if (in_is64) return launch_gather_tab_grouped_t<double2, float2>(jobs, njobs, s);
+    if (out_is64) return launch_gather_tab_grouped_t<float2, double2>(jobs, njobs, s);
+    return launch_gather_tab_grouped_t<float2, float2>(jobs, njobs, s);
+  }
   if (in_is64 && out_is64) return launch_gather_grouped_t<double2, double2>(jobs, njobs, s);
   if (in_is64) return launch_gather_grouped_t<double2, float2>(jobs, njobs, s);
   if (out_is64) return launch_gather_grouped_t<float2, double2>(jobs, njobs, s);
