@@ -369,21 +369,31 @@ cudaError_t launch_splitk(const T* A, const T* B, T* C, int64_t M, int64_t N, in
 // product with few 64-wide tiles is bound by the SMs it leaves idle and by the padding of its
 // edge tiles, not by loads: the launcher takes the largest tile that still gives every SM two.
 // The slices' partial sums are added in order.
+// The tiles in slices are bound by the latency of their loads: they take 64 k at a time and hold
+// the next 64 in registers meanwhile, and the K offsets of up to 512 columns are decomposed at
+// once (two-site map of a star at bond 32: 9.1 -> 6.3 us; 16 x 16 tiles, which fill the FP64
+// pipes, lose by it: 79 -> 100 us on the slices of a coupling tensor's adjoint at bond 75).
+// With `ov.on` an output (n, m) goes to ov's offsets instead of C[n][m]: the last step of a plan
+// then writes the result's leg order itself.
 template <int TM, int TN, int R, int KS>
 __global__ void __launch_bounds__(256) zgemm_view_kernel(const double2* __restrict__ T, GroupSpec mg, GroupSpec kg,
                                                          const double2* __restrict__ B, double2* __restrict__ C,
                                                          int64_t M, int64_t N, int64_t K, int64_t tiles_m,
                                                          int64_t ntiles, int64_t kchunk,
                                                          const int* __restrict__ a_flag,
-                                                         const int* __restrict__ b_flag, int token) {
+                                                         const int* __restrict__ b_flag, int token, OutView ov) {
+  constexpr bool kAhead = KS > 1;
+  constexpr int KB = kAhead ? 64 : BK, KOFF = kAhead ? 512 : BK;
+  constexpr int NA = TM * KB / 256, NB = TN * KB / 256;
   // slice blockIdx.y of the k range writes its partial product to C + blockIdx.y * M * N
   const int64_t kb = (int64_t)blockIdx.y * kchunk, ke = kb + kchunk < K ? kb + kchunk : K;
   C += (int64_t)blockIdx.y * M * N;
-  static_assert((TM / R) * (TN / R) * KS == 256 && BK % KS == 0, "one thread per R x R outputs and slice");
+  static_assert((TM / R) * (TN / R) * KS == 256 && KB % KS == 0, "one thread per R x R outputs and slice");
+  static_assert(TM * KB % 256 == 0 && TN * KB % 256 == 0 && KOFF % KB == 0, "whole loads per thread");
   if (a_flag && *a_flag != token && *b_flag == 0) return;
-  __shared__ double2 As[BK][TM + 1];
-  __shared__ double2 Bs[BK][TN + 1];
-  __shared__ int64_t offM[TM], offK[BK];
+  __shared__ double2 As[KB][TM + 1];
+  __shared__ double2 Bs[KB][TN + 1];
+  __shared__ int64_t offM[TM], offK[KOFF];
   const int tid = threadIdx.x;
   const int ks = tid / ((TM / R) * (TN / R)), q = tid % ((TM / R) * (TN / R));
   const int tx = q % (TM / R), ty = q / (TM / R);
@@ -395,36 +405,58 @@ __global__ void __launch_bounds__(256) zgemm_view_kernel(const double2* __restri
 #pragma unroll
       for (int j = 0; j < R; ++j) acc[i][j] = make_double2(0.0, 0.0);
     if (tid < TM) offM[tid] = m0 + tid < M ? decompose(m0 + tid, mg) : 0;
-    for (int64_t k0 = kb; k0 < ke; k0 += BK) {
-      if (tid < BK) offK[tid] = k0 + tid < ke ? decompose(k0 + tid, kg) : 0;
+    auto load_a = [&](int64_t k0, int64_t kq, int i) {
+      const int e = i * 256 + tid, r = e / KB, c = e % KB;
+      return (m0 + r < M && k0 + c < ke) ? T[offM[r] + offK[k0 - kq + c]] : CT<double2>::zero();
+    };
+    auto load_b = [&](int64_t k0, int i) {
+      const int e = i * 256 + tid, r = e / KB, c = e % KB;
+      return (n0 + r < N && k0 + c < ke) ? B[(n0 + r) * K + k0 + c] : CT<double2>::zero();
+    };
+    for (int64_t kq = kb; kq < ke; kq += KOFF) {
+      for (int c = tid; c < KOFF; c += 256) offK[c] = kq + c < ke ? decompose(kq + c, kg) : 0;
       __syncthreads();
-      for (int e = tid; e < TM * BK; e += 256) {
-        const int r = e / BK, c = e % BK;
-        As[c][r] = (m0 + r < M && k0 + c < ke) ? T[offM[r] + offK[c]] : CT<double2>::zero();
+      const int64_t kl = kq + KOFF < ke ? kq + KOFF : ke;
+      double2 ra[NA], rb[NB];
+      if constexpr (kAhead) {
+#pragma unroll
+        for (int i = 0; i < NA; ++i) ra[i] = load_a(kq, kq, i);
+#pragma unroll
+        for (int i = 0; i < NB; ++i) rb[i] = load_b(kq, i);
       }
-      for (int e = tid; e < TN * BK; e += 256) {
-        const int r = e / BK, c = e % BK;
-        Bs[c][r] = (n0 + r < N && k0 + c < ke) ? B[(n0 + r) * K + k0 + c] : CT<double2>::zero();
-      }
-      __syncthreads();
+      for (int64_t k0 = kq; k0 < kl; k0 += KB) {
+#pragma unroll
+        for (int i = 0; i < NA; ++i)
+          As[(i * 256 + tid) % KB][(i * 256 + tid) / KB] = kAhead ? ra[i] : load_a(k0, kq, i);
+#pragma unroll
+        for (int i = 0; i < NB; ++i)
+          Bs[(i * 256 + tid) % KB][(i * 256 + tid) / KB] = kAhead ? rb[i] : load_b(k0, i);
+        __syncthreads();
+        if (kAhead && k0 + KB < kl) {
+#pragma unroll
+          for (int i = 0; i < NA; ++i) ra[i] = load_a(k0 + KB, kq, i);
+#pragma unroll
+          for (int i = 0; i < NB; ++i) rb[i] = load_b(k0 + KB, i);
+        }
 #pragma unroll 4
-      for (int kk = ks; kk < BK; kk += KS) {
-        double2 a[R], b[R];
+        for (int kk = ks; kk < KB; kk += KS) {
+          double2 a[R], b[R];
 #pragma unroll
-        for (int i = 0; i < R; ++i) a[i] = As[kk][tx + (TM / R) * i];
+          for (int i = 0; i < R; ++i) a[i] = As[kk][tx + (TM / R) * i];
 #pragma unroll
-        for (int j = 0; j < R; ++j) b[j] = Bs[kk][ty + (TN / R) * j];
+          for (int j = 0; j < R; ++j) b[j] = Bs[kk][ty + (TN / R) * j];
 #pragma unroll
-        for (int i = 0; i < R; ++i)
+          for (int i = 0; i < R; ++i)
 #pragma unroll
-          for (int j = 0; j < R; ++j) {
-            acc[i][j].x = fma(a[i].x, b[j].x, acc[i][j].x);
-            acc[i][j].x = fma(-a[i].y, b[j].y, acc[i][j].x);
-            acc[i][j].y = fma(a[i].x, b[j].y, acc[i][j].y);
-            acc[i][j].y = fma(a[i].y, b[j].x, acc[i][j].y);
-          }
+            for (int j = 0; j < R; ++j) {
+              acc[i][j].x = fma(a[i].x, b[j].x, acc[i][j].x);
+              acc[i][j].x = fma(-a[i].y, b[j].y, acc[i][j].x);
+              acc[i][j].y = fma(a[i].x, b[j].y, acc[i][j].y);
+              acc[i][j].y = fma(a[i].y, b[j].x, acc[i][j].y);
+            }
+        }
+        __syncthreads();
       }
-      __syncthreads();
     }
     if constexpr (KS > 1) {  // one output per thread and slice: R == 1
       __shared__ double2 part[KS][TM * TN];
@@ -438,15 +470,18 @@ __global__ void __launch_bounds__(256) zgemm_view_kernel(const double2* __restri
       __syncthreads();
     }
     if (ks == 0) {
+      int64_t om[R], on[R];
 #pragma unroll
-      for (int j = 0; j < R; ++j) {
-        const int64_t n = n0 + ty + (TN / R) * j;
-#pragma unroll
-        for (int i = 0; i < R; ++i) {
-          const int64_t m = m0 + tx + (TM / R) * i;
-          if (m < M && n < N) C[n * M + m] = acc[i][j];
-        }
+      for (int i = 0; i < R; ++i) {
+        const int64_t m = m0 + tx + (TM / R) * i, n = n0 + ty + (TN / R) * i;
+        om[i] = ov.on && m < M ? decompose(m, ov.m) : m;
+        on[i] = ov.on ? (n < N ? decompose(n, ov.n) : 0) : n * M;
       }
+#pragma unroll
+      for (int j = 0; j < R; ++j)
+#pragma unroll
+        for (int i = 0; i < R; ++i)
+          if (m0 + tx + (TM / R) * i < M && n0 + ty + (TN / R) * j < N) C[on[j] + om[i]] = acc[i][j];
     }
     __syncthreads();
   }
@@ -455,12 +490,13 @@ __global__ void __launch_bounds__(256) zgemm_view_kernel(const double2* __restri
 template <int TM, int TN, int R, int KS>
 cudaError_t launch_view(const double2* T, const GroupSpec& mg, const GroupSpec& kg, const double2* B, double2* C,
                         int64_t M, int64_t N, int64_t K, int64_t kchunk, cudaStream_t s, const int* a_flag,
-                        const int* b_flag, int token) {
+                        const int* b_flag, int token, const OutView& ov) {
   const int64_t tm = (M + TM - 1) / TM, nt = tm * ((N + TN - 1) / TN);
   // a launch that usually has nothing to do keeps its grid small
   const int64_t grid = std::min<int64_t>(nt, a_flag ? 2 * 152 : (int64_t(1) << 30));
   const int64_t slices = (K + kchunk - 1) / kchunk;
-  zgemm_view_kernel<TM, TN, R, KS><<<dim3((unsigned)grid, (unsigned)slices), 256, 0, s>>>(T, mg, kg, B, C, M, N, K, tm, nt, kchunk, a_flag, b_flag, token);
+  zgemm_view_kernel<TM, TN, R, KS><<<dim3((unsigned)grid, (unsigned)slices), 256, 0, s>>>(
+      T, mg, kg, B, C, M, N, K, tm, nt, kchunk, a_flag, b_flag, token, ov);
   return cudaGetLastError();
 }
 
@@ -468,22 +504,23 @@ cudaError_t launch_view(const double2* T, const GroupSpec& mg, const GroupSpec& 
 
 cudaError_t launch_zgemm_view(const double2* T, const GroupSpec& mg, const GroupSpec& kg, const double2* B, double2* C,
                               int64_t M, int64_t N, int64_t K, cudaStream_t s, const int* a_flag, const int* b_flag,
-                              int token, int slices, double2* P) {
+                              int token, int slices, double2* P, const OutView& ov) {
   if (M <= 0 || N <= 0) return cudaSuccess;
   auto tiles = [&](int t) { return ((M + t - 1) / t) * ((N + t - 1) / t); };
-  if (tiles(64) >= 2 * 152) return launch_view<64, 64, 4, 1>(T, mg, kg, B, C, M, N, K, K, s, a_flag, b_flag, token);
-  if (tiles(32) >= 2 * 152) return launch_view<32, 32, 2, 1>(T, mg, kg, B, C, M, N, K, K, s, a_flag, b_flag, token);
-  if (tiles(16) >= 2 * 152) return launch_view<16, 16, 1, 1>(T, mg, kg, B, C, M, N, K, K, s, a_flag, b_flag, token);
+  if (tiles(64) >= 2 * 152) return launch_view<64, 64, 4, 1>(T, mg, kg, B, C, M, N, K, K, s, a_flag, b_flag, token, ov);
+  if (tiles(32) >= 2 * 152) return launch_view<32, 32, 2, 1>(T, mg, kg, B, C, M, N, K, K, s, a_flag, b_flag, token, ov);
+  if (tiles(16) >= 2 * 152) return launch_view<16, 16, 1, 1>(T, mg, kg, B, C, M, N, K, K, s, a_flag, b_flag, token, ov);
   if (slices > 1 && P) {
+    if (ov.on) return cudaErrorInvalidValue;  // slices are summed into C[n][m]
     const int64_t kchunk = ((K + slices - 1) / slices + BK - 1) / BK * BK;
-    cudaError_t e = launch_view<16, 16, 1, 1>(T, mg, kg, B, P, M, N, K, kchunk, s, a_flag, b_flag, token);
+    cudaError_t e = launch_view<16, 16, 1, 1>(T, mg, kg, B, P, M, N, K, kchunk, s, a_flag, b_flag, token, OutView());
     if (e != cudaSuccess) return e;
     const int64_t blocks = std::min<int64_t>((M * N + 255) / 256, 152 * 8);
     splitk_reduce_kernel<double2><<<(unsigned)blocks, 256, 0, s>>>(P, (int)((K + kchunk - 1) / kchunk), M * N, C);
     return cudaGetLastError();
   }
-  if (tiles(8) >= 2 * 152) return launch_view<8, 8, 1, 4>(T, mg, kg, B, C, M, N, K, K, s, a_flag, b_flag, token);
-  return launch_view<4, 4, 1, 16>(T, mg, kg, B, C, M, N, K, K, s, a_flag, b_flag, token);
+  if (tiles(8) >= 2 * 152) return launch_view<8, 8, 1, 4>(T, mg, kg, B, C, M, N, K, K, s, a_flag, b_flag, token, ov);
+  return launch_view<4, 4, 1, 16>(T, mg, kg, B, C, M, N, K, K, s, a_flag, b_flag, token, ov);
 }
 int zgemm_view_slices(int64_t M, int64_t N, int64_t K) {
   const int64_t t16 = ((M + 15) / 16) * ((N + 15) / 16), t4 = ((M + 3) / 4) * ((N + 3) / 4);

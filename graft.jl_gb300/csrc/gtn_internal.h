@@ -26,6 +26,12 @@ struct GroupSpec {
   int64_t str[GTN_MAXG];
 };
 
+// Where a product's output (n, m) goes: C[n][m], or the offsets of these groups (on != 0).
+struct OutView {
+  int on = 0;
+  GroupSpec n, m;
+};
+
 // Device error codes written to the context's error flag by bounded waits.
 enum : int { DEVERR_NONE = 0, DEVERR_TMA_TIMEOUT = 1, DEVERR_MMA_TIMEOUT = 2, DEVERR_EPI_TIMEOUT = 3,
              DEVERR_SELFTEST_TIMEOUT = 4 };
@@ -403,7 +409,8 @@ cudaError_t launch_pack_b_digits(const double2* B, int64_t N, int64_t K, void* o
 int zgemm_view_slices(int64_t M, int64_t N, int64_t K);
 cudaError_t launch_zgemm_view(const double2* T, const GroupSpec& mg, const GroupSpec& kg, const double2* B, double2* C,
                               int64_t M, int64_t N, int64_t K, cudaStream_t s, const int* a_flag = nullptr,
-                              const int* b_flag = nullptr, int token = 0, int slices = 1, double2* P = nullptr);
+                              const int* b_flag = nullptr, int token = 0, int slices = 1, double2* P = nullptr,
+                              const OutView& ov = OutView());
 bool tc_gemm_supported(int cc_major, int cc_minor);
 // Independent problems in one launch per kTcGroupMax problems (same product list for all).
 constexpr int kTcGroupMax = 64;
@@ -503,7 +510,7 @@ struct gtn_map_s {
   GroupSpec fin_mg, fin_kg;  // final permute of the last C into y order
   GatherTab fin_tab;         // its offset tables
   int64_t fin_M = 0, fin_K = 0;
-  bool fin_identity = false;
+  OutView out;  // the last step's outputs (n, m) in y
   double flops = 0;        // algorithmic FLOPs of the reference's env-first chain
   double exec_flops = 0;   // FLOPs of the executed (possibly grouped) chain
   int n_groups = 0;

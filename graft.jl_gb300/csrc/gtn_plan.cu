@@ -51,6 +51,25 @@ bool make_group(const std::vector<int64_t>& dims, const std::vector<int>& legs, 
   return true;
 }
 
+// Legs a0 .. a1 - 1 of a result with dims d and labels l (-1, -2, ...) at strides ystr[-l - 1].
+bool make_out_group(const std::vector<int64_t>& d, const std::vector<int>& l, const std::vector<int64_t>& ystr, int a0,
+                    int a1, GroupSpec* g) {
+  std::memset(g, 0, sizeof(*g));
+  for (int a = a0; a < a1; ++a) {
+    const int64_t st = ystr[-l[a] - 1];
+    if (d[a] == 1) continue;
+    if (g->n > 0 && g->str[g->n - 1] == st * d[a]) {
+      g->dim[g->n - 1] *= d[a];
+      g->str[g->n - 1] = st;
+    } else {
+      if (g->n == GTN_MAXG) return false;
+      g->dim[g->n] = d[a];
+      g->str[g->n++] = st;
+    }
+  }
+  return true;
+}
+
 int64_t prod(const std::vector<int64_t>& d, const std::vector<int>& legs) {
   int64_t p = 1;
   for (int l : legs) p *= d[l];
@@ -588,9 +607,13 @@ int plan_build(gtn_ctx ctx, int n, const int* ranks, const int64_t* dims, const 
     return set_err(ctx, GTN_ERR_UNSUPPORTED, "too many non-contiguous output leg groups");
   map->fin_K = R > 0 ? map->y_dims[R - 1] : 1;
   map->fin_M = map->y_elems / map->fin_K;
-  bool ident = true;
-  for (int a = 0; a < R; ++a) ident = ident && ypos[a] == a;
-  map->fin_identity = ident;
+  if (!map->steps.empty()) {  // the last step's legs [N..., M...] at their strides in y
+    std::vector<int64_t> ystr(R, 1);
+    for (int k = R - 2; k >= 0; --k) ystr[k] = ystr[k + 1] * map->y_dims[k + 1];
+    int nl = 0;  // legs of the N index
+    for (int64_t p = 1; p < map->steps.back().N && nl < R; ++nl) p *= DT[nl];
+    map->out.on = make_out_group(DT, LT, ystr, 0, nl, &map->out.n) && make_out_group(DT, LT, ystr, nl, R, &map->out.m);
+  }
   if (statics && !map->oneshot) {  // one-shot contractions skip the tables
     cudaError_t e = make_tab(map, map->fin_mg, map->fin_kg, map->fin_M, map->fin_K, &map->fin_tab);
     if (e != cudaSuccess) return set_err(ctx, GTN_ERR_CUDA, std::string("offset tables: ") + cudaGetErrorString(e));
@@ -783,11 +806,18 @@ int map_run(gtn_map map, int precision, const double2* x, double2* y) {
         }
       } else {
         const int slices = map->skbuf ? st.vslices : 1;
+        // the last step writes y in its leg order, unless slices are summed into C[n][m] or the
+        // step reads the input and y overlaps it
+        const double2* xe = x + map->x_elems;
+        const bool direct = i == nst - 1 && map->out.on && slices == 1 &&
+                            (i > 0 || !(x < y + map->y_elems && y < xe));
         prof_begin(s);
-        e = launch_zgemm_view(static_cast<const double2*>(cur), st.mg, st.kg, st.b64, static_cast<double2*>(out), st.M,
-                              st.N, st.K, s, nullptr, nullptr, 0, slices, static_cast<double2*>(map->skbuf));
+        e = launch_zgemm_view(static_cast<const double2*>(cur), st.mg, st.kg, st.b64,
+                              direct ? y : static_cast<double2*>(out), st.M, st.N, st.K, s, nullptr, nullptr, 0, slices,
+                              static_cast<double2*>(map->skbuf), direct ? map->out : OutView());
         prof_end(s, GTN_KERNEL_ZGEMM, 8.0 * st.macs);
         ctx->launches += slices > 1 ? 2 : 1;
+        if (direct && e == cudaSuccess) return GTN_OK;
       }
     } else {
       if (cur64 && (st.small || !tc)) {
