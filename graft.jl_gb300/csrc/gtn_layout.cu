@@ -651,10 +651,12 @@ __device__ __forceinline__ void cfma(float2& acc, float2 a, float2 b) {
 constexpr int kSmallSmemBytes = 48 * 1024;
 __host__ __device__ constexpr size_t small_offk_bytes(int K) { return ((size_t)K * sizeof(int64_t) + 15) / 16 * 16; }
 // Shared memory of the FP64 form: offsets, static and masks (less than 2 KB past
-// kSmallSmemBytes: N K <= 3072 and K <= 64).
-constexpr int kSmall64SmemBytes = kSmallSmemBytes + 2048;
-constexpr size_t small64_smem(int K, int N, int nb) {
-  return small_offk_bytes(K) + (size_t)N * K * 16 + (size_t)((N + nb - 1) / nb) * K * 4;
+// kSmallSmemBytes: N K <= 3072 and K <= 64), and kSmallAhead elements a thread.
+constexpr int kSmallAhead = 16;
+constexpr int kSmall64SmemBytes = kSmallSmemBytes + 2048 + kSmallAhead * 256 * 16;
+constexpr size_t small64_smem(int K, int N, int nb, int threads) {
+  return small_offk_bytes(K) + (size_t)N * K * 16 + (size_t)((N + nb - 1) / nb) * K * 4 +
+         (size_t)kSmallAhead * threads * 16;
 }
 
 // C[n][m] = sum_k T[offM(m) + offK(k)] * B[n][k]; B and the K offsets live in shared memory.
@@ -689,14 +691,32 @@ __device__ __forceinline__ void small_contract_body(const T* __restrict__ A, con
 }
 
 
+__device__ __forceinline__ void cp_async_el(float2* dst, const float2* src) {
+  asm volatile("cp.async.ca.shared.global [%0], [%1], 8;" ::"r"(static_cast<uint32_t>(__cvta_generic_to_shared(dst))),
+               "l"(src)
+               : "memory");
+}
+__device__ __forceinline__ void cp_async_el(double2* dst, const double2* src) {
+  asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(static_cast<uint32_t>(__cvta_generic_to_shared(dst))),
+               "l"(src)
+               : "memory");
+}
+__device__ __forceinline__ void cp_async_wait_all() { asm volatile("cp.async.wait_all;" ::: "memory"); }
+__device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
+template <int N> __device__ __forceinline__ void cp_async_wait() {  // all but the last N groups have arrived
+  asm volatile("cp.async.wait_group %0;" ::"n"(N) : "memory");
+}
+
 // The FP64 form.  FP64 FMAs (about two a clock and SM) bound this contraction, and the statics it
 // meets are mostly TTNO tensors, whose entries are mostly zero or purely real or imaginary:
 // per (column, group of NB outputs) a bit mask of the nonzero real and imaginary parts skips
 // the FMAs of the others, the same branch for the whole warp.  A product with an exact zero
 // changes a sum only if the other factor is infinite or NaN, so a warp that holds such a value
-// does all of them.  Up to 16 outputs a pass, so that N <= 16 reads the tensor once; four loads in
-// flight per thread.  Measured at M = 2.1e6, K = 50, N = 10 (Heisenberg TTNO tensor):
-// 6.72 -> 1.03 ms.
+// does all of them.  Up to 16 outputs a pass, so that N <= 16 reads the tensor once; every thread
+// stages its row's next kSmallAhead elements in shared memory by cp.async, which takes no
+// registers and keeps the loop over k small.  Measured at M = 2.1e6, K = 50, N = 10 (Heisenberg
+// TTNO tensor): 6.72 ms without the masks, 1.03 ms with them and four loads in registers (fp64
+// pipe 32 %, stalled on loads, instruction fetches and branches), 0.56 ms as here (2.0 GB moved).
 template <int NB>
 __device__ __forceinline__ void small_contract64_body(const double2* __restrict__ A, const GroupSpec& mg,
                                                       const GroupSpec& kg, int64_t M, int K, int N,
@@ -705,7 +725,9 @@ __device__ __forceinline__ void small_contract64_body(const double2* __restrict_
   extern __shared__ __align__(16) unsigned char smem_raw[];
   int64_t* offK = reinterpret_cast<int64_t*>(smem_raw);
   double2* Bs = reinterpret_cast<double2*>(smem_raw + small_offk_bytes(K));
-  uint32_t* mask = reinterpret_cast<uint32_t*>(Bs + (size_t)N * K);  // [ceil(N / NB)][K]: re bits, im bits << 16
+  double2* st = Bs + (size_t)N * K + threadIdx.x;  // [kSmallAhead][threads], this thread's column
+  uint32_t* mask = reinterpret_cast<uint32_t*>(Bs + (size_t)N * K + kSmallAhead * blockDim.x);
+  // [ceil(N / NB)][K]: re bits, im bits << 16
   const int ngrp = (N + NB - 1) / NB;
   for (int i = threadIdx.x; i < K; i += blockDim.x) offK[i] = decompose(i, kg);
   for (int i = threadIdx.x; i < N * K; i += blockDim.x) Bs[i] = B[i];
@@ -729,30 +751,40 @@ __device__ __forceinline__ void small_contract64_body(const double2* __restrict_
       double2 acc[NB];
 #pragma unroll
       for (int j = 0; j < NB; ++j) acc[j] = make_double2(0.0, 0.0);
-      for (int k0 = 0; k0 < K; k0 += 4) {
-        double2 t[4];
+#pragma unroll 1
+      for (int k = 0; k < kSmallAhead - 1; ++k) {
+        if (k < K) cp_async_el(st + k * blockDim.x, A + om + offK[k]);
+        cp_async_commit();
+      }
+#pragma unroll 1
+      for (int k = 0; k < K; ++k) {
+        cp_async_wait<kSmallAhead - 2>();
+        const double2 t = st[(k & (kSmallAhead - 1)) * blockDim.x];
+        // into the slot of k - 1, whose value has been used
+        const int ka = k + kSmallAhead - 1;
+        if (ka < K) cp_async_el(st + (ka & (kSmallAhead - 1)) * blockDim.x, A + om + offK[ka]);
+        cp_async_commit();
+        const bool odd = (__double2hiint(t.x) & 0x7ff00000) == 0x7ff00000 ||
+                         (__double2hiint(t.y) & 0x7ff00000) == 0x7ff00000;
+        uint32_t b = mask[g * K + k];
+        if (__any_sync(0xffffffffu, odd)) b = all | (all << 16);
+        const double2* bp = Bs + n0 * K + k;
 #pragma unroll
-        for (int q = 0; q < 4; ++q) t[q] = k0 + q < K ? A[om + offK[k0 + q]] : make_double2(0.0, 0.0);
+        for (int j4 = 0; j4 < NB; j4 += 4)
+          if (b & (0xf000fu << j4)) {
 #pragma unroll
-        for (int q = 0; q < 4; ++q) {
-          if (k0 + q >= K) break;
-          const bool odd = (__double2hiint(t[q].x) & 0x7ff00000) == 0x7ff00000 ||
-                           (__double2hiint(t[q].y) & 0x7ff00000) == 0x7ff00000;
-          uint32_t b = mask[g * K + k0 + q];
-          if (__any_sync(0xffffffffu, odd)) b = all | (all << 16);
-#pragma unroll
-          for (int j = 0; j < NB; ++j) {
-            if (b & (0x10001u << j)) {
-              const double2 v = Bs[(n0 + j) * K + k0 + q];
-              if (b & (1u << j)) acc[j].x = fma(t[q].x, v.x, acc[j].x);
-              if (b & (0x10000u << j)) {
-                acc[j].x = fma(-t[q].y, v.y, acc[j].x);
-                acc[j].y = fma(t[q].x, v.y, acc[j].y);
+            for (int j = j4; j < j4 + 4; ++j) {
+              if (b & (0x10001u << j)) {
+                const double2 v = bp[j * K];
+                if (b & (1u << j)) acc[j].x = fma(t.x, v.x, acc[j].x);
+                if (b & (0x10000u << j)) {
+                  acc[j].x = fma(-t.y, v.y, acc[j].x);
+                  acc[j].y = fma(t.x, v.y, acc[j].y);
+                }
+                if (b & (1u << j)) acc[j].y = fma(t.y, v.x, acc[j].y);
               }
-              if (b & (1u << j)) acc[j].y = fma(t[q].y, v.x, acc[j].y);
             }
           }
-        }
       }
       if (m < M) {
 #pragma unroll
@@ -800,9 +832,9 @@ cudaError_t launch_small(const T* A, const GroupSpec& mg, const GroupSpec& kg, i
       attr = true;
     }
     if (N <= 8) {
-      small_contract64_kernel<8><<<(unsigned)blocks, threads, small64_smem(K, N, 8), s>>>(A, mg, kg, M, K, N, B, C);
+      small_contract64_kernel<8><<<(unsigned)blocks, threads, small64_smem(K, N, 8, threads), s>>>(A, mg, kg, M, K, N, B, C);
     } else {
-      small_contract64_kernel<16><<<(unsigned)blocks, threads, small64_smem(K, N, 16), s>>>(A, mg, kg, M, K, N, B, C);
+      small_contract64_kernel<16><<<(unsigned)blocks, threads, small64_smem(K, N, 16, threads), s>>>(A, mg, kg, M, K, N, B, C);
     }
   } else {
     const int64_t blocks = std::min<int64_t>((M + 255) / 256, 152 * 16);
@@ -1351,17 +1383,6 @@ __device__ __forceinline__ float ld_peer_f32(const float* p, uint32_t rank) {
   asm volatile("ld.shared::cluster.f32 %0, [%1];" : "=f"(v) : "r"(ra) : "memory");
   return v;
 }
-__device__ __forceinline__ void cp_async_el(float2* dst, const float2* src) {
-  asm volatile("cp.async.ca.shared.global [%0], [%1], 8;" ::"r"(static_cast<uint32_t>(__cvta_generic_to_shared(dst))),
-               "l"(src)
-               : "memory");
-}
-__device__ __forceinline__ void cp_async_el(double2* dst, const double2* src) {
-  asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(static_cast<uint32_t>(__cvta_generic_to_shared(dst))),
-               "l"(src)
-               : "memory");
-}
-__device__ __forceinline__ void cp_async_wait_all() { asm volatile("cp.async.wait_all;" ::: "memory"); }
 
 template <typename Tin> __host__ __device__ constexpr int split_rows_pitch(int kc) { return kc | 1; }
 template <typename Tin> __host__ __device__ constexpr size_t split_rows_smem(int TR, int kc) {
@@ -1853,7 +1874,7 @@ static cudaError_t launch_small_grouped_t(const SmallJob* jobs, int njobs, cudaS
       blocks += (int)nb;
       const size_t need = small_offk_bytes(J.K) + (size_t)J.N * J.K * sizeof(T);
       if (need > (size_t)kSmallSmemBytes) return cudaErrorInvalidValue;
-      smem = std::max(smem, std::is_same<T, double2>::value ? small64_smem(J.K, J.N, 8) : need);
+      smem = std::max(smem, std::is_same<T, double2>::value ? small64_smem(J.K, J.N, 8, 256) : need);
     }
     g.blk_start[cnt] = blocks;
     g.n = cnt;

@@ -52,3 +52,22 @@ def test_one_step_map_in_place(ctx, labels):
     assert np.array_equal(ctx.download(d), ref)
     assert np.allclose(ref, S @ x if labels[0][0] == 1 else (x @ S).T, rtol=0, atol=1e-11)
     m.close()
+
+
+# the staged elements (16 a thread) at K around their number, N around the outputs of a pass
+@pytest.mark.parametrize("M", [1, 33, 300, 40001])
+@pytest.mark.parametrize("K", [1, 14, 15, 16, 17, 31, 64])
+@pytest.mark.parametrize("N", [1, 9, 17, 33])
+def test_narrow_products_skip_zeros(ctx, M, K, N):
+    rng = np.random.default_rng(M + K + N)
+    A, B = crandn(rng, (K, M)), crandn(rng, (K, N))
+    B = np.where(rng.random((K, N)) < 0.3, np.where(rng.random((K, N)) < 0.5, B.real, B), 0)
+    y = ctx.download(ctx.contract([ctx.upload(A), ctx.upload(B)], [[1, -1], [1, -2]], None, None,
+                                  _lib.PRECISIONS["fp64"]))
+    assert np.all(np.abs(y - A.T @ B) <= 2 * (2 * K + 2) * 2.0 ** -53 * np.sqrt(2) * (np.abs(A).T @ np.abs(B)))
+    A[K // 2, M - 1] = np.inf  # times a complex zero: NaN, in this row only
+    y = ctx.download(ctx.contract([ctx.upload(A), ctx.upload(B)], [[1, -1], [1, -2]], None, None,
+                                  _lib.PRECISIONS["fp64"]))
+    bad = np.zeros((M, N), dtype=bool)
+    bad[M - 1] = True
+    assert np.array_equal(~np.isfinite(y), bad)
