@@ -2,10 +2,11 @@
 // Jacobi rotations (Hestenes) on the whole chip: the truncated splits of sweeps at bond dimensions
 // of about 30 to 190, for which bidiagonalisation is a chain of latency-bound column steps.
 //
-//   W = Q R (W the tall side's matrix: A, or A^H of a wide A), L = R^H, L J = V S, so that
-//   W = (Q J) S V^H.  The triangular factor is what makes the rotations converge in 6 to 10 sweeps
-//   whatever the spectrum: on the columns of W itself a decaying spectrum, the usual one of a
-//   split, takes two to three times as many (they are all nearly parallel).
+//   W = Q R (W the tall side's matrix: A, or A^H of a wide A), R^H = P T, L = T^H, L J = V S, so
+//   that W = (Q V) S (P J)^H.  The triangular factors are what makes the rotations converge: on the
+//   columns of W itself a decaying spectrum, the usual one of a split, takes 28 sweeps (they are
+//   all nearly parallel), on R^H 12, on T^H 8 or 9 (Gaussian matrices: 12, 11, 10); a third
+//   factorisation saves less than it takes.
 //
 // Both parts are dataflow kernels, one CTA per column or column pair, all resident (cooperative
 // launches), that hand columns on through L2 without flags or fences: every 64-bit word travels
@@ -21,8 +22,10 @@
 // A pair counts as orthogonal when |a^H b| <= eps sqrt(n) |a| |b| (the rounding of the dot product
 // itself).  Cosine and phase of a rotation carry full precision (they keep the columns' norms); the
 // tangent is formed in FP32, its error only leaves 1e-7 of the overlap to the next sweep.
-// Measured against cuSOLVER's gesvd: singular values 1 .. 1e-8, 192 x 192 38.5 -> 12.7 ms, 300 x 300
-// 81 -> 26 ms; Gaussian 192 x 192 32 -> 9.1 ms, 96 x 400 16.5 -> 4.6 ms.
+// Measured against cuSOLVER's gesvd: singular values 1 .. 1e-8, 192 x 192 38.5 -> 11.8 ms, 300 x 300
+// 81 -> 22.7 ms, 96 x 400 with columns 1 .. 1e-6 16.5 -> 4.2 ms (one factorisation: 12.7, 26, 4.6).
+// On the 192 x 192 split of a DMRG step the second factorisation takes 1.25 ms and saves 4.4 of
+// 14.9 ms of sweeps.
 // Every wait is bounded (4 s, then a flag ends all CTAs).
 #include "gtn_internal.h"
 
@@ -176,12 +179,12 @@ __device__ __forceinline__ void reflect(double2 (&a)[kQE], const double2 (&v)[kQ
   }
 }
 
-// CTA k: column k of W (from the row-major A, scaled).  Reflector k as words of sequence 1 in
+// CTA k: column k of W (from the row-major A, scaled) or, without A, of the n x n words X.  Reflector k as words of sequence 1 in
 // refl[k * rows ..] (from row k on) and tau[k]; row k of R conjugated as column entries of L, and
 // the k-th unit column of J, as words of sequence 0 (both zeroed before).
 __global__ void __launch_bounds__(kT, 3)
-    jacobi_qr_kernel(const double2* __restrict__ A, int tall, int rows, int n, Word* refl, Word* tau, Word* L, Word* J,
-                     JacobiState* st, int* errflag) {
+    jacobi_qr_kernel(const double2* __restrict__ A, const Word* __restrict__ X, int tall, int rows, int n, Word* refl,
+                     Word* tau, Word* L, Word* J, JacobiState* st, int* errflag) {
   __shared__ double red[2][kT];
   __shared__ double tot[2];
   __shared__ double2 alpha;
@@ -192,8 +195,13 @@ __global__ void __launch_bounds__(kT, 3)
     const int x = tid + q * kT;
     a[q] = make_double2(0.0, 0.0);
     if (x < rows) {
-      const double2 t = tall ? A[(int64_t)x * n + k] : A[(int64_t)k * rows + x];
-      a[q] = make_double2(scaled(t.x, e), tall ? scaled(t.y, e) : -scaled(t.y, e));
+      if (A) {
+        const double2 t = tall ? A[(int64_t)x * n + k] : A[(int64_t)k * rows + x];
+        a[q] = make_double2(scaled(t.x, e), tall ? scaled(t.y, e) : -scaled(t.y, e));
+      } else {
+        const Word* w = X + ((int64_t)k * rows + x) * 2;
+        a[q] = make_double2(w[0].v, w[1].v);
+      }
     }
   }
   for (int j = 0; j < k; ++j) {
@@ -411,22 +419,20 @@ __global__ void __launch_bounds__(kT) jacobi_norms_kernel(const Word* __restrict
   if (threadIdx.x == 0) nrm[blockIdx.x] = sqrt(tot[0]);
 }
 
-// CTA i: the i-th largest triplet (positive value).  Long side: Q times column ord[i] of J; short
-// side: the unit column of L.  Tall A: U = long (m x r), Vh = short^H; wide: U = short, Vh = long^H.
+// CTA (i, 0): the long vector of the i-th largest triplet (positive value), Q times the unit column
+// ord[i] of L; CTA (i, 1): its short one, P times that column of J.  Tall A: U = long (m x r),
+// Vh = short^H; wide: U = short, Vh = long^H.
 __global__ void __launch_bounds__(kT, 3)
-    jacobi_vectors_kernel(const Word* __restrict__ refl, const Word* __restrict__ tau, const Word* __restrict__ L,
+    jacobi_vectors_kernel(const Word* __restrict__ refl0, const Word* __restrict__ tau0,
+                          const Word* __restrict__ refl1, const Word* __restrict__ tau1, const Word* __restrict__ L,
                           const Word* __restrict__ J, const double* __restrict__ nrm, const int* __restrict__ ord,
-                          int tall, int rows, int n, int r, double2* __restrict__ U, double2* __restrict__ Vh) {
+                          int tall, int rows0, int n, int r, double2* __restrict__ U, double2* __restrict__ Vh) {
   __shared__ double red[2][kT];
   __shared__ double tot[2];
-  const int i = blockIdx.x, c = ord[i], tid = threadIdx.x;
-  const double s = nrm[c];
-  for (int x = tid; x < n; x += kT) {
-    const Word* w = L + ((int64_t)c * n + x) * 2;
-    const double2 u = make_double2(w[0].v / s, w[1].v / s);
-    if (tall) Vh[(int64_t)i * n + x] = make_double2(u.x, -u.y);
-    else U[(int64_t)x * r + i] = u;
-  }
+  const bool is_long = blockIdx.y == 0;
+  const Word *refl = is_long ? refl0 : refl1, *tau = is_long ? tau0 : tau1, *src = is_long ? L : J;
+  const int i = blockIdx.x, c = ord[i], tid = threadIdx.x, rows = is_long ? rows0 : n;
+  const double s = is_long ? nrm[c] : 1.0;
   double2 a[kQE], v[kQE], nv[kQE];
   auto fetch = [&](int j, double2 (&t)[kQE]) {
 #pragma unroll
@@ -442,7 +448,8 @@ __global__ void __launch_bounds__(kT, 3)
 #pragma unroll
   for (int q = 0; q < kQE; ++q) {
     const int x = tid + q * kT;
-    a[q] = x < n ? make_double2(J[((int64_t)c * n + x) * 2].v, J[((int64_t)c * n + x) * 2 + 1].v) : make_double2(0.0, 0.0);
+    const Word* w = src + ((int64_t)c * n + x) * 2;
+    a[q] = x < n ? make_double2(w[0].v / s, w[1].v / s) : make_double2(0.0, 0.0);
   }
   fetch(n - 1, v);
   for (int j = n - 1; j >= 0; --j) {
@@ -451,11 +458,12 @@ __global__ void __launch_bounds__(kT, 3)
 #pragma unroll
     for (int q = 0; q < kQE; ++q) v[q] = nv[q];
   }
+  const bool to_u = (tall != 0) == is_long;
 #pragma unroll
   for (int q = 0; q < kQE; ++q) {
     const int x = tid + q * kT;
     if (x < rows) {
-      if (tall) U[(int64_t)x * r + i] = a[q];
+      if (to_u) U[(int64_t)x * r + i] = a[q];
       else Vh[(int64_t)i * rows + x] = make_double2(a[q].x, -a[q].y);
     }
   }
@@ -466,7 +474,7 @@ inline size_t up256(size_t b) { return (b + 255) / 256 * 256; }
 // The workspace's parts; the first `zeroed` bytes start as zero.
 struct Parts {
   JacobiState* st;
-  Word *refl, *tau, *L, *J, *rots;
+  Word *refl, *tau, *R, *refl2, *tau2, *L, *J, *rots;  // R: R^H of the first factorisation
   double* nrm;
   int* ord;
   size_t zeroed, bytes;
@@ -481,6 +489,9 @@ struct Parts {
     st = reinterpret_cast<JacobiState*>(take(sizeof(JacobiState)));
     refl = reinterpret_cast<Word*>(take(rows * n * 2 * sizeof(Word)));
     tau = reinterpret_cast<Word*>(take(n * 2 * sizeof(Word)));
+    R = reinterpret_cast<Word*>(take(n * n * 2 * sizeof(Word)));
+    refl2 = reinterpret_cast<Word*>(take(n * n * 2 * sizeof(Word)));
+    tau2 = reinterpret_cast<Word*>(take(n * 2 * sizeof(Word)));
     L = reinterpret_cast<Word*>(take(n * n * 2 * sizeof(Word)));
     J = reinterpret_cast<Word*>(take(n * n * 2 * sizeof(Word)));
     rots = reinterpret_cast<Word*>(take(n * ((n + 1) / 2) * 6 * sizeof(Word)));
@@ -512,8 +523,12 @@ int jacobi_svd_run(gtn_ctx ctx, int64_t m, int64_t n, const double2* A, void* ws
   jacobi_exponent_kernel<<<(unsigned)std::min<int64_t>((m * n + 255) / 256, 152 * 4), 256, 0, s>>>(A, m * n, w.st);
   GTN_CUDA_TRY(ctx, cudaGetLastError());
   int* errflag = ctx->d_errflag;
-  void* qargs[] = {&A, &tall, &rows, &k, &w.refl, &w.tau, &w.L, &w.J, &w.st, &errflag};
+  const Word* none = nullptr;
+  const double2* noA = nullptr;
+  void* qargs[] = {&A, &none, &tall, &rows, &k, &w.refl, &w.tau, &w.R, &w.J, &w.st, &errflag};
   GTN_CUDA_TRY(ctx, cudaLaunchCooperativeKernel((const void*)jacobi_qr_kernel, dim3((unsigned)k), dim3(kT), qargs, 0, s));
+  void* pargs[] = {&noA, &w.R, &tall, &k, &k, &w.refl2, &w.tau2, &w.L, &w.J, &w.st, &errflag};
+  GTN_CUDA_TRY(ctx, cudaLaunchCooperativeKernel((const void*)jacobi_qr_kernel, dim3((unsigned)k), dim3(kT), pargs, 0, s));
   // one CTA per pair of L and of J where they fit
   int gw = std::max(1, std::min((k + 1) / 2, sw_sm * ctx->sm_count / 2));
   void* args[] = {&w.L, &w.J, &k, &gw, &w.rots, &w.st, &errflag};
@@ -521,7 +536,7 @@ int jacobi_svd_run(gtn_ctx ctx, int64_t m, int64_t n, const double2* A, void* ws
                                                 args, 0, s));
   jacobi_norms_kernel<<<(unsigned)k, kT, 0, s>>>(w.L, k, w.nrm);
   GTN_CUDA_TRY(ctx, cudaGetLastError());
-  ctx->launches += 4;
+  ctx->launches += 5;
   std::vector<double> hn(k);
   JacobiState hst;
   GTN_CUDA_TRY(ctx, cudaMemcpyAsync(hn.data(), w.nrm, k * sizeof(double), cudaMemcpyDeviceToHost, s));
@@ -543,8 +558,8 @@ int jacobi_svd_run(gtn_ctx ctx, int64_t m, int64_t n, const double2* A, void* ws
 int jacobi_svd_store(gtn_ctx ctx, int64_t m, int64_t n, void* ws, int64_t r, double2* U, double2* Vh) {
   const int tall = m >= n ? 1 : 0, rows = (int)std::max(m, n), k = (int)std::min(m, n);
   const Parts w(ws, rows, k);
-  jacobi_vectors_kernel<<<(unsigned)r, kT, 0, ctx->stream>>>(w.refl, w.tau, w.L, w.J, w.nrm, w.ord, tall, rows, k,
-                                                            (int)r, U, Vh);
+  jacobi_vectors_kernel<<<dim3((unsigned)r, 2), kT, 0, ctx->stream>>>(w.refl, w.tau, w.refl2, w.tau2, w.L, w.J, w.nrm,
+                                                                     w.ord, tall, rows, k, (int)r, U, Vh);
   ctx->launches++;
   GTN_CUDA_TRY(ctx, cudaGetLastError());
   return GTN_OK;
