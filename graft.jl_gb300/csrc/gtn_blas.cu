@@ -126,6 +126,7 @@ template <bool F32>
 __global__ void __launch_bounds__(kDotThreads, 3) multidot_partial_kernel(const double2* __restrict__ V, int64_t ldv,
                                                                           int J, const double2* __restrict__ w,
                                                                           int64_t n, double2* __restrict__ part) {
+  chained_wait();
   __shared__ double sm[16 * kDotThreads];
   const int j0 = blockIdx.y * 8;
   switch (min(8, J - j0)) {
@@ -147,6 +148,7 @@ template <bool F32>
 __global__ void __launch_bounds__(kDotThreads) update_kernel(double2* __restrict__ w, const double2* __restrict__ V,
                                                              int64_t ldv, int J, const double2* __restrict__ coef,
                                                              int64_t n, double2* __restrict__ part) {
+  chained_wait();
   __shared__ double2 c[kMaxJ];
   __shared__ float2 cf[kMaxJ];
   __shared__ double sm[kDotThreads];
@@ -189,6 +191,7 @@ __global__ void __launch_bounds__(kDotThreads) update_kernel(double2* __restrict
 // w /= sqrt(nrm2) with the squared norm on the device (left alone where that is not positive).
 __global__ void __launch_bounds__(kDotThreads) unit_scale_kernel(double2* __restrict__ w,
                                                                  const double2* __restrict__ nrm2, int64_t n) {
+  chained_wait();
   __shared__ double f;
   if (threadIdx.x == 0) f = nrm2->x > 0.0 ? 1.0 / sqrt(nrm2->x) : 1.0;
   __syncthreads();
@@ -205,6 +208,7 @@ __global__ void __launch_bounds__(kDotThreads) unit_scale_kernel(double2* __rest
 __global__ void __launch_bounds__(128) multidot_final_kernel(const double2* __restrict__ part, int nblk, int J,
                                                              double2* __restrict__ out,
                                                              const int* __restrict__ errflag) {
+  chained_wait();
   const int j = blockIdx.x;
   double x = 0, y = 0;
   for (int b = threadIdx.x; b < nblk; b += 128) {
@@ -303,6 +307,7 @@ __global__ void restrict_leg_kernel(const double2* __restrict__ in, double2* __r
 }
 
 __global__ void conj_kernel(double2* __restrict__ x, int64_t n) {
+  chained_wait();
   for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n;
        i += (int64_t)gridDim.x * blockDim.x)
     x[i].y = -x[i].y;
@@ -450,9 +455,8 @@ static cudaError_t multidot(const double2* V, int64_t ldv, int J, const double2*
   if (J <= 0) return cudaSuccess;
   if (J > kMaxJ) return cudaErrorInvalidValue;
   const int nb = dot_blocks(n, nblk, J, scratch_cap);
-  multidot_partial_kernel<F32><<<dim3((unsigned)nb, (unsigned)((J + 7) / 8)), kDotThreads, 0, s>>>(
-      V, ldv, J, w, n, scratch);
-  multidot_final_kernel<<<J, 128, 0, s>>>(scratch, nb, J, out, nullptr);
+  launch_chained(multidot_partial_kernel<F32>, dim3((unsigned)nb, (unsigned)((J + 7) / 8)), dim3(kDotThreads), 0, s, V, ldv, J, w, n, scratch);
+  launch_chained(multidot_final_kernel, dim3(J), dim3(128), 0, s, scratch, nb, J, out, nullptr);
   return cudaGetLastError();
 }
 cudaError_t launch_multidot(const double2* V, int64_t ldv, int J, const double2* w, int64_t n, double2* out,
@@ -469,12 +473,12 @@ cudaError_t launch_update(double2* w, const double2* V, int64_t ldv, int J, cons
   if (J <= 0 || J > kMaxJ) return cudaErrorInvalidValue;
   const int nb = dot_blocks(n, nblk, 1, scratch_cap);
   double2* part = nrm2 ? scratch : nullptr;
-  (f32 ? update_kernel<true> : update_kernel<false>)<<<nb, kDotThreads, 0, s>>>(w, V, ldv, J, coef, n, part);
-  if (nrm2) multidot_final_kernel<<<1, 128, 0, s>>>(part, nb, 1, nrm2, errflag);
+  launch_chained((f32 ? update_kernel<true> : update_kernel<false>), dim3(nb), dim3(kDotThreads), 0, s, w, V, ldv, J, coef, n, part);
+  if (nrm2) launch_chained(multidot_final_kernel, dim3(1), dim3(128), 0, s, part, nb, 1, nrm2, errflag);
   return cudaGetLastError();
 }
 cudaError_t launch_unit_scale(double2* w, const double2* nrm2, int64_t n, cudaStream_t s) {
-  unit_scale_kernel<<<grid_for(n), kDotThreads, 0, s>>>(w, nrm2, n);
+  launch_chained(unit_scale_kernel, dim3(grid_for(n)), dim3(kDotThreads), 0, s, w, nrm2, n);
   return cudaGetLastError();
 }
 
@@ -522,7 +526,7 @@ cudaError_t launch_restrict_leg(const double2* in, double2* out, int64_t A, int6
 }
 
 cudaError_t launch_conj_inplace(double2* x, int64_t n, cudaStream_t s) {
-  conj_kernel<<<grid_for(n), 256, 0, s>>>(x, n);
+  launch_chained(conj_kernel, dim3(grid_for(n)), dim3(256), 0, s, x, n);
   return cudaGetLastError();
 }
 cudaError_t launch_transpose_c128(const double2* in, int64_t rows, int64_t cols, double2* out,

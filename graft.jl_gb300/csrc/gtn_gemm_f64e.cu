@@ -160,6 +160,7 @@ __global__ void __launch_bounds__(kThreads, 1)
                      int64_t M, int64_t N, int nkb, int64_t tiles_m, int64_t tiles_n, const float* __restrict__ a_exp,
                      const float* __restrict__ b_exp, const int* __restrict__ a_flag, const int* __restrict__ b_flag,
                      int token, longlong2* __restrict__ part, int* __restrict__ errflag) {
+  chained_wait();
   extern __shared__ __align__(1024) uint8_t smem_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) &
                                              ~static_cast<uintptr_t>(1023));
@@ -376,6 +377,7 @@ __global__ void __launch_bounds__(32 * kEpiWarps)
                        int64_t tiles_m, int64_t tiles_n, int G, const float* __restrict__ a_exp,
                        const float* __restrict__ b_exp, const int* __restrict__ a_flag, const int* __restrict__ b_flag,
                        int token) {
+  chained_wait();
   if (*a_flag == token || *b_flag != 0) return;
   constexpr int kPairs = kCols / 2, kT = 32 * kEpiWarps;
   const int64_t whole = tiles_m * tiles_n / G * G;
@@ -466,15 +468,14 @@ cudaError_t launch_f64e_gemm(const F64eGemmArgs& a, int sm_count, int* errflag, 
     }
     attr_set = true;
   }
-  kerns[(a.levels == 7 ? 2 : 0) + (share ? 1 : 0)]<<<(unsigned)grid, kThreads, kSmem, s>>>(
-      static_cast<const unsigned char*>(a.A), static_cast<const unsigned char*>(a.B), a.C, a.M, a.N, nkb, tm, tn,
+  launch_chained(kerns[(a.levels == 7 ? 2 : 0) + (share ? 1 : 0)], dim3((unsigned)grid), dim3(kThreads), kSmem, s, static_cast<const unsigned char*>(a.A), static_cast<const unsigned char*>(a.B), a.C, a.M, a.N, nkb, tm, tn,
       a.a_exp, a.b_exp, a.a_flag, a.b_flag, a.token, share ? static_cast<longlong2*>(a.part) : nullptr, errflag);
   cudaError_t e = cudaGetLastError();
   *launches = 1;
   if (e == cudaSuccess && share) {
     *launches = 2;
     const int64_t rest = tm * tn - tm * tn / grid * grid;
-    f64e_finish_kernel<<<(unsigned)(rest * (kCols / 2)), 32 * kEpiWarps, 0, s>>>(static_cast<const longlong2*>(a.part), a.C, a.M, a.N,
+    launch_chained(f64e_finish_kernel, dim3((unsigned)(rest * (kCols / 2))), dim3(32 * kEpiWarps), 0, s, static_cast<const longlong2*>(a.part), a.C, a.M, a.N,
                                                              nchunks, tm, tn, (int)grid, a.a_exp, a.b_exp, a.a_flag,
                                                              a.b_flag, a.token);
     e = cudaGetLastError();

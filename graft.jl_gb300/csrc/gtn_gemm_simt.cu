@@ -320,6 +320,7 @@ __global__ void __launch_bounds__(256) gemm_simt_splitk_kernel(const T* __restri
 
 template <typename T>
 __global__ void splitk_reduce_kernel(const T* __restrict__ P, int S, int64_t MN, T* __restrict__ C) {
+  chained_wait();
   for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < MN; i += (int64_t)gridDim.x * blockDim.x) {
     T acc = P[i];
     for (int z = 1; z < S; ++z) {
@@ -359,7 +360,7 @@ cudaError_t launch_splitk(const T* A, const T* B, T* C, int64_t M, int64_t N, in
   const int64_t MN = M * N;
   int64_t blocks = (MN + 255) / 256;
   if (blocks > 152 * 8) blocks = 152 * 8;
-  splitk_reduce_kernel<T><<<(unsigned)(blocks < 1 ? 1 : blocks), 256, 0, s>>>(P, Se, MN, C);
+  launch_chained(splitk_reduce_kernel<T>, dim3((unsigned)(blocks < 1 ? 1 : blocks)), dim3(256), 0, s, P, Se, MN, C);
   return cudaGetLastError();
 }
 
@@ -382,6 +383,7 @@ __global__ void __launch_bounds__(256) zgemm_view_kernel(const double2* __restri
                                                          int64_t ntiles, int64_t kchunk,
                                                          const int* __restrict__ a_flag,
                                                          const int* __restrict__ b_flag, int token, OutView ov) {
+  chained_wait();
   constexpr bool kAhead = KS > 1;
   constexpr int KB = kAhead ? 64 : BK, KOFF = kAhead ? 512 : BK;
   constexpr int NA = TM * KB / 256, NB = TN * KB / 256;
@@ -495,8 +497,7 @@ cudaError_t launch_view(const double2* T, const GroupSpec& mg, const GroupSpec& 
   // a launch that usually has nothing to do keeps its grid small
   const int64_t grid = std::min<int64_t>(nt, a_flag ? 2 * 152 : (int64_t(1) << 30));
   const int64_t slices = (K + kchunk - 1) / kchunk;
-  zgemm_view_kernel<TM, TN, R, KS><<<dim3((unsigned)grid, (unsigned)slices), 256, 0, s>>>(
-      T, mg, kg, B, C, M, N, K, tm, nt, kchunk, a_flag, b_flag, token, ov);
+  launch_chained(zgemm_view_kernel<TM, TN, R, KS>, dim3((unsigned)grid, (unsigned)slices), dim3(256), 0, s, T, mg, kg, B, C, M, N, K, tm, nt, kchunk, a_flag, b_flag, token, ov);
   return cudaGetLastError();
 }
 
@@ -516,7 +517,7 @@ cudaError_t launch_zgemm_view(const double2* T, const GroupSpec& mg, const Group
     cudaError_t e = launch_view<16, 16, 1, 1>(T, mg, kg, B, P, M, N, K, kchunk, s, a_flag, b_flag, token, OutView());
     if (e != cudaSuccess) return e;
     const int64_t blocks = std::min<int64_t>((M * N + 255) / 256, 152 * 8);
-    splitk_reduce_kernel<double2><<<(unsigned)blocks, 256, 0, s>>>(P, (int)((K + kchunk - 1) / kchunk), M * N, C);
+    launch_chained(splitk_reduce_kernel<double2>, dim3((unsigned)blocks), dim3(256), 0, s, P, (int)((K + kchunk - 1) / kchunk), M * N, C);
     return cudaGetLastError();
   }
   if (tiles(8) >= 2 * 152) return launch_view<8, 8, 1, 4>(T, mg, kg, B, C, M, N, K, K, s, a_flag, b_flag, token, ov);

@@ -405,6 +405,7 @@ __global__ void __launch_bounds__(kPsThreads, CPS)
     tc_gemm_ps_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB,
                       float2* __restrict__ C, int64_t M, int64_t N, int nkb, ProdList prods,
                       int* __restrict__ errflag, PlaneScales sc, int tiles_n) {
+  chained_wait();
   // N tile fastest: the CTAs that run together share their A tiles through L2
   tc_tile_ps<BN, P, CPS>(&tmA, &tmB, C, M, N, nkb, prods, (int)(blockIdx.x / tiles_n) * BM, (int)(blockIdx.x % tiles_n) * BN,
                     errflag, sc);
@@ -509,6 +510,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(128, 1)
     tc_gemm_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB,
                         float2* __restrict__ C, int64_t M, int64_t N, int nkb, ProdList prods,
                         int* __restrict__ errflag, PlaneScales sc, int tiles_n) {
+  chained_wait();
   using CF = CfgPair<P>;
   extern __shared__ __align__(1024) uint8_t smem_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) &
@@ -763,6 +765,7 @@ constexpr int kPersistThreads = 32 * (2 + kPersistEpiWarps);
 template <int BN, int P, int G>
 __global__ void __launch_bounds__(kPersistThreads, 1) tc_gemm_persist_kernel(const __grid_constant__ GroupedTc<G> g,
                                                                              int* __restrict__ errflag) {
+  chained_wait();
   using CF = CfgPersist<BN, P>;
   using B2 = Cfg2<BN, P, 1>;
   extern __shared__ __align__(1024) uint8_t smem_raw[];
@@ -1013,7 +1016,7 @@ cudaError_t launch_ps(const TcGemmArgs& a, int* errflag, cudaStream_t s, std::st
   const int64_t gy = (2 * a.N + BN - 1) / BN;
   if (gx * gy > 2147483647LL) return cudaErrorInvalidConfiguration;
   const PlaneScales sc{a.a_max, a.b_max, a.fp16};
-  tc_gemm_ps_kernel<BN, P, CPS><<<(unsigned)(gx * gy), kPsThreads, CF::SMEM, s>>>(tmA, tmB, a.C, a.M, a.N, nkb, pl, errflag, sc,
+  launch_chained(tc_gemm_ps_kernel<BN, P, CPS>, dim3((unsigned)(gx * gy)), dim3(kPsThreads), CF::SMEM, s, tmA, tmB, a.C, a.M, a.N, nkb, pl, errflag, sc,
                                                                      (int)gy);
   return cudaGetLastError();
 }
@@ -1080,7 +1083,7 @@ cudaError_t launch_persist_g(const TcGemmArgs* probs, int nprob, int* errflag, c
       g.prods.b[i] = i < probs[0].nprod ? probs[0].prod_b[i] : 0;
     }
     if (tiles == 0) continue;
-    tc_gemm_persist_kernel<BN, P, G><<<std::min(tiles, grid), kPersistThreads, CF::SMEM, s>>>(g, errflag);
+    launch_chained(tc_gemm_persist_kernel<BN, P, G>, dim3(std::min(tiles, grid)), dim3(kPersistThreads), CF::SMEM, s, g, errflag);
     cudaError_t e = cudaGetLastError();
     if (e != cudaSuccess) return e;
   }
@@ -1116,7 +1119,7 @@ cudaError_t launch_pair(const TcGemmArgs& a, int* errflag, cudaStream_t s, std::
   const int64_t tiles_n = (2 * a.N + CF::TILE_N - 1) / CF::TILE_N;
   if (2 * pairs_m * tiles_n > 2147483647LL) return cudaErrorInvalidConfiguration;
   const PlaneScales sc{a.a_max, a.b_max, a.fp16};
-  tc_gemm_pair_kernel<P><<<(unsigned)(2 * pairs_m * tiles_n), 128, CF::SMEM, s>>>(tmA, tmB, a.C, a.M, a.N, nkb, pl,
+  launch_chained(tc_gemm_pair_kernel<P>, dim3((unsigned)(2 * pairs_m * tiles_n)), dim3(128), CF::SMEM, s, tmA, tmB, a.C, a.M, a.N, nkb, pl,
                                                                                   errflag, sc, (int)tiles_n);
   return cudaGetLastError();
 }

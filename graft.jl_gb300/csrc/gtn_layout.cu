@@ -229,6 +229,7 @@ __device__ __forceinline__ void gather_tab_tile(const Tin* __restrict__ T, const
 template <typename Tin, class Writer, int TM, int TK>
 __global__ void __launch_bounds__(256) gather_tab_kernel(const Tin* __restrict__ T, TabOff off, int64_t M,
                                                          int64_t K, int64_t Kw, int m_fast, Writer w) {
+  chained_wait();
   __shared__ SmemTab<Tin, TM, TK> sm;
   gather_tab_tile<Tin, Writer, TM, TK>(T, off, M, K, Kw, m_fast, w, (int64_t)blockIdx.x * TM,
                                        (int64_t)blockIdx.y * TK, sm);
@@ -241,13 +242,11 @@ cudaError_t launch_gather_tab(const Tin* T, const int64_t* om, const int64_t* ok
   if (m_fast) {
     const int64_t gy = (Kw + 7) / 8, gx = (M + 255) / 256;
     if (gy > 65535 || gx > 2147483647LL) return cudaErrorInvalidConfiguration;
-    gather_tab_kernel<Tin, Writer, 256, 8><<<dim3((unsigned)gx, (unsigned)gy), dim3(32, 8), 0, s>>>(
-        T, TabOff{om, ok}, M, K, Kw, m_fast, w);
+    launch_chained(gather_tab_kernel<Tin, Writer, 256, 8>, dim3((unsigned)gx, (unsigned)gy), dim3(32, 8), 0, s, T, TabOff{om, ok}, M, K, Kw, m_fast, w);
   } else {
     const int64_t gy = (Kw + 31) / 32, gx = (M + 63) / 64;
     if (gy > 65535 || gx > 2147483647LL) return cudaErrorInvalidConfiguration;
-    gather_tab_kernel<Tin, Writer, 64, 32><<<dim3((unsigned)gx, (unsigned)gy), dim3(32, 8), 0, s>>>(
-        T, TabOff{om, ok}, M, K, Kw, m_fast, w);
+    launch_chained(gather_tab_kernel<Tin, Writer, 64, 32>, dim3((unsigned)gx, (unsigned)gy), dim3(32, 8), 0, s, T, TabOff{om, ok}, M, K, Kw, m_fast, w);
   }
   return cudaGetLastError();
 }
@@ -256,6 +255,7 @@ template <typename Tin, class Writer>
 __global__ void __launch_bounds__(256) gather_tile_kernel(const Tin* __restrict__ T, GroupSpec mg,
                                                           GroupSpec kg, int64_t M, int64_t K,
                                                           int64_t Kw, int m_fast, Writer w) {
+  chained_wait();
   __shared__ Smem32<Tin> sm;
   gather_tile<Tin, Writer>(T, mg, kg, M, K, Kw, m_fast, w, (int64_t)blockIdx.x * 32, (int64_t)blockIdx.y * 32, sm);
 }
@@ -274,7 +274,7 @@ cudaError_t launch_gather(const Tin* T, const GroupSpec& mg, const GroupSpec& kg
   const int64_t gx = (M + 31) / 32;
   if (gy > 65535 || gx > 2147483647LL) return cudaErrorInvalidConfiguration;
   dim3 grid((unsigned)gx, (unsigned)gy), block(32, 8);
-  gather_tile_kernel<Tin, Writer><<<grid, block, 0, s>>>(T, mg, kg, M, K, Kw,
+  launch_chained(gather_tile_kernel<Tin, Writer>, dim3(grid), dim3(block), 0, s, T, mg, kg, M, K, Kw,
                                                          choose_m_fast(mg, kg) ? 1 : 0, w);
   return cudaGetLastError();
 }
@@ -494,6 +494,7 @@ struct DigitRowWriter {
 __global__ void __launch_bounds__(256) pack_b_digits_kernel(const double2* __restrict__ B, int64_t N, int64_t K,
                                                             int64_t nkb, float* __restrict__ bexp,
                                                             unsigned char* __restrict__ out, int* flag) {
+  chained_wait();
   __shared__ float se[8];
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int64_t n0 = (int64_t)blockIdx.x * 8;
@@ -800,6 +801,7 @@ __global__ void __launch_bounds__(256, 2) small_contract64_kernel(const double2*
                                                                   GroupSpec kg, int64_t M, int K, int N,
                                                                   const double2* __restrict__ B,
                                                                   double2* __restrict__ C) {
+  chained_wait();
   small_contract64_body<NB>(A, mg, kg, M, K, N, B, C, blockIdx.x, gridDim.x);
 }
 
@@ -808,6 +810,7 @@ __global__ void __launch_bounds__(256) small_contract_kernel(const T* __restrict
                                                              GroupSpec kg, int64_t M, int K, int N,
                                                              const T* __restrict__ B,
                                                              T* __restrict__ C) {
+  chained_wait();
   small_contract_body<T, NB>(A, mg, kg, M, K, N, B, C, blockIdx.x, gridDim.x);
 }
 
@@ -832,13 +835,13 @@ cudaError_t launch_small(const T* A, const GroupSpec& mg, const GroupSpec& kg, i
       attr = true;
     }
     if (N <= 8) {
-      small_contract64_kernel<8><<<(unsigned)blocks, threads, small64_smem(K, N, 8, threads), s>>>(A, mg, kg, M, K, N, B, C);
+      launch_chained(small_contract64_kernel<8>, dim3((unsigned)blocks), dim3(threads), small64_smem(K, N, 8, threads), s, A, mg, kg, M, K, N, B, C);
     } else {
-      small_contract64_kernel<16><<<(unsigned)blocks, threads, small64_smem(K, N, 16, threads), s>>>(A, mg, kg, M, K, N, B, C);
+      launch_chained(small_contract64_kernel<16>, dim3((unsigned)blocks), dim3(threads), small64_smem(K, N, 16, threads), s, A, mg, kg, M, K, N, B, C);
     }
   } else {
     const int64_t blocks = std::min<int64_t>((M + 255) / 256, 152 * 16);
-    small_contract_kernel<T, 8><<<(unsigned)blocks, 256, smem, s>>>(A, mg, kg, M, K, N, B, C);
+    launch_chained(small_contract_kernel<T, 8>, dim3((unsigned)blocks), dim3(256), smem, s, A, mg, kg, M, K, N, B, C);
   }
   return cudaGetLastError();
 }
@@ -1393,6 +1396,7 @@ template <typename Tin, int TR, class Off, class W>
 __global__ void __launch_bounds__(256) split_rows_kernel(const Tin* __restrict__ T, Off off, int64_t M, int64_t K,
                                                          int64_t Kp, int kc, int cs, int m_fast, W w,
                                                          float* __restrict__ amax) {
+  chained_wait();
   extern __shared__ __align__(16) unsigned char smraw[];
   const int pitch = split_rows_pitch<Tin>(kc);  // odd: the row-strided staging stores spread over banks
   Tin* tile = reinterpret_cast<Tin*>(smraw);
@@ -1529,13 +1533,15 @@ cudaError_t launch_split_rows_t(const Tin* T, const Off& off, int64_t M, int64_t
   cfg.blockDim = dim3(256, 1, 1);
   cfg.dynamicSmemBytes = smem;
   cfg.stream = s;
-  cudaLaunchAttribute attrs[1];
+  cudaLaunchAttribute attrs[2];
+  attrs[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;  // as launch_chained
+  attrs[1].val.programmaticStreamSerializationAllowed = 1;
   attrs[0].id = cudaLaunchAttributeClusterDimension;
   attrs[0].val.clusterDim.x = (unsigned)cs;
   attrs[0].val.clusterDim.y = 1;
   attrs[0].val.clusterDim.z = 1;
   cfg.attrs = attrs;
-  cfg.numAttrs = 1;
+  cfg.numAttrs = 2;
   return cudaLaunchKernelEx(&cfg, kern, T, off, M, K, Kp, kc, cs, m_fast, w, amax);
 }
 
@@ -2022,7 +2028,7 @@ cudaError_t launch_pack_b_digits(const double2* B, int64_t N, int64_t K, void* o
   if (N <= 0) return cudaSuccess;
   const int64_t blocks = (N + 7) / 8;
   if (blocks > 2147483647LL) return cudaErrorInvalidConfiguration;
-  pack_b_digits_kernel<<<(unsigned)blocks, 256, 0, s>>>(B, N, K, (K + 7) / 8, bexp, static_cast<unsigned char*>(out),
+  launch_chained(pack_b_digits_kernel, dim3((unsigned)blocks), dim3(256), 0, s, B, N, K, (K + 7) / 8, bexp, static_cast<unsigned char*>(out),
                                                        flag);
   return cudaGetLastError();
 }
