@@ -1083,7 +1083,10 @@ cudaError_t launch_persist_g(const TcGemmArgs* probs, int nprob, int* errflag, c
       g.prods.b[i] = i < probs[0].nprod ? probs[0].prod_b[i] : 0;
     }
     if (tiles == 0) continue;
-    launch_chained(tc_gemm_persist_kernel<BN, P, G>, dim3(std::min(tiles, grid)), dim3(kPersistThreads), CF::SMEM, s, g, errflag);
+    // A long launch gains nothing from being chained, and its CTAs would take the SMs in the order in
+    // which the kernel before it leaves them (fp16x3 two-site map at d = 1024, 14 to 68 waves a step:
+    // 7.78 ms in order, 7.82 chained).
+    launch_chained_if(tiles <= 8 * grid, tc_gemm_persist_kernel<BN, P, G>, dim3(std::min(tiles, grid)), dim3(kPersistThreads), CF::SMEM, s, g, errflag);
     cudaError_t e = cudaGetLastError();
     if (e != cudaSuccess) return e;
   }

@@ -39,7 +39,8 @@ struct OutView {
 // kept: whatever is launched without this waits for the whole kernel as usual.  Saves about
 // 1.2 us a launch (two-site FP64 map of a chain at bond 250: 11 launches, 268 -> 255 us).
 template <class... P, class... A>
-inline cudaError_t launch_chained(void (*kern)(P...), dim3 grid, dim3 block, size_t smem, cudaStream_t s, A&&... args) {
+inline cudaError_t launch_chained_if(bool chained, void (*kern)(P...), dim3 grid, dim3 block, size_t smem,
+                                     cudaStream_t s, A&&... args) {
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = grid;
   cfg.blockDim = block;
@@ -49,8 +50,12 @@ inline cudaError_t launch_chained(void (*kern)(P...), dim3 grid, dim3 block, siz
   at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
   at[0].val.programmaticStreamSerializationAllowed = 1;
   cfg.attrs = at;
-  cfg.numAttrs = 1;
+  cfg.numAttrs = chained ? 1 : 0;
   return cudaLaunchKernelEx(&cfg, kern, std::forward<A>(args)...);
+}
+template <class... P, class... A>
+inline cudaError_t launch_chained(void (*kern)(P...), dim3 grid, dim3 block, size_t smem, cudaStream_t s, A&&... args) {
+  return launch_chained_if(true, kern, grid, block, smem, s, std::forward<A>(args)...);
 }
 #ifdef __CUDACC__
 __device__ __forceinline__ void chained_wait() {

@@ -173,9 +173,10 @@ __device__ __forceinline__ void gather_tile(const Tin* __restrict__ T, const Gro
 // before the transpose (the gathers are latency-bound at 32 x 32).
 constexpr int kTabRows = 64;
 
-// TM x TK tile of 2048 elements (8 loads in flight per thread).  64 x 32 in general; 256 x 8
-// when the rows are the unit-stride index, so that every k reads a 4 KB contiguous run
-// (a 32-wide tile over far-apart k legs touches 32 pages per tile).
+// TM x TK tile of 2048 elements (8 loads in flight per thread).  64 x 32 in general; 128 x 16
+// when the rows are the unit-stride index, so that every k reads a run of 1 or 2 KB (a 32-wide
+// tile over far-apart k legs touches 32 pages per tile) and every row is written in 256 bytes
+// (256 x 8: 64 uneven one-site maps 707 us, 702 so).
 template <typename Tin, int TM, int TK> struct SmemTab {
   int64_t offM[TM];
   int64_t offK[TK];
@@ -235,18 +236,23 @@ __global__ void __launch_bounds__(256) gather_tab_kernel(const Tin* __restrict__
                                        (int64_t)blockIdx.y * TK, sm);
 }
 
+// Gathers and splits of up to 2^24 elements (60 us) are chained launches.  Longer ones gain nothing
+// from it and lose some: fp16x3 two-site map at d = 1024 (splits of 34 to 168 million) 7.68 ms with
+// its launches in order, 7.82 all chained.
+inline bool chain_gather(int64_t M, int64_t K) { return M * K <= ((int64_t)1 << 24); }
+
 template <typename Tin, class Writer>
 cudaError_t launch_gather_tab(const Tin* T, const int64_t* om, const int64_t* ok, int64_t M, int64_t K, int64_t Kw,
                               int m_fast, const Writer& w, cudaStream_t s) {
   if (M <= 0 || Kw <= 0) return cudaSuccess;
   if (m_fast) {
-    const int64_t gy = (Kw + 7) / 8, gx = (M + 255) / 256;
+    const int64_t gy = (Kw + 15) / 16, gx = (M + 127) / 128;
     if (gy > 65535 || gx > 2147483647LL) return cudaErrorInvalidConfiguration;
-    launch_chained(gather_tab_kernel<Tin, Writer, 256, 8>, dim3((unsigned)gx, (unsigned)gy), dim3(32, 8), 0, s, T, TabOff{om, ok}, M, K, Kw, m_fast, w);
+    launch_chained_if(chain_gather(M, Kw), gather_tab_kernel<Tin, Writer, 128, 16>, dim3((unsigned)gx, (unsigned)gy), dim3(32, 8), 0, s, T, TabOff{om, ok}, M, K, Kw, m_fast, w);
   } else {
     const int64_t gy = (Kw + 31) / 32, gx = (M + 63) / 64;
     if (gy > 65535 || gx > 2147483647LL) return cudaErrorInvalidConfiguration;
-    launch_chained(gather_tab_kernel<Tin, Writer, 64, 32>, dim3((unsigned)gx, (unsigned)gy), dim3(32, 8), 0, s, T, TabOff{om, ok}, M, K, Kw, m_fast, w);
+    launch_chained_if(chain_gather(M, Kw), gather_tab_kernel<Tin, Writer, 64, 32>, dim3((unsigned)gx, (unsigned)gy), dim3(32, 8), 0, s, T, TabOff{om, ok}, M, K, Kw, m_fast, w);
   }
   return cudaGetLastError();
 }
@@ -274,7 +280,7 @@ cudaError_t launch_gather(const Tin* T, const GroupSpec& mg, const GroupSpec& kg
   const int64_t gx = (M + 31) / 32;
   if (gy > 65535 || gx > 2147483647LL) return cudaErrorInvalidConfiguration;
   dim3 grid((unsigned)gx, (unsigned)gy), block(32, 8);
-  launch_chained(gather_tile_kernel<Tin, Writer>, dim3(grid), dim3(block), 0, s, T, mg, kg, M, K, Kw,
+  launch_chained_if(chain_gather(M, Kw), gather_tile_kernel<Tin, Writer>, dim3(grid), dim3(block), 0, s, T, mg, kg, M, K, Kw,
                                                          choose_m_fast(mg, kg) ? 1 : 0, w);
   return cudaGetLastError();
 }
@@ -886,7 +892,7 @@ __global__ void __launch_bounds__(256) gather_grouped_kernel(const __grid_consta
 }
 
 // The same jobs with offset tables (maps that keep them): no index decomposition, and tiles of
-// 2048 elements with eight loads in flight per thread (64 x 32, or 256 x 8 where the rows are
+// 2048 elements with eight loads in flight per thread (64 x 32, or 128 x 16 where the rows are
 // the unit-stride index).  The 32 x 32 tiles above spend their time on 64-bit divisions and one
 // load's latency after the other: 64 uneven one-site maps, the longest split (320 MB moved)
 // 115 us there, 99 us here, and 66 us with the packed conversions and pairs of SplitWriter.
@@ -906,7 +912,7 @@ struct GatherTabJobsP {
 };
 template <typename Tin> union SmemTabs {
   SmemTab<Tin, 64, 32> a;
-  SmemTab<Tin, 256, 8> b;
+  SmemTab<Tin, 128, 16> b;
   __device__ SmemTabs() {}
 };
 template <typename Tin, class Writer>
@@ -915,7 +921,7 @@ __device__ __forceinline__ void gather_tab_job(const GatherTabJob& J, const Writ
   const Tin* T = static_cast<const Tin*>(J.T);
   const TabOff off{J.om, J.ok};
   if (J.m_fast)
-    gather_tab_tile<Tin, Writer, 256, 8>(T, off, J.M, J.K, J.Kw, 1, w, (int64_t)tm * 256, (int64_t)tk * 8, sm.b);
+    gather_tab_tile<Tin, Writer, 128, 16>(T, off, J.M, J.K, J.Kw, 1, w, (int64_t)tm * 128, (int64_t)tk * 16, sm.b);
   else
     gather_tab_tile<Tin, Writer, 64, 32>(T, off, J.M, J.K, J.Kw, 0, w, (int64_t)tm * 64, (int64_t)tk * 32, sm.a);
 }
@@ -1541,7 +1547,7 @@ cudaError_t launch_split_rows_t(const Tin* T, const Off& off, int64_t M, int64_t
   attrs[0].val.clusterDim.y = 1;
   attrs[0].val.clusterDim.z = 1;
   cfg.attrs = attrs;
-  cfg.numAttrs = 2;
+  cfg.numAttrs = chain_gather(M, Kp) ? 2 : 1;
   return cudaLaunchKernelEx(&cfg, kern, T, off, M, K, Kp, kc, cs, m_fast, w, amax);
 }
 
@@ -1767,7 +1773,7 @@ static cudaError_t launch_gather_tab_grouped_t(const GatherJob* jobs, int njobs,
     int64_t tiles = 0;
     for (int q = 0; q < cnt; ++q) {
       const GatherJob& J = jobs[base + q];
-      const int TM = J.tab.m_fast ? 256 : 64, TK = 2048 / TM;
+      const int TM = J.tab.m_fast ? 128 : 64, TK = 2048 / TM;
       g.j[q] = GatherTabJob{J.T, J.tab.om, J.tab.ok, J.out, J.amax, J.M, J.K, J.Kw, J.ld > 0 ? J.ld : J.Kw,
                             J.pstride, J.nplanes, J.tab.m_fast};
       g.tiles_m[q] = (int)((J.M + TM - 1) / TM);

@@ -1,6 +1,6 @@
 """More maps in a batch than one grouped launch takes (64 tensor-core problems, 128 table-driven
 gathers): the last map of a launch, the first of the next and every other match the single
-application, with rows and columns at the edges of the gather tiles (64 x 32, 256 x 8)."""
+application, with rows and columns at the edges of the gather tiles (64 x 32, 128 x 16)."""
 import numpy as np
 import pytest
 
