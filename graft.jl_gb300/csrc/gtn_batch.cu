@@ -49,7 +49,7 @@ int map_run_batched(gtn_map* maps_in, int n, int precision, const double2* const
   if (tc)
     for (gtn_map m : maps)
       for (auto& st : m->steps)
-        if (!st.small && (!st.bpl || st.bplanes != P || st.bfp16 != (f16 ? 1 : 0) || (f16 && !m->amax)))
+        if (!st.narrow && (!st.bpl || st.bplanes != P || st.bfp16 != (f16 ? 1 : 0) || (f16 && !m->amax)))
           return set_err(ctx, GTN_ERR_INVALID, "a batched map was not created for this tcgen05 precision");
   std::vector<const void*> cur(n);
   std::vector<bool> cur64(n, true);
@@ -65,7 +65,7 @@ int map_run_batched(gtn_map* maps_in, int n, int precision, const double2* const
     std::vector<GatherJob> conv;
     for (int i = 0; i < n; ++i) {
       const PlanStep& st0 = maps[i]->steps[0];
-      if (st0.small || !tc) {
+      if (st0.narrow || !tc) {
         GatherJob J;
         std::memset(&J, 0, sizeof(J));
         flat_groups(maps[i]->x_elems, &J.mg, &J.kg, &J.M, &J.K);
@@ -97,7 +97,7 @@ int map_run_batched(gtn_map* maps_in, int n, int precision, const double2* const
       void* out = (si & 1) ? m->buf1 : m->buf0;
       if (out == cur[i]) out = (out == m->buf0) ? m->buf1 : m->buf0;
       outs[i] = out;
-      if (st.small) {
+      if (st.narrow) {
         SmallJob J;
         J.A = cur[i];
         J.mg = st.mg;

@@ -495,7 +495,8 @@ int multidot_blocks(gtn_ctx ctx);
 // ---- plans (gtn_plan.cpp) ----------------------------------------------------------
 struct PlanStep {
   int operand;             // static operand absorbed
-  bool small;              // strided SIMT path (no permute)
+  bool narrow;             // fits the small-K kernel (no permute), which FP32 and batched steps take then
+  bool small;              // and takes it in a single FP64 application
   bool tc;                 // tcgen05 path (mixed precisions only)
   int64_t M, K, N, Kp;
   GroupSpec mg, kg;        // access of the running tensor as [M, K]

@@ -190,12 +190,26 @@ namespace {
 
 constexpr int64_t kMaxCombined = int64_t(1) << 22;  // elements of a pre-contracted static
 
+// Narrow products (K <= 64 and a static of at most 48 KB) run in the small-K kernel.  In an FP64 plan
+// only those do that may be a TTNO tensor (up to 512 entries) and keep the FP64 pipes busy for 6 us
+// if dense: an environment has no zeros to skip, and few rows, a thread each in passes of 16
+// outputs, leave the pipes waiting.  The others run in place on the FP64 pipes, not on digit planes:
+// those are accurate to a row's largest entry, which a short sparse sum can be far below.  One-site
+// map of the 31-site binary tree, small-K kernel against in place: bond 12 392 -> 43 us, 16 680 -> 92,
+// 24 1493 -> 261; two-site map of a star at bond 2 198 -> 9.6.
+bool narrow(double K, double N) {
+  return K <= kSmallK && small_contract_fits((int)K, (int)std::min(N, 1048576.0), sizeof(double2));
+}
+bool narrow_step(int prec, double M, double K, double N) {
+  return narrow(K, N) && !(prec == GTN_PREC_FP64 && (N * K > 512 || f64_pipe_time(M, N, K) < 10e-6));
+}
+
 double est_step_time(int prec, double M, double K, double N) {
   const bool fp64 = prec == GTN_PREC_FP64;
   const double e = fp64 ? 16.0 : 8.0;
   const double flops = 8.0 * M * K * N;
   const double hbm = 5e12;
-  const bool small = K <= kSmallK && small_contract_fits((int)K, (int)std::min(N, 1048576.0), sizeof(double2));
+  const bool small = narrow(K, N);
   double t = 5e-6;  // launch and tail
   if (small) return t + (M * K + M * N) * e / hbm + flops / (fp64 ? 1.1e12 : 15e12);
   if (fp64) return t + flops / 1.1e12 + (2 * M * K + M * N) * e / hbm;
@@ -216,9 +230,10 @@ double est_step_time(int prec, double M, double K, double N) {
 // and the digit planes in FP64; a one-shot contraction packs the absorbed operand too.
 double plan_step_time(int precision, double M, double K, double N, bool oneshot) {
   const double pack = oneshot ? 10e-6 + N * K * 90.0 / 4e12 : 0.0;
-  const bool small = K <= kSmallK && small_contract_fits((int)K, (int)std::min(N, 1048576.0), sizeof(double2));
+  const bool small = narrow_step(precision, M, K, N);
   if (precision != GTN_PREC_FP64 || small) return est_step_time(precision, M, K, N) + pack;
-  return std::min(f64e_time(M, N, K), f64_pipe_time(M, N, K)) + M * N * 16.0 / 5e12 + pack;
+  const double pipe = f64_pipe_time(M, N, K);
+  return (narrow(K, N) ? pipe : std::min(f64e_time(M, N, K), pipe)) + M * N * 16.0 / 5e12 + pack;
 }
 
 namespace {
@@ -516,9 +531,10 @@ int plan_build(gtn_ctx ctx, int n, const int* ranks, const int64_t* dims, const 
     st.macs = (double)st.M * (double)st.N * (double)st.K;
     if (!make_group(DT, freeT, &st.mg) || !make_group(DT, sh, &st.kg))
       return set_err(ctx, GTN_ERR_UNSUPPORTED, "too many non-contiguous leg groups");
-    st.small = st.K <= kSmallK && small_contract_fits((int)st.K, (int)std::min<int64_t>(st.N, 1 << 20), sizeof(double2));
+    st.narrow = narrow((double)st.K, (double)st.N);
+    st.small = narrow_step(precision, (double)st.M, (double)st.K, (double)st.N);
     st.tc = tc && !st.small;
-    st.dg = !st.small && st.K <= kF64eMaxK && ((f64e && statics) || (dg64 && f64e_time(st.M, st.N, st.K) < f64_pipe_time(st.M, st.N, st.K)));
+    st.dg = !st.small && (f64e || !st.narrow) && st.K <= kF64eMaxK && ((f64e && statics) || (dg64 && f64e_time(st.M, st.N, st.K) < f64_pipe_time(st.M, st.N, st.K)));
     st.Kp = ((st.K + 31) / 32) * 32;
     // C legs: S free (S order), then T free (T order)
     for (int b : freeS) { st.out_labels.push_back(LS[b]); st.out_dims.push_back(DS[b]); }
@@ -741,13 +757,13 @@ int map_run(gtn_map map, int precision, const double2* x, double2* y) {
   const bool tc = is_tc(precision);
   if (tc) {
     for (auto& st : map->steps)
-      if (!st.small && (!st.bpl || st.bplanes != nplanes_of(precision) || st.bfp16 != (is_fp16(precision) ? 1 : 0)))
+      if (!st.narrow && (!st.bpl || st.bplanes != nplanes_of(precision) || st.bfp16 != (is_fp16(precision) ? 1 : 0)))
         return set_err(ctx, GTN_ERR_INVALID, "map was not created for this tcgen05 precision");
   }
   const bool f64e = is_f64e(precision);
   if (f64e) {
     for (auto& st : map->steps)
-      if (!st.small && st.K <= kF64eMaxK && (!st.bdig || !map->amax))
+      if (!st.narrow && st.K <= kF64eMaxK && (!st.bdig || !map->amax))
         return set_err(ctx, GTN_ERR_INVALID, "map was not created for the FP64-grade tensor-core precision");
   }
   const bool fp64 = precision == GTN_PREC_FP64 || f64e;  // complex FP64 running tensors
@@ -820,7 +836,7 @@ int map_run(gtn_map map, int precision, const double2* x, double2* y) {
         if (direct && e == cudaSuccess) return GTN_OK;
       }
     } else {
-      if (cur64 && (st.small || !tc)) {
+      if (cur64 && (st.narrow || !tc)) {
         // the FP32 kernels read complex FP32: convert the FP64 input once
         void* conv = bufs[(i + 1) & 1];
         int64_t blocks = std::min<int64_t>((map->x_elems + 255) / 256, 152 * 8);
@@ -834,7 +850,7 @@ int map_run(gtn_map map, int precision, const double2* x, double2* y) {
         cur64 = false;
         if (e != cudaSuccess) break;
       }
-      if (st.small) {
+      if (st.narrow) {
         prof_begin(s);
         e = launch_small_contract_c64(static_cast<const float2*>(cur), st.mg, st.kg, st.M, (int)st.K,
                                       (int)st.N, st.b32, static_cast<float2*>(out), s);
