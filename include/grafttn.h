@@ -40,16 +40,17 @@ typedef enum {
 /* Arithmetic of a map application.  The Krylov vectors and all orthogonalisation are
  * FP64 in every mode; the mode selects how the contraction chain is computed. */
 typedef enum {
-  GTN_PREC_FP64 = 0,       /* complex FP64 throughout (DFMA SIMT kernels) */
+  GTN_PREC_FP64 = 0,       /* complex FP64 throughout: FP64 pipes, or exact sums of the 34 digit
+                              products of level <= 7 (base 256) where K > 64 and they are faster */
   GTN_PREC_BF16X6 = 1,     /* tcgen05: 3 bf16 slices per operand, 6 products, FP32 accum */
   GTN_PREC_BF16X3 = 2,     /* tcgen05: 2 bf16 slices per operand, 3 products, FP32 accum */
   GTN_PREC_FP32 = 3,       /* complex FP32 SIMT kernels (diagnostic mode) */
   GTN_PREC_FP16X3 = 4,     /* tcgen05: 2 fp16 slices per operand (22 bits, power-of-two row
                               scales), 3 products, FP32 accum */
-  GTN_PREC_FP64E = 5       /* FP64-grade on the tensor cores: 7 integer base-128 digits per
+  GTN_PREC_FP64E = 5       /* FP64-grade on the tensor cores: 7 integer base-256 digits per
                               operand (power-of-two row scales), the 28 digit products of
-                              level <= 6 summed exactly in FP32 over chunks of 256 k and
-                              combined in double-float; about 1e-14 relative (dense maps and
+                              level <= 6 summed exactly (FP32 over 128 or 256 k, then 64-bit
+                              integers); about 4e-16 in the 2-norm (dense maps and
                               one-shot contractions) */
 } gtn_precision;
 
@@ -71,8 +72,7 @@ int64_t gtn_ctx_launch_count(gtn_ctx ctx);
 int gtn_ctx_sync(gtn_ctx ctx);
 /* Precision of the matrix products inside the factorisations of this context (the Gram
  * matrix and the right factor of the truncated SVD's Gram route, gtn_svd_trunc):
- * GTN_PREC_FP64 (default, FP64 SIMT) or GTN_PREC_FP64E (the FP64-grade tensor-core GEMM,
- * about 1e-14 relative to sum |a||b|).  The eigen- and QR decompositions stay cuSOLVER FP64.
+ * GTN_PREC_FP64 (default) or GTN_PREC_FP64E, as for contractions.  The eigen- and QR decompositions stay cuSOLVER FP64.
  * No counterpart in the reference (its factorisations are LAPACK calls on the host). */
 int gtn_ctx_set_linalg_precision(gtn_ctx ctx, int precision);
 int gtn_ctx_linalg_precision(gtn_ctx ctx);
