@@ -139,11 +139,16 @@ __device__ __forceinline__ double rsqrt_step(double x, double r) {
   return fma(r, e * fma(e, 0.375, 0.5), r);
 }
 
+// Squared column norms below this are formed on a scaled column: above it, squares lost to
+// underflow (below 2^-1074 each) are less than 2^-160 of the sum, and its reciprocal is in range.
+constexpr double kTinySquare = 0x1p-900;
+__device__ __forceinline__ int exponent_of(double x) { return (__double2hiint(x) >> 20) & 0x7ff; }
+
 __global__ void jacobi_exponent_kernel(const double2* __restrict__ A, int64_t n, JacobiState* st) {
   int e = 0;
   for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x) {
     const double2 a = A[i];
-    e = max(e, max((__double2hiint(a.x) >> 20) & 0x7ff, (__double2hiint(a.y) >> 20) & 0x7ff));
+    e = max(e, max(exponent_of(a.x), exponent_of(a.y)));
   }
   for (int o = 16; o > 0; o >>= 1) e = max(e, __shfl_xor_sync(0xffffffffu, e, o));
   if ((threadIdx.x & 31) == 0) atomicMax(&st->max_exp, e);
@@ -188,6 +193,7 @@ __global__ void __launch_bounds__(kT, 3)
   __shared__ double red[2][kT];
   __shared__ double tot[2];
   __shared__ double2 alpha;
+  __shared__ int emax;
   const int k = blockIdx.x, tid = threadIdx.x, e = st->max_exp;
   double2 a[kQE], v[kQE];
 #pragma unroll
@@ -228,17 +234,51 @@ __global__ void __launch_bounds__(kT, 3)
   if (tid < 32) warp_sums<2>(red, tot);
   __syncthreads();
   // LAPACK's reflector: H = 1 - tau v v^H, H^H a = beta e_k, v_k = 1
-  const double2 al = alpha;
-  const double r2 = fma(al.x, al.x, fma(al.y, al.y, tot[0]));
+  double2 al = alpha;
+  double r2 = fma(al.x, al.x, fma(al.y, al.y, tot[0]));
+  bool tail = tot[0] != 0.0;
+  const bool tiny = r2 < kTinySquare;  // the same for every thread
+  int ec = 0;
+  if (tiny) {
+    // What is left of the column lies so far below the matrix's largest entry that its squares (or
+    // the reciprocal of their sum) leave the FP64 range: again on the column scaled by its own
+    // largest exponent.  A reflector depends only on the column's direction.
+    if (tid == 0) emax = 0;
+    __syncthreads();
+#pragma unroll
+    for (int q = 0; q < kQE; ++q) {
+      const int x = tid + q * kT;
+      if (x >= k && x < rows) atomicMax(&emax, max(exponent_of(a[q].x), exponent_of(a[q].y)));
+    }
+    __syncthreads();
+    ec = emax;
+    x2 = 0.0;
+#pragma unroll
+    for (int q = 0; q < kQE; ++q) {
+      const int x = tid + q * kT;
+      if (x < k) continue;
+      a[q] = make_double2(scaled(a[q].x, ec), scaled(a[q].y, ec));
+      if (x > k) x2 = fma(a[q].x, a[q].x, fma(a[q].y, a[q].y, x2));
+      if (x == k) alpha = a[q];
+    }
+    red[0][tid] = x2;
+    __syncthreads();
+    if (tid < 32) warp_sums<2>(red, tot);
+    __syncthreads();
+    al = alpha;
+    r2 = fma(al.x, al.x, fma(al.y, al.y, tot[0]));
+    tail = tot[0] != 0.0;
+  }
   double2 tk = make_double2(0.0, 0.0), sc = make_double2(0.0, 0.0);
   double beta = al.x;
-  if (tot[0] != 0.0 || al.y != 0.0) {
+  if (tail || al.y != 0.0) {
     beta = al.x >= 0.0 ? -sqrt(r2) : sqrt(r2);
     tk = make_double2((beta - al.x) / beta, -al.y / beta);
     const double2 d = make_double2(al.x - beta, al.y);
     const double i2 = 1.0 / fma(d.x, d.x, d.y * d.y);
     sc = make_double2(d.x * i2, -d.y * i2);
   }
+  if (tiny) beta = scalbn(beta, max(ec, 1) - 1023);
   if (tid < 2) st_word(tau + 2 * k + tid, tid == 0 ? tk.x : tk.y, 1);
 #pragma unroll
   for (int q = 0; q < kQE; ++q) {
@@ -544,6 +584,8 @@ int jacobi_svd_run(gtn_ctx ctx, int64_t m, int64_t n, const double2* A, void* ws
   const int rc = gtn_ctx_sync(ctx);
   if (rc != GTN_OK) return rc;
   if (hst.sweeps >= kMaxSweeps) return GTN_ERR_UNSUPPORTED;  // did not converge
+  for (double v : hn)
+    if (!std::isfinite(v)) return GTN_ERR_UNSUPPORTED;  // an infinity or NaN in the input: cuSOLVER's
   std::vector<int> ho(k);
   for (int i = 0; i < k; ++i) ho[i] = i;
   std::stable_sort(ho.begin(), ho.end(), [&](int a, int b) { return hn[a] > hn[b]; });
