@@ -141,7 +141,7 @@ int svd_small_launch(gtn_ctx ctx, int64_t m, int64_t n, const double2* A, double
 bool jacobi_svd_applies(int64_t m, int64_t n);
 size_t jacobi_svd_bytes(int64_t m, int64_t n);
 int jacobi_svd_run(gtn_ctx ctx, int64_t m, int64_t n, const double2* A, void* ws, std::vector<double>* S);
-int jacobi_svd_store(gtn_ctx ctx, int64_t m, int64_t n, void* ws, int64_t r, double2* U, double2* Vh);
+int jacobi_svd_store(gtn_ctx ctx, int64_t m, int64_t n, void* ws, int64_t r, int64_t nonzero, double2* U, double2* Vh);
 int qr_small(gtn_ctx ctx, int64_t m, int64_t n, const double2* A, double2* Q, double2* R);
 int qr_tall_cholesky(gtn_ctx ctx, int64_t m, int64_t n, const double2* A, double2* Q, double2* R);
 cudaError_t ctx_red(gtn_ctx ctx, size_t n2);   // ensure d_red/h_red hold n2 double2

@@ -186,7 +186,7 @@ __device__ __forceinline__ void reflect(double2 (&a)[kQE], const double2 (&v)[kQ
 
 // CTA k: column k of W (from the row-major A, scaled) or, without A, of the n x n words X.  Reflector k as words of sequence 1 in
 // refl[k * rows ..] (from row k on) and tau[k]; row k of R conjugated as column entries of L, and
-// the k-th unit column of J, as words of sequence 0 (both zeroed before).
+// the k-th unit column of J, as words of sequence 0 (both zeroed before; without L neither).
 __global__ void __launch_bounds__(kT, 3)
     jacobi_qr_kernel(const double2* __restrict__ A, const Word* __restrict__ X, int tall, int rows, int n, Word* refl,
                      Word* tau, Word* L, Word* J, JacobiState* st, int* errflag) {
@@ -289,6 +289,7 @@ __global__ void __launch_bounds__(kT, 3)
                                : make_double2(fma(sc.x, a[q].x, -sc.y * a[q].y), fma(sc.x, a[q].y, sc.y * a[q].x));
       st_complex(refl + ((int64_t)k * rows + x) * 2, u, 1);
     }
+    if (!L) continue;
     if (x < k) st_complex(L + ((int64_t)x * n + k) * 2, make_double2(a[q].x, -a[q].y), 0);
     if (x == k) {
       st_complex(L + ((int64_t)k * n + k) * 2, make_double2(beta, 0.0), 0);
@@ -459,21 +460,25 @@ __global__ void __launch_bounds__(kT) jacobi_norms_kernel(const Word* __restrict
   if (threadIdx.x == 0) nrm[blockIdx.x] = sqrt(tot[0]);
 }
 
-// CTA (i, 0): the long vector of the i-th largest triplet (positive value), Q times the unit column
-// ord[i] of L; CTA (i, 1): its short one, P times that column of J.  Tall A: U = long (m x r),
-// Vh = short^H; wide: U = short, Vh = long^H.
-__global__ void __launch_bounds__(kT, 3)
-    jacobi_vectors_kernel(const Word* __restrict__ refl0, const Word* __restrict__ tau0,
-                          const Word* __restrict__ refl1, const Word* __restrict__ tau1, const Word* __restrict__ L,
-                          const Word* __restrict__ J, const double* __restrict__ nrm, const int* __restrict__ ord,
-                          int tall, int rows0, int n, int r, double2* __restrict__ U, double2* __restrict__ Vh) {
-  __shared__ double red[2][kT];
-  __shared__ double tot[2];
-  const bool is_long = blockIdx.y == 0;
-  const Word *refl = is_long ? refl0 : refl1, *tau = is_long ? tau0 : tau1, *src = is_long ? L : J;
-  const int i = blockIdx.x, c = ord[i], tid = threadIdx.x, rows = is_long ? rows0 : n;
-  const double s = is_long ? nrm[c] : 1.0;
-  double2 a[kQE], v[kQE], nv[kQE];
+// The unit columns ord[0 .. p - 1] of L as words of sequence 0, then zero columns.
+__global__ void __launch_bounds__(kT) jacobi_unit_columns_kernel(const Word* __restrict__ L,
+                                                                 const double* __restrict__ nrm,
+                                                                 const int* __restrict__ ord, int n, int p,
+                                                                 Word* __restrict__ X) {
+  const int i = blockIdx.x, c = ord[i];
+  const double s = nrm[c];
+  for (int x = threadIdx.x; x < n; x += kT) {
+    const Word* w = L + ((int64_t)c * n + x) * 2;
+    st_complex(X + ((int64_t)i * n + x) * 2, i < p ? make_double2(w[0].v / s, w[1].v / s) : make_double2(0.0, 0.0), 0);
+  }
+}
+
+// a <- H_0 .. H_{count-1} a for the reflectors refl, tau of a `rows`-row matrix.
+__device__ __forceinline__ void apply_reflectors(double2 (&a)[kQE], const Word* __restrict__ refl,
+                                                 const Word* __restrict__ tau, int count, int rows, double (*red)[kT],
+                                                 double* tot) {
+  const int tid = threadIdx.x;
+  double2 v[kQE], nv[kQE];
   auto fetch = [&](int j, double2 (&t)[kQE]) {
 #pragma unroll
     for (int q = 0; q < kQE; ++q) {
@@ -485,19 +490,42 @@ __global__ void __launch_bounds__(kT, 3)
       }
     }
   };
-#pragma unroll
-  for (int q = 0; q < kQE; ++q) {
-    const int x = tid + q * kT;
-    const Word* w = src + ((int64_t)c * n + x) * 2;
-    a[q] = x < n ? make_double2(w[0].v / s, w[1].v / s) : make_double2(0.0, 0.0);
-  }
-  fetch(n - 1, v);
-  for (int j = n - 1; j >= 0; --j) {
+  fetch(count - 1, v);
+  for (int j = count - 1; j >= 0; --j) {
     fetch(j - 1, nv);  // in flight during the reflection
     reflect(a, v, make_double2(tau[2 * j].v, tau[2 * j + 1].v), red, tot);
 #pragma unroll
     for (int q = 0; q < kQE; ++q) v[q] = nv[q];
   }
+}
+
+// CTA (i, 0): the long vector of the i-th largest triplet, Q times the unit column ord[i] of L, or
+// for i >= p (a value of zero, which leaves no direction) Q times the i-th column of the completion
+// refl2, tau2 of the unit columns; CTA (i, 1): its short one, P times that column of J.  Tall A:
+// U = long (m x r), Vh = short^H; wide: U = short, Vh = long^H.
+__global__ void __launch_bounds__(kT, 3)
+    jacobi_vectors_kernel(const Word* __restrict__ refl0, const Word* __restrict__ tau0,
+                          const Word* __restrict__ refl1, const Word* __restrict__ tau1,
+                          const Word* __restrict__ refl2, const Word* __restrict__ tau2, const Word* __restrict__ L,
+                          const Word* __restrict__ J, const double* __restrict__ nrm, const int* __restrict__ ord,
+                          int tall, int rows0, int n, int r, int p, double2* __restrict__ U, double2* __restrict__ Vh) {
+  __shared__ double red[2][kT];
+  __shared__ double tot[2];
+  const bool is_long = blockIdx.y == 0;
+  const int i = blockIdx.x, c = ord[i], tid = threadIdx.x, rows = is_long ? rows0 : n;
+  const bool completed = is_long && i >= p;
+  const Word* src = is_long ? L : J;
+  const double s = is_long ? nrm[c] : 1.0;
+  double2 a[kQE];
+#pragma unroll
+  for (int q = 0; q < kQE; ++q) {
+    const int x = tid + q * kT;
+    const Word* w = src + ((int64_t)c * n + x) * 2;
+    a[q] = x >= n ? make_double2(0.0, 0.0)
+           : completed ? make_double2(x == i ? 1.0 : 0.0, 0.0) : make_double2(w[0].v / s, w[1].v / s);
+  }
+  if (completed) apply_reflectors(a, refl2, tau2, p, n, red, tot);
+  apply_reflectors(a, is_long ? refl0 : refl1, is_long ? tau0 : tau1, n, rows, red, tot);
   const bool to_u = (tall != 0) == is_long;
 #pragma unroll
   for (int q = 0; q < kQE; ++q) {
@@ -550,7 +578,8 @@ bool jacobi_svd_applies(int64_t m, int64_t n) {
 size_t jacobi_svd_bytes(int64_t m, int64_t n) { return Parts(nullptr, std::max(m, n), std::min(m, n)).bytes; }
 
 // Factorises and rotates; S (host, descending, k = min(m, n) values).  The workspace
-// (jacobi_svd_bytes) then holds what jacobi_svd_store makes the vectors of.
+// (jacobi_svd_bytes) then holds what jacobi_svd_store makes the vectors of; those of the values
+// from `nonzero` on complete the others to an orthonormal set.
 int jacobi_svd_run(gtn_ctx ctx, int64_t m, int64_t n, const double2* A, void* ws, std::vector<double>* S) {
   int tall = m >= n ? 1 : 0, rows = (int)std::max(m, n), k = (int)std::min(m, n);
   Parts w(ws, rows, k);
@@ -597,11 +626,26 @@ int jacobi_svd_run(gtn_ctx ctx, int64_t m, int64_t n, const double2* A, void* ws
   return GTN_OK;
 }
 
-int jacobi_svd_store(gtn_ctx ctx, int64_t m, int64_t n, void* ws, int64_t r, double2* U, double2* Vh) {
-  const int tall = m >= n ? 1 : 0, rows = (int)std::max(m, n), k = (int)std::min(m, n);
+int jacobi_svd_store(gtn_ctx ctx, int64_t m, int64_t n, void* ws, int64_t r, int64_t nonzero, double2* U, double2* Vh) {
+  const int tall = m >= n ? 1 : 0, rows = (int)std::max(m, n);
+  int k = (int)std::min(m, n), one = 1;
   const Parts w(ws, rows, k);
-  jacobi_vectors_kernel<<<dim3((unsigned)r, 2), kT, 0, ctx->stream>>>(w.refl, w.tau, w.refl2, w.tau2, w.L, w.J, w.nrm,
-                                                                     w.ord, tall, rows, k, (int)r, U, Vh);
+  cudaStream_t s = ctx->stream;
+  // the completion's reflectors lie where the rotations were, its matrix where R^H was
+  Word *refl = w.rots, *tau = w.rots + (int64_t)k * k * 2, *X = w.R, *none = nullptr;
+  if (nonzero > 0 && nonzero < r) {
+    GTN_CUDA_TRY(ctx, cudaMemsetAsync(refl, 0, (size_t)(k * k + k) * 2 * sizeof(Word), s));
+    jacobi_unit_columns_kernel<<<(unsigned)k, kT, 0, s>>>(w.L, w.nrm, w.ord, k, (int)nonzero, X);
+    GTN_CUDA_TRY(ctx, cudaGetLastError());
+    const double2* noA = nullptr;
+    int* errflag = ctx->d_errflag;
+    JacobiState* st = w.st;
+    void* args[] = {&noA, &X, &one, &k, &k, &refl, &tau, &none, &none, &st, &errflag};
+    GTN_CUDA_TRY(ctx, cudaLaunchCooperativeKernel((const void*)jacobi_qr_kernel, dim3((unsigned)k), dim3(kT), args, 0, s));
+    ctx->launches += 2;
+  }
+  jacobi_vectors_kernel<<<dim3((unsigned)r, 2), kT, 0, s>>>(w.refl, w.tau, w.refl2, w.tau2, refl, tau, w.L, w.J, w.nrm,
+                                                            w.ord, tall, rows, k, (int)r, (int)nonzero, U, Vh);
   ctx->launches++;
   GTN_CUDA_TRY(ctx, cudaGetLastError());
   return GTN_OK;

@@ -523,20 +523,20 @@ static int svd_jacobi(gtn_ctx ctx, int64_t m, int64_t n, const double2* A, int64
   std::vector<double> hs;
   if ((st = jacobi_svd_run(ctx, jm, jn, J, ws, &hs)) != GTN_OK) return st;
   const int64_t r = trunc_rank(hs, maxdim, atol, rtol, dw);
-  // a kept value of zero (or so small that products of its column underflow) needs an orthonormal completion,
-  // and NaN has no order: cuSOLVER's
-  if (!(hs[r - 1] > 1e-60 * hs[0])) return GTN_ERR_UNSUPPORTED;
+  // a kept value of zero, or so small that products of its column underflow, has no long vector of its own
+  int64_t nz = r;
+  while (nz > 0 && !(hs[nz - 1] > 1e-60 * hs[0])) --nz;
   double disc = 0;
   for (int64_t i = r; i < k; ++i) disc += hs[i] * hs[i];
   for (int64_t i = 0; i < r; ++i) S[i] = hs[i];
   *rank = r;
   if (discarded) *discarded = std::sqrt(disc);
   if (!qr) {
-    if ((st = jacobi_svd_store(ctx, m, n, ws, r, U, Vh)) != GTN_OK) return st;
+    if ((st = jacobi_svd_store(ctx, m, n, ws, r, nz, U, Vh)) != GTN_OK) return st;
     return gtn_ctx_sync(ctx);
   }
   // X = Q R = (Q U_R) S V_R^H with X = A, or A^H: then A = V_R S (Q U_R)^H
-  if ((st = jacobi_svd_store(ctx, k, k, ws, r, UR, VR)) != GTN_OK) return st;
+  if ((st = jacobi_svd_store(ctx, k, k, ws, r, nz, UR, VR)) != GTN_OK) return st;
   const int ranks[2] = {2, 2};
   const int64_t dims[4] = {lng, k, k, r};
   const int labels[4] = {-1, 1, 1, -2}, order[2] = {0, 1};

@@ -343,7 +343,8 @@ int gtn_expm_small(int m, const double* A, double* E);
  * U (m x r, row-major), S (r doubles, HOST), Vh (r x n, row-major) must hold
  * min(m,n) columns/rows of capacity.  *rank = r, *discarded = 2-norm of dropped s.
  * Routes: below min(m,n) = 384 one-sided Jacobi rotations (one CTA up to 4096 elements; else the
- * whole chip on a QR factor; cuSOLVER gesvd where a kept value is zero); above it, subspace iteration on
+ * whole chip on a QR factor; cuSOLVER gesvd where they do not converge or A is not finite); above it,
+ * subspace iteration on
  * maxdim + max(32, maxdim/2) vectors when four times that fits in min(m,n) and its
  * leading values settle (environment GTN_SVD_SUBSPACE=0 turns it off), else the Gram
  * matrix with Zheevd; rows of Vh are re-orthonormalised by a thin QR after both. */

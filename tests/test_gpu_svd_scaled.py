@@ -45,3 +45,46 @@ def test_columns_of_every_size(ctx):
     check(ctx, a * np.logspace(0, -300, 100)[None, :])
     check(ctx, a * np.logspace(-300, 0, 100)[None, :], maxdim=30)
     check(ctx, a * np.logspace(0, -300, 120)[:, None])
+
+
+def zero_padded(rng, m, n, zero_rows, zero_cols):
+    a = O.randn_c(rng, (m, n))
+    a[rng.permutation(m)[:zero_rows]] = 0
+    a[:, rng.permutation(n)[:zero_cols]] = 0
+    return a
+
+
+@pytest.mark.parametrize("m,n", [(100, 90), (90, 100), (67, 67), (900, 80), (80, 900)])
+def test_kept_values_of_zero(ctx, m, n):
+    rng = np.random.default_rng(n)
+    for zr, zc in [(0, 1), (1, 0), (13, 20), (min(m, n) - 1, 3)]:
+        check(ctx, zero_padded(rng, m, n, zr, zc))
+        check(ctx, zero_padded(rng, m, n, zr, zc), maxdim=min(m, n) - 1)
+    for z in (1, 17, min(m, n) - 1):  # padding at the end: values of exactly zero
+        a = O.randn_c(rng, (m, n))
+        if m >= n:
+            a[:, n - z:] = 0
+        else:
+            a[m - z:] = 0
+        check(ctx, a)
+        check(ctx, a, maxdim=min(m, n) - 1)
+    one = np.zeros((m, n), dtype=np.complex128)
+    one[3, 5] = 2j
+    check(ctx, one)
+    check(ctx, np.zeros_like(one) + np.diag(np.r_[1.0, np.zeros(max(m, n) - 1)])[:m, :n], maxdim=2)
+
+
+def test_zeros_cost_no_second_factorisation(ctx):
+    """A padded matrix takes about the time of a full one: the rotations' result is used (a second
+    factorisation, by bidiagonalisation, takes three times as long as they do)."""
+    import time
+    rng = np.random.default_rng(1)
+    mats = [ctx.upload(a) for a in (O.randn_c(rng, (192, 192)),
+                                  np.pad(O.randn_c(rng, (192, 180)), ((0, 0), (0, 12))))]
+    best = [1e9, 1e9]
+    for _ in range(4):
+        for i, a in enumerate(mats):
+            t = time.perf_counter()
+            ctx.svd_trunc(a)
+            best[i] = min(best[i], time.perf_counter() - t)
+    assert best[1] <= 2.0 * best[0], best
