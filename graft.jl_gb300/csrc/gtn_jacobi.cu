@@ -14,7 +14,7 @@
 // words it needs until they carry the number of its step.  With a version per column behind a fence
 // a hand-over took 6000 of a round's 12000 clocks (write drain, poll, load); FP64 itself, two FMAs
 // per clock and SM at a latency of about 60 clocks, is the rest.  Sums are trees for the same
-// reason, and a rotation's parameters take the short way below.
+// reason, and a rotation's parameters take two reciprocal square roots and an FP32 tangent.
 //   * QR: CTA k holds column k, applies the reflectors 0 .. k-1 as they appear, forms its own.
 //   * Jacobi: a round of the round-robin schedule rotates n / 2 disjoint pairs of columns of L, one
 //     CTA each; a second CTA per pair applies the same rotations to J a little later.  A sweep ends
@@ -126,17 +126,6 @@ __device__ __forceinline__ void warp_sums(const double (*red)[kT], double* tot) 
 #pragma unroll
   for (int o = G / 2; o > 0; o >>= 1) x[0] += __shfl_down_sync(0xffffffffu, x[0], o, G);
   if (l == 0) tot[v] = x[0];
-}
-
-__device__ __forceinline__ double rsqrt_approx(double x) {
-  double r;
-  asm("rsqrt.approx.ftz.f64 %0, %1;" : "=d"(r) : "d"(x));
-  return r;
-}
-// 1 / sqrt(x) to full precision from a seed of 22 bits: one cubic step.
-__device__ __forceinline__ double rsqrt_step(double x, double r) {
-  const double e = fma(-x * r, r, 1.0);
-  return fma(r, e * fma(e, 0.375, 0.5), r);
 }
 
 // Squared column norms below this are formed on a scaled column: above it, squares lost to
@@ -322,15 +311,14 @@ __device__ __forceinline__ void make_rotation(double A2, double B2, double gx, d
   R->u = make_double2(0.0, 0.0);
   R->d = make_double2(1.0, 0.0);
   if (!R->turn) return;
-  const double i0 = rsqrt_approx(g2);
+  const double ig = rsqrt(g2);
   // tangent of the smaller rotation, t = sgn / (|z| + sqrt(1 + z^2)), z = half / |g|
-  const double zd = fabs(half * i0);
+  const double zd = fabs(half * ig);
   const float z = (float)zd;
   double t = zd < 1e15 ? (double)__fdividef(1.f, z + __fsqrt_rn(fmaf(z, z, 1.f))) : 0.5 / zd;
   if (half < 0.0) t = -t;
   const double w = fma(t, t, 1.0);
-  const double c = rsqrt_step(w, rsqrt_approx(w)), s = t * c;
-  const double ig = rsqrt_step(g2, i0);
+  const double c = rsqrt(w), s = t * c;
   const double2 ph = make_double2(gx * ig, -gy * ig);  // e^{-i phi}
   R->c = c;
   R->s = s;
