@@ -460,15 +460,10 @@ cudaError_t launch_f64e_gemm(const F64eGemmArgs& a, int sm_count, int* errflag, 
                         const float*, const float*, const int*, const int*, int, longlong2*, int*);
   static const Kern kerns[4] = {f64e_gemm_kernel<8, false>, f64e_gemm_kernel<8, true>, f64e_gemm_kernel<7, false>,
                                 f64e_gemm_kernel<7, true>};
-  static bool attr_set = false;
-  if (!attr_set) {
-    for (Kern k : kerns) {
-      const cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmem);
-      if (e != cudaSuccess) return e;
-    }
-    attr_set = true;
-  }
-  launch_chained(kerns[(a.levels == 7 ? 2 : 0) + (share ? 1 : 0)], dim3((unsigned)grid), dim3(kThreads), kSmem, s, static_cast<const unsigned char*>(a.A), static_cast<const unsigned char*>(a.B), a.C, a.M, a.N, nkb, tm, tn,
+  static PerDeviceOnce opt_in[4];
+  const int which = (a.levels == 7 ? 2 : 0) + (share ? 1 : 0);
+  if (const cudaError_t e = smem_opt_in(opt_in[which], kerns[which], kSmem)) return e;
+  launch_chained(kerns[which], dim3((unsigned)grid), dim3(kThreads), kSmem, s, static_cast<const unsigned char*>(a.A), static_cast<const unsigned char*>(a.B), a.C, a.M, a.N, nkb, tm, tn,
       a.a_exp, a.b_exp, a.a_flag, a.b_flag, a.token, share ? static_cast<longlong2*>(a.part) : nullptr, errflag);
   cudaError_t e = cudaGetLastError();
   *launches = 1;

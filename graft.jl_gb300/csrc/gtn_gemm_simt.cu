@@ -212,13 +212,8 @@ size_t skinny_smem(const GemmJob& J) {
 
 template <typename T>
 cudaError_t launch_skinny(const GemmJob* jobs, int njobs, cudaStream_t s) {
-  static bool attr_set = false;
-  if (!attr_set) {
-    cudaError_t e = cudaFuncSetAttribute(gemm_skinny_grouped_kernel<T>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                         kSkinnyMaxSmem);
-    if (e != cudaSuccess) return e;
-    attr_set = true;
-  }
+  static PerDeviceOnce opt_in;
+  if (const cudaError_t e = smem_opt_in(opt_in, gemm_skinny_grouped_kernel<T>, kSkinnyMaxSmem)) return e;
   for (int base = 0; base < njobs; base += kGemmJobMax) {
     const int cnt = std::min(kGemmJobMax, njobs - base);
     SkinnyJobsP g;

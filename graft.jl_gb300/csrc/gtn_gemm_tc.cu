@@ -998,13 +998,8 @@ cudaError_t launch_ps(const TcGemmArgs& a, int* errflag, cudaStream_t s, std::st
   CUtensorMap tmA, tmB;
   if (!make_map(&tmA, a.A, a.Kp, a.M, a.a_planes, BM, why, BKE2)) return cudaErrorInvalidValue;
   if (!make_map(&tmB, a.B, a.Kp, 2 * a.N, a.b_planes, BN, why, BKE2)) return cudaErrorInvalidValue;
-  static bool attr_set = false;
-  if (!attr_set) {
-    cudaError_t e = cudaFuncSetAttribute(tc_gemm_ps_kernel<BN, P, CPS>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                         CF::SMEM);
-    if (e != cudaSuccess) return e;
-    attr_set = true;
-  }
+  static PerDeviceOnce opt_in;
+  if (const cudaError_t e = smem_opt_in(opt_in, tc_gemm_ps_kernel<BN, P, CPS>, CF::SMEM)) return e;
   ProdList pl;
   pl.n = a.nprod;
   for (int i = 0; i < 9; ++i) {
@@ -1038,13 +1033,8 @@ int device_sm_count() {
 template <int BN, int P, int G>
 cudaError_t launch_persist_g(const TcGemmArgs* probs, int nprob, int* errflag, cudaStream_t s, std::string* why) {
   using CF = Cfg2<BN, P>;
-  static bool attr_set = false;
-  if (!attr_set) {
-    cudaError_t e = cudaFuncSetAttribute(tc_gemm_persist_kernel<BN, P, G>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                         CF::SMEM);
-    if (e != cudaSuccess) return e;
-    attr_set = true;
-  }
+  static PerDeviceOnce opt_in;
+  if (const cudaError_t e = smem_opt_in(opt_in, tc_gemm_persist_kernel<BN, P, G>, CF::SMEM)) return e;
   const int grid = device_sm_count();
   auto tiles_n = [](const TcGemmArgs& a) { return (int)((2 * a.N + BN - 1) / BN); };
   auto width = [&](const TcGemmArgs& a) {
@@ -1104,13 +1094,8 @@ cudaError_t launch_pair(const TcGemmArgs& a, int* errflag, cudaStream_t s, std::
   CUtensorMap tmA, tmB;
   if (!make_map(&tmA, a.A, a.Kp, a.M, a.a_planes, CF::ROWS, why, BKE2)) return cudaErrorInvalidValue;
   if (!make_map(&tmB, a.B, a.Kp, 2 * a.N, a.b_planes, CF::ROWS, why, BKE2)) return cudaErrorInvalidValue;
-  static bool attr_set = false;
-  if (!attr_set) {
-    cudaError_t e = cudaFuncSetAttribute(tc_gemm_pair_kernel<P>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                         CF::SMEM);
-    if (e != cudaSuccess) return e;
-    attr_set = true;
-  }
+  static PerDeviceOnce opt_in;
+  if (const cudaError_t e = smem_opt_in(opt_in, tc_gemm_pair_kernel<P>, CF::SMEM)) return e;
   ProdList pl;
   pl.n = a.nprod;
   for (int i = 0; i < 9; ++i) {
@@ -1381,13 +1366,8 @@ cudaError_t launch_bn(const TcGemmArgs& a, int* errflag, cudaStream_t s, std::st
   CUtensorMap tmA, tmB;
   if (!make_map(&tmA, a.A, a.Kp, a.M, a.a_planes, BM, why)) return cudaErrorInvalidValue;
   if (!make_map(&tmB, a.B, a.Kp, 2 * a.N, a.b_planes, BN, why)) return cudaErrorInvalidValue;
-  static bool attr_set = false;
-  if (!attr_set) {
-    cudaError_t e = cudaFuncSetAttribute(tc_gemm_kernel<BN>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                         CF::SMEM);
-    if (e != cudaSuccess) return e;
-    attr_set = true;
-  }
+  static PerDeviceOnce opt_in;
+  if (const cudaError_t e = smem_opt_in(opt_in, tc_gemm_kernel<BN>, CF::SMEM)) return e;
   ProdList pl;
   pl.n = a.nprod;
   for (int i = 0; i < 9; ++i) {
@@ -1405,13 +1385,8 @@ cudaError_t launch_bn(const TcGemmArgs& a, int* errflag, cudaStream_t s, std::st
 template <int BN>
 cudaError_t launch_grouped_bn(const TcGemmArgs* probs, int nprob, int* errflag, cudaStream_t s, std::string* why) {
   using CF = Cfg<BN>;
-  static bool attr_set = false;
-  if (!attr_set) {
-    cudaError_t e = cudaFuncSetAttribute(tc_gemm_grouped_kernel<BN>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                         CF::SMEM);
-    if (e != cudaSuccess) return e;
-    attr_set = true;
-  }
+  static PerDeviceOnce opt_in;
+  if (const cudaError_t e = smem_opt_in(opt_in, tc_gemm_grouped_kernel<BN>, CF::SMEM)) return e;
   for (int base = 0; base < nprob; base += kTcGroupMax) {
     const int cnt = std::min(kTcGroupMax, nprob - base);
     GroupedTc<kTcGroupMax> g;

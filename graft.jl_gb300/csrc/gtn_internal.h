@@ -1,6 +1,8 @@
 // Internal declarations shared by the libgrafttn translation units.
 #pragma once
 
+#include "gtn_once.h"
+
 #include <utility>
 #include <cuda_runtime.h>
 #include <cuda_bf16.h>
@@ -56,6 +58,18 @@ inline cudaError_t launch_chained_if(bool chained, void (*kern)(P...), dim3 grid
 template <class... P, class... A>
 inline cudaError_t launch_chained(void (*kern)(P...), dim3 grid, dim3 block, size_t smem, cudaStream_t s, A&&... args) {
   return launch_chained_if(true, kern, grid, block, smem, s, std::forward<A>(args)...);
+}
+// A kernel's attribute, set once per device (it belongs to the kernel on the current device).
+template <class... P>
+inline cudaError_t func_attribute(PerDeviceOnce& once, void (*kern)(P...), cudaFuncAttribute attribute, int value) {
+  int dev = 0;
+  const cudaError_t e = cudaGetDevice(&dev);
+  return e != cudaSuccess ? e : once(dev, [&] { return cudaFuncSetAttribute(kern, attribute, value); });
+}
+// Opt in to more than 48 KB of dynamic shared memory.
+template <class... P>
+inline cudaError_t smem_opt_in(PerDeviceOnce& once, void (*kern)(P...), size_t bytes) {
+  return func_attribute(once, kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
 }
 #ifdef __CUDACC__
 __device__ __forceinline__ void chained_wait() {

@@ -830,19 +830,12 @@ cudaError_t launch_small(const T* A, const GroupSpec& mg, const GroupSpec& kg, i
     // narrow CTAs for short tensors: the FP64 pipes of all SMs share the rows
     const int threads = M >= 2 * 152 * 256 ? 256 : (M >= 2 * 152 * 64 ? 64 : 32);
     const int64_t blocks = std::min<int64_t>((M + threads - 1) / threads, 152 * 16);
-    static bool attr = false;
-    if (!attr) {
-      cudaError_t e = cudaFuncSetAttribute(small_contract64_kernel<8>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                           kSmall64SmemBytes);
-      if (e == cudaSuccess)
-        e = cudaFuncSetAttribute(small_contract64_kernel<16>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                 kSmall64SmemBytes);
-      if (e != cudaSuccess) return e;
-      attr = true;
-    }
+    static PerDeviceOnce opt_in8, opt_in16;
     if (N <= 8) {
+      if (const cudaError_t e = smem_opt_in(opt_in8, small_contract64_kernel<8>, kSmall64SmemBytes)) return e;
       launch_chained(small_contract64_kernel<8>, dim3((unsigned)blocks), dim3(threads), small64_smem(K, N, 8, threads), s, A, mg, kg, M, K, N, B, C);
     } else {
+      if (const cudaError_t e = smem_opt_in(opt_in16, small_contract64_kernel<16>, kSmall64SmemBytes)) return e;
       launch_chained(small_contract64_kernel<16>, dim3((unsigned)blocks), dim3(threads), small64_smem(K, N, 16, threads), s, A, mg, kg, M, K, N, B, C);
     }
   } else {
@@ -1525,13 +1518,9 @@ template <typename Tin, int TR, class Off, class W>
 cudaError_t launch_split_rows_t(const Tin* T, const Off& off, int64_t M, int64_t K, int64_t Kp, int kc, int cs,
                                 int m_fast, const W& w, float* amax, size_t smem, cudaStream_t s) {
   auto kern = split_rows_kernel<Tin, TR, Off, W>;
-  static bool attr = false;
-  if (!attr) {
-    cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, 112 * 1024);
-    if (e == cudaSuccess) e = cudaFuncSetAttribute(kern, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
-    if (e != cudaSuccess) return e;
-    attr = true;
-  }
+  static PerDeviceOnce opt_in, big_clusters;
+  if (const cudaError_t e = smem_opt_in(opt_in, kern, 112 * 1024)) return e;
+  if (const cudaError_t e = func_attribute(big_clusters, kern, cudaFuncAttributeNonPortableClusterSizeAllowed, 1)) return e;
   const int64_t tiles = (M + TR - 1) / TR;
   if (tiles * cs > 2147483647LL) return cudaErrorInvalidConfiguration;
   cudaLaunchConfig_t cfg = {};
@@ -1647,13 +1636,8 @@ namespace {
 template <typename Tin, typename T, int NPT, typename O>
 cudaError_t launch_band_t(const DevBand* bands, const DevBandWork* work, int nwork, const DevBandCol* cols,
                           const int64_t* rstr, const BlockBases& bases, size_t smem, cudaStream_t s) {
-  static bool attr_set = false;
-  if (!attr_set) {
-    cudaError_t e = cudaFuncSetAttribute(block_band_kernel<Tin, T, NPT, O>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                         kBandMaxSmem);
-    if (e != cudaSuccess) return e;
-    attr_set = true;
-  }
+  static PerDeviceOnce opt_in;
+  if (const cudaError_t e = smem_opt_in(opt_in, block_band_kernel<Tin, T, NPT, O>, kBandMaxSmem)) return e;
   block_band_kernel<Tin, T, NPT, O><<<nwork, 256, smem, s>>>(bands, work, cols, rstr, bases);
   return cudaGetLastError();
 }
@@ -1699,13 +1683,8 @@ namespace {
 template <typename Tin, bool F16>
 cudaError_t launch_split_band_t(const DevBand* bands, const DevBandWork* work, int nwork, const DevBandCol* cols,
                                 const int64_t* rstr, const BlockBases& bases, size_t smem, cudaStream_t s) {
-  static bool attr_set = false;
-  if (!attr_set) {
-    cudaError_t e = cudaFuncSetAttribute(block_split_band_kernel<Tin, F16>,
-                                         cudaFuncAttributeMaxDynamicSharedMemorySize, kBandMaxSmem);
-    if (e != cudaSuccess) return e;
-    attr_set = true;
-  }
+  static PerDeviceOnce opt_in;
+  if (const cudaError_t e = smem_opt_in(opt_in, block_split_band_kernel<Tin, F16>, kBandMaxSmem)) return e;
   block_split_band_kernel<Tin, F16><<<nwork, 256, smem, s>>>(bands, work, cols, rstr, bases);
   return cudaGetLastError();
 }
@@ -1864,13 +1843,8 @@ cudaError_t launch_rowmax_grouped(const GatherJob* jobs, int njobs, int in_is64,
 
 template <typename T>
 static cudaError_t launch_small_grouped_t(const SmallJob* jobs, int njobs, cudaStream_t s) {
-  static bool attr = false;
-  if (!attr) {
-    cudaError_t e = cudaFuncSetAttribute(small_grouped_kernel<T>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                         kSmall64SmemBytes);
-    if (e != cudaSuccess) return e;
-    attr = true;
-  }
+  static PerDeviceOnce opt_in;
+  if (const cudaError_t e = smem_opt_in(opt_in, small_grouped_kernel<T>, kSmall64SmemBytes)) return e;
   for (int base = 0; base < njobs; base += kGatherJobMax) {
     const int cnt = std::min(kGatherJobMax, njobs - base);
     SmallJobsP g;

@@ -518,13 +518,9 @@ size_t small_svd_smem(int64_t m, int64_t n) {
 
 int svd_small_launch(gtn_ctx ctx, int64_t m, int64_t n, const double2* A, double* S, double2* U, double2* Vh) {
   if (!small_svd_applies(m, n)) return GTN_ERR_UNSUPPORTED;
-  static bool attr = false;
-  if (!attr) {
-    if (cudaFuncSetAttribute(small_svd_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 140 * 1024) !=
-        cudaSuccess)
-      return set_err(ctx, GTN_ERR_CUDA, "svd: kernel attribute");
-    attr = true;
-  }
+  static PerDeviceOnce opt_in;
+  if (smem_opt_in(opt_in, small_svd_kernel, 140 * 1024) != cudaSuccess)
+    return set_err(ctx, GTN_ERR_CUDA, "svd: kernel attribute");
   small_svd_kernel<<<1, 256, small_svd_smem(m, n), ctx->stream>>>(A, (int)m, (int)n, S, U, Vh);
   ctx->launches++;
   const cudaError_t e = cudaGetLastError();
@@ -539,13 +535,9 @@ int qr_small(gtn_ctx ctx, int64_t m, int64_t n, const double2* A, double2* Q, do
   if (!small_qr_applies(m, n)) return GTN_ERR_UNSUPPORTED;
   const int64_t k = std::min(m, n);
   const size_t smem = (size_t)(m * n + m * k + k) * sizeof(double2) + 8 * sizeof(double);
-  static bool attr = false;
-  if (!attr) {
-    if (cudaFuncSetAttribute(small_qr_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 140 * 1024) !=
-        cudaSuccess)
-      return set_err(ctx, GTN_ERR_CUDA, "qr: kernel attribute");
-    attr = true;
-  }
+  static PerDeviceOnce opt_in;
+  if (smem_opt_in(opt_in, small_qr_kernel, 140 * 1024) != cudaSuccess)
+    return set_err(ctx, GTN_ERR_CUDA, "qr: kernel attribute");
   small_qr_kernel<<<1, 256, smem, ctx->stream>>>(A, (int)m, (int)n, Q, R);
   ctx->launches++;
   const cudaError_t e = cudaGetLastError();
@@ -576,12 +568,9 @@ int qr_tall_cholesky(gtn_ctx ctx, int64_t m, int64_t n, const double2* A, double
   double2* dRi = reinterpret_cast<double2*>(p + bT + bP + bG);
   const size_t smem_g = (size_t)TR * n * sizeof(double2);
   const size_t smem_r = (size_t)TR * (n + 1) * sizeof(double2) + (size_t)n * n * sizeof(double2);
-  static bool attr = false;
-  if (!attr) {
-    if (cudaFuncSetAttribute(tsqr_trsm, cudaFuncAttributeMaxDynamicSharedMemorySize, 100 * 1024) != cudaSuccess)
-      return set_err(ctx, GTN_ERR_CUDA, "qr: kernel attribute");
-    attr = true;
-  }
+  static PerDeviceOnce opt_in;
+  if (smem_opt_in(opt_in, tsqr_trsm, 100 * 1024) != cudaSuccess)
+    return set_err(ctx, GTN_ERR_CUDA, "qr: kernel attribute");
   std::vector<double2> hG((size_t)n * n);
   auto gram = [&](const double2* X, std::vector<cplx>& G) -> cudaError_t {
     tsqr_gram_partial<<<nparts, 256, smem_g, s>>>(X, m, ni, rpc, part);
