@@ -264,7 +264,6 @@ int gtn_ctx_destroy(gtn_ctx ctx) {
   for (auto& ev : ctx->step_ev)
     if (ev) cudaEventDestroy(ev);
   if (ctx->d_errflag) cudaFree(ctx->d_errflag);
-  if (ctx->f64e_part) cudaFree(ctx->f64e_part);
   if (ctx->own_stream) cudaStreamDestroy(ctx->stream);
   delete ctx;
   return GTN_OK;

@@ -434,7 +434,18 @@ double f64e_time(double M, double N, double K) {
   bool share;
   return 8e-6 + f64e_waves(M, N, K, 152, &share) + M * K * 60 / 4e12;
 }
-size_t f64e_part_bytes(int sm_count) { return (size_t)2 * std::max(1, sm_count) * kBM * kBN * sizeof(longlong2); }
+// CTAs of a product, and whether its last tiles are shared.
+static int64_t f64e_grid(int64_t M, int64_t N, int64_t K, int sm_count, bool* share) {
+  const int64_t sms = std::max(1, sm_count), tiles = ((M + kBM - 1) / kBM) * ((2 * N + kBN - 1) / kBN);
+  f64e_waves((double)M, (double)N, (double)K, (int)sms, share);
+  const int64_t chunks = (K + 8 * kChunkStages - 1) / (8 * kChunkStages);
+  return std::min(*share && tiles < sms ? tiles * chunks : tiles, sms);
+}
+size_t f64e_part_bytes(int64_t M, int64_t N, int64_t K, int sm_count) {
+  bool share;
+  const int64_t grid = f64e_grid(M, N, K, sm_count, &share);
+  return share ? (size_t)(2 * grid) * kBM * kBN * sizeof(longlong2) : 0;  // two segments a CTA
+}
 double f64_pipe_time(double M, double N, double K) { return 4e-6 + 8.0 * M * N * K / 1.15e12; }
 
 cudaError_t launch_f64e_gemm(const F64eGemmArgs& a, int sm_count, int* errflag, cudaStream_t s, std::string* why,
@@ -451,11 +462,13 @@ cudaError_t launch_f64e_gemm(const F64eGemmArgs& a, int sm_count, int* errflag, 
   }
   const int nkb = (int)((a.K + 7) / 8);
   const int64_t tm = (a.M + kBM - 1) / kBM, tn = (2 * a.N + kBN - 1) / kBN;
-  const int nchunks = (nkb + kChunkStages - 1) / kChunkStages, sms = std::max(1, sm_count);
+  const int nchunks = (nkb + kChunkStages - 1) / kChunkStages;
   bool share = false;
-  f64e_waves((double)a.M, (double)a.N, (double)a.K, sms, &share);
-  share = share && a.part;
-  const int64_t grid = std::min<int64_t>(share && tm * tn < sms ? tm * tn * nchunks : tm * tn, sms);
+  int64_t grid = f64e_grid(a.M, a.N, a.K, sm_count, &share);
+  if (share && !a.part) {
+    share = false;
+    grid = std::min<int64_t>(tm * tn, std::max(1, sm_count));
+  }
   using Kern = void (*)(const unsigned char*, const unsigned char*, double2*, int64_t, int64_t, int, int64_t, int64_t,
                         const float*, const float*, const int*, const int*, int, longlong2*, int*);
   static const Kern kerns[4] = {f64e_gemm_kernel<8, false>, f64e_gemm_kernel<8, true>, f64e_gemm_kernel<7, false>,

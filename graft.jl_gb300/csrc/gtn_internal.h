@@ -94,7 +94,6 @@ struct gtn_ctx_s {
   // out-of-range flags of the digit-plane products: product number t writes t to slot
   // t % kFbSlots, so no slot needs clearing between products (they are ordered on the stream)
   int* d_fbflag = nullptr;
-  void* f64e_part = nullptr;  // partial sums of the digit-plane products (first plan that has one)
   int fb_token = 0;
   int sm_count = 0;
   int cc_major = 0, cc_minor = 0;
@@ -435,11 +434,12 @@ struct F64eGemmArgs {
   const int* b_flag = nullptr;  // != 0: a row of B out of range
   int token = 0;
   int levels = 8;               // digit products d_i e_j with i + j < levels (7 or 8)
-  void* part = nullptr;         // f64e_part_bytes, or null: no tile is shared
+  void* part = nullptr;         // f64e_part_bytes of the product, or null: no tile is shared
 };
 cudaError_t launch_f64e_gemm(const F64eGemmArgs& a, int sm_count, int* errflag, cudaStream_t s, std::string* why,
                              int* launches);
-size_t f64e_part_bytes(int sm_count);  // partial sums of tiles that CTAs share
+// Bytes of partial sums of the tiles that CTAs share in a product (0: none are).
+size_t f64e_part_bytes(int64_t M, int64_t N, int64_t K, int sm_count);
 // Digit planes and row exponents of the running tensor's K-major view (c128; *flag = token when
 // a row is out of range), and of a static B [N][K] (*flag = 1 when a row is out of range).
 cudaError_t launch_split_digits_tab(const double2* T, const GatherTab& t, int64_t M, int64_t K, float* rexp, void* out,
@@ -568,6 +568,7 @@ struct gtn_map_s {
   int64_t max_apl = 0;     // largest split-plane staging (bf16 elements per plane * planes)
   int64_t max_mtc = 0;     // largest M of a tensor-core step (fp16 row maxima, digit row exponents)
   size_t max_adg = 0;      // largest digit-plane operand (bytes)
+  void* part = nullptr;    // partial sums of its digit-plane products (or null)
   int64_t max_splitk = 0;  // largest split-K partial-sum workspace (complex elements)
   bool oneshot = false;    // a one-shot contraction (gtn_contract): arena allocations, no tables
   char* arena = nullptr;   // allocations come from here first (one-shot contractions)

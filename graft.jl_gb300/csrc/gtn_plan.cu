@@ -138,9 +138,13 @@ int fill_offset_tables(gtn_map map) {
 // plan (a step without them stays on the FP64 pipe) and needed in an FP64E one.
 int pack_digits(gtn_map map, bool required) {
   gtn_ctx ctx = map->ctx;
-  if (!ctx->f64e_part && cudaMalloc(&ctx->f64e_part, f64e_part_bytes(ctx->sm_count)) != cudaSuccess) {
-    cudaGetLastError();  // without it no tile is shared
-    ctx->f64e_part = nullptr;
+  // partial sums of the map's own: applications of two maps, captured or on two threads, may overlap
+  size_t part = 0;
+  for (const PlanStep& st : map->steps)
+    if (st.dg) part = std::max(part, f64e_part_bytes(st.M, st.N, st.K, ctx->sm_count));
+  if (part > 0 && dalloc(map, &map->part, part) != cudaSuccess) {
+    cudaGetLastError();  // without them no tile is shared
+    map->part = nullptr;
   }
   int* flags = nullptr;
   cudaError_t e = dalloc(map, &flags, map->steps.size() * sizeof(int));
@@ -799,7 +803,7 @@ int map_run(gtn_map map, int precision, const double2* x, double2* y) {
         a.b_exp = st.bexp;
         a.token = ctx->fb_token;
         a.levels = f64e ? 7 : 8;
-        a.part = ctx->f64e_part;
+        a.part = map->part;
         a.a_flag = ctx->d_fbflag + ctx->fb_token % kFbSlots;
         a.b_flag = st.bflag;
         int* flag = ctx->d_fbflag + ctx->fb_token % kFbSlots;
