@@ -235,13 +235,12 @@ int gtn_ctx_create(int device, gtn_ctx* out) {
     return GTN_ERR_CUDA;
   }
   ctx->own_stream = true;
-  if (cudaMalloc(&ctx->d_errflag, (1 + kFbSlots) * sizeof(int)) != cudaSuccess ||
-      cudaMemset(ctx->d_errflag, 0, (1 + kFbSlots) * sizeof(int)) != cudaSuccess) {
+  if (cudaMalloc(&ctx->d_errflag, sizeof(int)) != cudaSuccess ||
+      cudaMemset(ctx->d_errflag, 0, sizeof(int)) != cudaSuccess) {
     cudaStreamDestroy(ctx->stream);
     delete ctx;
     return GTN_ERR_CUDA;
   }
-  ctx->d_fbflag = ctx->d_errflag + 1;
   if (ctx_red(ctx, 4096) != cudaSuccess) {
     cudaFree(ctx->d_errflag);
     cudaStreamDestroy(ctx->stream);

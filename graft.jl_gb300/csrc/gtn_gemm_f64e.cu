@@ -21,8 +21,9 @@
 // 2-norm, Gaussian operands: K = 65 5.7e-17 (FP64 pipe 3.7e-16), K = 5120 7.1e-17 (3.4e-15),
 // rows that decay from 1 to 1e-9 along k 1.3e-16 (5.4e-16) and 1.8e-16 (4.9e-15); L = 7 about
 // 3.6e-16 at every K.
-// A row with an infinity, a NaN or a magnitude beyond 2^+-450 has no digits: the split sets a
-// flag, this kernel returns and the FP64 kernel behind it computes the product.
+// A row with an infinity, a NaN or a magnitude beyond 2^+-450 has no digits: what this kernel makes
+// of it is overwritten by f64e_repair_kernel, which looks at the rows' exponents and leaves no trace
+// for a later product.
 //
 // Tile: 128 rows x 64 real columns (32 complex); stages of 16 real k hold all 7 planes of A
 // (28 KB) and of B' (14 KB), laid out by the split so that one contiguous bulk copy loads each
@@ -35,6 +36,7 @@
 // a tile while the next one's MMAs run.  Every mbarrier wait is bounded as in the other tcgen05
 // kernels.
 #include "gtn_internal.h"
+#include "gtn_group.h"
 #include "gtn_tcgen05.h"
 
 #include <algorithm>
@@ -158,8 +160,7 @@ template <int L, bool Split>
 __global__ void __launch_bounds__(kThreads, 1)
     f64e_gemm_kernel(const unsigned char* __restrict__ A, const unsigned char* __restrict__ B, double2* __restrict__ C,
                      int64_t M, int64_t N, int nkb, int64_t tiles_m, int64_t tiles_n, const float* __restrict__ a_exp,
-                     const float* __restrict__ b_exp, const int* __restrict__ a_flag, const int* __restrict__ b_flag,
-                     int token, longlong2* __restrict__ part, int* __restrict__ errflag) {
+                     const float* __restrict__ b_exp, longlong2* __restrict__ part, int* __restrict__ errflag) {
   chained_wait();
   extern __shared__ __align__(1024) uint8_t smem_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) &
@@ -171,7 +172,6 @@ __global__ void __launch_bounds__(kThreads, 1)
   __shared__ volatile int abort_flag;
   __shared__ int n_issued, n_consumed;
 
-  if (*a_flag == token || *b_flag != 0) return;  // the same for every thread of the launch
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int64_t ntiles = tiles_m * tiles_n;
   const int nchunks = (nkb + kChunkStages - 1) / kChunkStages;
@@ -375,10 +375,8 @@ __global__ void __launch_bounds__(kThreads, 1)
 __global__ void __launch_bounds__(32 * kEpiWarps)
     f64e_finish_kernel(const longlong2* __restrict__ part, double2* __restrict__ C, int64_t M, int64_t N, int nchunks,
                        int64_t tiles_m, int64_t tiles_n, int G, const float* __restrict__ a_exp,
-                       const float* __restrict__ b_exp, const int* __restrict__ a_flag, const int* __restrict__ b_flag,
-                       int token) {
+                       const float* __restrict__ b_exp) {
   chained_wait();
-  if (*a_flag == token || *b_flag != 0) return;
   constexpr int kPairs = kCols / 2, kT = 32 * kEpiWarps;
   const int64_t whole = tiles_m * tiles_n / G * G;
   // fewer than G tiles of at most 2^15 chunks are shared: 32 bits hold U b
@@ -411,6 +409,102 @@ __global__ void __launch_bounds__(32 * kEpiWarps)
   if (m < M && n < N) {
     const int es = (int)a_exp[m] + (int)b_exp[n];
     C[n * M + m] = make_double2(to_double(re.x, re.y, es), to_double(im.x, im.y, es));
+  }
+}
+
+// ---- outputs that the digit planes cannot give --------------------------------------------------
+// A CTA walks over tiles of kRM x kRN complex outputs and lists those to be summed again on the FP64
+// pipe: four a warp, the k range over its lanes, K offsets of kRK columns at a time.  Ordinary
+// operands list none, and a tile costs the reading of its rows' exponents.
+constexpr int kRM = 128, kRN = 64, kRK = 512, kRThreads = 256, kRPerWarp = 4;
+
+struct RepairArgs {
+  const double2* T;
+  const int64_t *om, *ok;  // offset tables, or null
+  GroupSpec mg, kg;
+  const double2* B;
+  double2* C;
+  int64_t M, N, K, tiles_m, ntiles;
+  const float *a_exp, *b_exp;
+};
+
+// Sum the listed outputs (n_local * kRM + m_local) of the tile at (m0, n0) again.
+__device__ __forceinline__ void repair_outputs(const RepairArgs& g, const uint16_t* list, int count, int64_t m0,
+                                               int64_t n0, int64_t* offK) {
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  constexpr int kPass = kRThreads / 32 * kRPerWarp;
+#pragma unroll 1
+  for (int base = 0; base < count; base += kPass) {
+    int64_t om[kRPerWarp];
+    const double2* b[kRPerWarp];
+    double2 acc[kRPerWarp];
+#pragma unroll
+    for (int j = 0; j < kRPerWarp; ++j) {
+      const int e = min(base + warp * kRPerWarp + j, count - 1);  // past the end: the last one again
+      const int64_t m = m0 + list[e] % kRM, n = n0 + list[e] / kRM;
+      om[j] = g.om ? g.om[m] : decompose(m, g.mg);
+      b[j] = g.B + n * g.K;
+      acc[j] = make_double2(0.0, 0.0);
+    }
+#pragma unroll 1
+    for (int64_t kq = 0; kq < g.K; kq += kRK) {
+      const int kv = (int)min((int64_t)kRK, g.K - kq);
+      __syncthreads();
+      for (int c = threadIdx.x; c < kv; c += kRThreads) offK[c] = g.ok ? g.ok[kq + c] : decompose(kq + c, g.kg);
+      __syncthreads();
+      for (int c = lane; c < kv; c += 32) {
+        double2 t[kRPerWarp], v[kRPerWarp];
+#pragma unroll
+        for (int j = 0; j < kRPerWarp; ++j) {
+          t[j] = g.T[om[j] + offK[c]];
+          v[j] = b[j][kq + c];
+        }
+#pragma unroll
+        for (int j = 0; j < kRPerWarp; ++j) {
+          acc[j].x = fma(t[j].x, v[j].x, acc[j].x);
+          acc[j].x = fma(-t[j].y, v[j].y, acc[j].x);
+          acc[j].y = fma(t[j].x, v[j].y, acc[j].y);
+          acc[j].y = fma(t[j].y, v[j].x, acc[j].y);
+        }
+      }
+    }
+#pragma unroll
+    for (int j = 0; j < kRPerWarp; ++j) {
+#pragma unroll
+      for (int o = 16; o > 0; o >>= 1) {
+        acc[j].x += __shfl_xor_sync(0xffffffffu, acc[j].x, o);
+        acc[j].y += __shfl_xor_sync(0xffffffffu, acc[j].y, o);
+      }
+      const int e = base + warp * kRPerWarp + j;
+      if (lane == 0 && e < count) g.C[(n0 + list[e] / kRM) * g.M + m0 + list[e] % kRM] = acc[j];
+    }
+  }
+}
+
+__global__ void __launch_bounds__(kRThreads) f64e_repair_kernel(const __grid_constant__ RepairArgs g) {
+  chained_wait();
+  __shared__ uint16_t list[kRM * kRN];
+  __shared__ int64_t offK[kRK];
+  __shared__ uint8_t bad[kRM + kRN];  // rows of A, then of B
+  __shared__ int count;
+  for (int64_t tile = blockIdx.x; tile < g.ntiles; tile += gridDim.x) {
+    const int64_t m0 = tile % g.tiles_m * kRM, n0 = tile / g.tiles_m * kRN;
+    bool any = false;
+    if (threadIdx.x < kRM + kRN) {
+      const bool is_a = threadIdx.x < kRM;
+      const int64_t r = is_a ? m0 + threadIdx.x : n0 + threadIdx.x - kRM;
+      any = r < (is_a ? g.M : g.N) && f64e_no_digits(is_a ? g.a_exp[r] : g.b_exp[r]);
+      bad[threadIdx.x] = any;
+    }
+    if (threadIdx.x == 0) count = 0;
+    if (!__syncthreads_or(any)) continue;
+    for (int e = threadIdx.x; e < kRM * kRN; e += kRThreads) {
+      const int ml = e % kRM, nl = e / kRM;
+      if (m0 + ml < g.M && n0 + nl < g.N && (bad[ml] || bad[kRM + nl])) list[atomicAdd(&count, 1)] = (uint16_t)e;
+    }
+    __syncthreads();
+    repair_outputs(g, list, count, m0, n0, offK);
+    __syncthreads();
   }
 }
 
@@ -452,7 +546,7 @@ cudaError_t launch_f64e_gemm(const F64eGemmArgs& a, int sm_count, int* errflag, 
                              int* launches) {
   *launches = 0;
   if (a.M <= 0 || a.N <= 0) return cudaSuccess;
-  if (!a.A || !a.B || !a.C || !a.a_exp || !a.b_exp || !a.a_flag || !a.b_flag || a.K <= 0 || a.K > kF64eMaxK) {
+  if (!a.A || !a.B || !a.C || !a.a_exp || !a.b_exp || a.K <= 0 || a.K > kF64eMaxK) {
     if (why) *why = "f64e_gemm: every operand given and K at most 2^21";
     return cudaErrorInvalidValue;
   }
@@ -470,23 +564,44 @@ cudaError_t launch_f64e_gemm(const F64eGemmArgs& a, int sm_count, int* errflag, 
     grid = std::min<int64_t>(tm * tn, std::max(1, sm_count));
   }
   using Kern = void (*)(const unsigned char*, const unsigned char*, double2*, int64_t, int64_t, int, int64_t, int64_t,
-                        const float*, const float*, const int*, const int*, int, longlong2*, int*);
+                        const float*, const float*, longlong2*, int*);
   static const Kern kerns[4] = {f64e_gemm_kernel<8, false>, f64e_gemm_kernel<8, true>, f64e_gemm_kernel<7, false>,
                                 f64e_gemm_kernel<7, true>};
   static PerDeviceOnce opt_in[4];
   const int which = (a.levels == 7 ? 2 : 0) + (share ? 1 : 0);
   if (const cudaError_t e = smem_opt_in(opt_in[which], kerns[which], kSmem)) return e;
   launch_chained(kerns[which], dim3((unsigned)grid), dim3(kThreads), kSmem, s, static_cast<const unsigned char*>(a.A), static_cast<const unsigned char*>(a.B), a.C, a.M, a.N, nkb, tm, tn,
-      a.a_exp, a.b_exp, a.a_flag, a.b_flag, a.token, share ? static_cast<longlong2*>(a.part) : nullptr, errflag);
+      a.a_exp, a.b_exp, share ? static_cast<longlong2*>(a.part) : nullptr, errflag);
   cudaError_t e = cudaGetLastError();
   *launches = 1;
   if (e == cudaSuccess && share) {
     *launches = 2;
     const int64_t rest = tm * tn - tm * tn / grid * grid;
     launch_chained(f64e_finish_kernel, dim3((unsigned)(rest * (kCols / 2))), dim3(32 * kEpiWarps), 0, s, static_cast<const longlong2*>(a.part), a.C, a.M, a.N,
-                                                             nchunks, tm, tn, (int)grid, a.a_exp, a.b_exp, a.a_flag,
-                                                             a.b_flag, a.token);
+                                                             nchunks, tm, tn, (int)grid, a.a_exp, a.b_exp);
     e = cudaGetLastError();
   }
   return e;
+}
+
+cudaError_t launch_f64e_repair(const F64eGemmArgs& a, const double2* T, const GatherTab& tab, const GroupSpec& mg,
+                               const GroupSpec& kg, const double2* B, int sm_count, cudaStream_t s) {
+  if (a.M <= 0 || a.N <= 0) return cudaSuccess;
+  RepairArgs g;
+  g.T = T;
+  g.om = tab.om;
+  g.ok = tab.ok;
+  g.mg = mg;
+  g.kg = kg;
+  g.B = B;
+  g.C = a.C;
+  g.M = a.M;
+  g.N = a.N;
+  g.K = a.K;
+  g.tiles_m = (a.M + kRM - 1) / kRM;
+  g.ntiles = g.tiles_m * ((a.N + kRN - 1) / kRN);
+  g.a_exp = a.a_exp;
+  g.b_exp = a.b_exp;
+  const int64_t grid = std::min<int64_t>(g.ntiles, 4 * std::max(1, sm_count));
+  return launch_chained(f64e_repair_kernel, dim3((unsigned)grid), dim3(kRThreads), 0, s, g);
 }

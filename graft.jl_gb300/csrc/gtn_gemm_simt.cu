@@ -375,9 +375,7 @@ template <int TM, int TN, int R, int KS>
 __global__ void __launch_bounds__(256) zgemm_view_kernel(const double2* __restrict__ T, GroupSpec mg, GroupSpec kg,
                                                          const double2* __restrict__ B, double2* __restrict__ C,
                                                          int64_t M, int64_t N, int64_t K, int64_t tiles_m,
-                                                         int64_t ntiles, int64_t kchunk,
-                                                         const int* __restrict__ a_flag,
-                                                         const int* __restrict__ b_flag, int token, OutView ov) {
+                                                         int64_t ntiles, int64_t kchunk, OutView ov) {
   chained_wait();
   constexpr bool kAhead = KS > 1;
   constexpr int KB = kAhead ? 64 : BK, KOFF = kAhead ? 512 : BK;
@@ -387,7 +385,6 @@ __global__ void __launch_bounds__(256) zgemm_view_kernel(const double2* __restri
   C += (int64_t)blockIdx.y * M * N;
   static_assert((TM / R) * (TN / R) * KS == 256 && KB % KS == 0, "one thread per R x R outputs and slice");
   static_assert(TM * KB % 256 == 0 && TN * KB % 256 == 0 && KOFF % KB == 0, "whole loads per thread");
-  if (a_flag && *a_flag != token && *b_flag == 0) return;
   __shared__ double2 As[KB][TM + 1];
   __shared__ double2 Bs[KB][TN + 1];
   __shared__ int64_t offM[TM], offK[KOFF];
@@ -486,37 +483,36 @@ __global__ void __launch_bounds__(256) zgemm_view_kernel(const double2* __restri
 
 template <int TM, int TN, int R, int KS>
 cudaError_t launch_view(const double2* T, const GroupSpec& mg, const GroupSpec& kg, const double2* B, double2* C,
-                        int64_t M, int64_t N, int64_t K, int64_t kchunk, cudaStream_t s, const int* a_flag,
-                        const int* b_flag, int token, const OutView& ov) {
+                        int64_t M, int64_t N, int64_t K, int64_t kchunk, cudaStream_t s,
+                        const OutView& ov) {
   const int64_t tm = (M + TM - 1) / TM, nt = tm * ((N + TN - 1) / TN);
-  // a launch that usually has nothing to do keeps its grid small
-  const int64_t grid = std::min<int64_t>(nt, a_flag ? 2 * 152 : (int64_t(1) << 30));
+  const int64_t grid = std::min<int64_t>(nt, int64_t(1) << 30);
   const int64_t slices = (K + kchunk - 1) / kchunk;
-  launch_chained(zgemm_view_kernel<TM, TN, R, KS>, dim3((unsigned)grid, (unsigned)slices), dim3(256), 0, s, T, mg, kg, B, C, M, N, K, tm, nt, kchunk, a_flag, b_flag, token, ov);
+  launch_chained(zgemm_view_kernel<TM, TN, R, KS>, dim3((unsigned)grid, (unsigned)slices), dim3(256), 0, s, T, mg, kg, B, C, M, N, K, tm, nt, kchunk, ov);
   return cudaGetLastError();
 }
 
 }  // namespace
 
 cudaError_t launch_zgemm_view(const double2* T, const GroupSpec& mg, const GroupSpec& kg, const double2* B, double2* C,
-                              int64_t M, int64_t N, int64_t K, cudaStream_t s, const int* a_flag, const int* b_flag,
-                              int token, int slices, double2* P, const OutView& ov) {
+                              int64_t M, int64_t N, int64_t K, cudaStream_t s, int slices,
+                              double2* P, const OutView& ov) {
   if (M <= 0 || N <= 0) return cudaSuccess;
   auto tiles = [&](int t) { return ((M + t - 1) / t) * ((N + t - 1) / t); };
-  if (tiles(64) >= 2 * 152) return launch_view<64, 64, 4, 1>(T, mg, kg, B, C, M, N, K, K, s, a_flag, b_flag, token, ov);
-  if (tiles(32) >= 2 * 152) return launch_view<32, 32, 2, 1>(T, mg, kg, B, C, M, N, K, K, s, a_flag, b_flag, token, ov);
-  if (tiles(16) >= 2 * 152) return launch_view<16, 16, 1, 1>(T, mg, kg, B, C, M, N, K, K, s, a_flag, b_flag, token, ov);
+  if (tiles(64) >= 2 * 152) return launch_view<64, 64, 4, 1>(T, mg, kg, B, C, M, N, K, K, s, ov);
+  if (tiles(32) >= 2 * 152) return launch_view<32, 32, 2, 1>(T, mg, kg, B, C, M, N, K, K, s, ov);
+  if (tiles(16) >= 2 * 152) return launch_view<16, 16, 1, 1>(T, mg, kg, B, C, M, N, K, K, s, ov);
   if (slices > 1 && P) {
     if (ov.on) return cudaErrorInvalidValue;  // slices are summed into C[n][m]
     const int64_t kchunk = ((K + slices - 1) / slices + BK - 1) / BK * BK;
-    cudaError_t e = launch_view<16, 16, 1, 1>(T, mg, kg, B, P, M, N, K, kchunk, s, a_flag, b_flag, token, OutView());
+    cudaError_t e = launch_view<16, 16, 1, 1>(T, mg, kg, B, P, M, N, K, kchunk, s, OutView());
     if (e != cudaSuccess) return e;
     const int64_t blocks = std::min<int64_t>((M * N + 255) / 256, 152 * 8);
     launch_chained(splitk_reduce_kernel<double2>, dim3((unsigned)blocks), dim3(256), 0, s, P, (int)((K + kchunk - 1) / kchunk), M * N, C);
     return cudaGetLastError();
   }
-  if (tiles(8) >= 2 * 152) return launch_view<8, 8, 1, 4>(T, mg, kg, B, C, M, N, K, K, s, a_flag, b_flag, token, ov);
-  return launch_view<4, 4, 1, 16>(T, mg, kg, B, C, M, N, K, K, s, a_flag, b_flag, token, ov);
+  if (tiles(8) >= 2 * 152) return launch_view<8, 8, 1, 4>(T, mg, kg, B, C, M, N, K, K, s, ov);
+  return launch_view<4, 4, 1, 16>(T, mg, kg, B, C, M, N, K, K, s, ov);
 }
 int zgemm_view_slices(int64_t M, int64_t N, int64_t K) {
   const int64_t t16 = ((M + 15) / 16) * ((N + 15) / 16), t4 = ((M + 3) / 4) * ((N + 3) / 4);

@@ -91,10 +91,6 @@ struct gtn_ctx_s {
   std::mutex err_mu;
   int64_t launches = 0;
   int* d_errflag = nullptr;
-  // out-of-range flags of the digit-plane products: product number t writes t to slot
-  // t % kFbSlots, so no slot needs clearing between products (they are ordered on the stream)
-  int* d_fbflag = nullptr;
-  int fb_token = 0;
   int sm_count = 0;
   int cc_major = 0, cc_minor = 0;
   // reduction scratch (device + pinned host)
@@ -119,8 +115,6 @@ struct gtn_ctx_s {
   std::multimap<size_t, void*> blk_free;
   size_t blk_cached = 0;
 };
-
-constexpr int kFbSlots = 1024;
 
 // ---- status helpers -------------------------------------------------------------
 int set_err(gtn_ctx ctx, int code, const std::string& msg);
@@ -407,12 +401,15 @@ cudaError_t launch_tc_gemm(const TcGemmArgs& a, int* errflag, cudaStream_t s, st
 // [row tile of 128][16 real k][plane][128][32 bytes], the real-expanded B' in blocks of 64
 // rows; row m of A scaled by 2^(1021 - a_exp[m]), complex row n of B by 2^(1021 - b_exp[n])
 // (biased exponents of the rows' largest entries).  A row whose exponent lies outside
-// [kF64eMinExp, kF64eMaxExp] (infinities, NaN, magnitudes beyond 2^+-450) sets a flag, the GEMM
-// then leaves C alone and the FP64 kernel launched behind it computes the product.
+// [kF64eMinExp, kF64eMaxExp] (infinities, NaN, magnitudes beyond 2^+-450) has no digits: its outputs
+// are computed again by launch_f64e_repair.
 constexpr int kF64eSlices = 7;
 constexpr int kF64eRowsA = 128, kF64eRowsB = 64;
 constexpr int64_t kF64eMaxK = int64_t(1) << 21;  // the 64-bit sums hold 2^22 real k
 constexpr int kF64eMinExp = 1023 - 450, kF64eMaxExp = 1023 + 450;
+__host__ __device__ inline bool f64e_no_digits(float E) {
+  return E != 0.f && !(E >= (float)kF64eMinExp && E <= (float)kF64eMaxExp);
+}
 inline size_t f64e_a_bytes(int64_t M, int64_t K) {
   return (size_t)((M + kF64eRowsA - 1) / kF64eRowsA) * ((K + 7) / 8) * kF64eSlices * kF64eRowsA * 32;
 }
@@ -430,9 +427,6 @@ struct F64eGemmArgs {
   int64_t M = 0, N = 0, K = 0;
   const float* a_exp = nullptr;
   const float* b_exp = nullptr;
-  const int* a_flag = nullptr;  // == token: a row of A out of range
-  const int* b_flag = nullptr;  // != 0: a row of B out of range
-  int token = 0;
   int levels = 8;               // digit products d_i e_j with i + j < levels (7 or 8)
   void* part = nullptr;         // f64e_part_bytes of the product, or null: no tile is shared
 };
@@ -440,22 +434,22 @@ cudaError_t launch_f64e_gemm(const F64eGemmArgs& a, int sm_count, int* errflag, 
                              int* launches);
 // Bytes of partial sums of the tiles that CTAs share in a product (0: none are).
 size_t f64e_part_bytes(int64_t M, int64_t N, int64_t K, int sm_count);
-// Digit planes and row exponents of the running tensor's K-major view (c128; *flag = token when
-// a row is out of range), and of a static B [N][K] (*flag = 1 when a row is out of range).
+// The outputs of rows without digits (of A or of B), each summed again on the FP64 pipe from the
+// operands: T read in place (offsets from the tables, or the groups where tab has none), B [N][K].
+cudaError_t launch_f64e_repair(const F64eGemmArgs& a, const double2* T, const GatherTab& tab, const GroupSpec& mg,
+                               const GroupSpec& kg, const double2* B, int sm_count, cudaStream_t s);
+// Digit planes and row exponents of the running tensor's K-major view (c128) and of a static B [N][K].
 cudaError_t launch_split_digits_tab(const double2* T, const GatherTab& t, int64_t M, int64_t K, float* rexp, void* out,
-                                    int* flag, int token, cudaStream_t s, int* launches);
+                                    cudaStream_t s, int* launches);
 cudaError_t launch_split_digits_grp(const double2* T, const GroupSpec& mg, const GroupSpec& kg, int64_t M, int64_t K,
-                                    float* rexp, void* out, int* flag, int token, cudaStream_t s, int* launches);
-cudaError_t launch_pack_b_digits(const double2* B, int64_t N, int64_t K, void* out, float* bexp, int* flag,
-                                 cudaStream_t s);
-// C[n][m] = sum_k T[offM(m) + offK(k)] B[n][k] on the FP64 pipe, T read in place; with a_flag
-// set the launch does its work only if *a_flag == token or *b_flag != 0.  With slices > 1 (of
-// zgemm_view_slices: few outputs, long K) the k range is cut into that many partial products
+                                    float* rexp, void* out, cudaStream_t s, int* launches);
+cudaError_t launch_pack_b_digits(const double2* B, int64_t N, int64_t K, void* out, float* bexp, cudaStream_t s);
+// C[n][m] = sum_k T[offM(m) + offK(k)] B[n][k] on the FP64 pipe, T read in place.  With slices > 1
+// (of zgemm_view_slices: few outputs, long K) the k range is cut into that many partial products
 // P[slice][n][m], summed in order.
 int zgemm_view_slices(int64_t M, int64_t N, int64_t K);
 cudaError_t launch_zgemm_view(const double2* T, const GroupSpec& mg, const GroupSpec& kg, const double2* B, double2* C,
-                              int64_t M, int64_t N, int64_t K, cudaStream_t s, const int* a_flag = nullptr,
-                              const int* b_flag = nullptr, int token = 0, int slices = 1, double2* P = nullptr,
+                              int64_t M, int64_t N, int64_t K, cudaStream_t s, int slices = 1, double2* P = nullptr,
                               const OutView& ov = OutView());
 bool tc_gemm_supported(int cc_major, int cc_minor);
 // Independent problems in one launch per kTcGroupMax problems (same product list for all).
@@ -532,7 +526,6 @@ struct PlanStep {
   bool dg = false;
   void* bdig = nullptr;
   float* bexp = nullptr;
-  int* bflag = nullptr;
   double macs = 0;
 };
 

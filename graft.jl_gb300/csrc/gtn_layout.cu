@@ -447,9 +447,6 @@ __device__ __forceinline__ int64_t digit_chunk(int64_t r, int64_t chunk, int row
   const int rr = (int)(r - rt * rows);
   return ((rt * nkb + (chunk >> 1)) * kF64eSlices * rows + rr) * 32 + (((int)chunk ^ (rr >> 2)) & 1) * 16;
 }
-__device__ __forceinline__ void digit_check(float E, int token, int* flag) {
-  if (E != 0.f && !(E >= (float)kF64eMinExp && E <= (float)kF64eMaxExp)) *flag = token;
-}
 
 // Element (m, k) of the A operand: its digits in the planes (4 bytes each).
 struct DigitWriter {
@@ -457,11 +454,8 @@ struct DigitWriter {
   unsigned char* out;
   int64_t nkb;
   const float* rexp;
-  int* flag;
-  int token;
   __device__ void operator()(int64_t m, int64_t k, double2 v) const {
     const float E = rexp[m];
-    digit_check(E, token, flag);
     const unsigned long long a = digit_word(v.x, (int)E), b = digit_word(v.y, (int)E);
     unsigned char* p = out + digit_chunk(m, k >> 2, kF64eRowsA, nkb) + (k & 3) * 4;
 #pragma unroll
@@ -473,11 +467,9 @@ struct DigitWriter {
 struct DigitRowWriter {
   unsigned char* out;
   int64_t nkb;
-  int* flag;
-  int token;
   using Mag = ExpMag;
   static constexpr int kCols = 4;
-  __device__ void row(float E) const { digit_check(E, token, flag); }
+  __device__ void row(float) const {}
   __device__ void operator()(int64_t m, int64_t k, const double2* v, float E) const {
     unsigned long long w[8];
 #pragma unroll
@@ -499,7 +491,7 @@ struct DigitRowWriter {
 // both real rows (the digits of -Bi are the negated digits of Bi).
 __global__ void __launch_bounds__(256) pack_b_digits_kernel(const double2* __restrict__ B, int64_t N, int64_t K,
                                                             int64_t nkb, float* __restrict__ bexp,
-                                                            unsigned char* __restrict__ out, int* flag) {
+                                                            unsigned char* __restrict__ out) {
   chained_wait();
   __shared__ float se[8];
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -513,10 +505,7 @@ __global__ void __launch_bounds__(256) pack_b_digits_kernel(const double2* __res
     for (int o = 16; o > 0; o >>= 1) x = fmaxf(x, __shfl_xor_sync(0xffffffffu, x, o));
     if (lane == 0) {
       se[warp] = x;
-      if (n < N) {
-        bexp[n] = x;
-        digit_check(x, 1, flag);
-      }
+      if (n < N) bexp[n] = x;
     }
   }
   __syncthreads();
@@ -1977,39 +1966,38 @@ cudaError_t launch_split16_rows_grp(const void* T, int is64, const GroupSpec& mg
 // split, or row exponents first and then the planes when a row is too long for it.
 template <class Off>
 static cudaError_t split_digits(const double2* T, const Off& off, int m_fast, const GroupSpec* mg, const GroupSpec* kg,
-                                int64_t M, int64_t K, float* rexp, unsigned char* out, int* flag, int token,
-                                cudaStream_t s, int* launches) {
+                                int64_t M, int64_t K, float* rexp, unsigned char* out, cudaStream_t s,
+                                int* launches) {
   const int64_t Kp = (K + 7) / 8 * 8, nkb = Kp / 8;
   bool done = false;
-  cudaError_t e = launch_split_rows(T, off, M, K, Kp, m_fast, DigitRowWriter{out, nkb, flag, token}, rexp, s, &done);
+  cudaError_t e = launch_split_rows(T, off, M, K, Kp, m_fast, DigitRowWriter{out, nkb}, rexp, s, &done);
   *launches = 1;
   if (e != cudaSuccess || done) return e;
   *launches = 2;
   e = launch_rowmax<ExpMag>(T, off, m_fast, M, K, rexp, s);
   if (e != cudaSuccess) return e;
-  const DigitWriter w{out, nkb, rexp, flag, token};
+  const DigitWriter w{out, nkb, rexp};
   if constexpr (std::is_same<Off, TabOff>::value)
     return launch_gather_tab(T, off.om, off.ok, M, K, Kp, m_fast, w, s);
   else
     return launch_gather(T, *mg, *kg, M, K, Kp, w, s);
 }
 cudaError_t launch_split_digits_tab(const double2* T, const GatherTab& t, int64_t M, int64_t K, float* rexp, void* out,
-                                    int* flag, int token, cudaStream_t s, int* launches) {
+                                    cudaStream_t s, int* launches) {
   return split_digits(T, TabOff{t.om, t.ok}, t.m_fast, nullptr, nullptr, M, K, rexp, static_cast<unsigned char*>(out),
-                      flag, token, s, launches);
+                      s, launches);
 }
 cudaError_t launch_split_digits_grp(const double2* T, const GroupSpec& mg, const GroupSpec& kg, int64_t M, int64_t K,
-                                    float* rexp, void* out, int* flag, int token, cudaStream_t s, int* launches) {
+                                    float* rexp, void* out, cudaStream_t s, int* launches) {
   return split_digits(T, GrpOffV{mg, kg}, choose_m_fast(mg, kg) ? 1 : 0, &mg, &kg, M, K, rexp,
-                      static_cast<unsigned char*>(out), flag, token, s, launches);
+                      static_cast<unsigned char*>(out), s, launches);
 }
-cudaError_t launch_pack_b_digits(const double2* B, int64_t N, int64_t K, void* out, float* bexp, int* flag,
+cudaError_t launch_pack_b_digits(const double2* B, int64_t N, int64_t K, void* out, float* bexp,
                                  cudaStream_t s) {
   if (N <= 0) return cudaSuccess;
   const int64_t blocks = (N + 7) / 8;
   if (blocks > 2147483647LL) return cudaErrorInvalidConfiguration;
-  launch_chained(pack_b_digits_kernel, dim3((unsigned)blocks), dim3(256), 0, s, B, N, K, (K + 7) / 8, bexp, static_cast<unsigned char*>(out),
-                                                       flag);
+  launch_chained(pack_b_digits_kernel, dim3((unsigned)blocks), dim3(256), 0, s, B, N, K, (K + 7) / 8, bexp, static_cast<unsigned char*>(out));
   return cudaGetLastError();
 }
 cudaError_t launch_gather_tab_to_c128(const void* T, int is64, const GatherTab& t, int64_t M, int64_t K, int64_t ldo,

@@ -146,9 +146,7 @@ int pack_digits(gtn_map map, bool required) {
     cudaGetLastError();  // without them no tile is shared
     map->part = nullptr;
   }
-  int* flags = nullptr;
-  cudaError_t e = dalloc(map, &flags, map->steps.size() * sizeof(int));
-  if (e == cudaSuccess) e = cudaMemsetAsync(flags, 0, map->steps.size() * sizeof(int), ctx->stream);
+  cudaError_t e = cudaSuccess;
   for (size_t i = 0; i < map->steps.size() && e == cudaSuccess; ++i) {
     PlanStep& st = map->steps[i];
     if (!st.dg) continue;
@@ -160,8 +158,7 @@ int pack_digits(gtn_map map, bool required) {
       cudaGetLastError();
       continue;
     }
-    st.bflag = flags + i;
-    e = launch_pack_b_digits(st.b64, st.N, st.K, planes, st.bexp, st.bflag, ctx->stream);
+    e = launch_pack_b_digits(st.b64, st.N, st.K, planes, st.bexp, ctx->stream);
     ctx->launches++;
     st.bdig = planes;
   }
@@ -789,9 +786,8 @@ int map_run(gtn_map map, int precision, const double2* x, double2* y) {
         ctx->launches++;
       } else if (st.bdig && map->amax) {
         // digit planes of the running tensor, the exact digit-product GEMM straight into
-        // complex FP64, and the FP64 kernel that takes over when a row was out of range
+        // complex FP64, and the outputs that the planes cannot give
         const double2* T = static_cast<const double2*>(cur);
-        ctx->fb_token = ctx->fb_token == INT32_MAX ? 1 : ctx->fb_token + 1;
         F64eGemmArgs a;
         a.A = map->abuf;
         a.B = st.bdig;
@@ -801,16 +797,12 @@ int map_run(gtn_map map, int precision, const double2* x, double2* y) {
         a.K = st.K;
         a.a_exp = map->amax;
         a.b_exp = st.bexp;
-        a.token = ctx->fb_token;
         a.levels = f64e ? 7 : 8;
         a.part = map->part;
-        a.a_flag = ctx->d_fbflag + ctx->fb_token % kFbSlots;
-        a.b_flag = st.bflag;
-        int* flag = ctx->d_fbflag + ctx->fb_token % kFbSlots;
         int nl = 0;
         prof_begin(s);
-        if (st.tab.om) e = launch_split_digits_tab(T, st.tab, st.M, st.K, map->amax, map->abuf, flag, a.token, s, &nl);
-        else e = launch_split_digits_grp(T, st.mg, st.kg, st.M, st.K, map->amax, map->abuf, flag, a.token, s, &nl);
+        if (st.tab.om) e = launch_split_digits_tab(T, st.tab, st.M, st.K, map->amax, map->abuf, s, &nl);
+        else e = launch_split_digits_grp(T, st.mg, st.kg, st.M, st.K, map->amax, map->abuf, s, &nl);
         prof_end(s, GTN_KERNEL_SPLIT, 0.0);
         ctx->launches += nl;
         if (e == cudaSuccess) {
@@ -820,7 +812,7 @@ int map_run(gtn_map map, int precision, const double2* x, double2* y) {
           prof_end(s, GTN_KERNEL_TC_GEMM, 8.0 * st.macs);
           if (e != cudaSuccess) return set_err(ctx, GTN_ERR_CUDA, "f64e_gemm: " + why + " " + cudaGetErrorString(e));
           prof_begin(s);
-          e = launch_zgemm_view(T, st.mg, st.kg, st.b64, a.C, st.M, st.N, st.K, s, a.a_flag, a.b_flag, a.token);
+          e = launch_f64e_repair(a, T, st.tab, st.mg, st.kg, st.b64, ctx->sm_count, s);
           prof_end(s, GTN_KERNEL_ZGEMM, 0.0);
           ctx->launches += nl + 1;
         }
@@ -833,7 +825,7 @@ int map_run(gtn_map map, int precision, const double2* x, double2* y) {
                             (i > 0 || !(x < y + map->y_elems && y < xe));
         prof_begin(s);
         e = launch_zgemm_view(static_cast<const double2*>(cur), st.mg, st.kg, st.b64,
-                              direct ? y : static_cast<double2*>(out), st.M, st.N, st.K, s, nullptr, nullptr, 0, slices,
+                              direct ? y : static_cast<double2*>(out), st.M, st.N, st.K, s, slices,
                               static_cast<double2*>(map->skbuf), direct ? map->out : OutView());
         prof_end(s, GTN_KERNEL_ZGEMM, 8.0 * st.macs);
         ctx->launches += slices > 1 ? 2 : 1;
