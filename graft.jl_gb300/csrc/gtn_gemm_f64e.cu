@@ -21,8 +21,8 @@
 // 2-norm, Gaussian operands: K = 65 5.7e-17 (FP64 pipe 3.7e-16), K = 5120 7.1e-17 (3.4e-15),
 // rows that decay from 1 to 1e-9 along k 1.3e-16 (5.4e-16) and 1.8e-16 (4.9e-15); L = 7 about
 // 3.6e-16 at every K.
-// A row with an infinity, a NaN or a magnitude beyond 2^+-450 has no digits: what this kernel makes
-// of it is overwritten by f64e_repair_kernel, which looks at the rows' exponents and leaves no trace
+// A row with an infinity, a NaN, nothing but subnormals or a magnitude beyond 2^+-450 has no digits:
+// what this kernel makes of it is overwritten by f64e_repair_kernel, which looks at the rows' exponents and leaves no trace
 // for a later product.
 //
 // Tile: 128 rows x 64 real columns (32 complex); stages of 16 real k hold all 7 planes of A

@@ -401,8 +401,8 @@ cudaError_t launch_tc_gemm(const TcGemmArgs& a, int* errflag, cudaStream_t s, st
 // [row tile of 128][16 real k][plane][128][32 bytes], the real-expanded B' in blocks of 64
 // rows; row m of A scaled by 2^(1021 - a_exp[m]), complex row n of B by 2^(1021 - b_exp[n])
 // (biased exponents of the rows' largest entries).  A row whose exponent lies outside
-// [kF64eMinExp, kF64eMaxExp] (infinities, NaN, magnitudes beyond 2^+-450) has no digits: its outputs
-// are computed again by launch_f64e_repair.
+// [kF64eMinExp, kF64eMaxExp] (infinities, NaN, subnormals, magnitudes beyond 2^+-450) has no digits:
+// its outputs are computed again by launch_f64e_repair.
 constexpr int kF64eSlices = 7;
 constexpr int kF64eRowsA = 128, kF64eRowsB = 64;
 constexpr int64_t kF64eMaxK = int64_t(1) << 21;  // the 64-bit sums hold 2^22 real k

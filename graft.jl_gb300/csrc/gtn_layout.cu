@@ -404,12 +404,14 @@ struct Split16RowWriter {
 // to every digit position turns the balanced digits into the bytes of one 56-bit number
 // (only the top one may reach 128 after the rounding), so a digit costs one byte extraction
 // and one FP32 add of 2^23 + byte instead of 64-bit shifts; |d_i| <= 128, exact in bf16.
-// Row "maxima" of these planes are the biased binary exponents of the largest entry (0 for a
-// zero or subnormal row, 2047 for a row with an infinity or NaN), held as floats.
+// Row "maxima" of these planes are the biased binary exponents of the largest entry (0 for a row of
+// zeros, 0.5 for one of subnormals, 2047 for a row with an infinity or NaN), held as floats.
 struct ExpMag {  // exponent of max(|re|, |im|)
   __device__ static float of(double2 v) {
-    const int a = (__double2hiint(v.x) >> 20) & 0x7ff, c = (__double2hiint(v.y) >> 20) & 0x7ff;
-    return (float)max(a, c);
+    const int hx = __double2hiint(v.x) & 0x7fffffff, hy = __double2hiint(v.y) & 0x7fffffff;
+    const int e = max(hx, hy) >> 20;
+    if (e != 0) return (float)e;
+    return (hx | hy | __double2loint(v.x) | __double2loint(v.y)) != 0 ? 0.5f : 0.f;
   }
 };
 

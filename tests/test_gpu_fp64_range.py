@@ -50,3 +50,16 @@ def test_a_replay_forgets_an_infinite_row():
         assert np.array_equal(replay(good), first)
         m.close()
         ctx.close()
+
+
+@pytest.mark.parametrize("prec", ["fp64", "fp64e"])
+def test_subnormal_rows_are_multiplied(ctx, prec):
+    rng = np.random.default_rng(5)
+    M, K, N = 300, 700, 200
+    A, B = crandn(rng, (M, K)), crandn(rng, (K, N)) * 1e100
+    A[3] *= 1e-310
+    got, ref = contract(ctx, A, B, prec), A @ B
+    assert np.abs(ref[3]).min() > 1e-213
+    assert np.all(np.abs(got - ref) <= 4 * K * 2.0 ** -52 * (np.abs(A) @ np.abs(B)))
+    got = contract(ctx, np.ascontiguousarray(B.T), np.ascontiguousarray(A.T), prec)
+    assert np.all(np.abs(got - ref.T) <= 4 * K * 2.0 ** -52 * (np.abs(A) @ np.abs(B)).T)
