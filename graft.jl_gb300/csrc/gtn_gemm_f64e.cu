@@ -16,7 +16,9 @@
 //     every 256, and add them with their weights into two 64-bit integers per output (units
 //     2^-72 and 2^-40): the sum over all k of the kept digit products is exact.  Its one rounding
 //     is the conversion to FP64 at the end, done on the integers' bits.
-// What is left out (levels from L on, digits beyond the seventh) does not grow with K, unlike the
+// In FP64 every output is checked against the bound of an FP64 sum and, where the digits may miss it,
+// summed again on the FP64 pipe (f64e_check_kernel, f64e_repair_kernel).  What is left out of the
+// others (levels from L on, digits beyond the seventh) does not grow with K, unlike the
 // rounding errors of FP64 fused multiply-adds.  Measured against extended precision, relative
 // 2-norm, Gaussian operands: K = 65 5.7e-17 (FP64 pipe 3.7e-16), K = 5120 7.1e-17 (3.4e-15),
 // rows that decay from 1 to 1e-9 along k 1.3e-16 (5.4e-16) and 1.8e-16 (4.9e-15); L = 7 about
@@ -413,10 +415,39 @@ __global__ void __launch_bounds__(32 * kEpiWarps)
 }
 
 // ---- outputs that the digit planes cannot give --------------------------------------------------
-// A CTA walks over tiles of kRM x kRN complex outputs and lists those to be summed again on the FP64
-// pipe: four a warp, the k range over its lanes, K offsets of kRK columns at a time.  Ordinary
-// operands list none, and a tile costs the reading of its rows' exponents.
-constexpr int kRM = 128, kRN = 64, kRK = 512, kRThreads = 256, kRPerWarp = 4;
+// A digit holds its entry to 2^-57 of the row's power of two, so an output is as accurate as its
+// rows' largest entries, which a sparse or graded sum can be far below.  With E the sum of
+//   2^-56 (alpha_k + beta_k) + 2^-62.6
+// over the k at which neither factor is zero (alpha, beta: magnitudes max(|re|, |im|) of the scaled
+// rows, at most 1/2; the last term for the levels left out), each part of an output is exact to E.
+// It stands where E <= 2 K 2^-53 sum alpha beta, the a-priori bound of K complex multiply-adds in
+// FP64 (N. J. Higham, Accuracy and Stability of Numerical Algorithms, 2nd ed., section 3.1); the others
+// are summed again on the FP64 pipe.
+//   * f64e_check_kernel looks for outputs with sum alpha beta below kSureSum, above which the bound
+//     holds whatever the entries.  Two rows with L of W entries more than W = 128 together that are at
+//     least 0.0508 have L products of 0.0026 in common: 28 are enough, and so the tiles of dense
+//     operands are done by counting (a row of 128 Gaussian entries has 110 such).  Of the others the
+//     sums are formed from bf16 magnitudes, 64 k at a time until all are above.  A sum of zero means
+//     that no two factors meet, and that the digit products are exact.  What remains is listed.
+//   * f64e_repair_kernel adds E and the magnitudes' products over the listed outputs' rows and sums
+//     those again whose bound does not hold.  Chunks of 32 listed outputs keep every SM at work where
+//     they come from few tiles (a state of Schmidt weights down to 1e-5 meets the identity
+//     channel of its environments, 4 of 24 tiles).
+// The sums have half of the digit product's rows, columns and k and one plane: mma.sync, which
+// needs no TMEM (the digit levels hold all of it), leaves them a small part of the step.
+// One-site map of a 31-site binary tree at D = 128 (M = 163840, N = 640, K = 128, digit product
+// 2423 us): the sums take 241 us, 148 us with tiles that end early, and counting 27 us.  Products of the
+// two-site map of a DMRG step at D = 96 (M = 384, N = 480, K = 96 and M = 384, N = 96, K = 480) with a
+// state of which 7 to 10 % of the outputs are summed again: check 9 and 15 us, repair 33 and 38 us
+// (with a CTA for each tile 1059 and 510 us together); 1 % of a Lanczos vector's: 24 us together.
+constexpr int kRM = kF64eCheckM, kRN = kF64eCheckN, kRThreads = 256;
+constexpr int kRKC = 64, kRStages = 2;              // complex k per stage (rows of 128 bytes)
+constexpr int kRStage = (kRM + kRN) * kRKC * 2;
+constexpr int kRSmem = kRStages * kRStage;
+static_assert(kRM * kRN * 2 <= kRStage, "a tile's list in a stage");
+// (2^-56 + 2^-62.6) K <= 2 K 2^-53 s from s = 0.0632 on; the rest covers the rounding of the sums
+constexpr float kSureSum = 0.0703f;
+constexpr int kSureMeets = 28;  // times 0.05078^2
 
 struct RepairArgs {
   const double2* T;
@@ -426,48 +457,242 @@ struct RepairArgs {
   double2* C;
   int64_t M, N, K, tiles_m, ntiles;
   const float *a_exp, *b_exp;
+  const uint16_t *a_mag, *b_mag;
+  const int* b_large;
+  uint16_t* lists;             // [tile][kRM kRN]: n_local kRM + m_local
+  unsigned long long* chunks;  // tile << 24 | first << 8 | length
+  int* count;                  // chunks
 };
 
-// Sum the listed outputs (n_local * kRM + m_local) of the tile at (m0, n0) again.
-__device__ __forceinline__ void repair_outputs(const RepairArgs& g, const uint16_t* list, int count, int64_t m0,
-                                               int64_t n0, int64_t* offK) {
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  constexpr int kPass = kRThreads / 32 * kRPerWarp;
+__global__ void __launch_bounds__(kRThreads, 3) f64e_check_kernel(const __grid_constant__ RepairArgs g) {
+  chained_wait();
+  extern __shared__ __align__(128) unsigned char rsmem[];
+  __shared__ int count, slot, large[kRM], least_row[kRThreads / 32];
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  const int wm = (warp & 3) * 32, wn = (warp >> 2) * 32;
+  const int64_t nkb = (g.K + 7) / 8;
+  const int nk = (int)((nkb + kRKC / 8 - 1) / (kRKC / 8));
+  const uint32_t s0 = smem_u32(rsmem);
+  auto ldmatrix = [&](uint32_t addr, uint32_t (&v)[4]) {
+    asm volatile("ldmatrix.sync.aligned.m8n8.x4.shared.b16 {%0, %1, %2, %3}, [%4];"
+                 : "=r"(v[0]), "=r"(v[1]), "=r"(v[2]), "=r"(v[3])
+                 : "r"(addr)
+                 : "memory");
+  };
+  // chunk kc of the tile at (m0, n0) into a stage: 16 bytes (8 k) of a row a time, rows on consecutive threads
+  auto load = [&](int64_t m0, int64_t n0, int kc, int stage) {
+    if (kc < nk) {
+      const uint32_t st = s0 + (uint32_t)(stage * kRStage);
+      auto put = [&](const uint16_t* mag, int64_t row, int64_t rows, int r, int c) {
+        const int64_t kb = (int64_t)kc * (kRKC / 8) + c;
+        const bool in = row < rows && kb < nkb;
+        asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(st + r * 128 + ((c ^ (r & 7)) << 4)),
+                     "l"(mag + (in ? (kb * rows + row) * 8 : 0)), "r"(in ? 16 : 0)
+                     : "memory");
+      };
+#pragma unroll
+      for (int i = 0; i < kRM * 8 / kRThreads; ++i) {
+        const int e = i * kRThreads + tid, r = e % kRM;
+        put(g.a_mag, m0 + r, g.M, r, e / kRM);
+      }
+#pragma unroll
+      for (int i = 0; i < kRN * 8 / kRThreads; ++i) {
+        const int e = i * kRThreads + tid, r = e % kRN;
+        put(g.b_mag, n0 + r, g.N, kRM + r, e / kRN);
+      }
+    }
+    asm volatile("cp.async.commit_group;" ::: "memory");
+  };
+  float acc[2][4][4];
+  auto multiply = [&](int stage) {
+    const uint32_t st = s0 + (uint32_t)(stage * kRStage);
+#pragma unroll
+    for (int ks = 0; ks < kRKC / 16; ++ks) {
+      uint32_t a[2][4], b[2][4];
+#pragma unroll
+      for (int i = 0; i < 2; ++i) {
+        const int r = wm + i * 16 + (lane & 15), c = ks * 2 + (lane >> 4);
+        ldmatrix(st + r * 128 + ((c ^ (r & 7)) << 4), a[i]);
+      }
+#pragma unroll
+      for (int j = 0; j < 2; ++j) {
+        const int r = kRM + wn + j * 16 + (lane & 7) + ((lane >> 4) << 3), c = ks * 2 + ((lane >> 3) & 1);
+        ldmatrix(st + r * 128 + ((c ^ (r & 7)) << 4), b[j]);
+      }
+#pragma unroll
+      for (int i = 0; i < 2; ++i)
+#pragma unroll
+        for (int j = 0; j < 4; ++j)
+          asm volatile(
+              "mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0, %1, %2, %3}, {%4, %5, %6, %7}, {%8, %9}, "
+              "{%0, %1, %2, %3};"
+              : "+f"(acc[i][j][0]), "+f"(acc[i][j][1]), "+f"(acc[i][j][2]), "+f"(acc[i][j][3])
+              : "r"(a[i][0]), "r"(a[i][1]), "r"(a[i][2]), "r"(a[i][3]), "r"(b[j >> 1][(j & 1) * 2]),
+                "r"(b[j >> 1][(j & 1) * 2 + 1]));
+    }
+  };
+  auto for_outputs = [&](auto f) {  // f(m_local, n_local, sum)
+#pragma unroll
+    for (int i = 0; i < 2; ++i)
+#pragma unroll
+      for (int j = 0; j < 4; ++j)
+#pragma unroll
+        for (int e = 0; e < 4; ++e)
+          f(wm + i * 16 + (lane >> 2) + (e >> 1) * 8, wn + j * 8 + 2 * (lane & 3) + (e & 1), acc[i][j][e]);
+  };
+  uint16_t* list = reinterpret_cast<uint16_t*>(rsmem);
+  const int window = (int)min(g.K, (int64_t)kF64eWindow), wkb = (int)min(nkb, (int64_t)(kF64eWindow / 8));
+  // a CTA's tiles: a range with the column tiles of a row tile behind each other
+  const unsigned tiles_n = (unsigned)(g.ntiles / g.tiles_m);
+  const unsigned end = (unsigned)(g.ntiles * (blockIdx.x + 1) / gridDim.x);
+  unsigned row = ~0u;
 #pragma unroll 1
-  for (int base = 0; base < count; base += kPass) {
+  for (unsigned t = (unsigned)(g.ntiles * blockIdx.x / gridDim.x); t < end; ++t) {
+    const unsigned tm = t / tiles_n, tn = t - tm * tiles_n;
+    const int64_t m0 = (int64_t)tm * kRM, n0 = (int64_t)tn * kRN;
+    const int mlim = (int)min((int64_t)kRM, g.M - m0), nlim = (int)min((int64_t)kRN, g.N - n0);
+    // A CTA of one tile forms the sums at once: counting is worth its latency from the second one on
+    // (two-site map of a chain at D = 250, 160 tiles: 287 us with it, 283 without).
+    if (g.ntiles > gridDim.x && tm != row) {  // large entries of the row tile, two threads a row
+      row = tm;
+      if (tid < kRM) large[tid] = 0;
+      __syncthreads();
+      const int r = tid % kRM;
+      int c = 0;
+      if (r < mlim)
+#pragma unroll 4
+        for (int kb = tid / kRM; kb < wkb; kb += 2) {
+          const uint4 u = *reinterpret_cast<const uint4*>(g.a_mag + (kb * g.M + m0 + r) * 8);
+          const uint32_t x[4] = {u.x, u.y, u.z, u.w};
+#pragma unroll
+          for (int q = 0; q < 4; ++q) {
+            const uint32_t lo = x[q] & 0xffffu, hi = x[q] >> 16;
+            c += (lo >= kF64eLarge) + (hi >= kF64eLarge);
+            if (lo > 0x7f80u) c = kF64eNoCount;
+          }
+        }
+      atomicAdd(&large[r], r < mlim ? c : window);
+      __syncthreads();
+      int least = large[r];
+#pragma unroll
+      for (int o = 16; o > 0; o >>= 1) least = min(least, __shfl_xor_sync(0xffffffffu, least, o));
+      if (lane == 0) least_row[warp] = least;
+      __syncthreads();
+    }
+    if (g.ntiles > gridDim.x) {  // every output of the tile sure by the numbers of large entries?
+      int a = least_row[0];
+#pragma unroll
+      for (int q = 1; q < kRM / 32; ++q) a = min(a, least_row[q]);
+      const bool few = tid < nlim && a + g.b_large[n0 + tid] < window + kSureMeets;
+      if (!__syncthreads_or(few)) continue;
+    }
+#pragma unroll
+    for (int p = 0; p < kRStages - 1; ++p) load(m0, n0, p, p);
+    if (tid == 0) count = 0;
+    for_outputs([&](int, int, float& s) { s = 0.f; });
+    if (mlim < kRM || nlim < kRN)  // outputs beyond the edges are sure (or NaN)
+      for_outputs([&](int ml, int nl, float& s) { s = ml < mlim && nl < nlim ? 0.f : 1.f; });
+    bool done = false;
+#pragma unroll 1
+    for (int kc = 0; kc < nk && !done; ++kc) {
+      load(m0, n0, kc + kRStages - 1, (kc + kRStages - 1) % kRStages);  // where chunk kc - 1 was
+      asm volatile("cp.async.wait_group %0;" ::"n"(kRStages - 1) : "memory");
+      __syncthreads();
+      multiply(kc % kRStages);
+      bool sure = true;
+      for_outputs([&](int, int, float& s) { sure = sure && s >= kSureSum; });  // (never for NaN)
+      done = __syncthreads_and(sure);  // and the stage may be written again
+    }
+    asm volatile("cp.async.wait_all;" ::: "memory");
+    __syncthreads();
+    if (done) continue;
+    uint32_t doubtful = 0, bit = 1;
+    for_outputs([&](int ml, int nl, float& s) {
+      if (!(s >= kSureSum) && s != 0.f && ml < mlim && nl < nlim) doubtful |= bit;
+      bit <<= 1;
+    });
+    int at = __popc(doubtful), total = at;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+      const int x = __shfl_up_sync(0xffffffffu, total, o);
+      if (lane >= o) total += x;
+    }
+    at = total - at;  // of the lanes before
+    int first = 0;
+    if (lane == 31 && total > 0) first = atomicAdd(&count, total);
+    at += __shfl_sync(0xffffffffu, first, 31);
+    bit = 1;
+    for_outputs([&](int ml, int nl, float&) {
+      if (doubtful & bit) list[at++] = (uint16_t)(nl * kRM + ml);
+      bit <<= 1;
+    });
+    __syncthreads();
+    const int n = count, nch = (n + kF64eCheckChunk - 1) / kF64eCheckChunk;
+    if (n > 0) {
+      if (tid == 0) slot = atomicAdd(g.count, nch);
+      for (int e = tid; e < n; e += kRThreads) g.lists[(int64_t)t * (kRM * kRN) + e] = list[e];
+      __syncthreads();
+      for (int c = tid; c < nch; c += kRThreads)
+        g.chunks[slot + c] = (unsigned long long)t << 24 | (unsigned long long)(c * kF64eCheckChunk) << 8 |
+                             (unsigned long long)min(kF64eCheckChunk, n - c * kF64eCheckChunk);
+    }
+    __syncthreads();
+  }
+}
+
+constexpr int kRPerWarp = 4;                        // outputs a warp sums at a time
+constexpr int kPThreads = 4 * kF64eCheckChunk;      // four threads for each output of a chunk
+
+// Sum the listed outputs (n_local kRM + m_local) of the tile at (m0, n0) again: kRPerWarp a warp, the k
+// range over its lanes.  Warps work by themselves: the latency of their loads is what this takes.
+template <int Threads>
+__device__ __forceinline__ void repair_outputs(const RepairArgs& g, const uint16_t* list, int count, int64_t m0,
+                                               int64_t n0) {
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  auto offset = [&](int64_t k) { return g.ok ? g.ok[k] : decompose(k, g.kg); };
+#pragma unroll 1
+  for (int base = warp * kRPerWarp; base < count; base += Threads / 32 * kRPerWarp) {
     int64_t om[kRPerWarp];
     const double2* b[kRPerWarp];
     double2 acc[kRPerWarp];
 #pragma unroll
     for (int j = 0; j < kRPerWarp; ++j) {
-      const int e = min(base + warp * kRPerWarp + j, count - 1);  // past the end: the last one again
-      const int64_t m = m0 + list[e] % kRM, n = n0 + list[e] / kRM;
+      const int id = list[min(base + j, count - 1)];  // past the end: the last one again
+      const int64_t m = m0 + id % kRM;
       om[j] = g.om ? g.om[m] : decompose(m, g.mg);
-      b[j] = g.B + n * g.K;
+      b[j] = g.B + (n0 + id / kRM) * g.K;
       acc[j] = make_double2(0.0, 0.0);
     }
+    auto add = [&](double2& s, double2 t, double2 v) {
+      s.x = fma(t.x, v.x, s.x);
+      s.x = fma(-t.y, v.y, s.x);
+      s.y = fma(t.x, v.y, s.y);
+      s.y = fma(t.y, v.x, s.y);
+    };
+    int64_t k = lane;
 #pragma unroll 1
-    for (int64_t kq = 0; kq < g.K; kq += kRK) {
-      const int kv = (int)min((int64_t)kRK, g.K - kq);
-      __syncthreads();
-      for (int c = threadIdx.x; c < kv; c += kRThreads) offK[c] = g.ok ? g.ok[kq + c] : decompose(kq + c, g.kg);
-      __syncthreads();
-      for (int c = lane; c < kv; c += 32) {
-        double2 t[kRPerWarp], v[kRPerWarp];
+    for (; k + 32 < g.K; k += 64) {
+      const int64_t o0 = offset(k), o1 = offset(k + 32);
+      double2 t[2][kRPerWarp], v[2][kRPerWarp];
 #pragma unroll
-        for (int j = 0; j < kRPerWarp; ++j) {
-          t[j] = g.T[om[j] + offK[c]];
-          v[j] = b[j][kq + c];
-        }
+      for (int j = 0; j < kRPerWarp; ++j) {
+        t[0][j] = g.T[om[j] + o0];
+        v[0][j] = b[j][k];
+        t[1][j] = g.T[om[j] + o1];
+        v[1][j] = b[j][k + 32];
+      }
 #pragma unroll
-        for (int j = 0; j < kRPerWarp; ++j) {
-          acc[j].x = fma(t[j].x, v[j].x, acc[j].x);
-          acc[j].x = fma(-t[j].y, v[j].y, acc[j].x);
-          acc[j].y = fma(t[j].x, v[j].y, acc[j].y);
-          acc[j].y = fma(t[j].y, v[j].x, acc[j].y);
-        }
+      for (int j = 0; j < kRPerWarp; ++j) {
+        add(acc[j], t[0][j], v[0][j]);
+        add(acc[j], t[1][j], v[1][j]);
       }
     }
+    if (k < g.K) {
+      const int64_t o = offset(k);
+#pragma unroll
+      for (int j = 0; j < kRPerWarp; ++j) add(acc[j], g.T[om[j] + o], b[j][k]);
+    }
+    __syncwarp();
 #pragma unroll
     for (int j = 0; j < kRPerWarp; ++j) {
 #pragma unroll
@@ -475,16 +700,69 @@ __device__ __forceinline__ void repair_outputs(const RepairArgs& g, const uint16
         acc[j].x += __shfl_xor_sync(0xffffffffu, acc[j].x, o);
         acc[j].y += __shfl_xor_sync(0xffffffffu, acc[j].y, o);
       }
-      const int e = base + warp * kRPerWarp + j;
-      if (lane == 0 && e < count) g.C[(n0 + list[e] / kRM) * g.M + m0 + list[e] % kRM] = acc[j];
+      if (lane == 0 && base + j < count) {
+        const int id = list[base + j];
+        g.C[(n0 + id / kRM) * g.M + m0 + id % kRM] = acc[j];
+      }
     }
   }
 }
 
-__global__ void __launch_bounds__(kRThreads) f64e_repair_kernel(const __grid_constant__ RepairArgs g) {
+// Checked products: the chunks of f64e_check_kernel.  Of a chunk's outputs those whose bound does not
+// hold, four threads each, are summed again.
+__global__ void __launch_bounds__(kPThreads, 4) f64e_repair_kernel(const __grid_constant__ RepairArgs g) {
+  chained_wait();
+  __shared__ uint16_t again[kF64eCheckChunk];
+  __shared__ int count;
+  const int nch = *g.count, l = threadIdx.x & 3, e = threadIdx.x >> 2;
+  const int64_t nkb = (g.K + 7) / 8, tiles_n = g.ntiles / g.tiles_m;
+#pragma unroll 1
+  for (int c = blockIdx.x; c < nch; c += gridDim.x) {
+    const unsigned long long ch = g.chunks[c];
+    const int64_t tile = (int64_t)(ch >> 24);
+    const int n = (int)(ch & 0xff), first = (int)(ch >> 8 & 0xffff);
+    const int64_t m0 = tile / tiles_n * kRM, n0 = tile % tiles_n * kRN;
+    const int id = g.lists[tile * (kRM * kRN) + first + min(e, n - 1)];
+    const uint16_t *a = g.a_mag + (m0 + id % kRM) * 8, *b = g.b_mag + (n0 + id / kRM) * 8;
+    float prod = 0.f, sum = 0.f, met = 0.f;
+#pragma unroll 4
+    for (int64_t kb = l; kb < nkb; kb += 4) {
+      const uint4 u = *reinterpret_cast<const uint4*>(a + kb * g.M * 8);
+      const uint4 v = *reinterpret_cast<const uint4*>(b + kb * g.N * 8);
+      const uint32_t x[4] = {u.x, u.y, u.z, u.w}, y[4] = {v.x, v.y, v.z, v.w};
+#pragma unroll
+      for (int q = 0; q < 8; ++q) {
+        const float al = __uint_as_float(q & 1 ? x[q >> 1] & 0xffff0000u : x[q >> 1] << 16);
+        const float be = __uint_as_float(q & 1 ? y[q >> 1] & 0xffff0000u : y[q >> 1] << 16);
+        const bool both = al != 0.f && be != 0.f;
+        prod = fmaf(al, be, prod);
+        sum += both ? al + be : 0.f;
+        met += both ? 1.f : 0.f;
+      }
+    }
+    __syncwarp();
+#pragma unroll
+    for (int o = 2; o > 0; o >>= 1) {
+      prod += __shfl_xor_sync(0xffffffffu, prod, o);
+      sum += __shfl_xor_sync(0xffffffffu, sum, o);
+      met += __shfl_xor_sync(0xffffffffu, met, o);
+    }
+    __syncthreads();  // the last chunk's list has been used
+    if (threadIdx.x == 0) count = 0;
+    __syncthreads();
+    // E / (2 * 2^-53): 2^-4 and 2^-10.6, with the rounding of the magnitudes and sums (NaN: a row
+    // without digits)
+    const bool holds = prod * (float)g.K >= fmaf(0.064f, sum, 0.00066f * met);
+    if (l == 0 && e < n && !holds) again[atomicAdd(&count, 1)] = (uint16_t)id;
+    __syncthreads();
+    repair_outputs<kPThreads>(g, again, count, m0, n0);
+  }
+}
+
+// Others (FP64E): the outputs of rows without digits, found by the rows' exponents tile by tile.
+__global__ void __launch_bounds__(kRThreads) f64e_rows_kernel(const __grid_constant__ RepairArgs g) {
   chained_wait();
   __shared__ uint16_t list[kRM * kRN];
-  __shared__ int64_t offK[kRK];
   __shared__ uint8_t bad[kRM + kRN];  // rows of A, then of B
   __shared__ int count;
   for (int64_t tile = blockIdx.x; tile < g.ntiles; tile += gridDim.x) {
@@ -503,7 +781,7 @@ __global__ void __launch_bounds__(kRThreads) f64e_repair_kernel(const __grid_con
       if (m0 + ml < g.M && n0 + nl < g.N && (bad[ml] || bad[kRM + nl])) list[atomicAdd(&count, 1)] = (uint16_t)e;
     }
     __syncthreads();
-    repair_outputs(g, list, count, m0, n0, offK);
+    repair_outputs<kRThreads>(g, list, count, m0, n0);
     __syncthreads();
   }
 }
@@ -523,10 +801,11 @@ static double f64e_waves(double M, double N, double K, int sms, bool* share) {
   *share = rest > 0 && chunks > 1 && cut < tile;
   return std::floor(tiles / sms) * tile + (rest > 0 ? std::min(tile, cut) : 0.0);
 }
-// Digit planes: the split and the launches, then the waves of tiles.  FP64 pipe: 1.15 TFLOP/s.
+// Digit planes: the split, the check and the launches, then the waves of tiles.  FP64 pipe: 1.15
+// TFLOP/s.
 double f64e_time(double M, double N, double K) {
   bool share;
-  return 8e-6 + f64e_waves(M, N, K, 152, &share) + M * K * 60 / 4e12;
+  return 12e-6 + f64e_waves(M, N, K, 152, &share) + M * K * 60 / 4e12;
 }
 // CTAs of a product, and whether its last tiles are shared.
 static int64_t f64e_grid(int64_t M, int64_t N, int64_t K, int sm_count, bool* share) {
@@ -585,9 +864,10 @@ cudaError_t launch_f64e_gemm(const F64eGemmArgs& a, int sm_count, int* errflag, 
 }
 
 cudaError_t launch_f64e_repair(const F64eGemmArgs& a, const double2* T, const GatherTab& tab, const GroupSpec& mg,
-                               const GroupSpec& kg, const double2* B, int sm_count, cudaStream_t s) {
+                               const GroupSpec& kg, const double2* B, int sm_count, cudaStream_t s, int* launches) {
+  *launches = 0;
   if (a.M <= 0 || a.N <= 0) return cudaSuccess;
-  RepairArgs g;
+  RepairArgs g = {};
   g.T = T;
   g.om = tab.om;
   g.ok = tab.ok;
@@ -602,6 +882,22 @@ cudaError_t launch_f64e_repair(const F64eGemmArgs& a, const double2* T, const Ga
   g.ntiles = g.tiles_m * ((a.N + kRN - 1) / kRN);
   g.a_exp = a.a_exp;
   g.b_exp = a.b_exp;
-  const int64_t grid = std::min<int64_t>(g.ntiles, 4 * std::max(1, sm_count));
-  return launch_chained(f64e_repair_kernel, dim3((unsigned)grid), dim3(kRThreads), 0, s, g);
+  const int sms = std::max(1, sm_count);
+  if (!a.a_mag) {
+    *launches = 1;
+    return launch_chained(f64e_rows_kernel, dim3((unsigned)std::min<int64_t>(g.ntiles, 4 * sms)), dim3(kRThreads), 0, s, g);
+  }
+  g.a_mag = a.a_mag;
+  g.b_mag = a.b_mag;
+  g.b_large = a.b_large;
+  g.count = a.count;
+  g.lists = static_cast<uint16_t*>(const_cast<void*>(a.A));
+  g.chunks = reinterpret_cast<unsigned long long*>(g.lists + g.ntiles * kRM * kRN);
+  static PerDeviceOnce opt_in;
+  if (const cudaError_t e = smem_opt_in(opt_in, f64e_check_kernel, kRSmem)) return e;
+  *launches = 2;
+  cudaError_t e = launch_chained(f64e_check_kernel, dim3((unsigned)std::min<int64_t>(g.ntiles, 3 * sms)),
+                                 dim3(kRThreads), kRSmem, s, g);
+  if (e == cudaSuccess) e = launch_chained(f64e_repair_kernel, dim3((unsigned)(4 * sms)), dim3(kPThreads), 0, s, g);
+  return e;
 }

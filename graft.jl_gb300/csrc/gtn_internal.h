@@ -7,6 +7,7 @@
 #include <cuda_runtime.h>
 #include <cuda_bf16.h>
 #include <cuda_fp16.h>
+#include <algorithm>
 #include <atomic>
 #include <cstdint>
 #include <cstring>
@@ -413,6 +414,25 @@ __host__ __device__ inline bool f64e_no_digits(float E) {
 inline size_t f64e_a_bytes(int64_t M, int64_t K) {
   return (size_t)((M + kF64eRowsA - 1) / kF64eRowsA) * ((K + 7) / 8) * kF64eSlices * kF64eRowsA * 32;
 }
+// The check of FP64 products: magnitudes of an operand's entries (bf16, [k / 8][row][k % 8]); the
+// lists of doubtful outputs, over tiles of kF64eCheckM x kF64eCheckN, which take the place of A's planes
+// once the product is there; a count before A's magnitudes.
+constexpr int kF64eCheckM = 128, kF64eCheckN = 64, kF64eCheckChunk = 32;
+// Entries among a row's first kF64eWindow that are at least kF64eLarge (bf16 bits of 0.0508): where two
+// rows have L of W entries more than W together, L of them meet.  A row without digits counts as
+// far below none.
+constexpr int kF64eWindow = 128, kF64eNoCount = -(1 << 20);
+constexpr uint32_t kF64eLarge = 0x3d50;
+inline size_t f64e_mag_bytes(int64_t rows, int64_t K) { return ((size_t)rows * ((K + 7) / 8) * 16 + 255) / 256 * 256; }
+inline size_t f64e_check_offset(int64_t M, int64_t N, int64_t K, size_t a_bytes) {
+  const size_t tiles = (size_t)((M + kF64eCheckM - 1) / kF64eCheckM) * ((N + kF64eCheckN - 1) / kF64eCheckN);
+  const size_t outputs = (size_t)kF64eCheckM * kF64eCheckN;
+  const size_t lists = tiles * (outputs * 2 + outputs / kF64eCheckChunk * 8);
+  return (std::max(lists, a_bytes) + 255) / 256 * 256;
+}
+inline size_t f64e_check_bytes(int64_t M, int64_t N, int64_t K, size_t a_bytes) {
+  return f64e_check_offset(M, N, K, a_bytes) + 256 + f64e_mag_bytes(M, K);
+}
 inline size_t f64e_b_bytes(int64_t N, int64_t K) {
   return (size_t)((2 * N + kF64eRowsB - 1) / kF64eRowsB) * ((K + 7) / 8) * kF64eSlices * kF64eRowsB * 32;
 }
@@ -427,6 +447,10 @@ struct F64eGemmArgs {
   int64_t M = 0, N = 0, K = 0;
   const float* a_exp = nullptr;
   const float* b_exp = nullptr;
+  const uint16_t* a_mag = nullptr;  // magnitudes: the outputs are checked; null: they are not
+  const uint16_t* b_mag = nullptr;
+  const int* b_large = nullptr;     // large entries of B's rows
+  int* count = nullptr;             // of the check, zeroed by the split; its lists take A's place
   int levels = 8;               // digit products d_i e_j with i + j < levels (7 or 8)
   void* part = nullptr;         // f64e_part_bytes of the product, or null: no tile is shared
 };
@@ -434,16 +458,19 @@ cudaError_t launch_f64e_gemm(const F64eGemmArgs& a, int sm_count, int* errflag, 
                              int* launches);
 // Bytes of partial sums of the tiles that CTAs share in a product (0: none are).
 size_t f64e_part_bytes(int64_t M, int64_t N, int64_t K, int sm_count);
-// The outputs of rows without digits (of A or of B), each summed again on the FP64 pipe from the
-// operands: T read in place (offsets from the tables, or the groups where tab has none), B [N][K].
+// The outputs of rows without digits (of A or of B), and with magnitudes those whose digit products
+// may miss the bound 2 K 2^-53 sum_k |a_k| |b_k| of an FP64 sum, each summed again on the FP64 pipe from
+// the operands: T read in place (offsets from the tables, or the groups where tab has none), B [N][K].
 cudaError_t launch_f64e_repair(const F64eGemmArgs& a, const double2* T, const GatherTab& tab, const GroupSpec& mg,
-                               const GroupSpec& kg, const double2* B, int sm_count, cudaStream_t s);
+                               const GroupSpec& kg, const double2* B, int sm_count, cudaStream_t s, int* launches);
 // Digit planes and row exponents of the running tensor's K-major view (c128) and of a static B [N][K].
 cudaError_t launch_split_digits_tab(const double2* T, const GatherTab& t, int64_t M, int64_t K, float* rexp, void* out,
-                                    cudaStream_t s, int* launches);
+                                    uint16_t* mag, int* count, cudaStream_t s, int* launches);
 cudaError_t launch_split_digits_grp(const double2* T, const GroupSpec& mg, const GroupSpec& kg, int64_t M, int64_t K,
-                                    float* rexp, void* out, cudaStream_t s, int* launches);
-cudaError_t launch_pack_b_digits(const double2* B, int64_t N, int64_t K, void* out, float* bexp, cudaStream_t s);
+                                    float* rexp, void* out, uint16_t* mag, int* count, cudaStream_t s,
+                                    int* launches);
+cudaError_t launch_pack_b_digits(const double2* B, int64_t N, int64_t K, void* out, float* bexp, uint16_t* mag,
+                                 int* large, cudaStream_t s);
 // C[n][m] = sum_k T[offM(m) + offK(k)] B[n][k] on the FP64 pipe, T read in place.  With slices > 1
 // (of zgemm_view_slices: few outputs, long K) the k range is cut into that many partial products
 // P[slice][n][m], summed in order.
@@ -526,6 +553,8 @@ struct PlanStep {
   bool dg = false;
   void* bdig = nullptr;
   float* bexp = nullptr;
+  uint16_t* bmag = nullptr;  // magnitudes of the static and the large ones' number (FP64 applications)
+  int* blarge = nullptr;
   double macs = 0;
 };
 

@@ -388,7 +388,7 @@ struct Split16Writer {
 struct Split16RowWriter {
   using Mag = AbsMag;
   static constexpr int kCols = 2;
-  __device__ void row(float) const {}
+  __device__ void row(int64_t) const {}
   __half* out;
   int64_t ld2;
   int64_t pstride;
@@ -440,6 +440,14 @@ __device__ __forceinline__ uint32_t digit_pair(unsigned long long a, unsigned lo
   }
   return __byte_perm(__float_as_uint(fa), __float_as_uint(fb), 0x7632);  // the bf16 halves: exact
 }
+// max(|re|, |im|) of a value under row exponent E (in [1/4, 1/2) for the row's largest) as bf16 bits,
+// rounded down and at least 2^-60 unless it is zero; NaN throughout a row without digits.
+__device__ __forceinline__ uint32_t digit_mag(double2 v, float E) {
+  const uint32_t hx = __double2hiint(v.x) & 0x7fffffff, hy = __double2hiint(v.y) & 0x7fffffff;
+  if (f64e_no_digits(E)) return 0x7fc0u;
+  if ((hx | hy | __double2loint(v.x) | __double2loint(v.y)) == 0u) return 0u;
+  return (uint32_t)max((int)(max(hx, hy) >> 13) - (((int)E - 125) << 7), (127 - 60) << 7);
+}
 // Byte offset, within the digit planes of an operand with `rows` rows per tile, of plane 0 of
 // the 16-byte chunk `chunk` (8 real k) of row r: blocks [row tile][16 k][plane][rows][32 bytes],
 // each (row tile, 16 k) block contiguous so that one bulk copy loads a pipeline stage; the
@@ -450,10 +458,19 @@ __device__ __forceinline__ int64_t digit_chunk(int64_t r, int64_t chunk, int row
   return ((rt * nkb + (chunk >> 1)) * kF64eSlices * rows + rr) * 32 + (((int)chunk ^ (rr >> 2)) & 1) * 16;
 }
 
-// Element (m, k) of the A operand: its digits in the planes (4 bytes each).
+// Element (m, k) of the A operand: its digits in the planes (4 bytes each) and, where the product is
+// checked, its magnitude in mag[k / 8][m][k % 8] (rows of one k block behind each other: whole
+// sectors for the threads of a split, and for the check's loads).  The count of the check's chunks
+// starts at zero.
+struct DigitCheck {
+  uint16_t* mag;  // null: not checked
+  int* count;
+  int64_t rows;
+};
 struct DigitWriter {
   static constexpr bool kPair = false;
   unsigned char* out;
+  DigitCheck chk;
   int64_t nkb;
   const float* rexp;
   __device__ void operator()(int64_t m, int64_t k, double2 v) const {
@@ -462,16 +479,23 @@ struct DigitWriter {
     unsigned char* p = out + digit_chunk(m, k >> 2, kF64eRowsA, nkb) + (k & 3) * 4;
 #pragma unroll
     for (int i = 0; i < kF64eSlices; ++i) *reinterpret_cast<uint32_t*>(p + i * kF64eRowsA * 32) = digit_pair(a, b, i);
+    if (chk.mag) {
+      chk.mag[((k >> 3) * chk.rows + m) * 8 + (k & 7)] = (uint16_t)digit_mag(v, E);
+      if (m == 0 && k == 0) *chk.count = 0;
+    }
   }
 };
 // The same for four adjacent columns (k a multiple of 4), the row exponent in hand: one
 // 16-byte store per plane.
 struct DigitRowWriter {
   unsigned char* out;
+  DigitCheck chk;
   int64_t nkb;
   using Mag = ExpMag;
   static constexpr int kCols = 4;
-  __device__ void row(float) const {}
+  __device__ void row(int64_t m) const {
+    if (m == 0 && chk.mag) *chk.count = 0;
+  }
   __device__ void operator()(int64_t m, int64_t k, const double2* v, float E) const {
     unsigned long long w[8];
 #pragma unroll
@@ -485,17 +509,22 @@ struct DigitRowWriter {
       *reinterpret_cast<uint4*>(p + i * kF64eRowsA * 32) =
           make_uint4(digit_pair(w[0], w[1], i), digit_pair(w[2], w[3], i), digit_pair(w[4], w[5], i),
                      digit_pair(w[6], w[7], i));
+    if (chk.mag)
+      *reinterpret_cast<uint2*>(chk.mag + ((k >> 3) * chk.rows + m) * 8 + (k & 7)) =
+          make_uint2(digit_mag(v[0], E) | digit_mag(v[1], E) << 16, digit_mag(v[2], E) | digit_mag(v[3], E) << 16);
   }
 };
 
 // B' = [[Br, -Bi], [Bi, Br]] of a static B [N][K]: CTA b takes the complex rows 8b .. 8b + 7,
 // one warp per row for the exponents, then every thread the digits of 4 columns of a row for
-// both real rows (the digits of -Bi are the negated digits of Bi).
+// both real rows (the digits of -Bi are the negated digits of Bi) and, given mag, their magnitudes.
 __global__ void __launch_bounds__(256) pack_b_digits_kernel(const double2* __restrict__ B, int64_t N, int64_t K,
                                                             int64_t nkb, float* __restrict__ bexp,
-                                                            unsigned char* __restrict__ out) {
+                                                            unsigned char* __restrict__ out,
+                                                            uint16_t* __restrict__ mag, int* __restrict__ large) {
   chained_wait();
   __shared__ float se[8];
+  __shared__ int nlarge[8];
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int64_t n0 = (int64_t)blockIdx.x * 8;
   {
@@ -507,6 +536,7 @@ __global__ void __launch_bounds__(256) pack_b_digits_kernel(const double2* __res
     for (int o = 16; o > 0; o >>= 1) x = fmaxf(x, __shfl_xor_sync(0xffffffffu, x, o));
     if (lane == 0) {
       se[warp] = x;
+      nlarge[warp] = f64e_no_digits(x) ? kF64eNoCount : 0;
       if (n < N) bexp[n] = x;
     }
   }
@@ -519,11 +549,18 @@ __global__ void __launch_bounds__(256) pack_b_digits_kernel(const double2* __res
     const int64_t chunk = (e >> 4) * 2 + (e & 1), k = chunk * 4, n = n0 + r;
     const int E = (int)se[r];
     unsigned long long w[8];
+    uint32_t g[4];
 #pragma unroll
     for (int j = 0; j < 4; ++j) {
       const double2 v = k + j < K ? B[n * K + k + j] : make_double2(0.0, 0.0);
       w[2 * j] = digit_word(v.x, E);
       w[2 * j + 1] = digit_word(v.y, E);
+      g[j] = digit_mag(v, se[r]);
+    }
+    if (mag) {
+      *reinterpret_cast<uint2*>(mag + ((k >> 3) * N + n) * 8 + (k & 7)) = make_uint2(g[0] | g[1] << 16, g[2] | g[3] << 16);
+      if (k < kF64eWindow)
+        atomicAdd(&nlarge[r], (g[0] >= kF64eLarge) + (g[1] >= kF64eLarge) + (g[2] >= kF64eLarge) + (g[3] >= kF64eLarge));
     }
     // (the two real rows share a swizzle group: 2n and 2n + 1 differ in bit 0 only)
     unsigned char* p = out + digit_chunk(2 * n, chunk, kF64eRowsB, nkb);
@@ -541,6 +578,9 @@ __global__ void __launch_bounds__(256) pack_b_digits_kernel(const double2* __res
       *reinterpret_cast<uint4*>(o + 32) = make_uint4(t[0], t[1], t[2], t[3]);
     }
   }
+  if (!mag) return;
+  __syncthreads();
+  if (threadIdx.x < nr) large[n0 + threadIdx.x] = nlarge[threadIdx.x];
 }
 
 // amax[m] = max over k of max(|re|, |im|) of the K-major gather (atomic max of the
@@ -1445,7 +1485,7 @@ __global__ void __launch_bounds__(256) split_rows_kernel(const Tin* __restrict__
   }
   if (rank == 0 && tid < TR && m0 + tid < M) {
     amax[m0 + tid] = rmax[tid];
-    w.row(rmax[tid]);
+    w.row(m0 + tid);
   }
   const int nrows = (int)min((int64_t)TR, M - m0);
   if constexpr (W::kCols == 4) {
@@ -1968,38 +2008,41 @@ cudaError_t launch_split16_rows_grp(const void* T, int is64, const GroupSpec& mg
 // split, or row exponents first and then the planes when a row is too long for it.
 template <class Off>
 static cudaError_t split_digits(const double2* T, const Off& off, int m_fast, const GroupSpec* mg, const GroupSpec* kg,
-                                int64_t M, int64_t K, float* rexp, unsigned char* out, cudaStream_t s,
-                                int* launches) {
+                                int64_t M, int64_t K, float* rexp, unsigned char* out, uint16_t* mag,
+                                int* count, cudaStream_t s, int* launches) {
   const int64_t Kp = (K + 7) / 8 * 8, nkb = Kp / 8;
+  const DigitCheck chk{mag, count, M};
   bool done = false;
-  cudaError_t e = launch_split_rows(T, off, M, K, Kp, m_fast, DigitRowWriter{out, nkb}, rexp, s, &done);
+  cudaError_t e = launch_split_rows(T, off, M, K, Kp, m_fast, DigitRowWriter{out, chk, nkb}, rexp, s, &done);
   *launches = 1;
   if (e != cudaSuccess || done) return e;
   *launches = 2;
   e = launch_rowmax<ExpMag>(T, off, m_fast, M, K, rexp, s);
   if (e != cudaSuccess) return e;
-  const DigitWriter w{out, nkb, rexp};
+  const DigitWriter w{out, chk, nkb, rexp};
   if constexpr (std::is_same<Off, TabOff>::value)
     return launch_gather_tab(T, off.om, off.ok, M, K, Kp, m_fast, w, s);
   else
     return launch_gather(T, *mg, *kg, M, K, Kp, w, s);
 }
 cudaError_t launch_split_digits_tab(const double2* T, const GatherTab& t, int64_t M, int64_t K, float* rexp, void* out,
-                                    cudaStream_t s, int* launches) {
+                                    uint16_t* mag, int* count, cudaStream_t s, int* launches) {
   return split_digits(T, TabOff{t.om, t.ok}, t.m_fast, nullptr, nullptr, M, K, rexp, static_cast<unsigned char*>(out),
-                      s, launches);
+                      mag, count, s, launches);
 }
 cudaError_t launch_split_digits_grp(const double2* T, const GroupSpec& mg, const GroupSpec& kg, int64_t M, int64_t K,
-                                    float* rexp, void* out, cudaStream_t s, int* launches) {
+                                    float* rexp, void* out, uint16_t* mag, int* count, cudaStream_t s,
+                                    int* launches) {
   return split_digits(T, GrpOffV{mg, kg}, choose_m_fast(mg, kg) ? 1 : 0, &mg, &kg, M, K, rexp,
-                      static_cast<unsigned char*>(out), s, launches);
+                      static_cast<unsigned char*>(out), mag, count, s, launches);
 }
 cudaError_t launch_pack_b_digits(const double2* B, int64_t N, int64_t K, void* out, float* bexp,
-                                 cudaStream_t s) {
+                                 uint16_t* mag, int* large, cudaStream_t s) {
   if (N <= 0) return cudaSuccess;
   const int64_t blocks = (N + 7) / 8;
   if (blocks > 2147483647LL) return cudaErrorInvalidConfiguration;
-  launch_chained(pack_b_digits_kernel, dim3((unsigned)blocks), dim3(256), 0, s, B, N, K, (K + 7) / 8, bexp, static_cast<unsigned char*>(out));
+  launch_chained(pack_b_digits_kernel, dim3((unsigned)blocks), dim3(256), 0, s, B, N, K, (K + 7) / 8, bexp, static_cast<unsigned char*>(out),
+                 mag, large);
   return cudaGetLastError();
 }
 cudaError_t launch_gather_tab_to_c128(const void* T, int is64, const GatherTab& t, int64_t M, int64_t K, int64_t ldo,

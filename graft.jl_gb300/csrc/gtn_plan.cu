@@ -136,7 +136,8 @@ int fill_offset_tables(gtn_map map) {
 
 // Digit planes of the statics of the plan's digit-plane steps.  They are optional in an FP64
 // plan (a step without them stays on the FP64 pipe) and needed in an FP64E one.
-int pack_digits(gtn_map map, bool required) {
+// mags: with the magnitudes that FP64 applications check their products by.
+int pack_digits(gtn_map map, bool required, bool mags) {
   gtn_ctx ctx = map->ctx;
   // partial sums of the map's own: applications of two maps, captured or on two threads, may overlap
   size_t part = 0;
@@ -153,12 +154,14 @@ int pack_digits(gtn_map map, bool required) {
     void* planes = nullptr;
     cudaError_t a = dalloc(map, &planes, f64e_b_bytes(st.N, st.K));
     if (a == cudaSuccess) a = dalloc(map, &st.bexp, (size_t)st.N * sizeof(float));
+    if (a == cudaSuccess && mags) a = dalloc(map, &st.bmag, f64e_mag_bytes(st.N, st.K));
+    if (a == cudaSuccess && mags) a = dalloc(map, &st.blarge, (size_t)st.N * sizeof(int));
     if (a != cudaSuccess) {
       if (required) return set_err(ctx, GTN_ERR_MEMORY, "static packing allocation failed");
       cudaGetLastError();
       continue;
     }
-    e = launch_pack_b_digits(st.b64, st.N, st.K, planes, st.bexp, ctx->stream);
+    e = launch_pack_b_digits(st.b64, st.N, st.K, planes, st.bexp, st.bmag, st.blarge, ctx->stream);
     ctx->launches++;
     st.bdig = planes;
   }
@@ -195,7 +198,8 @@ constexpr int64_t kMaxCombined = int64_t(1) << 22;  // elements of a pre-contrac
 // only those do that may be a TTNO tensor (up to 512 entries) and keep the FP64 pipes busy for 6 us
 // if dense: an environment has no zeros to skip, and few rows, a thread each in passes of 16
 // outputs, leave the pipes waiting.  The others run in place on the FP64 pipes, not on digit planes:
-// those are accurate to a row's largest entry, which a short sparse sum can be far below.  One-site
+// those are accurate to a row's largest entry, which a short sparse sum can be far below, and many of
+// its outputs would be summed again.  One-site
 // map of the 31-site binary tree, small-K kernel against in place: bond 12 392 -> 43 us, 16 680 -> 92,
 // 24 1493 -> 261; two-site map of a star at bond 2 198 -> 9.6.
 bool narrow(double K, double N) {
@@ -398,6 +402,8 @@ int plan_build(gtn_ctx ctx, int n, const int* ranks, const int64_t* dims, const 
   // FP64 plans that own a workspace run their long products on the tensor cores too
   const bool dg64 = precision == GTN_PREC_FP64 && alloc_ws && statics && tc_gemm_supported(ctx->cc_major, ctx->cc_minor);
 
+  const bool mags = !(f64e && map->oneshot);  // (a one-shot FP64E contraction is never applied in FP64)
+
   // ---- the reference's env-first chain and the grouped chain we execute ------------------
   ChainOp X{L[0], D[0]};
   std::vector<ChainOp> base;
@@ -546,7 +552,10 @@ int plan_build(gtn_ctx ctx, int n, const int* ranks, const int64_t* dims, const 
       map->max_a = std::max(map->max_a, st.M * st.K);
       if (st.tc) map->max_apl = std::max(map->max_apl, (int64_t)P * st.M * 2 * st.Kp);
       if (st.tc || st.dg) map->max_mtc = std::max(map->max_mtc, st.M);
-      if (st.dg) map->max_adg = std::max(map->max_adg, f64e_a_bytes(st.M, st.K));
+      if (st.dg) {
+        const size_t planes = f64e_a_bytes(st.M, st.K);
+        map->max_adg = std::max(map->max_adg, mags ? f64e_check_bytes(st.M, st.N, st.K, planes) : planes);
+      }
       st.splitk = gemm_splitk_slices(st.M, st.N, st.K);
       st.vslices = zgemm_view_slices(st.M, st.N, st.K);
       const int sk = std::max(st.splitk, st.vslices);
@@ -688,7 +697,7 @@ int plan_build(gtn_ctx ctx, int n, const int* ranks, const int64_t* dims, const 
                         cudaSuccess)
     return set_err(ctx, GTN_ERR_MEMORY, "map workspace allocation failed");
   if (statics && map->max_adg > 0) {
-    const int st = pack_digits(map, f64e);
+    const int st = pack_digits(map, f64e, mags);
     if (st != GTN_OK) return st;
   }
   if (map->fp64_alt) {
@@ -798,11 +807,19 @@ int map_run(gtn_map map, int precision, const double2* x, double2* y) {
         a.a_exp = map->amax;
         a.b_exp = st.bexp;
         a.levels = f64e ? 7 : 8;
+        uint16_t* mag = nullptr;
+        if (!f64e) {  // FP64: count and magnitudes of the check behind the planes
+          char* chk = static_cast<char*>(map->abuf) + f64e_check_offset(st.M, st.N, st.K, f64e_a_bytes(st.M, st.K));
+          a.count = reinterpret_cast<int*>(chk);
+          a.a_mag = mag = reinterpret_cast<uint16_t*>(chk + 256);
+          a.b_mag = st.bmag;
+          a.b_large = st.blarge;
+        }
         a.part = map->part;
         int nl = 0;
         prof_begin(s);
-        if (st.tab.om) e = launch_split_digits_tab(T, st.tab, st.M, st.K, map->amax, map->abuf, s, &nl);
-        else e = launch_split_digits_grp(T, st.mg, st.kg, st.M, st.K, map->amax, map->abuf, s, &nl);
+        if (st.tab.om) e = launch_split_digits_tab(T, st.tab, st.M, st.K, map->amax, map->abuf, mag, a.count, s, &nl);
+        else e = launch_split_digits_grp(T, st.mg, st.kg, st.M, st.K, map->amax, map->abuf, mag, a.count, s, &nl);
         prof_end(s, GTN_KERNEL_SPLIT, 0.0);
         ctx->launches += nl;
         if (e == cudaSuccess) {
@@ -812,9 +829,10 @@ int map_run(gtn_map map, int precision, const double2* x, double2* y) {
           prof_end(s, GTN_KERNEL_TC_GEMM, 8.0 * st.macs);
           if (e != cudaSuccess) return set_err(ctx, GTN_ERR_CUDA, "f64e_gemm: " + why + " " + cudaGetErrorString(e));
           prof_begin(s);
-          e = launch_f64e_repair(a, T, st.tab, st.mg, st.kg, st.b64, ctx->sm_count, s);
+          int nr = 0;
+          e = launch_f64e_repair(a, T, st.tab, st.mg, st.kg, st.b64, ctx->sm_count, s, &nr);
           prof_end(s, GTN_KERNEL_ZGEMM, 0.0);
-          ctx->launches += nl + 1;
+          ctx->launches += nl + nr;
         }
       } else {
         const int slices = map->skbuf ? st.vslices : 1;

@@ -40,8 +40,11 @@ typedef enum {
 /* Arithmetic of a map application.  The Krylov vectors and all orthogonalisation are
  * FP64 in every mode; the mode selects how the contraction chain is computed. */
 typedef enum {
-  GTN_PREC_FP64 = 0,       /* complex FP64 throughout: FP64 pipes, or exact sums of the 34 digit
-                              products of level <= 7 (base 256) where K > 64 and they are faster */
+  GTN_PREC_FP64 = 0,       /* complex FP64: each part of a sum of K products is within
+                              2 K 2^-53 sum |a||b| of the exact one, the bound of FP64 multiply-adds.
+                              Long sums run as exact sums of the 34 digit products of level <= 7 (base
+                              256) where that is faster than the FP64 pipes; the outputs that the
+                              digits may give less accurately are summed on the FP64 pipes */
   GTN_PREC_BF16X6 = 1,     /* tcgen05: 3 bf16 slices per operand, 6 products, FP32 accum */
   GTN_PREC_BF16X3 = 2,     /* tcgen05: 2 bf16 slices per operand, 3 products, FP32 accum */
   GTN_PREC_FP32 = 3,       /* complex FP32 SIMT kernels (diagnostic mode) */
@@ -50,8 +53,9 @@ typedef enum {
   GTN_PREC_FP64E = 5       /* FP64-grade on the tensor cores: 7 integer base-256 digits per
                               operand (power-of-two row scales), the 28 digit products of
                               level <= 6 summed exactly (FP32 over 128 or 256 k, then 64-bit
-                              integers); about 4e-16 in the 2-norm (dense maps and
-                              one-shot contractions) */
+                              integers); about 4e-16 in the 2-norm: accurate to the rows'
+                              largest entries, not to each output's own terms (dense maps
+                              and one-shot contractions) */
 } gtn_precision;
 
 typedef struct gtn_ctx_s* gtn_ctx;
