@@ -227,13 +227,19 @@ __device__ __forceinline__ void gather_tab_tile(const Tin* __restrict__ T, const
     }
   }
 }
+// A grid of gx row tiles and gy k tiles; more k tiles than grid.y holds go on in grid.z (the last
+// layer's tiles beyond gy have no elements).
+inline dim3 k_grid(int64_t gx, int64_t gy) {
+  return dim3((unsigned)gx, (unsigned)std::min<int64_t>(gy, 65535), (unsigned)((gy + 65534) / 65535));
+}
+__device__ __forceinline__ int64_t k_tile() { return (int64_t)blockIdx.z * 65535 + blockIdx.y; }
+
 template <typename Tin, class Writer, int TM, int TK>
 __global__ void __launch_bounds__(256) gather_tab_kernel(const Tin* __restrict__ T, TabOff off, int64_t M,
                                                          int64_t K, int64_t Kw, int m_fast, Writer w) {
   chained_wait();
   __shared__ SmemTab<Tin, TM, TK> sm;
-  gather_tab_tile<Tin, Writer, TM, TK>(T, off, M, K, Kw, m_fast, w, (int64_t)blockIdx.x * TM,
-                                       (int64_t)blockIdx.y * TK, sm);
+  gather_tab_tile<Tin, Writer, TM, TK>(T, off, M, K, Kw, m_fast, w, (int64_t)blockIdx.x * TM, k_tile() * TK, sm);
 }
 
 // Gathers and splits of up to 2^24 elements (60 us) are chained launches.  Longer ones gain nothing
@@ -247,12 +253,12 @@ cudaError_t launch_gather_tab(const Tin* T, const int64_t* om, const int64_t* ok
   if (M <= 0 || Kw <= 0) return cudaSuccess;
   if (m_fast) {
     const int64_t gy = (Kw + 15) / 16, gx = (M + 127) / 128;
-    if (gy > 65535 || gx > 2147483647LL) return cudaErrorInvalidConfiguration;
-    launch_chained_if(chain_gather(M, Kw), gather_tab_kernel<Tin, Writer, 128, 16>, dim3((unsigned)gx, (unsigned)gy), dim3(32, 8), 0, s, T, TabOff{om, ok}, M, K, Kw, m_fast, w);
+    if (gx > 2147483647LL) return cudaErrorInvalidConfiguration;
+    launch_chained_if(chain_gather(M, Kw), gather_tab_kernel<Tin, Writer, 128, 16>, k_grid(gx, gy), dim3(32, 8), 0, s, T, TabOff{om, ok}, M, K, Kw, m_fast, w);
   } else {
     const int64_t gy = (Kw + 31) / 32, gx = (M + 63) / 64;
-    if (gy > 65535 || gx > 2147483647LL) return cudaErrorInvalidConfiguration;
-    launch_chained_if(chain_gather(M, Kw), gather_tab_kernel<Tin, Writer, 64, 32>, dim3((unsigned)gx, (unsigned)gy), dim3(32, 8), 0, s, T, TabOff{om, ok}, M, K, Kw, m_fast, w);
+    if (gx > 2147483647LL) return cudaErrorInvalidConfiguration;
+    launch_chained_if(chain_gather(M, Kw), gather_tab_kernel<Tin, Writer, 64, 32>, k_grid(gx, gy), dim3(32, 8), 0, s, T, TabOff{om, ok}, M, K, Kw, m_fast, w);
   }
   return cudaGetLastError();
 }
@@ -633,7 +639,7 @@ __device__ __forceinline__ void rowmax_tile(const Tin* __restrict__ T, const Off
 template <typename Tin, class Off, int TM, int TK, class Mag>
 __global__ void __launch_bounds__(256) rowmax_kernel(const Tin* __restrict__ T, Off off, int64_t M, int64_t K,
                                                      int m_fast, float* __restrict__ amax) {
-  rowmax_tile<Tin, Off, TM, TK, Mag>(T, off, M, K, m_fast, amax, (int64_t)blockIdx.x * TM, (int64_t)blockIdx.y * TK);
+  rowmax_tile<Tin, Off, TM, TK, Mag>(T, off, M, K, m_fast, amax, (int64_t)blockIdx.x * TM, k_tile() * TK);
 }
 
 // bmax[n] = max over k of max(|re|, |im|) of B[n][:], one CTA per row
@@ -1946,14 +1952,12 @@ static cudaError_t launch_rowmax(const Tin* T, const Off& off, int m_fast, int64
   if (e != cudaSuccess || K <= 0) return e;
   if (m_fast) {
     const int64_t gx = (M + 255) / 256, gy = (K + 7) / 8;
-    if (gy > 65535 || gx > 2147483647LL) return cudaErrorInvalidConfiguration;
-    rowmax_kernel<Tin, Off, 256, 8, Mag><<<dim3((unsigned)gx, (unsigned)gy), dim3(32, 8), 0, s>>>(T, off, M, K,
-                                                                                                m_fast, amax);
+    if (gx > 2147483647LL) return cudaErrorInvalidConfiguration;
+    rowmax_kernel<Tin, Off, 256, 8, Mag><<<k_grid(gx, gy), dim3(32, 8), 0, s>>>(T, off, M, K, m_fast, amax);
   } else {
     const int64_t gx = (M + 63) / 64, gy = (K + 31) / 32;
-    if (gy > 65535 || gx > 2147483647LL) return cudaErrorInvalidConfiguration;
-    rowmax_kernel<Tin, Off, 64, 32, Mag><<<dim3((unsigned)gx, (unsigned)gy), dim3(32, 8), 0, s>>>(T, off, M, K,
-                                                                                                m_fast, amax);
+    if (gx > 2147483647LL) return cudaErrorInvalidConfiguration;
+    rowmax_kernel<Tin, Off, 64, 32, Mag><<<k_grid(gx, gy), dim3(32, 8), 0, s>>>(T, off, M, K, m_fast, amax);
   }
   return cudaGetLastError();
 }

@@ -63,3 +63,27 @@ def test_subnormal_rows_are_multiplied(ctx, prec):
     assert np.all(np.abs(got - ref) <= 4 * K * 2.0 ** -52 * (np.abs(A) @ np.abs(B)))
     got = contract(ctx, np.ascontiguousarray(B.T), np.ascontiguousarray(A.T), prec)
     assert np.all(np.abs(got - ref.T) <= 4 * K * 2.0 ** -52 * (np.abs(A) @ np.abs(B)).T)
+
+
+@pytest.mark.parametrize("K", [524281, 600001, 2097120])
+def test_very_long_sums(ctx, K):
+    """Products of more than 2^19 terms, the summed index slow and fast in memory."""
+    rng = np.random.default_rng(1)
+    A, B = crandn(rng, (K, 40)), crandn(rng, (K, 33))
+    ref = A.T @ B
+    tol = 4 * K * 2.0 ** -52 * (np.abs(A).T @ np.abs(B))
+    for la, a in (([1, -1], A), ([-1, 1], A.T)):
+        got = ctx.download(ctx.contract([ctx.upload(a), ctx.upload(B)], [la, [1, -2]], None, None,
+                                        _lib.PRECISIONS["fp64"]))
+        assert np.all(np.abs(got - ref) <= tol)
+
+
+def test_very_long_sums_of_a_map(ctx):
+    """The same with offset tables, beyond 2^20 terms."""
+    K = 1048600
+    rng = np.random.default_rng(2)
+    A, B = crandn(rng, (K, 40)), crandn(rng, (K, 33))
+    m = EffectiveMap(ctx, A.shape, [[1, -1], [1, -2]], [0, 1], [ctx.upload(B)], "fp64")
+    got = ctx.download(m(ctx.upload(A)))
+    m.close()
+    assert np.all(np.abs(got - A.T @ B) <= 4 * K * 2.0 ** -52 * (np.abs(A).T @ np.abs(B)))
