@@ -458,8 +458,8 @@ int gtn_contract(gtn_ctx ctx, int n_operands, const int* ranks, const int64_t* d
 // The label graph is rewritten: ybar takes the output legs (new positive labels), the legs
 // op_slot shared become output legs -1..-r in op_slot's leg order, every other operand's
 // conj flag flips.  Without an order the chain starts at ybar and is the cheapest one of all
-// (VjpNetwork); a network too large for the search, or a chain refused for its memory, takes the
-// greedy chain.
+// (VjpNetwork); a network too large for the search, or a chain refused for its memory or its leg
+// groups, takes the greedy chain.
 int gtn_contract_vjp(gtn_ctx ctx, int n_operands, const int* ranks, const int64_t* dims, const int* labels,
                      const int* conj, const int* order, const void* const* operands, int slot, const void* ybar,
                      void* out, int precision) {
@@ -530,7 +530,8 @@ int gtn_contract_vjp(gtn_ctx ctx, int n_operands, const int* ranks, const int64_
     const std::vector<int> ord = net.cheapest_chain(precision);
     const int st = gtn_contract(ctx, nn, nr.data(), nd.data(), nl.data(), nc.data(), ord.data(), np.data(), out,
                                 precision);
-    if (st != GTN_ERR_MEMORY) return st;  // else: the greedy chain, whose tensors may be smaller
+    // a chain refused for the memory of its tensors or for their leg groups: the greedy one may pass
+    if (st != GTN_ERR_MEMORY && st != GTN_ERR_UNSUPPORTED) return st;
     cudaGetLastError();
   }
   const std::vector<int> ord = net.greedy_chain();
