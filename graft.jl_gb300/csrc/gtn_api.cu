@@ -1,5 +1,6 @@
 // C ABI entry points: contexts, maps, one-shot contractions, permutations and vector helpers.
 #include "gtn_internal.h"
+#include "gtn_vjp_chain.h"
 
 #include <algorithm>
 #include <cstdlib>
@@ -111,107 +112,6 @@ int map_busy_error(gtn_map_s* map) {
   return set_err(map->ctx, GTN_ERR_INVALID,
                  "map is in use by another call: a map is not reentrant (one map per host thread)");
 }
-
-namespace {
-// The rewritten network of an adjoint (operand 0 = the cotangent) and its chains from operand 0.
-constexpr int kVjpSearchMax = 13;  // operands up to which every left-deep chain is compared
-struct VjpNetwork {
-  struct Leg {
-    int label;
-    int64_t dim;
-  };
-  std::vector<std::vector<Leg>> op;
-  VjpNetwork(int n, const std::vector<int>& ranks, const std::vector<int64_t>& dims, const std::vector<int>& labels)
-      : op(n) {
-    size_t o = 0;
-    for (int i = 0; i < n; ++i)
-      for (int r = 0; r < ranks[i]; ++r, ++o) op[i].push_back(Leg{labels[o], dims[o]});
-  }
-  // Absorb operand q into a tensor with the legs cur: the step's (M, K, N) and the new legs.
-  static bool absorb(const std::vector<Leg>& cur, const std::vector<Leg>& q, double* M, double* K, double* N,
-                     std::vector<Leg>* next) {
-    *M = *K = *N = 1;
-    bool shared = false;
-    next->clear();
-    auto has = [](const std::vector<Leg>& legs, int l) {
-      return l > 0 && std::any_of(legs.begin(), legs.end(), [l](const Leg& x) { return x.label == l; });
-    };
-    for (const Leg& l : cur) {
-      if (has(q, l.label)) { *K *= (double)l.dim; shared = true; }
-      else { *M *= (double)l.dim; next->push_back(l); }
-    }
-    for (const Leg& l : q)
-      if (!has(cur, l.label)) { *N *= (double)l.dim; next->push_back(l); }
-    return shared;
-  }
-  // The chain of least modelled time: the legs of a partial chain depend only on the set of its
-  // operands, so the best way to every set is built from the sets with one operand less.  The
-  // greedy chain it replaces (largest contracted extent first) took up to five times the
-  // multiply-adds: site and operator adjoints of a degree-3 node at bond 75, 50.2 -> 3.24 ms.
-  std::vector<int> cheapest_chain(int precision) const {
-    const int n = (int)op.size() - 1;
-    struct State {
-      double cost = -1;
-      int last = -1;
-      std::vector<Leg> legs;
-    };
-    std::vector<State> st(size_t(1) << n);
-    st[0].cost = 0;
-    st[0].legs = op[0];
-    for (uint32_t mask = 0; mask + 1 < (1u << n); ++mask) {
-      if (st[mask].cost < 0) continue;
-      for (int pass = 0, found = 0; pass < 2 && !found; ++pass)  // outer products only if nothing connects
-        for (int b = 0; b < n; ++b) {
-          if (mask >> b & 1u) continue;
-          double M, K, N;
-          std::vector<Leg> next;
-          if (!absorb(st[mask].legs, op[b + 1], &M, &K, &N, &next) && pass == 0) continue;
-          found = 1;
-          State& t = st[mask | 1u << b];
-          const double c = st[mask].cost + plan_step_time(precision, M, K, N, true);
-          if (t.cost < 0 || c < t.cost) {
-            t.cost = c;
-            t.last = b;
-            t.legs.swap(next);
-          }
-        }
-    }
-    std::vector<int> ord(n + 1, 0);
-    for (uint32_t mask = (1u << n) - 1, i = n; mask; --i) {
-      ord[i] = st[mask].last + 1;
-      mask &= ~(1u << st[mask].last);
-    }
-    return ord;
-  }
-  // Always the operand sharing the largest contracted extent (ties: the smaller result).
-  std::vector<int> greedy_chain() const {
-    const int n = (int)op.size();
-    std::vector<Leg> cur = op[0], next;
-    std::vector<int> ord(1, 0);
-    std::vector<bool> used(n, false);
-    for (int step = 1; step < n; ++step) {
-      int best = -1;
-      double best_shared = -1, best_size = 0;
-      for (int q = 1; q < n; ++q) {
-        if (used[q]) continue;
-        double M, K, N;
-        const double shared = absorb(cur, op[q], &M, &K, &N, &next) ? K : 0;
-        if (shared > best_shared || (shared == best_shared && M * N < best_size)) {
-          best = q;
-          best_shared = shared;
-          best_size = M * N;
-        }
-      }
-      double M, K, N;
-      absorb(cur, op[best], &M, &K, &N, &next);
-      cur.swap(next);
-      used[best] = true;
-      ord.push_back(best);
-    }
-    return ord;
-  }
-};
-}  // namespace
 
 extern "C" {
 
@@ -526,16 +426,16 @@ int gtn_contract_vjp(gtn_ctx ctx, int n_operands, const int* ranks, const int64_
   if (order)
     return gtn_contract(ctx, nn, nr.data(), nd.data(), nl.data(), nc.data(), order, np.data(), out, precision);
   const VjpNetwork net(nn, nr, nd, nl);
-  if (nn <= kVjpSearchMax) {
-    const std::vector<int> ord = net.cheapest_chain(precision);
+  const auto step_time = [precision](double M, double K, double N) { return plan_step_time(precision, M, K, N, true); };
+  const std::vector<int> greedy = net.greedy_chain(), ord = net.cheapest_chain(greedy, step_time);
+  if (ord != greedy) {
     const int st = gtn_contract(ctx, nn, nr.data(), nd.data(), nl.data(), nc.data(), ord.data(), np.data(), out,
                                 precision);
     // a chain refused for the memory of its tensors or for their leg groups: the greedy one may pass
     if (st != GTN_ERR_MEMORY && st != GTN_ERR_UNSUPPORTED) return st;
     cudaGetLastError();
   }
-  const std::vector<int> ord = net.greedy_chain();
-  return gtn_contract(ctx, nn, nr.data(), nd.data(), nl.data(), nc.data(), ord.data(), np.data(), out, precision);
+  return gtn_contract(ctx, nn, nr.data(), nd.data(), nl.data(), nc.data(), greedy.data(), np.data(), out, precision);
 }
 
 int gtn_permute(gtn_ctx ctx, int rank, const int64_t* dims, const int* perm, const void* in, void* out) {

@@ -289,7 +289,8 @@ int gtn_contract(gtn_ctx ctx, int n_operands, const int* ranks, const int64_t* d
  * for every perturbation of op_slot as it enters the contraction (after its conj flag):
  * G = contract(ybar, conj(op_i), i != slot).  It runs through the same contraction engine
  * (tcgen05 steps in the mixed precisions).  order (may be NULL) orders the rewritten
- * operand list [ybar, op_i for i != slot]; NULL picks the cheapest chain from ybar. */
+ * operand list [ybar, op_i for i != slot]; NULL picks the chain from ybar of least
+ * modelled time, or a greedy one where looking for it takes longer than it can save. */
 int gtn_contract_vjp(gtn_ctx ctx, int n_operands, const int* ranks, const int64_t* dims, const int* labels,
                      const int* conj, const int* order, const void* const* operands, int slot, const void* ybar,
                      void* out, int precision);
