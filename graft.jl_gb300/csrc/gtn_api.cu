@@ -323,8 +323,12 @@ int gtn_contract(gtn_ctx ctx, int n_operands, const int* ranks, const int64_t* d
     if (ctx->carena) cudaFree(ctx->carena);
     ctx->carena = nullptr;
     ctx->carena_cap = 0;
-    if (cudaMalloc(&ctx->carena, ctx->carena_need) == cudaSuccess) ctx->carena_cap = ctx->carena_need;
-    else ctx->carena = nullptr;
+    if (cudaMalloc(&ctx->carena, ctx->carena_need) == cudaSuccess) {
+      ctx->carena_cap = ctx->carena_need;
+    } else {
+      ctx->carena = nullptr;
+      cudaGetLastError();  // no arena: the launches below do not report its refusal
+    }
   }
   gtn_map map = new (std::nothrow) gtn_map_s();
   if (!map) return set_err(ctx, GTN_ERR_MEMORY, "host allocation failed");

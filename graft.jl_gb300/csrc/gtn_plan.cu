@@ -669,6 +669,8 @@ int plan_build(gtn_ctx ctx, int n, const int* ranks, const int64_t* dims, const 
     max_sk = std::max(max_sk, map->fp64_alt->max_splitk);
   }
   const size_t tbytes = (size_t)max_t * sizeof(double2);
+  // (a one-shot FP64 contraction runs on digit planes or reads its tensors in place: no K-major copy)
+  if (map->oneshot && precision == GTN_PREC_FP64) max_a = 0;
   size_t abytes = std::max<size_t>((size_t)max_a * sizeof(double2), (size_t)map->max_apl * sizeof(__nv_bfloat16));
   size_t freeb = 0, totalb = 0;
   if (map->oneshot) freeb = SIZE_MAX;  // one-shot contraction: the arena or a failing cudaMalloc decides
@@ -676,23 +678,37 @@ int plan_build(gtn_ctx ctx, int n, const int* ranks, const int64_t* dims, const 
     cudaMemGetInfo(&freeb, &totalb);
     freeb += ctx->blk_cached;  // cached blocks are reused or given back on demand
   }
-  if (dg64 && map->max_adg > abytes && 2 * tbytes + map->max_adg + (size_t)(1u << 30) > freeb) {
-    // the digit planes do not fit: the FP64 pipe, which reads the running tensor in place, runs
+  // Without the memory for its digit planes an FP64 plan runs on the FP64 pipe, which reads the running
+  // tensor in place.
+  auto no_digits = [&] {
     for (auto& st : map->steps) st.dg = false;
     map->max_adg = 0;
-  }
-  abytes = std::max(abytes, map->max_adg);
-  const size_t need = 2 * tbytes + abytes + (size_t)(1u << 30);
+  };
+  size_t planes = 0;  // of the statics
+  for (const auto& st : map->steps)
+    if (st.dg) planes += f64e_b_bytes(st.N, st.K) + f64e_mag_bytes(st.N, st.K);
+  if (dg64 && map->max_adg > 0 &&
+      2 * tbytes + std::max(abytes, map->max_adg) + planes + (size_t)(1u << 30) > freeb)
+    no_digits();
+  const size_t need = 2 * tbytes + std::max(abytes, map->max_adg) + (size_t)(1u << 30);
   if (need > freeb)
     return set_err(ctx, GTN_ERR_MEMORY, "memory admission refused: map workspace " +
                                             std::to_string(need >> 20) + " MiB > free " +
                                             std::to_string(freeb >> 20) + " MiB");
-  if (dalloc(map, &map->buf0, tbytes) != cudaSuccess || dalloc(map, &map->buf1, tbytes) != cudaSuccess ||
-      dalloc(map, &map->abuf, std::max<size_t>(abytes, 256)) != cudaSuccess)
+  if (dalloc(map, &map->buf0, tbytes) != cudaSuccess || dalloc(map, &map->buf1, tbytes) != cudaSuccess)
     return set_err(ctx, GTN_ERR_MEMORY, "map workspace allocation failed");
-  if ((is_fp16(precision) || map->max_adg > 0) && map->max_mtc > 0 &&
-      dalloc(map, &map->amax, (size_t)map->max_mtc * sizeof(float)) != cudaSuccess)
-    return set_err(ctx, GTN_ERR_MEMORY, "map workspace allocation failed");
+  auto stage = [&] {
+    return dalloc(map, &map->abuf, std::max<size_t>(std::max(abytes, map->max_adg), 256)) == cudaSuccess &&
+           (!(is_fp16(precision) || map->max_adg > 0) || map->max_mtc <= 0 ||
+            dalloc(map, &map->amax, (size_t)map->max_mtc * sizeof(float)) == cudaSuccess);
+  };
+  bool staged = stage();
+  if (!staged && dg64 && map->max_adg > 0) {
+    cudaGetLastError();
+    no_digits();
+    staged = stage();
+  }
+  if (!staged) return set_err(ctx, GTN_ERR_MEMORY, "map workspace allocation failed");
   if (max_sk > 0 && dalloc(map, reinterpret_cast<double2**>(&map->skbuf), (size_t)max_sk * sizeof(double2)) !=
                         cudaSuccess)
     return set_err(ctx, GTN_ERR_MEMORY, "map workspace allocation failed");
