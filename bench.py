@@ -8,7 +8,8 @@ TTNO, w = 5).  Inputs are seeded synthetic tensors of exactly those shapes.
 
   python bench.py [--gpus N] [--steps K] [--warmup W] [--impl ours|reference]
 
-Prints one JSON line.  ``--impl reference`` times the CPU restatement of the reference
+Prints one JSON line (at most LINE_BYTES) on stdout; the segments' own records and the tile
+choices go to stderr as a second one.  ``--impl reference`` times the CPU restatement of the reference
 path (numpy/OpenBLAS on all host cores) on the same workload.
 """
 from __future__ import annotations
@@ -368,6 +369,39 @@ def bench_batched(ctx, steps):
             "launches_per_batched_apply": launches, "tflops_batched": flops / ms_b / 1e9, "max_rel_err_vs_oracle": err}
 
 
+LINE_BYTES = 4000  # a record of the run's output keeps its last kilobytes: the line has to be among them
+SEGMENTS = ("kernels", "tc_tile_choices", "dmrg_segment", "gradient", "other_mixed_modes", "grouping_ab",
+            "u1_blocksparse", "batched_eff_h1")
+
+
+def headline(line):
+    """(the line to print, the detail behind it): the segments' records become one figure each."""
+    detail = {k: line[k] for k in SEGMENTS if k in line}
+    line = {k: v for k, v in line.items() if k not in detail}
+
+    def pick(name, *path):
+        v = detail.get(name)
+        for key in path:
+            v = v.get(key) if isinstance(v, dict) else None
+        return v
+    short = {
+        "dmrg_step_fp64_over_mixed": pick("dmrg_segment", "time_ratio_fp64_over_mixed"),
+        "dmrg_step_mixed_s": pick("dmrg_segment", "runs", "fp16x3", "total_s"),
+        "site_gradients_fp64_s": pick("gradient", "site_gradients", "fp64", "s"),
+        "bf16x6_applies_per_s": pick("other_mixed_modes", "bf16x6", "value"),
+        "env_first_ms_per_apply": pick("grouping_ab", "env_first_ms_per_apply"),
+        "u1_fp16x3_applies_per_s": pick("u1_blocksparse", "fp16x3", "applies_per_s"),
+        "u1_fp64_applies_per_s": pick("u1_blocksparse", "fp64", "applies_per_s"),
+        "batched_64_ms": pick("batched_eff_h1", "ms_batched_graph"),
+        "tile_choices": len(detail["tc_tile_choices"]) if "tc_tile_choices" in detail else None,
+    }
+    line["segments"] = {k: v for k, v in short.items() if v is not None}
+    errors = {k: v["error"][:100] for k, v in detail.items() if isinstance(v, dict) and "error" in v}
+    if errors:
+        line["segment_errors"] = errors
+    return line, detail
+
+
 def run_ours(args, rank, world):
     import torch
     import grafttn as G
@@ -611,6 +645,8 @@ def run_ours(args, rank, world):
     if gradient is not None:
         line["gradient"] = gradient
     line.update(extra)
+    line, detail = headline(line)
+    print(json.dumps({"detail": detail}), file=sys.stderr, flush=True)
     print(json.dumps(line), flush=True)
     if not parity_ok:
         sys.exit(f"parity failure: fp64 vs oracle {fp64_vs_oracle:.3e} (bound 1e-12), "
