@@ -444,10 +444,13 @@ constexpr int kRM = kF64eCheckM, kRN = kF64eCheckN, kRThreads = 256;
 constexpr int kRKC = 64, kRStages = 2;              // complex k per stage (rows of 128 bytes)
 constexpr int kRStage = (kRM + kRN) * kRKC * 2;
 constexpr int kRSmem = kRStages * kRStage;
-static_assert(kRM * kRN * 2 <= kRStage, "a tile's list in a stage");
+static_assert(kRM * kRN * 2 + (kRM + kRN) * 4 <= kRSmem, "a tile's list and sums over the stages");
 // (2^-56 + 2^-62.6) K <= 2 K 2^-53 s from s = 0.0632 on; the rest covers the rounding of the sums
 constexpr float kSureSum = 0.0703f;
 constexpr int kSureMeets = 28;  // times 0.05078^2
+// E / (2 2^-53): 2^-4 (alpha + beta) and 2^-10.6, with the rounding of the magnitudes and sums
+constexpr float kMagError = 0.064f, kLevelError = 0.00066f;
+constexpr int kRowSumBlocks = 512;  // K up to 4096: longer sums are above kSureSum or far below
 
 struct RepairArgs {
   const double2* T;
@@ -541,6 +544,7 @@ __global__ void __launch_bounds__(kRThreads, 3) f64e_check_kernel(const __grid_c
           f(wm + i * 16 + (lane >> 2) + (e >> 1) * 8, wn + j * 8 + 2 * (lane & 3) + (e & 1), acc[i][j][e]);
   };
   uint16_t* list = reinterpret_cast<uint16_t*>(rsmem);
+  float* row_sum = reinterpret_cast<float*>(rsmem + kRM * kRN * 2);  // of the rows of A, then of B
   const int window = (int)min(g.K, (int64_t)kF64eWindow), wkb = (int)min(nkb, (int64_t)(kF64eWindow / 8));
   // a CTA's tiles: a range with the column tiles of a row tile behind each other
   const unsigned tiles_n = (unsigned)(g.ntiles / g.tiles_m);
@@ -606,9 +610,34 @@ __global__ void __launch_bounds__(kRThreads, 3) f64e_check_kernel(const __grid_c
     asm volatile("cp.async.wait_all;" ::: "memory");
     __syncthreads();
     if (done) continue;
+    // the bound again with the rows' own sums in place of K halves (a thread a row; short sums, and
+    // graded rows, gain by it)
+    const bool sums = nkb <= kRowSumBlocks;
+    if (sums) {
+      if (tid < kRM + kRN) {
+        const bool is_a = tid < kRM;
+        const int64_t rows = is_a ? g.M : g.N, row_at = is_a ? m0 + tid : n0 + tid - kRM;
+        const uint16_t* mag = (is_a ? g.a_mag : g.b_mag) + row_at * 8;
+        float x = 0.f;
+        if (row_at < rows)
+#pragma unroll 8
+          for (int kb = 0; kb < (int)nkb; ++kb) {
+            const uint4 u = *reinterpret_cast<const uint4*>(mag + kb * rows * 8);
+            x += ((__uint_as_float(u.x << 16) + __uint_as_float(u.x & 0xffff0000u)) +
+                  (__uint_as_float(u.y << 16) + __uint_as_float(u.y & 0xffff0000u))) +
+                 ((__uint_as_float(u.z << 16) + __uint_as_float(u.z & 0xffff0000u)) +
+                  (__uint_as_float(u.w << 16) + __uint_as_float(u.w & 0xffff0000u)));
+          }
+        row_sum[tid] = kMagError * x;
+      }
+      __syncthreads();
+    }
+    const float levels = kLevelError * (float)g.K;
     uint32_t doubtful = 0, bit = 1;
     for_outputs([&](int ml, int nl, float& s) {
-      if (!(s >= kSureSum) && s != 0.f && ml < mlim && nl < nlim) doubtful |= bit;
+      if (!(s >= kSureSum) && s != 0.f && ml < mlim && nl < nlim &&
+          !(sums && s * (float)g.K >= row_sum[ml] + row_sum[kRM + nl] + levels))
+        doubtful |= bit;
       bit <<= 1;
     });
     int at = __popc(doubtful), total = at;
@@ -750,9 +779,7 @@ __global__ void __launch_bounds__(kPThreads, 4) f64e_repair_kernel(const __grid_
     __syncthreads();  // the last chunk's list has been used
     if (threadIdx.x == 0) count = 0;
     __syncthreads();
-    // E / (2 * 2^-53): 2^-4 and 2^-10.6, with the rounding of the magnitudes and sums (NaN: a row
-    // without digits)
-    const bool holds = prod * (float)g.K >= fmaf(0.064f, sum, 0.00066f * met);
+    const bool holds = prod * (float)g.K >= fmaf(kMagError, sum, kLevelError * met);  // (NaN: a row without digits)
     if (l == 0 && e < n && !holds) again[atomicAdd(&count, 1)] = (uint16_t)id;
     __syncthreads();
     repair_outputs<kPThreads>(g, again, count, m0, n0);
