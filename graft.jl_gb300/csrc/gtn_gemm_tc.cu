@@ -1075,7 +1075,7 @@ cudaError_t launch_persist_g(const TcGemmArgs* probs, int nprob, int* errflag, c
     if (tiles == 0) continue;
     // A long launch gains nothing from being chained, and its CTAs would take the SMs in the order in
     // which the kernel before it leaves them (fp16x3 two-site map at d = 1024, 14 to 68 waves a step:
-    // 7.78 ms in order, 7.82 chained).
+    // 7.78 ms in order, 7.82 chained, which is within the runs' scatter).
     launch_chained_if(tiles <= 8 * grid, tc_gemm_persist_kernel<BN, P, G>, dim3(std::min(tiles, grid)), dim3(kPersistThreads), CF::SMEM, s, g, errflag);
     cudaError_t e = cudaGetLastError();
     if (e != cudaSuccess) return e;

@@ -452,8 +452,9 @@ class EnvCache:
     used eviction (envcache.jl:571-594); evicted environments are recomputed on demand."""
 
     def __init__(self, topo, max_env_bytes=None, precision="fp64"):
-        """``precision`` of the environment contractions: "fp64" (FP64 SIMT kernels) or
-        "fp64e" (the FP64-grade digit products on the tensor cores, about 1e-14)."""
+        """``precision`` of the environment contractions: "fp64" (every entry within the bound of
+        an FP64 sum) or "fp64e" (digit products on the tensor cores alone, about 4e-16 in the
+        2-norm; entries far below their rows' largest are less accurate)."""
         from collections import OrderedDict
         self.topo = topo
         self.precision = _lib.PRECISIONS[precision] if isinstance(precision, str) else precision
