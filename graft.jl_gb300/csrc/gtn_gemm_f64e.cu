@@ -429,17 +429,23 @@ __global__ void __launch_bounds__(32 * kEpiWarps)
 //     operands are done by counting (a row of 128 Gaussian entries has 110 such).  Of the others the
 //     sums are formed from bf16 magnitudes, 64 k at a time until all are above.  A sum of zero means
 //     that no two factors meet, and that the digit products are exact.  What remains is listed.
-//   * f64e_repair_kernel adds E and the magnitudes' products over the listed outputs' rows and sums
-//     those again whose bound does not hold.  Chunks of 32 listed outputs keep every SM at work where
-//     they come from few tiles (a state of Schmidt weights down to 1e-5 meets the identity
-//     channel of its environments, 4 of 24 tiles).
+//   * f64e_repair_kernel adds E and the magnitudes' products over the listed outputs' rows.  Where the
+//     bound does not hold it adds the products of A's first and B's eighth digits to the output, by
+//     which B's entries count to 2^-65 and E becomes the sum of
+//       2^-56 beta_k + 2^-64 + min(2^-62.6, 2^-12.6 min(alpha_k, beta_k))
+//     (the last for the levels left out: a factor below 2^-50 has few digits to meet them).  That is
+//     what the identity channel of an environment wants, one entry of 1 and others of rounding size.
+//     Where it is not enough either the output is summed again.  Chunks of 32 listed outputs keep every
+//     SM at work where they come from few tiles.
 // The sums have half of the digit product's rows, columns and k and one plane: mma.sync, which
 // needs no TMEM (the digit levels hold all of it), leaves them a small part of the step.
 // One-site map of a 31-site binary tree at D = 128 (M = 163840, N = 640, K = 128, digit product
 // 2423 us): the sums take 241 us, 148 us with tiles that end early, and counting 27 us.  Products of the
 // two-site map of a DMRG step at D = 96 (M = 384, N = 480, K = 96 and M = 384, N = 96, K = 480) with a
-// state of which 7 to 10 % of the outputs are summed again: check 9 and 15 us, repair 33 and 38 us
-// (with a CTA for each tile 1059 and 510 us together); 1 % of a Lanczos vector's: 24 us together.
+// state of which 7 to 10 % of the outputs miss the bound: check 11 and 19 us, repair 26 and 48 us (with
+// a CTA for each tile 1059 and 510 us together); 1 % of a Lanczos vector's: 23 us together.  Environments
+// of a random state at D = 128 (M = 163840, N = 640, K = 128; 6.4 % miss it, 2.4 % with eighth digits
+// too): 5.9 ms, 10.5 ms with every one of them summed again, 93 ms on the FP64 pipe.
 constexpr int kRM = kF64eCheckM, kRN = kF64eCheckN, kRThreads = 256;
 constexpr int kRKC = 64, kRStages = 2;              // complex k per stage (rows of 128 bytes)
 constexpr int kRStage = (kRM + kRN) * kRKC * 2;
@@ -450,6 +456,7 @@ constexpr float kSureSum = 0.0703f;
 constexpr int kSureMeets = 28;  // times 0.05078^2
 // E / (2 2^-53): 2^-4 (alpha + beta) and 2^-10.6, with the rounding of the magnitudes and sums
 constexpr float kMagError = 0.064f, kLevelError = 0.00066f;
+constexpr float kLowError = 0.000247f, kSmallError = 7.35e11f;  // 2^-12, 2^39.4
 constexpr int kRowSumBlocks = 512;  // K up to 4096: longer sums are above kSureSum or far below
 
 struct RepairArgs {
@@ -462,6 +469,8 @@ struct RepairArgs {
   const float *a_exp, *b_exp;
   const uint16_t *a_mag, *b_mag;
   const int* b_large;
+  const uint32_t* b_low;
+  const unsigned char* planes;  // of A
   uint16_t* lists;             // [tile][kRM kRN]: n_local kRM + m_local
   unsigned long long* chunks;  // tile << 24 | first << 8 | length
   int* count;                  // chunks
@@ -737,52 +746,77 @@ __device__ __forceinline__ void repair_outputs(const RepairArgs& g, const uint16
   }
 }
 
-// Checked products: the chunks of f64e_check_kernel.  Of a chunk's outputs those whose bound does not
-// hold, four threads each, are summed again.
+// Two bf16 in a word: the first (even k, or the real part) and the second.
+__device__ __forceinline__ float lo16(uint32_t w) { return __uint_as_float(w << 16); }
+__device__ __forceinline__ float hi16(uint32_t w) { return __uint_as_float(w & 0xffff0000u); }
+__device__ __forceinline__ float sum4(float x) {  // over the four threads of an output
+  x += __shfl_xor_sync(0xffffffffu, x, 2);
+  return x + __shfl_xor_sync(0xffffffffu, x, 1);
+}
+
+// Checked products: the chunks of f64e_check_kernel, four threads for each output.  Each decides
+// between the output as it is, with B's eighth digits, and a sum on the FP64 pipe.
 __global__ void __launch_bounds__(kPThreads, 4) f64e_repair_kernel(const __grid_constant__ RepairArgs g) {
   chained_wait();
   __shared__ uint16_t again[kF64eCheckChunk];
-  __shared__ int count;
+  __shared__ int nagain;
   const int nch = *g.count, l = threadIdx.x & 3, e = threadIdx.x >> 2;
   const int64_t nkb = (g.K + 7) / 8, tiles_n = g.ntiles / g.tiles_m;
 #pragma unroll 1
   for (int c = blockIdx.x; c < nch; c += gridDim.x) {
     const unsigned long long ch = g.chunks[c];
     const int64_t tile = (int64_t)(ch >> 24);
-    const int n = (int)(ch & 0xff), first = (int)(ch >> 8 & 0xffff);
+    const int count = (int)(ch & 0xff), first = (int)(ch >> 8 & 0xffff);
     const int64_t m0 = tile / tiles_n * kRM, n0 = tile % tiles_n * kRN;
-    const int id = g.lists[tile * (kRM * kRN) + first + min(e, n - 1)];
-    const uint16_t *a = g.a_mag + (m0 + id % kRM) * 8, *b = g.b_mag + (n0 + id / kRM) * 8;
-    float prod = 0.f, sum = 0.f, met = 0.f;
-#pragma unroll 4
-    for (int64_t kb = l; kb < nkb; kb += 4) {
-      const uint4 u = *reinterpret_cast<const uint4*>(a + kb * g.M * 8);
-      const uint4 v = *reinterpret_cast<const uint4*>(b + kb * g.N * 8);
-      const uint32_t x[4] = {u.x, u.y, u.z, u.w}, y[4] = {v.x, v.y, v.z, v.w};
+    const int id = g.lists[tile * (kRM * kRN) + first + min(e, count - 1)], rr = id % kRM;
+    const int64_t m = m0 + rr, n = n0 + id / kRM;
+    const unsigned char* a = g.planes + (m0 / kBM * nkb * kS * kBM + rr) * 32;  // A's first digits
+    const uint32_t* b = g.b_low + n * 8 * nkb;
+    const uint16_t *am = g.a_mag + m * 8, *bm = g.b_mag + n * 8;
+    float re = 0.f, im = 0.f, prod = 0.f, alpha = 0.f, beta = 0.f, met = 0.f, left = 0.f;
+#pragma unroll 2
+    for (int64_t q = l; q < 2 * nkb; q += 4) {  // four k
+      const uint4 u = *reinterpret_cast<const uint4*>(a + (q >> 1) * (kS * kPlaneA) + (((int)q ^ (rr >> 2)) & 1) * 16);
+      const uint4 v = *reinterpret_cast<const uint4*>(b + q * 4);
+      const uint2 x = *reinterpret_cast<const uint2*>(am + (q >> 1) * g.M * 8 + (q & 1) * 4);
+      const uint2 y = *reinterpret_cast<const uint2*>(bm + (q >> 1) * g.N * 8 + (q & 1) * 4);
+      const uint32_t d[4] = {u.x, u.y, u.z, u.w}, t[4] = {v.x, v.y, v.z, v.w}, xs[2] = {x.x, x.y}, ys[2] = {y.x, y.y};
 #pragma unroll
-      for (int q = 0; q < 8; ++q) {
-        const float al = __uint_as_float(q & 1 ? x[q >> 1] & 0xffff0000u : x[q >> 1] << 16);
-        const float be = __uint_as_float(q & 1 ? y[q >> 1] & 0xffff0000u : y[q >> 1] << 16);
+      for (int p = 0; p < 4; ++p) {
+        re = fmaf(lo16(d[p]), lo16(t[p]), fmaf(-hi16(d[p]), hi16(t[p]), re));
+        im = fmaf(lo16(d[p]), hi16(t[p]), fmaf(hi16(d[p]), lo16(t[p]), im));
+        const float al = p & 1 ? hi16(xs[p >> 1]) : lo16(xs[p >> 1]), be = p & 1 ? hi16(ys[p >> 1]) : lo16(ys[p >> 1]);
         const bool both = al != 0.f && be != 0.f;
         prod = fmaf(al, be, prod);
-        sum += both ? al + be : 0.f;
+        alpha += both ? al : 0.f;
+        beta += both ? be : 0.f;
         met += both ? 1.f : 0.f;
+        left += both ? fminf(kLevelError, kSmallError * fminf(al, be)) : 0.f;
       }
     }
     __syncwarp();
-#pragma unroll
-    for (int o = 2; o > 0; o >>= 1) {
-      prod += __shfl_xor_sync(0xffffffffu, prod, o);
-      sum += __shfl_xor_sync(0xffffffffu, sum, o);
-      met += __shfl_xor_sync(0xffffffffu, met, o);
-    }
+    re = sum4(re);
+    im = sum4(im);
+    prod = sum4(prod) * (float)g.K;
+    alpha = sum4(alpha);
+    beta = sum4(beta);
+    met = sum4(met);
+    left = sum4(left);
     __syncthreads();  // the last chunk's list has been used
-    if (threadIdx.x == 0) count = 0;
+    if (threadIdx.x == 0) nagain = 0;
     __syncthreads();
-    const bool holds = prod * (float)g.K >= fmaf(kMagError, sum, kLevelError * met);  // (NaN: a row without digits)
-    if (l == 0 && e < n && !holds) again[atomicAdd(&count, 1)] = (uint16_t)id;
+    // (no bound holds with NaN, the magnitudes of a row without digits)
+    if (l == 0 && e < count && !(prod >= fmaf(kMagError, alpha + beta, kLevelError * met))) {
+      if (prod >= fmaf(kMagError, beta, fmaf(kLowError, met, left))) {  // units of 2^-72 of the scaled rows
+        const int scale = (int)g.a_exp[m] + (int)g.b_exp[n] - 2 * 1021 - 72;
+        double2* y = g.C + n * g.M + m;
+        *y = make_double2(y->x + scalbn((double)re, scale), y->y + scalbn((double)im, scale));
+      } else {
+        again[atomicAdd(&nagain, 1)] = (uint16_t)id;
+      }
+    }
     __syncthreads();
-    repair_outputs<kPThreads>(g, again, count, m0, n0);
+    repair_outputs<kPThreads>(g, again, nagain, m0, n0);
   }
 }
 
@@ -918,7 +952,9 @@ cudaError_t launch_f64e_repair(const F64eGemmArgs& a, const double2* T, const Ga
   g.b_mag = a.b_mag;
   g.b_large = a.b_large;
   g.count = a.count;
-  g.lists = static_cast<uint16_t*>(const_cast<void*>(a.A));
+  g.b_low = a.b_low;
+  g.planes = static_cast<const unsigned char*>(a.A);
+  g.lists = static_cast<uint16_t*>(a.lists);
   g.chunks = reinterpret_cast<unsigned long long*>(g.lists + g.ntiles * kRM * kRN);
   static PerDeviceOnce opt_in;
   if (const cudaError_t e = smem_opt_in(opt_in, f64e_check_kernel, kRSmem)) return e;

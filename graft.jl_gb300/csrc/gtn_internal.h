@@ -415,8 +415,7 @@ inline size_t f64e_a_bytes(int64_t M, int64_t K) {
   return (size_t)((M + kF64eRowsA - 1) / kF64eRowsA) * ((K + 7) / 8) * kF64eSlices * kF64eRowsA * 32;
 }
 // The check of FP64 products: magnitudes of an operand's entries (bf16, [k / 8][row][k % 8]); the
-// lists of doubtful outputs, over tiles of kF64eCheckM x kF64eCheckN, which take the place of A's planes
-// once the product is there; a count before A's magnitudes.
+// lists of doubtful outputs, over tiles of kF64eCheckM x kF64eCheckN; the eighth digits of B.
 constexpr int kF64eCheckM = 128, kF64eCheckN = 64, kF64eCheckChunk = 32;
 // Entries among a row's first kF64eWindow that are at least kF64eLarge (bf16 bits of 0.0508): where two
 // rows have L of W entries more than W together, L of them meet.  A row without digits counts as
@@ -424,14 +423,14 @@ constexpr int kF64eCheckM = 128, kF64eCheckN = 64, kF64eCheckChunk = 32;
 constexpr int kF64eWindow = 128, kF64eNoCount = -(1 << 20);
 constexpr uint32_t kF64eLarge = 0x3d50;
 inline size_t f64e_mag_bytes(int64_t rows, int64_t K) { return ((size_t)rows * ((K + 7) / 8) * 16 + 255) / 256 * 256; }
-inline size_t f64e_check_offset(int64_t M, int64_t N, int64_t K, size_t a_bytes) {
+inline size_t f64e_low_bytes(int64_t N, int64_t K) { return (size_t)N * ((K + 7) / 8) * 32; }
+inline size_t f64e_list_bytes(int64_t M, int64_t N) {
   const size_t tiles = (size_t)((M + kF64eCheckM - 1) / kF64eCheckM) * ((N + kF64eCheckN - 1) / kF64eCheckN);
-  const size_t outputs = (size_t)kF64eCheckM * kF64eCheckN;
-  const size_t lists = tiles * (outputs * 2 + outputs / kF64eCheckChunk * 8);
-  return (std::max(lists, a_bytes) + 255) / 256 * 256;
+  return tiles * kF64eCheckM * kF64eCheckN / kF64eCheckChunk * (kF64eCheckChunk * 2 + 8);
 }
-inline size_t f64e_check_bytes(int64_t M, int64_t N, int64_t K, size_t a_bytes) {
-  return f64e_check_offset(M, N, K, a_bytes) + 256 + f64e_mag_bytes(M, K);
+// What an FP64 step keeps in its staging buffer behind A's planes: a count, A's magnitudes, the lists.
+inline size_t f64e_check_bytes(int64_t M, int64_t N, int64_t K) {
+  return 256 + f64e_mag_bytes(M, K) + f64e_list_bytes(M, N);
 }
 inline size_t f64e_b_bytes(int64_t N, int64_t K) {
   return (size_t)((2 * N + kF64eRowsB - 1) / kF64eRowsB) * ((K + 7) / 8) * kF64eSlices * kF64eRowsB * 32;
@@ -450,7 +449,9 @@ struct F64eGemmArgs {
   const uint16_t* a_mag = nullptr;  // magnitudes: the outputs are checked; null: they are not
   const uint16_t* b_mag = nullptr;
   const int* b_large = nullptr;     // large entries of B's rows
-  int* count = nullptr;             // of the check, zeroed by the split; its lists take A's place
+  const uint32_t* b_low = nullptr;  // their eighth digits
+  int* count = nullptr;             // of the check, zeroed by the split
+  void* lists = nullptr;            // of the check
   int levels = 8;               // digit products d_i e_j with i + j < levels (7 or 8)
   void* part = nullptr;         // f64e_part_bytes of the product, or null: no tile is shared
 };
@@ -470,7 +471,7 @@ cudaError_t launch_split_digits_grp(const double2* T, const GroupSpec& mg, const
                                     float* rexp, void* out, uint16_t* mag, int* count, cudaStream_t s,
                                     int* launches);
 cudaError_t launch_pack_b_digits(const double2* B, int64_t N, int64_t K, void* out, float* bexp, uint16_t* mag,
-                                 int* large, cudaStream_t s);
+                                 int* large, uint32_t* low, cudaStream_t s);
 // C[n][m] = sum_k T[offM(m) + offK(k)] B[n][k] on the FP64 pipe, T read in place.  With slices > 1
 // (of zgemm_view_slices: few outputs, long K) the k range is cut into that many partial products
 // P[slice][n][m], summed in order.
@@ -555,6 +556,7 @@ struct PlanStep {
   float* bexp = nullptr;
   uint16_t* bmag = nullptr;  // magnitudes of the static and the large ones' number (FP64 applications)
   int* blarge = nullptr;
+  uint32_t* blow = nullptr;  // and its eighth digits
   double macs = 0;
 };
 

@@ -156,12 +156,13 @@ int pack_digits(gtn_map map, bool required, bool mags) {
     if (a == cudaSuccess) a = dalloc(map, &st.bexp, (size_t)st.N * sizeof(float));
     if (a == cudaSuccess && mags) a = dalloc(map, &st.bmag, f64e_mag_bytes(st.N, st.K));
     if (a == cudaSuccess && mags) a = dalloc(map, &st.blarge, (size_t)st.N * sizeof(int));
+    if (a == cudaSuccess && mags) a = dalloc(map, &st.blow, f64e_low_bytes(st.N, st.K));
     if (a != cudaSuccess) {
       if (required) return set_err(ctx, GTN_ERR_MEMORY, "static packing allocation failed");
       cudaGetLastError();
       continue;
     }
-    e = launch_pack_b_digits(st.b64, st.N, st.K, planes, st.bexp, st.bmag, st.blarge, ctx->stream);
+    e = launch_pack_b_digits(st.b64, st.N, st.K, planes, st.bexp, st.bmag, st.blarge, st.blow, ctx->stream);
     ctx->launches++;
     st.bdig = planes;
   }
@@ -558,7 +559,7 @@ int plan_build(gtn_ctx ctx, int n, const int* ranks, const int64_t* dims, const 
       if (st.tc || st.dg) map->max_mtc = std::max(map->max_mtc, st.M);
       if (st.dg) {
         const size_t planes = f64e_a_bytes(st.M, st.K);
-        map->max_adg = std::max(map->max_adg, mags ? f64e_check_bytes(st.M, st.N, st.K, planes) : planes);
+        map->max_adg = std::max(map->max_adg, planes + (mags ? f64e_check_bytes(st.M, st.N, st.K) : 0));
       }
       st.splitk = gemm_splitk_slices(st.M, st.N, st.K);
       st.vslices = zgemm_view_slices(st.M, st.N, st.K);
@@ -690,7 +691,7 @@ int plan_build(gtn_ctx ctx, int n, const int* ranks, const int64_t* dims, const 
   };
   size_t planes = 0;  // of the statics
   for (const auto& st : map->steps)
-    if (st.dg) planes += f64e_b_bytes(st.N, st.K) + f64e_mag_bytes(st.N, st.K);
+    if (st.dg) planes += f64e_b_bytes(st.N, st.K) + f64e_mag_bytes(st.N, st.K) + f64e_low_bytes(st.N, st.K);
   if (dg64 && map->max_adg > 0 &&
       2 * tbytes + std::max(abytes, map->max_adg) + planes + (size_t)(1u << 30) > freeb)
     no_digits();
@@ -828,10 +829,12 @@ int map_run(gtn_map map, int precision, const double2* x, double2* y) {
         a.b_exp = st.bexp;
         a.levels = f64e ? 7 : 8;
         uint16_t* mag = nullptr;
-        if (!f64e) {  // FP64: count and magnitudes of the check behind the planes
-          char* chk = static_cast<char*>(map->abuf) + f64e_check_offset(st.M, st.N, st.K, f64e_a_bytes(st.M, st.K));
+        if (!f64e) {  // FP64: count, magnitudes and lists of the check behind the planes
+          char* chk = static_cast<char*>(map->abuf) + f64e_a_bytes(st.M, st.K);
           a.count = reinterpret_cast<int*>(chk);
           a.a_mag = mag = reinterpret_cast<uint16_t*>(chk + 256);
+          a.lists = chk + 256 + f64e_mag_bytes(st.M, st.K);
+          a.b_low = st.blow;
           a.b_mag = st.bmag;
           a.b_large = st.blarge;
         }

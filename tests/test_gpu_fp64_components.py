@@ -104,3 +104,17 @@ def test_a_map_with_decaying_input(ctx):
         # two steps of at most w D terms, each with the bound of its own sum; numpy's as well
         tol = 2 * 2 * (2 * w * D + 4) * 2.0 ** -53 * np.sqrt(2) * mag
         assert np.all(np.abs(got - ref) <= tol)
+
+
+@pytest.mark.parametrize("M,K,N", [(300, 128, 300), (1000, 77, 154), (129, 1030, 1100)])
+def test_noisy_identity_meets_flat_and_graded_rows(ctx, M, K, N):
+    """Columns with one large entry among rounding noise of several sizes: the eighth digits decide."""
+    rng = np.random.default_rng(K)
+    A = crandn(rng, (M, K))
+    A[1::3] *= np.logspace(0, -8, K)
+    A[2::7] *= 10.0 ** rng.uniform(-20, 0, (len(A[2::7]), K))
+    B = np.zeros((K, N), dtype=complex)
+    B[np.arange(N) % K, np.arange(N)] = np.exp(1j * rng.uniform(0, 6, N)) * 10.0 ** rng.uniform(-3, 3, N)
+    for noise in (1e-15, 1e-16, 1e-17, 1e-19):
+        check(ctx, A, B + noise * np.abs(B).max(0) * crandn(rng, (K, N)), K)
+        check(ctx, A, B + noise * np.abs(B).max(0) * 10.0 ** rng.uniform(-6, 0, (K, N)), K)
