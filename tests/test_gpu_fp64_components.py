@@ -118,3 +118,17 @@ def test_noisy_identity_meets_flat_and_graded_rows(ctx, M, K, N):
     for noise in (1e-15, 1e-16, 1e-17, 1e-19):
         check(ctx, A, B + noise * np.abs(B).max(0) * crandn(rng, (K, N)), K)
         check(ctx, A, B + noise * np.abs(B).max(0) * 10.0 ** rng.uniform(-6, 0, (K, N)), K)
+
+
+@pytest.mark.parametrize("tiny", [1e-10, 1e-18, 1e-30, 1e-100])
+def test_the_only_terms_that_meet_are_tiny(ctx, tiny):
+    """Rows and columns whose large entries meet zeros: the product of two tiny ones is all there is."""
+    rng = np.random.default_rng(3)
+    M, K, N = 300, 700, 200
+    A, B = np.zeros((M, K), dtype=complex), np.zeros((K, N), dtype=complex)
+    A[:, :300], B[400:, :] = crandn(rng, (M, 300)), crandn(rng, (300, N))
+    check(ctx, A, B, K)  # nothing meets
+    A[:, 350], B[350, :] = tiny * crandn(rng, M), tiny * crandn(rng, N)
+    check(ctx, A, B, K)
+    A[::2, 399], B[399, ::3] = tiny, -tiny
+    check(ctx, A, B, K)
