@@ -39,6 +39,7 @@
 // kernels.
 #include "gtn_internal.h"
 #include "gtn_group.h"
+#include "gtn_digits.h"
 #include "gtn_tcgen05.h"
 
 #include <algorithm>
@@ -442,7 +443,7 @@ __global__ void __launch_bounds__(32 * kEpiWarps)
 // One-site map of a 31-site binary tree at D = 128 (M = 163840, N = 640, K = 128, digit product
 // 2423 us): the sums take 241 us, 148 us with tiles that end early, and counting 27 us.  Products of the
 // two-site map of a DMRG step at D = 96 (M = 384, N = 480, K = 96 and M = 384, N = 96, K = 480) with a
-// state of which 7 to 10 % of the outputs miss the bound: check 11 and 19 us, repair 26 and 48 us (with
+// state of which 7 to 10 % of the outputs miss the bound: check 11 and 19 us, repair 27 and 50 us (with
 // a CTA for each tile 1059 and 510 us together); 1 % of a Lanczos vector's: 23 us together.  Environments
 // of a random state at D = 128 (M = 163840, N = 640, K = 128; 6.4 % miss it, 2.4 % with eighth digits
 // too): 5.9 ms, 10.5 ms with every one of them summed again, 93 ms on the FP64 pipe.
@@ -470,6 +471,7 @@ struct RepairArgs {
   const uint16_t *a_mag, *b_mag;
   const int* b_large;
   const uint32_t* b_low;
+  int low_all;
   const unsigned char* planes;  // of A
   uint16_t* lists;             // [tile][kRM kRN]: n_local kRM + m_local
   unsigned long long* chunks;  // tile << 24 | first << 8 | length
@@ -772,19 +774,37 @@ __global__ void __launch_bounds__(kPThreads, 4) f64e_repair_kernel(const __grid_
     const int64_t m = m0 + rr, n = n0 + id / kRM;
     const unsigned char* a = g.planes + (m0 / kBM * nkb * kS * kBM + rr) * 32;  // A's first digits
     const uint32_t* b = g.b_low + n * 8 * nkb;
+    const bool kept = f64e_low_kept(g.b_large[n], g.K, g.low_all);
+    const int eb = (int)g.b_exp[n];
     const uint16_t *am = g.a_mag + m * 8, *bm = g.b_mag + n * 8;
     float re = 0.f, im = 0.f, prod = 0.f, alpha = 0.f, beta = 0.f, met = 0.f, left = 0.f;
 #pragma unroll 2
     for (int64_t q = l; q < 2 * nkb; q += 4) {  // four k
       const uint4 u = *reinterpret_cast<const uint4*>(a + (q >> 1) * (kS * kPlaneA) + (((int)q ^ (rr >> 2)) & 1) * 16);
-      const uint4 v = *reinterpret_cast<const uint4*>(b + q * 4);
       const uint2 x = *reinterpret_cast<const uint2*>(am + (q >> 1) * g.M * 8 + (q & 1) * 4);
       const uint2 y = *reinterpret_cast<const uint2*>(bm + (q >> 1) * g.N * 8 + (q & 1) * 4);
-      const uint32_t d[4] = {u.x, u.y, u.z, u.w}, t[4] = {v.x, v.y, v.z, v.w}, xs[2] = {x.x, x.y}, ys[2] = {y.x, y.y};
+      const uint32_t d[4] = {u.x, u.y, u.z, u.w}, xs[2] = {x.x, x.y}, ys[2] = {y.x, y.y};
+      float tr[4], ti[4];
+      if (kept) {
+        const uint4 v = *reinterpret_cast<const uint4*>(b + q * 4);
+        const uint32_t t[4] = {v.x, v.y, v.z, v.w};
+#pragma unroll
+        for (int p = 0; p < 4; ++p) {
+          tr[p] = lo16(t[p]);
+          ti[p] = hi16(t[p]);
+        }
+      } else {
+#pragma unroll
+        for (int p = 0; p < 4; ++p) {
+          const double2 v = q * 4 + p < g.K ? g.B[n * g.K + q * 4 + p] : make_double2(0.0, 0.0);
+          tr[p] = (float)low_digit(v.x, eb);
+          ti[p] = (float)low_digit(v.y, eb);
+        }
+      }
 #pragma unroll
       for (int p = 0; p < 4; ++p) {
-        re = fmaf(lo16(d[p]), lo16(t[p]), fmaf(-hi16(d[p]), hi16(t[p]), re));
-        im = fmaf(lo16(d[p]), hi16(t[p]), fmaf(hi16(d[p]), lo16(t[p]), im));
+        re = fmaf(lo16(d[p]), tr[p], fmaf(-hi16(d[p]), ti[p], re));
+        im = fmaf(lo16(d[p]), ti[p], fmaf(hi16(d[p]), tr[p], im));
         const float al = p & 1 ? hi16(xs[p >> 1]) : lo16(xs[p >> 1]), be = p & 1 ? hi16(ys[p >> 1]) : lo16(ys[p >> 1]);
         const bool both = al != 0.f && be != 0.f;
         prod = fmaf(al, be, prod);
@@ -953,6 +973,7 @@ cudaError_t launch_f64e_repair(const F64eGemmArgs& a, const double2* T, const Ga
   g.b_large = a.b_large;
   g.count = a.count;
   g.b_low = a.b_low;
+  g.low_all = a.low_all;
   g.planes = static_cast<const unsigned char*>(a.A);
   g.lists = static_cast<uint16_t*>(a.lists);
   g.chunks = reinterpret_cast<unsigned long long*>(g.lists + g.ntiles * kRM * kRN);

@@ -423,6 +423,13 @@ constexpr int kF64eCheckM = 128, kF64eCheckN = 64, kF64eCheckChunk = 32;
 constexpr int kF64eWindow = 128, kF64eNoCount = -(1 << 20);
 constexpr uint32_t kF64eLarge = 0x3d50;
 inline size_t f64e_mag_bytes(int64_t rows, int64_t K) { return ((size_t)rows * ((K + 7) / 8) * 16 + 255) / 256 * 256; }
+// Whether a row of B with that many large entries keeps its eighth digits (others are formed where
+// an output wants them).  A map's statics, packed once, keep all; an operand of a one-shot contraction
+// only rows of half as many large entries as they have entries or fewer: the products of dense rows
+// are sure, and the digits of all rows took 5 of 156 us of an environment at D = 193.
+__host__ __device__ inline bool f64e_low_kept(int large, int64_t K, int all) {
+  return all || (large >= 0 && 2 * large < (K < kF64eWindow ? (int)K : kF64eWindow));
+}
 inline size_t f64e_low_bytes(int64_t N, int64_t K) { return (size_t)N * ((K + 7) / 8) * 32; }
 inline size_t f64e_list_bytes(int64_t M, int64_t N) {
   const size_t tiles = (size_t)((M + kF64eCheckM - 1) / kF64eCheckM) * ((N + kF64eCheckN - 1) / kF64eCheckN);
@@ -449,7 +456,8 @@ struct F64eGemmArgs {
   const uint16_t* a_mag = nullptr;  // magnitudes: the outputs are checked; null: they are not
   const uint16_t* b_mag = nullptr;
   const int* b_large = nullptr;     // large entries of B's rows
-  const uint32_t* b_low = nullptr;  // their eighth digits
+  const uint32_t* b_low = nullptr;  // eighth digits of those that keep them (low_all: of all)
+  int low_all = 0;
   int* count = nullptr;             // of the check, zeroed by the split
   void* lists = nullptr;            // of the check
   int levels = 8;               // digit products d_i e_j with i + j < levels (7 or 8)
@@ -471,7 +479,7 @@ cudaError_t launch_split_digits_grp(const double2* T, const GroupSpec& mg, const
                                     float* rexp, void* out, uint16_t* mag, int* count, cudaStream_t s,
                                     int* launches);
 cudaError_t launch_pack_b_digits(const double2* B, int64_t N, int64_t K, void* out, float* bexp, uint16_t* mag,
-                                 int* large, uint32_t* low, cudaStream_t s);
+                                 int* large, uint32_t* low, int low_all, cudaStream_t s);
 // C[n][m] = sum_k T[offM(m) + offK(k)] B[n][k] on the FP64 pipe, T read in place.  With slices > 1
 // (of zgemm_view_slices: few outputs, long K) the k range is cut into that many partial products
 // P[slice][n][m], summed in order.
@@ -556,7 +564,7 @@ struct PlanStep {
   float* bexp = nullptr;
   uint16_t* bmag = nullptr;  // magnitudes of the static and the large ones' number (FP64 applications)
   int* blarge = nullptr;
-  uint32_t* blow = nullptr;  // and its eighth digits
+  uint32_t* blow = nullptr;  // and eighth digits
   double macs = 0;
 };
 

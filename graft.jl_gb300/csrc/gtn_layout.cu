@@ -4,6 +4,7 @@
 // side are coalesced.
 #include "gtn_internal.h"
 #include "gtn_group.h"
+#include "gtn_digits.h"
 
 #include <algorithm>
 #include <cstdlib>
@@ -432,16 +433,6 @@ __device__ __forceinline__ unsigned long long digit_word(double x, int E) {
   if (e != 0 && r < 60) N = r <= 0 ? mant << -r : (mant + (1ull << (r - 1))) >> r;
   return 0x80808080808080ull + (bits < 0 ? 0ull - N : N);
 }
-// The eighth digit of x under row exponent E: what digit_word rounds off, in units of 2^-64.
-__device__ __forceinline__ int low_digit(double x, int E) {
-  const long long bits = __double_as_longlong(x);
-  const int e = (int)((bits >> 52) & 0x7ff), r = E - e - 2;
-  if (e == 0 || r <= 0 || r >= 62) return 0;
-  const long long mant = (bits & 0xFFFFFFFFFFFFFll) | (1ll << 52);
-  const long long rest = mant - (r < 60 ? ((mant + (1ll << (r - 1))) >> r) << r : 0);
-  const int d = r >= 9 ? (int)((rest + (1ll << (r - 9))) >> (r - 8)) : (int)(rest << (8 - r));
-  return bits < 0 ? -d : d;
-}
 // Digits i of two numbers as a bf16 pair (first in the low half).
 __device__ __forceinline__ uint32_t digit_pair(unsigned long long a, unsigned long long b, int i) {
   float fa, fb;
@@ -538,7 +529,7 @@ __global__ void __launch_bounds__(256) pack_b_digits_kernel(const double2* __res
                                                             int64_t nkb, float* __restrict__ bexp,
                                                             unsigned char* __restrict__ out,
                                                             uint16_t* __restrict__ mag, int* __restrict__ large,
-                                                            uint32_t* __restrict__ low) {
+                                                            uint32_t* __restrict__ low, int low_all) {
   chained_wait();
   __shared__ float se[8];
   __shared__ int nlarge[8];
@@ -566,19 +557,16 @@ __global__ void __launch_bounds__(256) pack_b_digits_kernel(const double2* __res
     const int64_t chunk = (e >> 4) * 2 + (e & 1), k = chunk * 4, n = n0 + r;
     const int E = (int)se[r];
     unsigned long long w[8];
-    uint32_t g[4], low4[4];
+    uint32_t g[4];
 #pragma unroll
     for (int j = 0; j < 4; ++j) {
       const double2 v = k + j < K ? B[n * K + k + j] : make_double2(0.0, 0.0);
       w[2 * j] = digit_word(v.x, E);
       w[2 * j + 1] = digit_word(v.y, E);
       g[j] = digit_mag(v, se[r]);
-      const __nv_bfloat162 ld = __floats2bfloat162_rn((float)low_digit(v.x, E), (float)low_digit(v.y, E));
-      low4[j] = *reinterpret_cast<const uint32_t*>(&ld);
     }
     if (mag) {
       *reinterpret_cast<uint2*>(mag + ((k >> 3) * N + n) * 8 + (k & 7)) = make_uint2(g[0] | g[1] << 16, g[2] | g[3] << 16);
-      *reinterpret_cast<uint4*>(low + n * 8 * nkb + k) = make_uint4(low4[0], low4[1], low4[2], low4[3]);
       if (k < kF64eWindow)
         atomicAdd(&nlarge[r], (g[0] >= kF64eLarge) + (g[1] >= kF64eLarge) + (g[2] >= kF64eLarge) + (g[3] >= kF64eLarge));
     }
@@ -601,6 +589,20 @@ __global__ void __launch_bounds__(256) pack_b_digits_kernel(const double2* __res
   if (!mag) return;
   __syncthreads();
   if (threadIdx.x < nr) large[n0 + threadIdx.x] = nlarge[threadIdx.x];
+  for (int64_t e = threadIdx.x; e < total; e += 256) {
+    const int r = (int)((e >> 1) & 7);
+    if (r >= nr || !f64e_low_kept(nlarge[r], K, low_all)) continue;
+    const int64_t k = ((e >> 4) * 2 + (e & 1)) * 4, n = n0 + r;
+    const int E = (int)se[r];
+    uint32_t w[4];
+#pragma unroll
+    for (int j = 0; j < 4; ++j) {
+      const double2 v = k + j < K ? B[n * K + k + j] : make_double2(0.0, 0.0);
+      const __nv_bfloat162 d = __floats2bfloat162_rn((float)low_digit(v.x, E), (float)low_digit(v.y, E));
+      w[j] = *reinterpret_cast<const uint32_t*>(&d);
+    }
+    *reinterpret_cast<uint4*>(low + n * 8 * nkb + k) = make_uint4(w[0], w[1], w[2], w[3]);
+  }
 }
 
 // amax[m] = max over k of max(|re|, |im|) of the K-major gather (atomic max of the
@@ -2055,12 +2057,13 @@ cudaError_t launch_split_digits_grp(const double2* T, const GroupSpec& mg, const
                       static_cast<unsigned char*>(out), mag, count, s, launches);
 }
 cudaError_t launch_pack_b_digits(const double2* B, int64_t N, int64_t K, void* out, float* bexp,
-                                 uint16_t* mag, int* large, uint32_t* low, cudaStream_t s) {
+                                 uint16_t* mag, int* large, uint32_t* low, int low_all,
+                                 cudaStream_t s) {
   if (N <= 0) return cudaSuccess;
   const int64_t blocks = (N + 7) / 8;
   if (blocks > 2147483647LL) return cudaErrorInvalidConfiguration;
   launch_chained(pack_b_digits_kernel, dim3((unsigned)blocks), dim3(256), 0, s, B, N, K, (K + 7) / 8, bexp, static_cast<unsigned char*>(out),
-                 mag, large, low);
+                 mag, large, low, low_all);
   return cudaGetLastError();
 }
 cudaError_t launch_gather_tab_to_c128(const void* T, int is64, const GatherTab& t, int64_t M, int64_t K, int64_t ldo,

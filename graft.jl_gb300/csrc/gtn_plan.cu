@@ -162,7 +162,8 @@ int pack_digits(gtn_map map, bool required, bool mags) {
       cudaGetLastError();
       continue;
     }
-    e = launch_pack_b_digits(st.b64, st.N, st.K, planes, st.bexp, st.bmag, st.blarge, st.blow, ctx->stream);
+    e = launch_pack_b_digits(st.b64, st.N, st.K, planes, st.bexp, st.bmag, st.blarge, st.blow, map->oneshot ? 0 : 1,
+                             ctx->stream);
     ctx->launches++;
     st.bdig = planes;
   }
@@ -835,6 +836,7 @@ int map_run(gtn_map map, int precision, const double2* x, double2* y) {
           a.a_mag = mag = reinterpret_cast<uint16_t*>(chk + 256);
           a.lists = chk + 256 + f64e_mag_bytes(st.M, st.K);
           a.b_low = st.blow;
+          a.low_all = map->oneshot ? 0 : 1;
           a.b_mag = st.bmag;
           a.b_large = st.blarge;
         }
